@@ -16,6 +16,25 @@
 
 using namespace epik2;
 
+// A device buffer that only grows.
+struct GrowBuf {
+  void* p = nullptr;
+  size_t cap = 0;
+  cudaError_t need(size_t bytes) {
+    if (bytes <= cap) return cudaSuccess;
+    drop();
+    const cudaError_t e = cudaMalloc(&p, bytes);
+    if (e == cudaSuccess) cap = bytes;
+    else p = nullptr;
+    return e;
+  }
+  void drop() {
+    if (p) cudaFree(p);
+    p = nullptr;
+    cap = 0;
+  }
+};
+
 struct epik2_ctx {
   int device = 0;
   cudaStream_t stream = nullptr;      // current stream (own or caller's)
@@ -73,6 +92,11 @@ struct epik2_ctx {
   BestSlot* d_rep_res = nullptr;
   Rescored* d_rep_resc = nullptr;
   int64_t rep_cap = 0, rep_slot_cap = 0;
+  // split search workspace (grown, bounded by kSplitChunkBytes plus the searched datasets' own
+  // bits; given back when another allocation needs the room and with the context)
+  GrowBuf sp_rows, sp_lists, sp_cp, sp_tiles, sp_small, sp_slots;
+  unsigned char* h_small = nullptr;  // pinned image of the uploaded part of sp_small, and results
+  size_t h_small_cap = 0;
 };
 
 constexpr size_t kMaxPlans = 32;  // cached batched plans per context
@@ -141,6 +165,16 @@ void drop_spare(epik2_ctx* ctx) {
   ctx->spare_bytes = 0;
 }
 
+size_t split_bytes(const epik2_ctx* ctx) {
+  return ctx->sp_rows.cap + ctx->sp_lists.cap + ctx->sp_cp.cap + ctx->sp_tiles.cap + ctx->sp_small.cap +
+         ctx->sp_slots.cap;
+}
+
+void drop_split(epik2_ctx* ctx) {
+  for (GrowBuf* b : {&ctx->sp_rows, &ctx->sp_lists, &ctx->sp_cp, &ctx->sp_tiles, &ctx->sp_small, &ctx->sp_slots})
+    b->drop();
+}
+
 // A dataset allocation of at least `bytes`: the context's spare block when it fits without
 // more than doubling the footprint, else a new one (the spare is released first).
 cudaError_t take_block(epik2_ctx* ctx, size_t bytes, void** out, size_t* got) {
@@ -153,7 +187,14 @@ cudaError_t take_block(epik2_ctx* ctx, size_t bytes, void** out, size_t* got) {
   }
   drop_spare(ctx);
   *got = bytes;
-  return cudaMalloc(out, bytes);
+  cudaError_t e = cudaMalloc(out, bytes);
+  if (e == cudaErrorMemoryAllocation && split_bytes(ctx) > 0) {  // the search workspace gives way
+    cudaGetLastError();
+    cudaStreamSynchronize(ctx->stream);
+    drop_split(ctx);
+    e = cudaMalloc(out, bytes);
+  }
+  return e;
 }
 
 struct Layout {
@@ -351,6 +392,10 @@ void complete_config(const epik2_tune& t, bool can_fp4, bool can_overlap, int& e
 
 int run_scan(epik2_ctx* ctx, DevDataset& d, const epik2_opts* opts, uint32_t* dump_tables, float* dump_scores,
              BestSlot* best_out);
+constexpr int kSplitNoRoom = 1;  // run_split: the workspace does not fit (the caller takes the other kernels)
+bool split_fits(const DevDataset& d);
+int run_split(epik2_ctx* ctx, const std::vector<DevDataset*>& ds, int64_t ib, int64_t ie, int top_k,
+              uint32_t* dump_tables, float* dump_scores, BestSlot* best_out);
 
 // Pair groups of first index i: j0 = i+1, i+5, ... while j0 <= m-2.
 int64_t groups_of(int64_t m, int64_t i) { return (i <= m - 3) ? (m - 2 - i + kPairsPerWarp) / kPairsPerWarp : 0; }
@@ -382,6 +427,16 @@ int run_scan(epik2_ctx* ctx, DevDataset& d, const epik2_opts* opts, uint32_t* du
   const bool can_overlap = fp4_exact(d) && pipe_fits(d.n_controls, d.n_cases);
   if (ov == 2 && !can_overlap)
     return fail(ctx, EPIK2_E_TOO_LARGE, "overlapped kernel: classes of at most 65535 samples");
+  // Nothing pinned beyond the format: the genotype-split kernel wherever its 16-bit cells hold
+  // (it is the fastest at every shape measured); the other kernels for larger classes.
+  if ((engine == 0 || engine == 3) && kw == 0 && pt == 0 && ov == 0 && split_fits(d)) {
+    const int r = run_split(ctx, {&d}, ib, ie, top_k, dump_tables, dump_scores, best_out);
+    if (r != kSplitNoRoom) {
+      if (r) return r;
+      ctx->stats.last_scan_words = d.w0 + d.w1;
+      return collect_topk(ctx, d, opts, top_k, tc_pair_blocks(ctx->tc_blocks) * split_score_warps());
+    }
+  }
   if (engine == 0 || ((engine == 2 || engine == 3) && kw == 0)) {
     epik2_tune t{};
     int r = tuned(ctx, d, &t);
@@ -685,6 +740,212 @@ int64_t triplets_before(int64_t m, int64_t ie) {
   int64_t t = 0;
   for (int64_t i = 0; i < ie; i++) t += (m - 1 - i) * (m - 2 - i) / 2;
   return t;
+}
+
+// ---- genotype-split search (scan_split.cu) ----
+
+// Its cells are 16-bit halves of a word: classes of at most 65535 samples.
+bool split_fits(const DevDataset& d) { return d.n_snps >= 3 && d.n_controls <= 65535 && d.n_cases <= 65535; }
+
+// Compacted planes of the first SNPs searched per launch: launches of the large workload then
+// last 6 ms or more, and their ends (one tile, about 10 us) stay below 0.3 %.
+constexpr size_t kSplitChunkBytes = (size_t)768 << 20;
+// Planes of the first SNPs whose tiles are interleaved in the queue: what may stay in L2 (126 MB)
+// beside the margins.
+constexpr size_t kSplitRunBytes = (size_t)40 << 20;
+
+// Best triplet of each dataset over first indices [ib, ie) (clipped to the dataset).  top_k > 1
+// (one dataset): candidates in ctx->d_cand, split_score_warps() lists per CTA.
+int run_split(epik2_ctx* ctx, const std::vector<DevDataset*>& ds, int64_t ib, int64_t ie, int top_k,
+              uint32_t* dump_tables, float* dump_scores, BestSlot* best_out) {
+  const int n_jobs = (int)ds.size();
+  const int grid = tc_pair_blocks(ctx->tc_blocks), per_job = grid * split_score_warps();
+  struct Chunk {
+    int rec0, n_recs, run0, n_runs, max_quads, max_cols, max_blocks;
+  };
+  std::vector<SplitJob> jobs((size_t)n_jobs);
+  std::vector<SplitRec> recs;
+  std::vector<SplitRun> runs;
+  std::vector<Chunk> chunks;
+  size_t rows_bytes = 0, cp_max = 0, lists_max = 0, tiles_max = 0;
+  size_t cp = 0, lists = 0, tiles = 0;  // of the current chunk: bytes, bytes, descriptors
+  int64_t trip = 0;
+  for (int b = 0; b < n_jobs; b++) {
+    const DevDataset& d = *ds[(size_t)b];
+    SplitJob& J = jobs[(size_t)b];
+    J = SplitJob{};
+    J.planes = d.planes;
+    J.singles = d.singles;
+    J.pairs = d.pairs;
+    J.lut = d.lut;
+    J.tri = d.tri;
+    J.m = (int32_t)d.n_snps;
+    J.m_pad = (int32_t)d.m_pad;
+    J.mwp = (int32_t)((d.m_pad / 32 + 3) / 4 * 4);
+    J.w0 = (int32_t)d.w0;
+    J.w1 = (int32_t)d.w1;
+    J.n0 = (int32_t)d.n_controls;
+    J.n1 = (int32_t)d.n_cases;
+    const ScreenConsts sc = screen_constants(d.n_controls, d.n_cases);
+    J.coef = sc.coef;
+    J.bias = sc.bias;
+    J.theta1 = sc.theta1;
+    J.theta2 = sc.theta2;
+    J.c = sc.c;
+    J.base = sc.base;
+    J.rows = reinterpret_cast<const uint2*>(rows_bytes);  // offset, made an address below
+    rows_bytes += align_up((size_t)(32 * (d.w0 + d.w1)) * J.mwp * 8, 256);
+    const int64_t m = d.n_snps;
+    const int max_quads = (int)(2 * d.n_samples / 3 / 128) + 5;  // the dropped genotype is the most frequent
+    const int64_t i0 = std::max<int64_t>(ib, 0), i1 = std::min<int64_t>(ie, m - 2);
+    size_t run_bytes = 0;
+    for (int64_t i = i0; i < i1; i++) {
+      SplitRec r{};
+      r.job = b;
+      r.i = (int32_t)i;
+      r.qlo = (int32_t)((i + 1) / 32 / 4 * 4);
+      r.mlen = 32 * (J.mwp - r.qlo);
+      const size_t rec_cp = (size_t)max_quads * r.mlen * 32, rec_list = (size_t)max_quads * 128 * 4;
+      const bool new_chunk = chunks.empty() || cp + rec_cp > kSplitChunkBytes || recs.size() - chunks.back().rec0 >= (1u << 23);
+      if (new_chunk) {
+        chunks.push_back(Chunk{(int)recs.size(), 0, (int)runs.size(), 0, 0, 0, 0});
+        cp = lists = tiles = 0;
+      }
+      Chunk& c = chunks.back();
+      const size_t est = (size_t)((max_quads * 5 + 7) / 8) * r.mlen * 32;  // usual size: 0.41 of the samples
+      if (new_chunk || runs.empty() || recs[(size_t)runs.back().rec0 + c.rec0].job != b || run_bytes + est > kSplitRunBytes) {
+        runs.push_back(SplitRun{(int32_t)recs.size() - c.rec0, 0});
+        c.n_runs++;
+        run_bytes = 0;
+      }
+      run_bytes += est;
+      runs.back().n++;
+      r.cp_off = (int64_t)(cp / 16);
+      r.list_off = (int64_t)(lists / 4);
+      cp += rec_cp;
+      lists += rec_list;
+      const int64_t left = m - 2 - i;  // SNPs j from i + 1 to m - 2
+      const int64_t blocks = (left + kSplitJ - 1) / kSplitJ;
+      tiles += (size_t)(blocks + (blocks * left - kSplitJ * blocks * (blocks - 1) / 2) / kSplitK + 1);
+      trip += (m - 1 - i) * (m - 2 - i) / 2;
+      c.n_recs++;
+      c.max_quads = std::max(c.max_quads, max_quads);
+      c.max_cols = std::max(c.max_cols, r.mlen / 32);
+      c.max_blocks = std::max(c.max_blocks, (int)blocks);
+      cp_max = std::max(cp_max, cp);
+      lists_max = std::max(lists_max, lists);
+      tiles_max = std::max(tiles_max, tiles);
+      recs.push_back(r);
+    }
+  }
+  // device: [jobs][recs][runs] uploaded, then [cursors, counters of every chunk][thresholds][results]
+  const size_t o_recs = align_up(sizeof(SplitJob) * jobs.size(), 256);
+  const size_t o_runs = o_recs + align_up(sizeof(SplitRec) * std::max<size_t>(recs.size(), 1), 256);
+  const size_t up_bytes = o_runs + align_up(sizeof(SplitRun) * std::max<size_t>(runs.size(), 1), 256);
+  const size_t o_cur = up_bytes, cur_bytes = align_up(8 * std::max<size_t>(chunks.size(), 1) + 4, 256);
+  const size_t o_thr = o_cur + cur_bytes, thr_bytes = align_up(4 * jobs.size(), 256);
+  const size_t o_res = o_thr + thr_bytes, res_bytes = align_up(sizeof(BestSlot) * jobs.size(), 256);
+  auto reserve = [&]() {
+    cudaError_t e = ctx->sp_small.need(o_res + res_bytes);
+    if (e == cudaSuccess) e = ctx->sp_slots.need(sizeof(BestSlot) * (size_t)n_jobs * per_job);
+    if (e == cudaSuccess) e = ctx->sp_rows.need(std::max<size_t>(rows_bytes, 256));
+    if (e == cudaSuccess) e = ctx->sp_lists.need(std::max<size_t>(lists_max, 256));
+    if (e == cudaSuccess) e = ctx->sp_cp.need(std::max<size_t>(cp_max, 256));
+    if (e == cudaSuccess) e = ctx->sp_tiles.need(8 * std::max<size_t>(tiles_max, 32));
+    return e;
+  };
+  cudaError_t e = reserve();
+  if (e == cudaErrorMemoryAllocation) {
+    cudaGetLastError();
+    drop_spare(ctx);
+    e = reserve();
+  }
+  if (e == cudaErrorMemoryAllocation) {
+    cudaGetLastError();
+    drop_split(ctx);
+    return kSplitNoRoom;
+  }
+  CK(ctx, e, "search workspace");
+  const size_t h_need = up_bytes + res_bytes + 256;
+  if (h_need > ctx->h_small_cap) {
+    cudaFreeHost(ctx->h_small);
+    ctx->h_small = nullptr;
+    ctx->h_small_cap = 0;
+    CK(ctx, cudaMallocHost(&ctx->h_small, 2 * h_need), "pinned search tables");
+    ctx->h_small_cap = 2 * h_need;
+  }
+  unsigned char* const dev = static_cast<unsigned char*>(ctx->sp_small.p);
+  for (SplitJob& J : jobs)
+    J.rows = reinterpret_cast<const uint2*>(static_cast<char*>(ctx->sp_rows.p) + reinterpret_cast<size_t>(J.rows));
+  memcpy(ctx->h_small, jobs.data(), sizeof(SplitJob) * jobs.size());
+  if (!recs.empty()) memcpy(ctx->h_small + o_recs, recs.data(), sizeof(SplitRec) * recs.size());
+  if (!runs.empty()) memcpy(ctx->h_small + o_runs, runs.data(), sizeof(SplitRun) * runs.size());
+  const SplitJob* d_jobs = reinterpret_cast<const SplitJob*>(dev);
+  SplitRec* d_recs = reinterpret_cast<SplitRec*>(dev + o_recs);
+  const SplitRun* d_runs = reinterpret_cast<const SplitRun*>(dev + o_runs);
+  unsigned* d_cur = reinterpret_cast<unsigned*>(dev + o_cur);  // per chunk: tile count, tickets; then the error word
+  int* d_err = reinterpret_cast<int*>(d_cur + 2 * chunks.size());
+  unsigned* d_thr = reinterpret_cast<unsigned*>(dev + o_thr);
+  BestSlot* d_res = reinterpret_cast<BestSlot*>(dev + o_res);
+  BestSlot* d_slots = static_cast<BestSlot*>(ctx->sp_slots.p);
+  CK(ctx, cudaEventRecord(ctx->ev_start, ctx->stream), "event");
+  CK(ctx, cudaMemcpyAsync(dev, ctx->h_small, up_bytes, cudaMemcpyHostToDevice, ctx->stream), "upload search tables");
+  ctx->stats.h2d_bytes += up_bytes;
+  CK(ctx, cudaMemsetAsync(d_cur, 0, cur_bytes, ctx->stream), "reset counters");
+  CK(ctx, cudaMemsetAsync(d_thr, 0x7F, thr_bytes, ctx->stream), "reset thresholds");  // 3.4e38 as FP32
+  CK(ctx, launch_fill_slots(d_slots, (int64_t)n_jobs * per_job, ctx->stream), "reset slots");
+  ctx->stats.kernel_launches += 2;
+  if (top_k > 1) {
+    CK(ctx, launch_fill_slots(ctx->d_cand, (int64_t)grid * split_score_warps() * 32, ctx->stream), "reset candidates");
+    ctx->stats.kernel_launches += 1;
+  }
+  for (const SplitJob& J : jobs) {
+    CK(ctx, launch_split_rows(J, const_cast<uint2*>(J.rows), ctx->stream), "sample rows");
+    ctx->stats.kernel_launches += 1;
+  }
+  for (size_t x = 0; x < chunks.size(); x++) {
+    const Chunk& c = chunks[x];
+    CK(ctx, launch_split_prepare(d_jobs, d_recs + c.rec0, c.n_recs, c.max_quads, c.max_cols,
+                                 static_cast<int32_t*>(ctx->sp_lists.p), static_cast<uint4*>(ctx->sp_cp.p),
+                                 ctx->stream),
+       "split planes");
+    CK(ctx, launch_split_tiles(d_jobs, d_recs + c.rec0, d_runs + c.run0, c.n_runs, c.max_blocks,
+                               static_cast<uint64_t*>(ctx->sp_tiles.p), d_cur + 2 * x, ctx->stream),
+       "tile queue");
+    SplitParams p{};
+    p.jobs = d_jobs;
+    p.recs = d_recs + c.rec0;
+    p.cp = static_cast<const uint4*>(ctx->sp_cp.p);
+    p.tiles = static_cast<const uint64_t*>(ctx->sp_tiles.p);
+    p.n_tiles = d_cur + 2 * x;
+    p.counter = d_cur + 2 * x + 1;
+    p.thr = d_thr;
+    p.job_slots = d_slots;
+    p.top_k = top_k;
+    p.cand = ctx->d_cand;
+    p.dump_tables = dump_tables;
+    p.dump_scores = dump_scores;
+    p.err = d_err;
+    p.wait_limit = ctx->wait_limit;
+    CK(ctx, launch_scan_split(p, grid, dump_tables != nullptr, ctx->stream), "split search kernel");
+    ctx->stats.kernel_launches += 4;
+  }
+  CK(ctx, launch_reduce_jobs(d_slots, n_jobs, per_job, d_res, ctx->stream), "reduce kernel");
+  CK(ctx, cudaEventRecord(ctx->ev_stop, ctx->stream), "event");
+  BestSlot* h_res = reinterpret_cast<BestSlot*>(ctx->h_small + up_bytes);
+  int* h_err = reinterpret_cast<int*>(ctx->h_small + up_bytes + res_bytes);
+  CK(ctx, cudaMemcpyAsync(h_res, d_res, sizeof(BestSlot) * (size_t)n_jobs, cudaMemcpyDeviceToHost, ctx->stream),
+     "read results");
+  CK(ctx, cudaMemcpyAsync(h_err, d_err, 4, cudaMemcpyDeviceToHost, ctx->stream), "read error word");
+  ctx->stats.d2h_bytes += sizeof(BestSlot) * (size_t)n_jobs + 4;
+  CK(ctx, cudaStreamSynchronize(ctx->stream), "search");
+  if (*h_err) return fail(ctx, EPIK2_E_TIMEOUT, "tensor-core scan: a bounded wait expired");
+  float kms = 0.0f;
+  CK(ctx, cudaEventElapsedTime(&kms, ctx->ev_start, ctx->ev_stop), "event time");
+  ctx->stats.last_scan_kernel_ms = kms;
+  ctx->stats.last_scan_triplets = trip;
+  memcpy(best_out, h_res, sizeof(BestSlot) * (size_t)n_jobs);
+  return EPIK2_OK;
 }
 
 // Autotuner: time each candidate on a slice of the dataset (first indices [0, ie) holding
@@ -1046,6 +1307,8 @@ void epik2_destroy(epik2_ctx* ctx) {
   for (auto& kv : ctx->datasets) cudaFree(kv.second->block);
   ctx->datasets.clear();
   cudaFree(ctx->spare_block);
+  drop_split(ctx);
+  cudaFreeHost(ctx->h_small);
   cudaFree(ctx->d_counter);
   cudaFree(ctx->d_slots);
   cudaFree(ctx->d_best);
@@ -1079,7 +1342,8 @@ int epik2_mem_info(const epik2_ctx* ctx, size_t* free_bytes, size_t* total_bytes
   if (!ctx || !free_bytes || !total_bytes) return EPIK2_E_INVALID;
   cudaSetDevice(ctx->device);
   if (cudaMemGetInfo(free_bytes, total_bytes) != cudaSuccess) return EPIK2_E_CUDA;
-  *free_bytes += ctx->spare_bytes;  // the context's spare allocation is reused or released on demand
+  // the context's spare allocation and search workspace are reused or released on demand
+  *free_bytes += ctx->spare_bytes + split_bytes(ctx);
   return EPIK2_OK;
 }
 
@@ -1192,7 +1456,7 @@ int epik2_load_u8(epik2_ctx* ctx, const uint8_t* geno, const uint8_t* pheno, int
   if (!reuse) {
     size_t fr = 0, tot = 0;
     CK(ctx, cudaMemGetInfo(&fr, &tot), "mem info");
-    if (L.total + (size_t)(256u << 20) > fr + ctx->spare_bytes)
+    if (L.total + (size_t)(256u << 20) > fr + ctx->spare_bytes + split_bytes(ctx))
       return fail(ctx, EPIK2_E_NOMEM, "dataset does not fit in free device memory");
   }
   std::unique_ptr<DevDataset> d(new DevDataset());
@@ -1280,7 +1544,7 @@ int epik2_load_replicate(epik2_ctx* ctx, int32_t base_dataset_id, const uint8_t*
   if (!(ctx->spare_block && ctx->spare_bytes >= L.total && ctx->spare_bytes <= 2 * L.total)) {
     size_t fr = 0, tot = 0;  // a new allocation: ask for free memory (about a millisecond)
     CK(ctx, cudaMemGetInfo(&fr, &tot), "mem info");
-    if (L.total + (size_t)(256u << 20) > fr + ctx->spare_bytes)
+    if (L.total + (size_t)(256u << 20) > fr + ctx->spare_bytes + split_bytes(ctx))
       return fail(ctx, EPIK2_E_NOMEM, "replicate does not fit in free device memory");
   }
   std::unique_ptr<DevDataset> d(new DevDataset());
@@ -1538,7 +1802,7 @@ int epik2_scan_replicates(epik2_ctx* ctx, int32_t dataset_id, const uint8_t* phe
   if (!(ctx->spare_block && ctx->spare_bytes >= rep_bytes * (size_t)want)) {
     size_t fr = 0, tot = 0;
     CK(ctx, cudaMemGetInfo(&fr, &tot), "mem info");
-    fr += ctx->spare_bytes;
+    fr += ctx->spare_bytes + split_bytes(ctx);
     fit = ((int64_t)fr - ((int64_t)1 << 30)) / (int64_t)rep_bytes;
   }
   const int32_t group = (int32_t)std::max<int64_t>(1, std::min<int64_t>(fit, want));

@@ -143,6 +143,80 @@ struct TcParams {
   int32_t n_reps;
 };
 
+// ---- genotype-split search (scan_split.cu) ----
+constexpr int kSplitK = 128;   // SNPs k per tile (64 per CTA of the pair)
+constexpr int kSplitJ = 56;    // SNPs j per tile
+constexpr int kSplitSlots = 3; // tiles in flight per CTA pair: scored, in tensor memory, produced
+
+// Constants of the screening bound for a class split (screen_constants).
+struct ScreenConsts {
+  uint32_t coef;           // bytes (128 - kp, -kp): 128 D = (128 - kp) a - kp b + bias
+  int32_t bias;            // 64 - kp
+  float theta1, theta2;    // of 128 D
+  float c;                 // of (128 D)^2 / den
+  float base;
+};
+// One dataset of a split search.
+struct SplitJob {
+  const uint2* planes;
+  const uint2* rows;       // [32*(w0+w1)][mwp] {g0, g1} bits of 32 SNPs per entry, class-sorted samples
+  const uint32_t* singles;
+  const uint4* pairs;
+  const float* lut;
+  int64_t tri;
+  int32_t m, m_pad, mwp, w0, w1, n0, n1;
+  uint32_t coef;           // ScreenConsts
+  int32_t bias;
+  float theta1, theta2, c, base;
+  int32_t pad[7];
+};
+static_assert(sizeof(SplitJob) == 128, "copied as 32 words per tile");
+
+// One first SNP i of a job: where its compacted planes and sample lists lie in the workspace
+// (host) and how its samples split (k_split_lists).  The samples of each class are taken in two
+// groups, those with genotype gA of SNP i and those with gB (gA < gB; the third genotype gC, the
+// most frequent, follows from the margins); group order: class 0 gA, class 0 gB, class 1 gA,
+// class 1 gB, each padded to quads of 128 samples, at least one quad.
+struct SplitRec {
+  int64_t cp_off;          // compacted planes: uint4 index of quad 0, SNP 32*qlo
+  int64_t list_off;        // sample lists: index of the first entry
+  int32_t job, i;
+  int32_t qlo;             // first 32-SNP column kept (SNPs below are never j or k)
+  int32_t mlen;            // SNPs per quad row
+  int32_t qend[4];         // end of each group, in quads
+  int32_t genos;           // gA | gB << 2 | gC << 4
+  int32_t pad[3];
+};
+static_assert(sizeof(SplitRec) == 64, "copied as 16 words per tile");
+
+// Consecutive records of one job whose tiles are interleaved in the queue.
+struct SplitRun {
+  int32_t rec0, n;
+};
+
+// Tile descriptor: record (bits 0-23), j block u (24-41: j0 = i + 1 + 56u), k block t (42-57:
+// k0 = j0 + 1 + 128t).
+__host__ __device__ inline uint64_t pack_split_tile(uint32_t rec, uint32_t u, uint32_t t) {
+  return (uint64_t)rec | ((uint64_t)u << 24) | ((uint64_t)t << 42);
+}
+
+struct SplitParams {
+  const SplitJob* jobs;
+  const SplitRec* recs;
+  const uint4* cp;               // compacted planes: per quad and SNP two uint4 (4 words of g0, of g1)
+  const uint64_t* tiles;
+  const unsigned* n_tiles;
+  unsigned* counter;
+  unsigned* thr;                 // [job] bits of the lowest score found (top-k: of a score that top_k reach)
+  BestSlot* job_slots;           // [job][grid]
+  int32_t top_k;
+  BestSlot* cand;                // [scoring warps of the grid][32]
+  uint32_t* dump_tables;
+  float* dump_scores;
+  int* err;
+  long long wait_limit;
+};
+
 // Kernel launchers (scan_int.cu / scan_tc.cu / encode.cu); all asynchronous on `stream`.
 cudaError_t launch_encode(const DevDataset& d, cudaStream_t stream);
 cudaError_t launch_counts(const DevDataset& d, cudaStream_t stream, bool pairs = true);
@@ -150,6 +224,18 @@ cudaError_t launch_counts(const DevDataset& d, cudaStream_t stream, bool pairs =
 cudaError_t launch_pairs_tc(const TcParams& p, int blocks, cudaStream_t stream);
 // replicate form of the CTA-pair FP4 search (16 words per stage): see TcParams::n_reps
 cudaError_t launch_scan_reps(const TcParams& p, int blocks, cudaStream_t stream);
+int split_score_warps();  // scoring warps per CTA of the split search
+cudaError_t split_configure();
+// rows (sample-major bits) of one job from its planes
+cudaError_t launch_split_rows(const SplitJob& j, uint2* rows, cudaStream_t stream);
+// sample lists and group ends of records [0, n); then their compacted planes (at most max_quads
+// quads and max_cols 32-SNP columns each)
+cudaError_t launch_split_prepare(const SplitJob* jobs, SplitRec* recs, int n, int max_quads, int max_cols,
+                                 int32_t* lists, uint4* cp, cudaStream_t stream);
+// tile queue of a run list; *cursor (zeroed by the caller) receives the tile count
+cudaError_t launch_split_tiles(const SplitJob* jobs, const SplitRec* recs, const SplitRun* runs, int n_runs,
+                               int max_blocks, uint64_t* tiles, unsigned* cursor, cudaStream_t stream);
+cudaError_t launch_scan_split(const SplitParams& p, int blocks, bool dump, cudaStream_t stream);
 cudaError_t launch_scan_int(const ScanParams& p, int blocks, bool dump, cudaStream_t stream);
 cudaError_t launch_reduce_best(const BestSlot* slots, int n, BestSlot* out, cudaStream_t stream);
 cudaError_t launch_tables(const DevDataset& d, const uint32_t* triplets, int64_t n, uint32_t* out,
@@ -178,6 +264,7 @@ cudaError_t launch_rescore_jobs(const TcJob* jobs, const BestSlot* best, int n, 
 int tc_warps_per_block();
 
 // Host helpers (host_data.cpp).
+ScreenConsts screen_constants(int64_t n0, int64_t n1);
 void build_k2_lut(int64_t n_max, float* lut);
 void build_k2_lut_range(int64_t n_begin, int64_t n_end, float* out);  // out[n - n_begin], n in [begin, end)
 void build_k2_lut64(int64_t n_max, double* lut);

@@ -1,0 +1,1101 @@
+// Genotype-split tensor-core search (tcgen05 block-scaled FP4 on CTA pairs, sm_100a).
+//
+// Same result as k_scan_tc, the integer engine and the reference's kernel_epi
+// (GPU/v4.cpp:295-594): exact tables, K2 in the reference's FP32 order, lowest (score, i, j, k).
+//
+// Two things make it cheaper than counting the 8 cells of (i, j, k) over all samples:
+//
+// 1. For a fixed first SNP i the samples of a class are sorted by their genotype of i, and only
+//    the two rarer genotypes are counted:
+//      D_g[(k, c)][(j, b)] = sum over the samples of group g of x_c(k) x_b(j),  b, c in {0, 1},
+//    four products per triplet and sample of a counted group instead of eight per sample.  The
+//    counted groups hold at most 2/3 of the samples (0.41 on average for minor-allele frequencies
+//    uniform in [0.05, 0.5]); the cells of the most frequent genotype follow from the (j, k)
+//    margins by inclusion-exclusion, as the cells with genotype 2 of j or k do.  No operand holds
+//    a product of two SNPs any more: both are plain indicator rows.  The sorting itself is one
+//    pass of bit transposes per i (k_split_lists, k_split_planes), 3-5 % of a search.
+// 2. A triplet's 27 cells are first put through a lower bound of K2 (screen_constants in
+//    host_data.cpp: one reciprocal per cell and a few FP32 operations, no table).  Only where the
+//    bound does not exceed the best score found so far (of the whole launch) is the score computed
+//    in the reference's arithmetic.  The bound is below the score by 2 to 4 on average; 0.002 % to
+//    0.04 % of the warps' steps go on to the score.
+//
+// Warp roles of a CTA (512 threads), concurrent from tile to tile:
+//   warps 0-5   produce: expand the compacted bit planes into the operand ring (warps 0-3 the 64
+//               SNPs k of this CTA, 4-5 its 28 SNPs j), 256 samples per stage, 4 stages
+//   warp 6      issues the products (even CTA)
+//   warp 7      schedules: takes tiles from the queue, publishes descriptor, record and job
+//   warps 8-15  score: copy a tile's four accumulators out of tensor memory into a 16-bit staging
+//               buffer (class 0 in the low, class 1 in the high half of a word), which frees them
+//               for the next tile, then complete, screen and select while that tile counts
+// Classes of at most 65535 samples (the 16-bit halves).
+//
+// What bounds it: the issue slots of the scoring warps (about 320 instructions per 32 triplets)
+// and, from about 8192 samples on, the round trip of a ring stage (stores, arrival in the even CTA,
+// products, commit).  Cost of the parts of that round trip, which set the roles and hand-offs above
+// (clocks, measured alone): a commit of four products 560; an arrival in the other CTA 133, and
+// 447 with a cluster-scope release; issuing four products and their commit 330 from a converged
+// warp, 610 from a lane-0 branch.
+// Measured against k_scan_tc on CTA pairs (kernel time of a whole search): 1024 x 8192 14.1 -> 5.1
+// ms, 3072 x 4096 265 -> 102 ms, 2048 x 8192 103 -> 34.5 ms, an eighth of 4096 x 16384 144 -> 45 ms.
+//
+// Every mbarrier wait is bounded; on expiry the kernel sets an error word and ends.
+#include <cfloat>
+
+#include "epik2_internal.h"
+#include "scan_common.cuh"
+#include "tc_ptx.cuh"
+
+namespace epik2 {
+
+// ------------------------------------------------------------------ sorting by genotype of i
+
+// 32 x 32 bit transpose across a warp: lane l, bit b -> lane b, bit l.
+__device__ __forceinline__ uint32_t transpose32(uint32_t x, int lane) {
+#pragma unroll
+  for (int j = 16; j > 0; j >>= 1) {
+    const uint32_t m = j == 16 ? 0x0000FFFFu : j == 8 ? 0x00FF00FFu : j == 4 ? 0x0F0F0F0Fu : j == 2 ? 0x33333333u : 0x55555555u;
+    const uint32_t y = __shfl_xor_sync(kFull, x, j);
+    x = (lane & j) ? ((x & ~m) | ((y >> j) & m)) : ((x & m) | ((y & m) << j));
+  }
+  return x;
+}
+
+// rows[32w + b][q] from planes[w][32q ..]: one warp per class word and four 32-SNP columns.
+__global__ void __launch_bounds__(256) k_split_rows(const uint2* __restrict__ planes, uint2* __restrict__ rows,
+                                                    int64_t m_pad, int mwp, int64_t words) {
+  const int lane = threadIdx.x & 31;
+  const int nq = mwp / 4;
+  const int64_t unit = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5);
+  const int64_t w = unit / nq;
+  const int q = 4 * (int)(unit - w * nq);
+  if (w >= words) return;
+  uint2 v[4];
+#pragma unroll
+  for (int t = 0; t < 4; t++) {
+    const int64_t snp = 32 * (int64_t)(q + t) + lane;
+    v[t] = snp < m_pad ? __ldg(planes + w * m_pad + snp) : make_uint2(0, 0);
+  }
+#pragma unroll
+  for (int t = 0; t < 4; t++) {
+    v[t].x = transpose32(v[t].x, lane);
+    v[t].y = transpose32(v[t].y, lane);
+  }
+  uint4* dst = reinterpret_cast<uint4*>(rows + (32 * w + lane) * (int64_t)mwp + q);
+  dst[0] = make_uint4(v[0].x, v[0].y, v[1].x, v[1].y);
+  dst[1] = make_uint4(v[2].x, v[2].y, v[3].x, v[3].y);
+}
+
+// Sample lists of one record per block: the row numbers of each group's samples, -1 up to the
+// end of its last quad.
+constexpr int kListThreads = 256;
+__global__ void __launch_bounds__(kListThreads) k_split_lists(const SplitJob* __restrict__ jobs, SplitRec* __restrict__ recs,
+                                                              int32_t* __restrict__ lists) {
+  __shared__ uint2 s_sum[kListThreads / 32];
+  SplitRec& rec = recs[blockIdx.x];
+  const SplitJob& J = jobs[rec.job];
+  const int i = rec.i, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  int n[2][3];
+#pragma unroll
+  for (int c = 0; c < 2; c++) {
+    n[c][0] = (int)J.singles[((int64_t)c * J.m_pad + i) * 2];
+    n[c][1] = (int)J.singles[((int64_t)c * J.m_pad + i) * 2 + 1];
+    n[c][2] = (c ? J.n1 : J.n0) - n[c][0] - n[c][1];
+  }
+  const int t0 = n[0][0] + n[1][0], t1 = n[0][1] + n[1][1], t2 = n[0][2] + n[1][2];
+  const int gC = (t0 >= t1 && t0 >= t2) ? 0 : (t1 >= t2 ? 1 : 2);
+  const int gA = gC == 0 ? 1 : 0, gB = gC == 2 ? 1 : 2;
+  int qend[4], q = 0;
+#pragma unroll
+  for (int g = 0; g < 4; g++) {
+    const int cnt = n[g >> 1][(g & 1) ? gB : gA];
+    q += cnt > 0 ? (cnt + 127) / 128 : 1;
+    qend[g] = q;
+  }
+  if (tid < 4) rec.qend[tid] = qend[tid];
+  if (tid == 4) rec.genos = gA | (gB << 2) | (gC << 4);
+  int32_t* list = lists + rec.list_off;
+#pragma unroll 1
+  for (int c = 0; c < 2; c++) {
+    const int words = c ? J.w1 : J.w0, wb = c ? J.w0 : 0, ncls = c ? J.n1 : J.n0;
+    int posA = 128 * (c ? qend[1] : 0), posB = 128 * (c ? qend[2] : qend[0]);
+    for (int base = 0; base < words; base += kListThreads) {
+      const int w = base + tid;
+      uint32_t ma = 0, mb = 0;
+      if (w < words) {
+        const uint2 v = __ldg(J.planes + (int64_t)(wb + w) * J.m_pad + i);
+        const int left = ncls - 32 * w;
+        const uint32_t valid = left >= 32 ? kFull : ((1u << left) - 1u);
+        const uint32_t m2 = ~(v.x | v.y) & valid;
+        ma = gA == 0 ? v.x : v.y;
+        mb = gB == 1 ? v.y : m2;
+      }
+      const int ca = __popc(ma), cb = __popc(mb);
+      int xa = ca, xb = cb;  // inclusive sums over the block
+#pragma unroll
+      for (int off = 1; off < 32; off <<= 1) {
+        const int ya = __shfl_up_sync(kFull, xa, off), yb = __shfl_up_sync(kFull, xb, off);
+        if (lane >= off) {
+          xa += ya;
+          xb += yb;
+        }
+      }
+      if (lane == 31) s_sum[warp] = make_uint2((uint32_t)xa, (uint32_t)xb);
+      __syncthreads();
+      int ba = 0, bb = 0, ta = 0, tb = 0;
+#pragma unroll
+      for (int x = 0; x < kListThreads / 32; x++) {
+        const uint2 v = s_sum[x];
+        if (x < warp) {
+          ba += (int)v.x;
+          bb += (int)v.y;
+        }
+        ta += (int)v.x;
+        tb += (int)v.y;
+      }
+      int pa = posA + ba + xa - ca, pb = posB + bb + xb - cb;
+      const int row = 32 * (wb + w);
+      while (ma) {
+        list[pa++] = row + __ffs(ma) - 1;
+        ma &= ma - 1;
+      }
+      while (mb) {
+        list[pb++] = row + __ffs(mb) - 1;
+        mb &= mb - 1;
+      }
+      posA += ta;
+      posB += tb;
+      __syncthreads();
+    }
+    const int endA = 128 * (c ? qend[2] : qend[0]), endB = 128 * (c ? qend[3] : qend[1]);
+    for (int x = posA + tid; x < endA; x += kListThreads) list[x] = -1;
+    for (int x = posB + tid; x < endB; x += kListThreads) list[x] = -1;
+  }
+}
+
+// Compacted planes: one warp per record, quad and four 32-SNP columns.  Lane l gathers the row
+// pieces (32 bytes) of four samples, the warp transposes them and lane l writes the 32 bytes of
+// SNP 32q + l: its four words of g0, then of g1.  Bound by the transposes (shuffles).
+__global__ void __launch_bounds__(256) k_split_planes(const SplitJob* __restrict__ jobs, const SplitRec* __restrict__ recs,
+                                                      const int32_t* __restrict__ lists, uint4* __restrict__ cp) {
+  const SplitRec& rec = recs[blockIdx.y];
+  const int lane = threadIdx.x & 31;
+  const int ncol = rec.mlen / 128;
+  const int unit = blockIdx.x * 8 + (threadIdx.x >> 5);
+  const int quad = unit / ncol, col = unit - quad * ncol;
+  if (quad >= rec.qend[3]) return;
+  const SplitJob& J = jobs[rec.job];
+  const int q = rec.qlo + 4 * col;
+  uint32_t x[4][4], y[4][4];  // [column][word]
+  int s[4];
+#pragma unroll
+  for (int w = 0; w < 4; w++) s[w] = __ldg(lists + rec.list_off + 128 * quad + 32 * w + lane);
+#pragma unroll
+  for (int w = 0; w < 4; w++) {
+    uint4 a = make_uint4(0, 0, 0, 0), b = a;
+    if (s[w] >= 0) {
+      const uint4* src = reinterpret_cast<const uint4*>(J.rows + (int64_t)s[w] * J.mwp + q);
+      a = __ldg(src);
+      b = __ldg(src + 1);
+    }
+    x[0][w] = a.x; y[0][w] = a.y; x[1][w] = a.z; y[1][w] = a.w;
+    x[2][w] = b.x; y[2][w] = b.y; x[3][w] = b.z; y[3][w] = b.w;
+  }
+  uint4* dst = cp + rec.cp_off + 2 * ((int64_t)quad * rec.mlen + 128 * col + lane);
+#pragma unroll
+  for (int t = 0; t < 4; t++) {
+#pragma unroll
+    for (int w = 0; w < 4; w++) {
+      x[t][w] = transpose32(x[t][w], lane);
+      y[t][w] = transpose32(y[t][w], lane);
+    }
+    dst[64 * t] = make_uint4(x[t][0], x[t][1], x[t][2], x[t][3]);
+    dst[64 * t + 1] = make_uint4(y[t][0], y[t][1], y[t][2], y[t][3]);
+  }
+}
+
+// Tile queue: one block per run of records and j block u; the run's tiles of that j block follow
+// one another record by record, so the CTAs working at the same time share the (j, k) margins
+// through L2.  The blocks take their place in the queue from the cursor (any order is correct).
+__global__ void __launch_bounds__(128) k_split_tiles(const SplitJob* __restrict__ jobs, const SplitRec* __restrict__ recs,
+                                                     const SplitRun* __restrict__ runs, uint64_t* __restrict__ tiles,
+                                                     unsigned* __restrict__ cursor) {
+  __shared__ unsigned s_base;
+  const SplitRun run = runs[blockIdx.y];
+  const int u = blockIdx.x;
+  const int m = jobs[recs[run.rec0].job].m;
+  auto count = [&](int i) { return (int)tiles_of_pair_block((int64_t)i + 1 + kSplitJ * u, m, kSplitK); };
+  if (count(recs[run.rec0].i) == 0) return;  // the run's smallest i has the most tiles
+  unsigned total = 0;
+  for (int r = threadIdx.x; r < run.n; r += blockDim.x) total += (unsigned)count(recs[run.rec0 + r].i);
+  // block sum through a shared accumulator (few records per run)
+  __shared__ unsigned s_total;
+  if (threadIdx.x == 0) s_total = 0;
+  __syncthreads();
+  if (total) atomicAdd(&s_total, total);
+  __syncthreads();
+  if (threadIdx.x == 0) s_base = atomicAdd(cursor, s_total);
+  __syncthreads();
+  unsigned at = s_base;
+  for (int r = 0; r < run.n; r++) {
+    const int n = count(recs[run.rec0 + r].i);
+    for (int t = threadIdx.x; t < n; t += blockDim.x)
+      tiles[at + t] = pack_split_tile((uint32_t)(run.rec0 + r), (uint32_t)u, (uint32_t)t);
+    at += (unsigned)n;
+  }
+}
+
+// ------------------------------------------------------------------ the search kernel
+
+constexpr int kSProd = 6;            // producing warps
+constexpr int kSScore = 8;           // scoring warps (the last ones): four pairs of warps
+constexpr int kSPairs = kSScore / 2;
+constexpr int kSPairJ = 28;          // SNPs j scored by a pair (x 32 SNPs k)
+constexpr int kSFirstScore = kSProd + 2;
+constexpr int kSThreads = 32 * (kSFirstScore + kSScore);
+constexpr int kSStages = 4;
+constexpr int kSRowBytes = 128;      // 8 words of 32 samples, E2M1
+constexpr uint32_t kSSbo = 8 * kSRowBytes;
+constexpr int kSHalfJ = kSplitJ / 2; // SNPs j expanded by each CTA
+constexpr int kSStageA = 128 * kSRowBytes;
+constexpr int kSStageBytes = (128 + 2 * kSHalfJ) * kSRowBytes;
+constexpr int kSStagingOff = kSStages * kSStageBytes;  // E[c][j][k]: uint4 words (u, b) = (A,0) (A,1) (B,0) (B,1)
+constexpr int kSStagingBytes = 2 * kSplitJ * 64 * 16;
+// Per pair of scoring warps: the margins of its SNPs j.
+constexpr int kSPairOff = kSStagingOff + kSStagingBytes;
+constexpr int kMargWords = 28;       // per g_j: forms of (A, g_j), (B, g_j), g_j, 2 unused; offset of row j of the pair table
+constexpr int kSPairBytes = kSPairJ * kMargWords * 4;
+constexpr int kSSlotOff = kSPairOff + kSPairs * kSPairBytes;
+constexpr int kSSlotBytes = 64 + 128 + 16;        // record, job, descriptor
+constexpr int kSBarOff = kSSlotOff + kSplitSlots * kSSlotBytes;
+constexpr int kSSmemBytes = kSBarOff + 256;
+static_assert(kSSmemBytes <= 232448 - 1024, "shared memory of one CTA");
+static_assert(kSPairBytes % 16 == 0 && kSStagingOff % 128 == 0, "alignment");
+
+constexpr int kCFull = 0, kCEmpty = 4, kCAcc = 8, kCDrained = 9, kCHand = 10, kCDesc = 13, kCRel = 16, kCFinal = 19;
+// Accumulators of group g: columns [112g, 112g + 112).  Scale factors (UE8M0, per row and K group):
+// columns [448, 480) for the first two K groups of a quad (2 and 1), [480, 512) for the others (1/2).
+constexpr uint32_t kSSfCol = 448;
+constexpr uint32_t kScale01 = 0x7F807F80u, kScale23 = 0x7E7E7E7Eu;
+// kind::mxf4, M = 256 (pair), N = 112, K = 64; E2M1 operands, UE8M0 scales, FP32 accumulators
+constexpr uint32_t kSIdesc = (1u << 7) | (1u << 10) | ((112u >> 3) << 17) | (1u << 23) | ((256u >> 4) << 24);
+
+// Issued by one elected lane of a converged warp with warp-uniform operands: an instruction then
+// takes 8 clocks to issue; from a lane-0 branch it takes 44 (every operand is moved to the uniform
+// registers first), and the products of a stage 610 clocks instead of 330.
+__device__ __forceinline__ void split_mma(uint32_t d_tmem, uint64_t a, uint64_t b, uint32_t accumulate, uint32_t sfa,
+                                          uint32_t sfb) {
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "elect.sync _|q, 0xffffffff;\n\t"
+      "@q tcgen05.mma.cta_group::2.kind::mxf4.block_scale.scale_vec::2X [%0], %1, %2, %3, [%5], [%6], p;\n\t}\n" ::"r"(
+          d_tmem),
+      "l"(a), "l"(b), "r"(kSIdesc), "r"(accumulate), "r"(sfa), "r"(sfb));
+}
+// Arrival on a barrier of the other CTA.  The stores it announces are to this CTA's own shared
+// memory and for its own tensor core (fence.proxy.async before), so no cluster-scope release: that
+// one waits for earlier accesses of the thread and costs several hundred clocks per stage.
+__device__ __forceinline__ void bar_arrive_remote(uint32_t cluster_addr) {
+  asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
+}
+__device__ __forceinline__ void split_commit(uint32_t bar) {
+  asm volatile(
+      "{\n\t.reg .pred q;\n\t"
+      "elect.sync _|q, 0xffffffff;\n\t"
+      "@q tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;\n\t}\n" ::"r"(
+          bar),
+      "h"((uint16_t)3)
+      : "memory");
+}
+
+__device__ __forceinline__ void tmem_ld2(uint32_t addr, uint32_t (&r)[2]) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x2.b32 {%0, %1}, [%2];" : "=r"(r[0]), "=r"(r[1]) : "r"(addr));
+}
+
+// 128 sample bits of one SNP and genotype -> four K groups of 32 E2M1 elements.  Group q holds bit q
+// of every nibble of the four words: 0.5, 1 and 2 for q = 0, 1, 2 without a shift, and q = 3 moved
+// to 2 (bit 3 is the sign).  Both operands hold the same values, so the products are 1/4, 1, 4 and
+// 4; the scale factors of the K groups (kScale01, kScale23) make them 1.
+__device__ __forceinline__ void store_quad(uint32_t at, uint4 w) {
+  sts128(at, make_uint4(w.x & 0x11111111u, w.y & 0x11111111u, w.z & 0x11111111u, w.w & 0x11111111u));
+  sts128(at + 128, make_uint4(w.x & 0x22222222u, w.y & 0x22222222u, w.z & 0x22222222u, w.w & 0x22222222u));
+  sts128(at + 256, make_uint4(w.x & 0x44444444u, w.y & 0x44444444u, w.z & 0x44444444u, w.w & 0x44444444u));
+  sts128(at + 384, make_uint4((w.x >> 1) & 0x44444444u, (w.y >> 1) & 0x44444444u, (w.z >> 1) & 0x44444444u,
+                              (w.w >> 1) & 0x44444444u));
+}
+
+__device__ __forceinline__ uint4 lds128(uint32_t saddr) {
+  uint4 v;
+  asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(saddr));
+  return v;
+}
+
+__device__ __forceinline__ void pair_sync(int id) { asm volatile("bar.sync %0, 64;" ::"r"(id) : "memory"); }
+
+__device__ __forceinline__ float rcp_approx(float x) {
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+}
+
+// w.lo * coef.byte0 + w.hi * coef.byte1 + c, unsigned halves, signed bytes
+__device__ __forceinline__ int dot2(uint32_t w, uint32_t coef, int c) {
+  int r;
+  asm("dp2a.lo.u32.s32 %0, %1, %2, %3;" : "=r"(r) : "r"(w), "r"(coef), "r"(c));
+  return r;
+}
+
+// The two linear forms of a cell (a controls, b cases) that the screening bound needs, as integers:
+// n = N = a + b + 1 and d = 128 D = 128 (a + 1/2) - kp N.  A margin over x cells holds the sums of
+// its cells' forms, so that cells complete by subtraction.
+struct Form {
+  int n, d;
+};
+__device__ __forceinline__ Form operator-(Form x, Form y) { return Form{x.n - y.n, x.d - y.d}; }
+struct FormOf {  // counts (class 0 low half, class 1 high half) of a sum over `cells` cells -> forms
+  uint32_t coef;   // bytes (128 - kp, -kp)
+  int bias;        // 64 - kp
+  __device__ __forceinline__ Form operator()(uint32_t w, int cells) const {
+    return Form{dot2(w, 0x0101u, cells), dot2(w, coef, bias * cells)};
+  }
+};
+
+// Lower bound of K2 (screen_constants in host_data.cpp), cell by cell: per cell two conversions,
+// one reciprocal, four FP32 operations and half an integer addition.
+struct Screen {
+  float theta1, theta2;  // of 128 D
+  float acc;
+  uint32_t bits;         // sum of the cells' log2 (N - theta1 D), from below, in units of 2^-23
+  template <int kN>
+  __device__ __forceinline__ void cells(const Form (&f)[kN]) {
+    float D[kN], P[kN], r[kN];
+#pragma unroll
+    for (int x = 0; x < kN; x++) {
+      D[x] = (float)f[x].d;
+      P[x] = fmaf(D[x], -theta1, (float)f[x].n);
+    }
+#pragma unroll
+    for (int x = 0; x < kN; x++) r[x] = rcp_approx(fmaf(fabsf(D[x]), -theta2, P[x]));
+#pragma unroll
+    for (int x = 0; x + 1 < kN; x += 2) bits += __float_as_uint(P[x]) + __float_as_uint(P[x + 1]);
+    if (kN & 1) bits += __float_as_uint(P[kN - 1]);
+#pragma unroll
+    for (int x = 0; x < kN; x++) acc = fmaf(D[x] * r[x], D[x], acc);
+  }
+};
+
+// The nine cells of one genotype of j from those with g_k = 0 and 1 of the two counted genotypes of
+// i (f[0], f[1]: A; f[3], f[4]: B) and the margins: (A, j), (B, j), j, and (j, k) with g_k = 0 and 1.
+// f[6 ..]: C.
+__device__ __forceinline__ void row_forms(Form ijA, Form ijB, Form nj, Form jk0, Form jk1, Form (&f)[9]) {
+  f[2] = ijA - f[0] - f[1];
+  f[5] = ijB - f[3] - f[4];
+  f[6] = jk0 - f[0] - f[3];
+  f[7] = jk1 - f[1] - f[4];
+  f[8] = nj - jk0 - jk1 - f[2] - f[5];
+}
+
+// Cells of one counted genotype of i from its four counts: t[3b + c].
+__device__ __forceinline__ void counted_cells(uint32_t t00, uint32_t t01, uint32_t t10, uint32_t t11, uint32_t ij0,
+                                              uint32_t ij1, uint32_t ij2, uint32_t ik0, uint32_t ik1, uint32_t (&t)[9]) {
+  t[0] = t00;
+  t[1] = t01;
+  t[2] = ij0 - t00 - t01;
+  t[3] = t10;
+  t[4] = t11;
+  t[5] = ij1 - t10 - t11;
+  t[6] = ik0 - t00 - t10;
+  t[7] = ik1 - t01 - t11;
+  t[8] = ij2 - t[6] - t[7];
+}
+
+// Cells of the genotype of i that was not counted: (j, k) margins less the counted cells' sums.
+__device__ __forceinline__ void dropped_cells(uint4 jk, uint32_t nj0, uint32_t nj1, uint32_t nj2, uint32_t nk0,
+                                              uint32_t nk1, const uint32_t (&a)[9], const uint32_t (&b)[9],
+                                              uint32_t (&t)[9]) {
+  const uint32_t m02 = nj0 - jk.x - jk.y, m12 = nj1 - jk.z - jk.w;
+  const uint32_t m20 = nk0 - jk.x - jk.z, m21 = nk1 - jk.y - jk.w, m22 = nj2 - m20 - m21;
+  t[0] = jk.x - a[0] - b[0];
+  t[1] = jk.y - a[1] - b[1];
+  t[2] = m02 - a[2] - b[2];
+  t[3] = jk.z - a[3] - b[3];
+  t[4] = jk.w - a[4] - b[4];
+  t[5] = m12 - a[5] - b[5];
+  t[6] = m20 - a[6] - b[6];
+  t[7] = m21 - a[7] - b[7];
+  t[8] = m22 - a[8] - b[8];
+}
+
+// Counts (g_i = g, g_x = 0 and 1) from a pair's counts and the singles of x.
+__device__ __forceinline__ void by_genotype(uint4 c0, uint4 c1, uint32_t n0, uint32_t n1, int g, uint32_t& x0, uint32_t& x1) {
+  const uint32_t a0 = c0.x | (c1.x << 16), a1 = c0.y | (c1.y << 16), b0 = c0.z | (c1.z << 16), b1 = c0.w | (c1.w << 16);
+  x0 = g == 0 ? a0 : g == 1 ? b0 : n0 - a0 - b0;
+  x1 = g == 0 ? a1 : g == 1 ? b1 : n1 - a1 - b1;
+}
+
+// K2 of triplet (i, j, k) in the reference's arithmetic and order from its eight staged words per
+// class (e0: g_k = 0, e1: g_k = 1) and the margins in device memory; its table where one is
+// wanted.  Not inlined: the search takes it for a few triplets in a million.
+__device__ __noinline__ float exact_score(uint4 e0, uint4 e1, const SplitJob* J, int i, int j, int k, int genos,
+                                          uint32_t* table) {
+  const int gA = genos & 3, gB = (genos >> 2) & 3, gC = genos >> 4;
+  const int64_t m_pad = J->m_pad;
+  auto single = [&](int x, uint32_t& n0, uint32_t& n1) {
+    const uint2 a = __ldg(reinterpret_cast<const uint2*>(J->singles) + x), b = __ldg(reinterpret_cast<const uint2*>(J->singles) + m_pad + x);
+    n0 = a.x | (b.x << 16);
+    n1 = a.y | (b.y << 16);
+  };
+  const uint32_t all = (uint32_t)J->n0 | ((uint32_t)J->n1 << 16);
+  uint32_t ni[3], nj[3], nk[3];
+  single(i, ni[0], ni[1]);
+  single(j, nj[0], nj[1]);
+  single(k, nk[0], nk[1]);
+  ni[2] = all - ni[0] - ni[1];
+  nj[2] = all - nj[0] - nj[1];
+  const uint4* pij = J->pairs + tri_offset(m_pad, i, j);
+  const uint4* pik = J->pairs + tri_offset(m_pad, i, k);
+  const uint4* pjk = J->pairs + tri_offset(m_pad, j, k);
+  const uint4 ij0 = __ldg(pij), ij1 = __ldg(pij + J->tri), ik0 = __ldg(pik), ik1 = __ldg(pik + J->tri);
+  const uint4 jk0 = __ldg(pjk), jk1 = __ldg(pjk + J->tri);
+  const uint4 jk = make_uint4(jk0.x | (jk1.x << 16), jk0.y | (jk1.y << 16), jk0.z | (jk1.z << 16), jk0.w | (jk1.w << 16));
+  uint32_t t[3][9], x0, x1, y0, y1;
+  by_genotype(ij0, ij1, nj[0], nj[1], gA, x0, x1);
+  by_genotype(ik0, ik1, nk[0], nk[1], gA, y0, y1);
+  counted_cells(e0.x, e1.x, e0.y, e1.y, x0, x1, (gA == 0 ? ni[0] : ni[1]) - x0 - x1, y0, y1, t[0]);
+  by_genotype(ij0, ij1, nj[0], nj[1], gB, x0, x1);
+  by_genotype(ik0, ik1, nk[0], nk[1], gB, y0, y1);
+  counted_cells(e0.z, e1.z, e0.w, e1.w, x0, x1, (gB == 1 ? ni[1] : ni[2]) - x0 - x1, y0, y1, t[1]);
+  dropped_cells(jk, nj[0], nj[1], nj[2], nk[0], nk[1], t[0], t[1], t[2]);
+  const float* __restrict__ lut = J->lut;
+  float score = 0.0f;
+#pragma unroll
+  for (int g = 0; g < 3; g++) {
+#pragma unroll
+    for (int c = 0; c < 9; c++) {
+      const uint32_t w = g == gC ? t[2][c] : ((g == 0 || (g == 1 && gC == 0)) ? t[0][c] : t[1][c]);
+      const uint32_t a = w & 0xFFFFu, b = w >> 16;
+      const float d = __fsub_rn(__ldg(lut + a + b + 1), __ldg(lut + a));
+      score = __fadd_rn(score, __fsub_rn(d, __ldg(lut + b)));
+      if (table) {
+        table[9 * g + c] = a;
+        table[27 + 9 * g + c] = b;
+      }
+    }
+  }
+  return fabsf(score);
+}
+
+template <bool kDump, bool kTopK>
+__global__ void __launch_bounds__(kSThreads, 1) k_scan_split(const SplitParams p) {
+  extern __shared__ __align__(1024) unsigned char smem[];
+  __shared__ uint32_t s_tmem;
+  __shared__ long long s_hand[kSplitSlots];  // odd CTA: descriptors handed over by the even CTA
+  __shared__ int s_abort, s_fail[kSPairs];         // s_fail: one per pair of scoring warps
+  const int tid = threadIdx.x, warp = __shfl_sync(kFull, tid >> 5, 0), lane = tid & 31;
+  const uint32_t crank = cluster_rank();
+  const bool even = crank == 0;
+  const uint32_t sbase = smem_u32(smem), bar0 = sbase + kSBarOff;
+  auto bar = [&](int slot) { return bar0 + 8u * (uint32_t)slot; };
+  auto slot_rec = [&](uint32_t t) { return reinterpret_cast<const SplitRec*>(smem + kSSlotOff + (t % kSplitSlots) * kSSlotBytes); };
+  auto slot_job = [&](uint32_t t) { return reinterpret_cast<const SplitJob*>(smem + kSSlotOff + (t % kSplitSlots) * kSSlotBytes + 64); };
+  auto slot_desc = [&](uint32_t t) { return reinterpret_cast<volatile long long*>(smem + kSSlotOff + (t % kSplitSlots) * kSSlotBytes + 192); };
+  const long long wl = p.wait_limit > 0 ? p.wait_limit : kWaitLimit;
+  volatile int* abort_flag = &s_abort;
+
+  if (tid == 0) {
+    for (int s = 0; s < kSStages; s++) {
+      bar_init(bar(kCFull + s), 2 * kSProd);  // both CTAs' producing warps arrive in the even one
+      bar_init(bar(kCEmpty + s), 1);
+    }
+    bar_init(bar(kCAcc), 1);
+    bar_init(bar(kCDrained), kSScore + (even ? 1 : 0));
+    for (int s = 0; s < kSplitSlots; s++) {
+      bar_init(bar(kCHand + s), 1);
+      bar_init(bar(kCDesc + s), 1);
+      bar_init(bar(kCRel + s), kSScore);
+    }
+    bar_init(bar(kCFinal), 1);
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    s_abort = 0;
+    for (int x = 0; x < kSPairs; x++) s_fail[x] = 0;
+  }
+  cluster_sync_all();
+  if (warp == 0) {
+    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&s_tmem)), "r"(512u)
+                 : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem = __shfl_sync(kFull, s_tmem, 0);
+  if (warp < 4) {
+    const uint32_t ta = tmem + ((uint32_t)(32 * warp) << 16) + kSSfCol;
+    tmem_st16_fill(ta, kScale01);
+    tmem_st16_fill(ta + 16, kScale01);
+    tmem_st16_fill(ta + 32, kScale23);
+    tmem_st16_fill(ta + 48, kScale23);
+    tmem_wait_st();
+  }
+  tc_fence_before();
+  __syncthreads();
+  cluster_sync_all();
+  tc_fence_after();
+
+  if (warp < kSProd) {
+    // ================= producing warps =================
+    // A: rows 64c + kk of this CTA's 64 SNPs k; B: rows 28b + jj of its 28 SNPs j.  A warp takes
+    // one quad (4 words) of a stage for 32 SNPs: 32 bytes loaded, 8 x 16 bytes stored per lane.
+    const bool isA = warp < 4;
+    const int sub = isA ? warp >> 1 : warp - 4;
+    const int x = isA ? 32 * (warp & 1) + lane : lane;           // row of genotype 0
+    const int row1 = x + (isA ? 64 : kSHalfJ);                   // row of genotype 1
+    const bool mine = isA || lane < kSHalfJ;
+    const uint32_t off_base = (isA ? 0u : (uint32_t)kSStageA) + 512u * (uint32_t)sub;
+    const uint32_t off0 = off_base + (uint32_t)(x >> 3) * kSSbo + (uint32_t)(x & 7) * 16;
+    const uint32_t off1 = off_base + (uint32_t)(row1 >> 3) * kSSbo + (uint32_t)(row1 & 7) * 16;
+    uint32_t g = 0;
+    for (uint32_t t = 0;; t++) {
+      const bool got = bar_wait(bar(kCDesc + (int)(t % kSplitSlots)), (t / kSplitSlots) & 1u, wl);
+      if (__any_sync(kFull, !got)) {
+        *abort_flag = 1;
+        break;
+      }
+      const long long desc = *slot_desc(t);
+      if (desc < 0) break;
+      const SplitRec* R = slot_rec(t);
+      const int nq = R->qend[3], nst = (nq + 1) / 2, mlen = R->mlen;
+      const int j0 = R->i + 1 + kSplitJ * (int)(((uint64_t)desc >> 24) & 0x3FFFF);
+      const int k0 = j0 + 1 + kSplitK * (int)(((uint64_t)desc >> 42) & 0xFFFF);
+      const int snp = (isA ? k0 + 64 * (int)crank : j0 + kSHalfJ * (int)crank) + x - 32 * R->qlo;
+      const bool on = mine && snp < mlen;
+      const uint4* src = p.cp + R->cp_off + 2 * ((int64_t)sub * mlen + (on ? snp : 0));
+      const int64_t step = 4 * (int64_t)mlen;
+      // loads run four stages ahead of their use
+      uint4 va[4], vb[4];
+      auto load = [&](int st, uint4& a, uint4& b) {
+        if (on && 2 * st + sub < nq) {
+          const uint4* s = src + st * step;
+          a = __ldg(s);
+          b = __ldg(s + 1);
+        }
+      };
+#pragma unroll
+      for (int u = 0; u < 4; u++) {
+        va[u] = vb[u] = make_uint4(0, 0, 0, 0);
+        load(u, va[u], vb[u]);
+      }
+      bool bad = false;
+      for (int st0 = 0; st0 < nst && !bad; st0 += 4) {
+#pragma unroll
+        for (int u = 0; u < 4; u++) {
+          const int st = st0 + u;
+          if (st < nst && !bad) {
+            const uint32_t gg = g + (uint32_t)st;
+            const int s = (int)(gg % kSStages);
+            const uint32_t use = gg / kSStages;
+            bad = __any_sync(kFull, use > 0 && !bar_wait(bar(kCEmpty + s), (use & 1u) ^ 1u, wl));
+            if (!bad) {
+              if (on && 2 * st + sub < nq) {
+                const uint32_t at = sbase + (uint32_t)(s * kSStageBytes);
+                store_quad(at + off0, va[u]);
+                store_quad(at + off1, vb[u]);
+              }
+              load(st + 4, va[u], vb[u]);
+              fence_proxy_async();
+              __syncwarp();
+              if (lane == 0) {
+                if (even) bar_arrive(bar(kCFull + s));
+                else bar_arrive_remote(map_cta(bar(kCFull + s), 0));
+              }
+            }
+          }
+        }
+      }
+      if (bad) {
+        *abort_flag = 1;
+        break;
+      }
+      g += (uint32_t)nst;
+    }
+  } else if (warp == kSProd) {
+    // ================= issuing warp (of the even CTA; the odd one passes its "drained" on) ======
+    uint32_t g = 0;
+    for (uint32_t t = 0;; t++) {
+      bool bad = !bar_wait(bar(kCDesc + (int)(t % kSplitSlots)), (t / kSplitSlots) & 1u, wl);
+      if (__any_sync(kFull, bad)) {
+        *abort_flag = 1;
+        break;
+      }
+      if (__shfl_sync(kFull, *slot_desc(t), 0) < 0) break;
+      const SplitRec* R = slot_rec(t);
+      const int e0 = __shfl_sync(kFull, R->qend[0], 0), e1 = __shfl_sync(kFull, R->qend[1], 0);
+      const int e2 = __shfl_sync(kFull, R->qend[2], 0), nq = __shfl_sync(kFull, R->qend[3], 0), nst = (nq + 1) / 2;
+      if (t > 0) {  // the previous tile's accumulators have been copied out
+        if (even) {
+          bad = !bar_wait(bar(kCDrained), (t - 1) & 1u, wl);
+        } else {
+          bad = !bar_wait(bar(kCDrained), (t - 1) & 1u, wl);
+          if (!bad && lane == 0) bar_arrive_cluster(map_cta(bar(kCDrained), 0));
+        }
+      }
+      bad = __any_sync(kFull, bad);
+      if (!even && !bad) continue;  // the odd CTA's operands go to the same products
+      for (int st = 0; st < nst && !bad; st++) {
+        const uint32_t gg = g + (uint32_t)st;
+        const int s = (int)(gg % kSStages);
+        const uint32_t use = gg / kSStages;
+        bad = __any_sync(kFull, !bar_wait(bar(kCFull + s), use & 1u, wl));
+        if (bad) break;
+        tc_fence_after();
+        const uint32_t sA = sbase + (uint32_t)(s * kSStageBytes), sB = sA + kSStageA;
+        const uint64_t da = smem_desc(sA, kSSbo), db = smem_desc(sB, kSSbo);
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+          const int q = 2 * st + h;
+          if (q < nq) {
+            const int grp = (q >= e0) + (q >= e1) + (q >= e2);
+            const bool first = q == 0 || q == e0 || q == e1 || q == e2;
+            const uint32_t d = tmem + 112u * (uint32_t)grp;
+            split_mma(d, da + 32u * h, db + 32u * h, first ? 0u : 1u, tmem + kSSfCol, tmem + kSSfCol + 16);
+            split_mma(d, da + 32u * h + 16u, db + 32u * h + 16u, 1u, tmem + kSSfCol + 32, tmem + kSSfCol + 48);
+          }
+        }
+        split_commit(bar(kCEmpty + s));
+        if (st == nst - 1) split_commit(bar(kCAcc));
+      }
+      if (bad) {
+        *abort_flag = 1;
+        break;
+      }
+      g += (uint32_t)nst;
+    }
+  } else if (warp == kSProd + 1) {
+    // ================= scheduling warp =================
+    // Even CTA: ticket -> descriptor, handed to the odd CTA; both publish descriptor, record and
+    // job of tile t in slot t % 3, free again once tile t - 3 has been scored.
+    const unsigned n_tiles = *reinterpret_cast<const volatile unsigned*>(p.n_tiles);
+    for (uint32_t t = 0;; t++) {
+      const int sl = (int)(t % kSplitSlots);
+      const uint32_t ph = (t / kSplitSlots) & 1u;
+      long long d = -1;
+      bool bad = false;
+      if (lane == 0) {
+        if (!even) {
+          if (bar_wait_cluster(bar(kCHand + sl), ph, wl)) d = *reinterpret_cast<volatile long long*>(&s_hand[sl]);
+          else bad = true;
+        }
+        if (t >= kSplitSlots && !bad) bad = !bar_wait(bar(kCRel + sl), ph ^ 1u, wl);
+        if (even && !bad) {
+          const unsigned ticket = atomicAdd(p.counter, 1u);
+          if (ticket < n_tiles && !*abort_flag) d = (long long)__ldg(p.tiles + ticket);
+        }
+      }
+      bad = __any_sync(kFull, bad);
+      if (bad) {
+        *abort_flag = 1;
+        d = -1;
+      }
+      d = __shfl_sync(kFull, d, 0);
+      if (even && lane == 0) {
+        st_cluster_s64(map_cta(smem_u32(&s_hand[sl]), 1), d);
+        bar_arrive_cluster(map_cta(bar(kCHand + sl), 1));
+      }
+      uint32_t* sw = reinterpret_cast<uint32_t*>(smem + kSSlotOff + sl * kSSlotBytes);
+      if (d >= 0) {
+        const SplitRec* R = p.recs + ((uint64_t)d & 0xFFFFFF);
+        if (lane < 16) sw[lane] = reinterpret_cast<const uint32_t*>(R)[lane];
+        const SplitJob* J = p.jobs + R->job;
+        sw[16 + lane] = reinterpret_cast<const uint32_t*>(J)[lane];
+      }
+      if (lane == 0) *slot_desc(t) = d;
+      __syncwarp();
+      if (lane == 0) bar_arrive(bar(kCDesc + sl));
+      if (d < 0) break;
+    }
+  } else if (warp >= kSFirstScore) {
+    // ================= scoring warps =================
+    // Warp (c, kh, part): drains rows c of the SNPs k 32kh.. and columns of a third of the SNPs
+    // j; the pair of warps with the same (kh, part) shares its part of the staging buffer and its margins
+    // and nothing else, so the pairs go from tile to tile by themselves (less than a tile apart).
+    const int sw = warp - kSFirstScore;
+    const int quarter = warp & 3, kh = quarter & 1, c = quarter >> 1, part = sw >> 2;
+    const int pt = 32 * c + lane;  // thread of the pair
+    const int pair = kh + 2 * part, pbar = 1 + pair;
+    const int pj = 28 * part, nj = 28;  // its SNPs j in the tile
+    volatile int* const fail = &s_fail[pair];
+    int* const marg = reinterpret_cast<int*>(smem + kSPairOff + pair * kSPairBytes);
+    float best_s = FLT_MAX, list_s = FLT_MAX;
+    unsigned long long best_k = ~0ull, list_k = ~0ull;
+    unsigned thr = 0x7F7F7F7Fu, known = thr;  // bits of the score to reach; of the one last read
+    if (kTopK) {  // continue the lists of the earlier launches of this search
+      const BestSlot& e = p.cand[((int64_t)blockIdx.x * kSScore + sw) * 32 + lane];
+      list_s = e.score;
+      list_k = e.key;
+    }
+    int cur_job = -1;
+    auto flush_job = [&](int jb) {  // this warp's best of job jb into its slot
+#pragma unroll
+      for (int off = 16; off > 0; off >>= 1) {
+        const float os = __shfl_xor_sync(kFull, best_s, off);
+        const unsigned long long ok = __shfl_xor_sync(kFull, best_k, off);
+        if (better(os, ok, best_s, best_k)) {
+          best_s = os;
+          best_k = ok;
+        }
+      }
+      if (lane == 0) {
+        BestSlot& slot = p.job_slots[((int64_t)jb * gridDim.x + blockIdx.x) * kSScore + sw];
+        if (better(best_s, best_k, slot.score, slot.key)) {
+          slot.score = best_s;
+          slot.key = best_k;
+        }
+      }
+      best_s = FLT_MAX;
+      best_k = ~0ull;
+    };
+    long long desc = -1;
+    bool got = bar_wait(bar(kCDesc), 0, wl);
+    if (got) desc = *slot_desc(0);
+    for (uint32_t t = 0;; t++) {
+      bool ok = got;
+      const SplitRec* R = slot_rec(t);
+      const SplitJob* J = slot_job(t);
+      int i = 0, m = 0, jp = 0, kb = 0;  // first SNP, SNPs; first SNP j and k of the pair
+      // margins of this thread's SNP k and, in the pair's first threads, of a SNP j: in flight while the
+      // tile's products complete and its accumulators are copied
+      uint4 ik0, ik1, ij0, ij1;
+      uint2 sk0, sk1, sj0, sj1, si0, si1;
+      if (ok && desc >= 0) {
+        i = R->i;
+        m = J->m;
+        jp = i + 1 + kSplitJ * (int)(((uint64_t)desc >> 24) & 0x3FFFF);
+        kb = jp + 1 + kSplitK * (int)(((uint64_t)desc >> 42) & 0xFFFF) + 64 * (int)crank + 32 * kh;
+        jp += pj;
+        const int64_t m_pad = J->m_pad;
+        const uint4* pi = J->pairs + tri_offset(m_pad, i, i + 1) - (i + 1);  // + x: pair (i, x)
+        const uint2* si = reinterpret_cast<const uint2*>(J->singles);
+        const int xk = min(kb + lane, m - 1), xj = min(jp + (pt < nj ? pt : 0), m - 1);  // both > i
+        ik0 = __ldg(pi + xk);
+        ik1 = __ldg(pi + J->tri + xk);
+        sk0 = __ldg(si + xk);
+        sk1 = __ldg(si + m_pad + xk);
+        ij0 = __ldg(pi + xj);
+        ij1 = __ldg(pi + J->tri + xj);
+        sj0 = __ldg(si + xj);
+        sj1 = __ldg(si + m_pad + xj);
+        si0 = __ldg(si + i);
+        si1 = __ldg(si + m_pad + i);
+        if (lane == 0) known = *reinterpret_cast<volatile unsigned*>(p.thr + R->job);
+        ok = bar_wait(bar(kCAcc), t & 1u, wl);
+      }
+      // Both warps leave together or not at all: the pair's flag is written only before this
+      // barrier and read only between it and the next one.
+      if (!ok) *abort_flag = 1;
+      if (!ok || *abort_flag) *fail = 1;
+      pair_sync(pbar);  // both warps are done with the staging buffer and the margins
+      if (desc < 0 || *fail) break;
+      known = __shfl_sync(kFull, known, 0);
+      if (R->job != cur_job) {
+        if (cur_job >= 0) flush_job(cur_job);
+        cur_job = R->job;
+        thr = known;
+      }
+      thr = min(thr, known);
+      const int genos = R->genos, gA = genos & 3, gB = (genos >> 2) & 3;
+      tc_fence_after();
+      // accumulators -> staging
+      const uint32_t Ek = sbase + kSStagingOff + (uint32_t)((pj * 64 + 32 * kh + lane) * 16);
+      {
+        const uint32_t ta = tmem + ((uint32_t)(32 * quarter) << 16);
+        const uint32_t dst = Ek + (uint32_t)(c * kSplitJ * 64 * 16);
+#pragma unroll 1
+        for (int jj = 0; jj < nj; jj += 2) {
+          const uint32_t tc = ta + (uint32_t)(pj + jj + (pj + jj >= kSHalfJ ? kSHalfJ : 0));  // SNP j of half h: 28h further
+          uint32_t v[4][2][2];
+#pragma unroll
+          for (int g = 0; g < 4; g++)
+#pragma unroll
+            for (int b = 0; b < 2; b++) tmem_ld2(tc + (uint32_t)(112 * g + kSHalfJ * b), v[g][b]);
+          tmem_wait_ld();
+          const float magic = 8388608.0f;
+#pragma unroll
+          for (int q = 0; q < 2; q++) {
+            uint32_t w[4];
+#pragma unroll
+            for (int ub = 0; ub < 4; ub++) {
+              const uint32_t lo = __float_as_uint(__uint_as_float(v[ub >> 1][ub & 1][q]) + magic);
+              const uint32_t hi = __float_as_uint(__uint_as_float(v[2 + (ub >> 1)][ub & 1][q]) + magic);
+              w[ub] = prmt(lo, hi, 0x5410u);
+            }
+            sts128(dst + (uint32_t)((jj + q) * 64 * 16), make_uint4(w[0], w[1], w[2], w[3]));
+          }
+        }
+      }
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) bar_arrive(bar(kCDrained));
+      // margins as forms: per j into shared memory, per k (this thread's) in registers
+      const uint32_t ntot = (uint32_t)J->n0 | ((uint32_t)J->n1 << 16);
+      const FormOf form{J->coef, J->bias};
+      if (pt < nj) {
+        const uint32_t i0 = si0.x | (si1.x << 16), i1 = si0.y | (si1.y << 16);
+        const uint32_t nA = gA == 0 ? i0 : i1, nB = gB == 1 ? i1 : ntot - i0 - i1;
+        const uint32_t n0 = sj0.x | (sj1.x << 16), n1 = sj0.y | (sj1.y << 16);
+        uint32_t wA[3], wB[3];
+        const uint32_t wj[3] = {n0, n1, ntot - n0 - n1};
+        by_genotype(ij0, ij1, n0, n1, gA, wA[0], wA[1]);
+        by_genotype(ij0, ij1, n0, n1, gB, wB[0], wB[1]);
+        wA[2] = nA - wA[0] - wA[1];
+        wB[2] = nB - wB[0] - wB[1];
+        int* o = marg + kMargWords * pt;
+#pragma unroll
+        for (int b = 0; b < 3; b++) {
+          const Form x = form(wA[b], 3), y = form(wB[b], 3), z = form(wj[b], 9);
+          *reinterpret_cast<int4*>(o + 8 * b) = make_int4(x.n, x.d, y.n, y.d);
+          *reinterpret_cast<int2*>(o + 8 * b + 4) = make_int2(z.n, z.d);
+        }
+        const int64_t j = min(jp + pt, m - 1);
+        const int64_t jo = j * (J->m_pad - 1) - (j * (j - 1)) / 2 - j - 1;
+        *reinterpret_cast<int2*>(o + 24) = make_int2((int)(uint32_t)jo, (int)(uint32_t)((uint64_t)jo >> 32));
+      }
+      Form kA0, kA1, kB0, kB1, nk0, nk1;
+      {
+        const uint32_t n0 = sk0.x | (sk1.x << 16), n1 = sk0.y | (sk1.y << 16);
+        uint32_t x0, x1;
+        by_genotype(ik0, ik1, n0, n1, gA, x0, x1);
+        kA0 = form(x0, 3);
+        kA1 = form(x1, 3);
+        by_genotype(ik0, ik1, n0, n1, gB, x0, x1);
+        kB0 = form(x0, 3);
+        kB1 = form(x1, 3);
+        nk0 = form(n0, 9);
+        nk1 = form(n1, 9);
+      }
+      pair_sync(pbar);  // staging rows and margins are in place
+      // complete, screen, select: lane = k, this warp's j = c, c + 2, ...
+      const int k = kb + lane;
+      const uint4* pairs = J->pairs + k;
+      const int64_t tri = J->tri;
+      auto load_jk = [&](int jj, uint4& a, uint4& b) {
+        a = b = make_uint4(0, 0, 0, 0);
+        if (jj < nj && jp + jj < m && k < m && k > jp + jj) {
+          const uint2 o = *reinterpret_cast<const uint2*>(marg + kMargWords * jj + 24);
+          const uint4* q = pairs + (int64_t)(((uint64_t)o.y << 32) | o.x);
+          a = __ldg(q);
+          b = __ldg(q + tri);
+        }
+      };
+      Screen scr;
+      scr.theta1 = J->theta1;
+      scr.theta2 = J->theta2;
+      const float coef = J->c, base = J->base;
+      uint4 jk0, jk1;
+      load_jk(c, jk0, jk1);
+      if (kb < m) {
+#pragma unroll 1
+        for (int jj = c; jj < nj; jj += 2) {
+          const int j = jp + jj;
+          if (j >= m || kb + 31 <= j) break;  // no valid lane from here on
+          const bool valid = k < m && k > j;
+          const uint4 e0 = lds128(Ek + (uint32_t)(jj * 64 * 16));
+          const uint4 e1 = lds128(Ek + (uint32_t)((kSplitJ + jj) * 64 * 16));
+          bool want = valid;
+          if (kDump) {
+            load_jk(jj + 2, jk0, jk1);
+          } else {
+            const uint32_t w00 = prmt(jk0.x, jk1.x, 0x5410u), w01 = prmt(jk0.y, jk1.y, 0x5410u);
+            const uint32_t w10 = prmt(jk0.z, jk1.z, 0x5410u), w11 = prmt(jk0.w, jk1.w, 0x5410u);
+            load_jk(jj + 2, jk0, jk1);
+            const int4* mj = reinterpret_cast<const int4*>(marg + kMargWords * jj);
+            auto margins = [&](int b, Form& ijA, Form& ijB, Form& nj_b) {
+              const int4 x = mj[2 * b];
+              const int2 y = *reinterpret_cast<const int2*>(mj + 2 * b + 1);
+              ijA = Form{x.x, x.y};
+              ijB = Form{x.z, x.w};
+              nj_b = Form{y.x, y.y};
+            };
+            scr.acc = 0.0f;
+            scr.bits = 0u;
+            Form ijA, ijB, nj_b, r0[9], r1[9], r2[9];
+            const Form q00 = form(w00, 3), q01 = form(w01, 3), q10 = form(w10, 3), q11 = form(w11, 3);
+            margins(0, ijA, ijB, nj_b);
+            r0[0] = form(e0.x, 1);
+            r0[1] = form(e1.x, 1);
+            r0[3] = form(e0.z, 1);
+            r0[4] = form(e1.z, 1);
+            row_forms(ijA, ijB, nj_b, q00, q01, r0);
+            scr.cells(r0);
+            margins(1, ijA, ijB, nj_b);
+            r1[0] = form(e0.y, 1);
+            r1[1] = form(e1.y, 1);
+            r1[3] = form(e0.w, 1);
+            r1[4] = form(e1.w, 1);
+            row_forms(ijA, ijB, nj_b, q10, q11, r1);
+            scr.cells(r1);
+            margins(2, ijA, ijB, nj_b);
+            r2[0] = kA0 - r0[0] - r1[0];
+            r2[1] = kA1 - r0[1] - r1[1];
+            r2[3] = kB0 - r0[3] - r1[3];
+            r2[4] = kB1 - r0[4] - r1[4];
+            row_forms(ijA, ijB, nj_b, nk0 - q00 - q10, nk1 - q01 - q11, r2);
+            scr.cells(r2);
+            // sum of logs: bits - 27 * 127 * 2^23 (modulo 2^32) in units of 2^-23 / log2 e * 2
+            const float lg = __uint2float_rn(scr.bits - 27u * 0x3F800000u);
+            const float low = fmaf(4.1315582e-8f, lg, -coef * scr.acc);
+            float reach = __uint_as_float(thr);
+            if (kTopK) reach = fminf(reach, __shfl_sync(kFull, list_s, 31));
+            want = valid && !(low >= reach - base);  // not a number: take the exact path
+          }
+          if (!__any_sync(kFull, want)) continue;
+          float sc = FLT_MAX;
+          unsigned long long key = ~0ull;
+          if (want) {
+            uint32_t table[kDump ? 54 : 1];
+            sc = exact_score(e0, e1, J, R->i, j, k, R->genos, kDump ? table : nullptr);
+            const int i1 = R->i;
+            key = pack_key((uint64_t)i1, (uint64_t)j, (uint64_t)k);
+            if (kDump) {
+              const int64_t ti = triplet_index(m, i1, j, k);
+#pragma unroll
+              for (int x = 0; x < 54; x++) p.dump_tables[ti * 54 + x] = table[kDump ? x : 0];
+              p.dump_scores[ti] = sc;
+            }
+            if (better(sc, key, best_s, best_k)) {
+              best_s = sc;
+              best_k = key;
+            }
+          }
+          unsigned reach = __float_as_uint(sc);  // FLT_MAX where not wanted
+          if (kTopK) {
+            const float ts = __shfl_sync(kFull, list_s, 31);
+            const unsigned long long tk = __shfl_sync(kFull, list_k, 31);
+            unsigned todo = __ballot_sync(kFull, want && better(sc, key, ts, tk));
+            while (todo) {
+              const int src = __ffs(todo) - 1;
+              todo &= todo - 1;
+              const float cs = __shfl_sync(kFull, sc, src);
+              const unsigned long long ck = __shfl_sync(kFull, key, src);
+              const float ts2 = __shfl_sync(kFull, list_s, 31);
+              const unsigned long long tk2 = __shfl_sync(kFull, list_k, 31);
+              if (better(cs, ck, ts2, tk2)) warp_list_insert(list_s, list_k, cs, ck, lane);
+            }
+            // 32 triplets reach this warp's last entry: no triplet above it is among the best 32
+            reach = __float_as_uint(__shfl_sync(kFull, list_s, 31));
+          }
+          reach = __reduce_min_sync(kFull, reach);
+          if (reach < thr) {
+            if (lane == 0) thr = min(reach, atomicMin(p.thr + cur_job, reach));
+            thr = __shfl_sync(kFull, thr, 0);
+          }
+        }
+      }
+      __syncwarp();
+      if (lane == 0) bar_arrive(bar(kCRel + (int)(t % kSplitSlots)));  // done with tile t's slot
+      got = bar_wait(bar(kCDesc + (int)((t + 1) % kSplitSlots)), ((t + 1) / kSplitSlots) & 1u, wl);
+      desc = got ? *slot_desc(t + 1) : -1;
+    }
+    if (cur_job >= 0) flush_job(cur_job);
+    if (kTopK) {
+      BestSlot& e = p.cand[((int64_t)blockIdx.x * kSScore + sw) * 32 + lane];
+      e.score = list_s;
+      e.key = list_k;
+    }
+  }
+
+  // ---- teardown: every role has left its loop; tensor memory is released only after every
+  // product has completed (bounded wait on one more commit)
+  if (warp == kSProd && lane == 0) {
+    if (even) mma_commit_pair(bar(kCFinal));
+    if (!bar_wait(bar(kCFinal), 0, wl)) s_abort = 1;
+  }
+  tc_fence_before();
+  __syncthreads();
+  if (s_abort && tid == 0) atomicExch(p.err, 1);
+  cluster_sync_all();
+  if (warp == 0) {
+    tc_fence_after();
+    asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512u) : "memory");
+  }
+}
+
+int split_score_warps() { return kSScore; }
+
+template <bool kD, bool kT>
+static cudaError_t split_set_smem() {
+  return cudaFuncSetAttribute(k_scan_split<kD, kT>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSSmemBytes);
+}
+
+cudaError_t split_configure() {
+  static bool configured = false;
+  if (configured) return cudaSuccess;
+  cudaError_t e = split_set_smem<false, false>();
+  if (e == cudaSuccess) e = split_set_smem<true, false>();
+  if (e == cudaSuccess) e = split_set_smem<false, true>();
+  if (e == cudaSuccess) configured = true;
+  return e;
+}
+
+cudaError_t launch_split_rows(const SplitJob& j, uint2* rows, cudaStream_t stream) {
+  const int64_t words = (int64_t)j.w0 + j.w1, units = words * (j.mwp / 4);
+  if (units == 0) return cudaSuccess;
+  k_split_rows<<<(unsigned)((units + 7) / 8), 256, 0, stream>>>(j.planes, rows, j.m_pad, j.mwp, words);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_split_prepare(const SplitJob* jobs, SplitRec* recs, int n, int max_quads, int max_cols,
+                                 int32_t* lists, uint4* cp, cudaStream_t stream) {
+  if (n <= 0) return cudaSuccess;
+  k_split_lists<<<(unsigned)n, kListThreads, 0, stream>>>(jobs, recs, lists);
+  cudaError_t e = cudaGetLastError();
+  if (e != cudaSuccess) return e;
+  const int64_t units = (int64_t)max_quads * ((max_cols + 3) / 4);
+  for (int at = 0; at < n; at += 65535) {
+    const int c = n - at < 65535 ? n - at : 65535;
+    k_split_planes<<<dim3((unsigned)((units + 7) / 8), (unsigned)c), 256, 0, stream>>>(jobs, recs + at, lists, cp);
+    e = cudaGetLastError();
+    if (e != cudaSuccess) return e;
+  }
+  return cudaSuccess;
+}
+
+cudaError_t launch_split_tiles(const SplitJob* jobs, const SplitRec* recs, const SplitRun* runs, int n_runs,
+                               int max_blocks, uint64_t* tiles, unsigned* cursor, cudaStream_t stream) {
+  if (n_runs <= 0 || max_blocks <= 0) return cudaSuccess;
+  for (int at = 0; at < n_runs; at += 65535) {
+    const int c = n_runs - at < 65535 ? n_runs - at : 65535;
+    k_split_tiles<<<dim3((unsigned)max_blocks, (unsigned)c), 128, 0, stream>>>(jobs, recs, runs + at, tiles, cursor);
+    const cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess) return e;
+  }
+  return cudaSuccess;
+}
+
+template <bool kD, bool kT>
+static cudaError_t launch_split(const SplitParams& p, int blocks, cudaStream_t stream) {
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3((unsigned)blocks);
+  cfg.blockDim = dim3(kSThreads);
+  cfg.dynamicSmemBytes = kSSmemBytes;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = 2;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, k_scan_split<kD, kT>, p);
+}
+
+cudaError_t launch_scan_split(const SplitParams& p, int blocks, bool dump, cudaStream_t stream) {
+  const cudaError_t ce = split_configure();
+  if (ce != cudaSuccess) return ce;
+  const cudaError_t e = dump ? launch_split<true, false>(p, blocks & ~1, stream)
+                        : p.top_k > 1 ? launch_split<false, true>(p, blocks & ~1, stream)
+                                      : launch_split<false, false>(p, blocks & ~1, stream);
+  return e != cudaSuccess ? e : cudaGetLastError();
+}
+
+}  // namespace epik2
