@@ -159,7 +159,7 @@ struct ScreenConsts {
 // One dataset of a split search.
 struct SplitJob {
   const uint2* planes;
-  const uint2* rows;       // [32*(w0+w1)][mwp] {g0, g1} bits of 32 SNPs per entry, class-sorted samples
+  uint2* rows;             // [32*(w0+w1)][mwp] {g0, g1} bits of 32 SNPs per entry, class-sorted samples
   const uint32_t* singles;
   const uint4* pairs;
   const float* lut;
@@ -226,8 +226,9 @@ cudaError_t launch_pairs_tc(const TcParams& p, int blocks, cudaStream_t stream);
 cudaError_t launch_scan_reps(const TcParams& p, int blocks, cudaStream_t stream);
 int split_score_warps();  // scoring warps per CTA of the split search
 cudaError_t split_configure();
-// rows (sample-major bits) of one job from its planes
-cudaError_t launch_split_rows(const SplitJob& j, uint2* rows, cudaStream_t stream);
+// rows (sample-major bits) of every job (at most 65535) from its planes; max_units: the most class
+// words x four 32-SNP columns of a job
+cudaError_t launch_split_rows(const SplitJob* jobs, int n_jobs, int64_t max_units, cudaStream_t stream);
 // sample lists and group ends of records [0, n); then their compacted planes (at most max_quads
 // quads and max_cols 32-SNP columns each)
 cudaError_t launch_split_prepare(const SplitJob* jobs, SplitRec* recs, int n, int max_quads, int max_cols,

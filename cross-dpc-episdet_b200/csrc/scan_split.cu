@@ -61,10 +61,14 @@ __device__ __forceinline__ uint32_t transpose32(uint32_t x, int lane) {
   return x;
 }
 
-// rows[32w + b][q] from planes[w][32q ..]: one warp per class word and four 32-SNP columns.
-__global__ void __launch_bounds__(256) k_split_rows(const uint2* __restrict__ planes, uint2* __restrict__ rows,
-                                                    int64_t m_pad, int mwp, int64_t words) {
-  const int lane = threadIdx.x & 31;
+// rows[32w + b][q] from planes[w][32q ..] of job blockIdx.y: one warp per class word and four
+// 32-SNP columns.
+__global__ void __launch_bounds__(256) k_split_rows(const SplitJob* __restrict__ jobs) {
+  const SplitJob& J = jobs[blockIdx.y];
+  const uint2* __restrict__ planes = J.planes;
+  uint2* __restrict__ rows = J.rows;
+  const int64_t m_pad = J.m_pad, words = (int64_t)J.w0 + J.w1;
+  const int lane = threadIdx.x & 31, mwp = J.mwp;
   const int nq = mwp / 4;
   const int64_t unit = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5);
   const int64_t w = unit / nq;
@@ -1037,10 +1041,9 @@ cudaError_t split_configure() {
   return e;
 }
 
-cudaError_t launch_split_rows(const SplitJob& j, uint2* rows, cudaStream_t stream) {
-  const int64_t words = (int64_t)j.w0 + j.w1, units = words * (j.mwp / 4);
-  if (units == 0) return cudaSuccess;
-  k_split_rows<<<(unsigned)((units + 7) / 8), 256, 0, stream>>>(j.planes, rows, j.m_pad, j.mwp, words);
+cudaError_t launch_split_rows(const SplitJob* jobs, int n_jobs, int64_t max_units, cudaStream_t stream) {
+  if (n_jobs <= 0 || max_units <= 0) return cudaSuccess;
+  k_split_rows<<<dim3((unsigned)((max_units + 7) / 8), (unsigned)n_jobs), 256, 0, stream>>>(jobs);
   return cudaGetLastError();
 }
 

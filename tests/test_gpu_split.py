@@ -120,3 +120,37 @@ def test_ranges_and_topk_agree_with_the_integer_engine(auto):
         assert e.value.status == epik2.E_INVALID
     finally:
         auto.unload(did)
+
+
+def test_batch_and_replicates_equal_separate_searches(auto):
+    """Datasets of many shapes, and phenotypes of very different class sizes, in one search each."""
+    data = [O.gen_hwe(40 + t, S, M, c) for t, (S, M, c) in enumerate(
+        [(300, 20, 140), (64, 3, 32), (2047, 70, 1500), (500, 131, 250), (40, 12, 0), (3001, 33, 3000), (129, 187, 64)])]
+    ids = [auto.load(g, p) for g, p in data]
+    try:
+        for rescore in (0, 1):
+            got = auto.scan_batch(ids, rescore_fp64=rescore)
+            for (g, p), b in zip(data, got):
+                r = O.scan(g, p)
+                assert b.ijk == r["ijk"] and f32_bits(b.score) == f32_bits(r["score"])
+                if rescore:
+                    assert b.score_fp64 == O.k2_fp64(O.scan(g, p, with_tables=True)["tables"][_index(g.shape[1], *b.ijk)])
+    finally:
+        for d in ids:
+            auto.unload(d)
+    g, p = O.gen_hwe(90, 900, 66, 400)
+    rng = np.random.default_rng(3)
+    reps = np.stack([rng.permutation(p), np.zeros_like(p), np.ones_like(p), (rng.random(900) < 0.03).astype(np.uint8)])
+    did = auto.load(g, p)
+    try:
+        for q, b in zip(reps, auto.scan_replicates(did, reps)):
+            r = O.scan(g, q)
+            assert b.ijk == r["ijk"] and f32_bits(b.score) == f32_bits(r["score"])
+    finally:
+        auto.unload(did)
+
+
+def _index(m, i, j, k):
+    before_i = sum((m - 1 - a) * (m - 2 - a) // 2 for a in range(i))
+    before_j = sum(m - 1 - b for b in range(i + 1, j))
+    return before_i + before_j + k - j - 1
