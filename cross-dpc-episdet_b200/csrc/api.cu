@@ -92,8 +92,8 @@ struct epik2_ctx {
   BestSlot* d_rep_res = nullptr;
   Rescored* d_rep_resc = nullptr;
   int64_t rep_cap = 0, rep_slot_cap = 0;
-  // split search workspace (grown, bounded by kSplitChunkBytes plus the searched datasets' own
-  // bits; given back when another allocation needs the room and with the context)
+  // split search workspace (kept while it is at most kSplitKeepBytes; given back when another
+  // allocation needs the room and with the context)
   GrowBuf sp_rows, sp_lists, sp_cp, sp_tiles, sp_small, sp_slots;
   unsigned char* h_small = nullptr;  // pinned image of the uploaded part of sp_small, and results
   size_t h_small_cap = 0;
@@ -750,6 +750,8 @@ bool split_fits(const DevDataset& d) { return d.n_snps >= 3 && d.n_controls <= 6
 // Compacted planes of the first SNPs searched per launch: launches of the large workload then
 // last 6 ms or more, and their ends (one tile, about 10 us) stay below 0.3 %.
 constexpr size_t kSplitChunkBytes = (size_t)768 << 20;
+// A larger workspace of a part is released after the search that needed it.
+constexpr size_t kSplitKeepBytes = (size_t)1 << 30;
 // Planes of the first SNPs whose tiles are interleaved in the queue: what may stay in L2 (126 MB)
 // beside the margins.
 constexpr size_t kSplitRunBytes = (size_t)40 << 20;
@@ -770,7 +772,7 @@ int run_split(epik2_ctx* ctx, const std::vector<DevDataset*>& ds, int64_t ib, in
   std::vector<Chunk> chunks;
   size_t rows_bytes = 0, cp_max = 0, lists_max = 0, tiles_max = 0;
   size_t cp = 0, lists = 0, tiles = 0;  // of the current chunk: bytes, bytes, descriptors
-  int64_t trip = 0, rows_units = 0;
+  int64_t trip = 0, rows_units = 0, max_tri = 0;
   // datasets with the most samples first: their tiles last longest, the short ones fill the end
   std::vector<int> order((size_t)n_jobs);
   for (int b = 0; b < n_jobs; b++) order[(size_t)b] = b;
@@ -801,6 +803,9 @@ int run_split(epik2_ctx* ctx, const std::vector<DevDataset*>& ds, int64_t ib, in
     J.rows = reinterpret_cast<uint2*>(rows_bytes);  // offset, made an address below
     rows_units = std::max(rows_units, (d.w0 + d.w1) * (J.mwp / 4));
     rows_bytes += align_up((size_t)(32 * (d.w0 + d.w1)) * J.mwp * 8, 256);
+    J.pairs16 = reinterpret_cast<uint4*>(rows_bytes);
+    rows_bytes += align_up((size_t)d.tri * 16, 256);
+    max_tri = std::max(max_tri, d.tri);
     const int64_t m = d.n_snps;
     const int max_quads = (int)(2 * d.n_samples / 3 / 128) + 5;  // the dropped genotype is the most frequent
     const int64_t i0 = std::max<int64_t>(ib, 0), i1 = std::min<int64_t>(ie, m - 2);
@@ -858,7 +863,7 @@ int run_split(epik2_ctx* ctx, const std::vector<DevDataset*>& ds, int64_t ib, in
     if (e == cudaSuccess) e = ctx->sp_slots.need(sizeof(BestSlot) * (size_t)n_jobs * per_job);
     if (e == cudaSuccess) e = ctx->sp_rows.need(std::max<size_t>(rows_bytes, 256));
     if (e == cudaSuccess) e = ctx->sp_lists.need(std::max<size_t>(lists_max, 256));
-    if (e == cudaSuccess) e = ctx->sp_cp.need(std::max<size_t>(cp_max, 256));
+    if (e == cudaSuccess) e = ctx->sp_cp.need(cp_max + 8192);  // tiles past the last SNP read up to 128 columns on
     if (e == cudaSuccess) e = ctx->sp_tiles.need(8 * std::max<size_t>(tiles_max, 32));
     return e;
   };
@@ -883,8 +888,10 @@ int run_split(epik2_ctx* ctx, const std::vector<DevDataset*>& ds, int64_t ib, in
     ctx->h_small_cap = 2 * h_need;
   }
   unsigned char* const dev = static_cast<unsigned char*>(ctx->sp_small.p);
-  for (SplitJob& J : jobs)
+  for (SplitJob& J : jobs) {
     J.rows = reinterpret_cast<uint2*>(static_cast<char*>(ctx->sp_rows.p) + reinterpret_cast<size_t>(J.rows));
+    J.pairs16 = reinterpret_cast<uint4*>(static_cast<char*>(ctx->sp_rows.p) + reinterpret_cast<size_t>(J.pairs16));
+  }
   memcpy(ctx->h_small, jobs.data(), sizeof(SplitJob) * jobs.size());
   if (!recs.empty()) memcpy(ctx->h_small + o_recs, recs.data(), sizeof(SplitRec) * recs.size());
   if (!runs.empty()) memcpy(ctx->h_small + o_runs, runs.data(), sizeof(SplitRun) * runs.size());
@@ -910,12 +917,13 @@ int run_split(epik2_ctx* ctx, const std::vector<DevDataset*>& ds, int64_t ib, in
   CK(ctx, cudaMemsetAsync(d_cur, 0, cur_bytes, ctx->stream), "reset counters");
   CK(ctx, cudaMemsetAsync(d_thr, 0x7F, thr_bytes, ctx->stream), "reset thresholds");  // 3.4e38 as FP32
   CK(ctx, launch_fill_slots(d_slots, (int64_t)n_jobs * per_job, ctx->stream), "reset slots");
-  ctx->stats.kernel_launches += 2;
+  ctx->stats.kernel_launches += 4;
   if (top_k > 1) {
     CK(ctx, launch_fill_slots(ctx->d_cand, (int64_t)grid * split_score_warps() * 32, ctx->stream), "reset candidates");
     ctx->stats.kernel_launches += 1;
   }
   CK(ctx, launch_split_rows(d_jobs, n_jobs, rows_units, ctx->stream), "sample rows");
+  CK(ctx, launch_split_pairs(d_jobs, n_jobs, max_tri, ctx->stream), "packed margins");
   for (size_t x = 0; x < chunks.size(); x++) {
     const Chunk& c = chunks[x];
     CK(ctx, launch_split_prepare(d_jobs, d_recs + c.rec0, c.n_recs, c.max_quads, c.max_cols,
@@ -958,7 +966,10 @@ int run_split(epik2_ctx* ctx, const std::vector<DevDataset*>& ds, int64_t ib, in
      "read results");
   CK(ctx, cudaMemcpyAsync(h_err, d_err, 4, cudaMemcpyDeviceToHost, ctx->stream), "read error word");
   ctx->stats.d2h_bytes += sizeof(BestSlot) * (size_t)n_jobs + 4;
-  CK(ctx, cudaStreamSynchronize(ctx->stream), "search");
+  const cudaError_t done = cudaStreamSynchronize(ctx->stream);
+  for (GrowBuf* b : {&ctx->sp_rows, &ctx->sp_lists, &ctx->sp_tiles})
+    if (b->cap > kSplitKeepBytes) b->drop();
+  CK(ctx, done, "search");
   if (*h_err) return fail(ctx, EPIK2_E_TIMEOUT, "tensor-core scan: a bounded wait expired");
   float kms = 0.0f;
   CK(ctx, cudaEventElapsedTime(&kms, ctx->ev_start, ctx->ev_stop), "event time");

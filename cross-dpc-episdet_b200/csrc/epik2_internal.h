@@ -150,10 +150,10 @@ constexpr int kSplitSlots = 3; // tiles in flight per CTA pair: scored, in tenso
 
 // Constants of the screening bound for a class split (screen_constants).
 struct ScreenConsts {
-  uint32_t coef;           // bytes (128 - kp, -kp): 128 D = (128 - kp) a - kp b + bias
-  int32_t bias;            // 64 - kp
-  float theta1, theta2;    // of 128 D
-  float c;                 // of (128 D)^2 / den
+  uint32_t coef;           // bytes (64 - kp, -kp): 64 D = (64 - kp) a - kp b + bias
+  int32_t bias;            // 32 - kp
+  float theta1, theta2;    // of 64 D
+  float c;                 // of (64 D)^2 / den
   float base;
 };
 // One dataset of a split search.
@@ -162,13 +162,14 @@ struct SplitJob {
   uint2* rows;             // [32*(w0+w1)][mwp] {g0, g1} bits of 32 SNPs per entry, class-sorted samples
   const uint32_t* singles;
   const uint4* pairs;
+  uint4* pairs16;          // `pairs` with both classes' counts in one word
   const float* lut;
   int64_t tri;
   int32_t m, m_pad, mwp, w0, w1, n0, n1;
   uint32_t coef;           // ScreenConsts
   int32_t bias;
   float theta1, theta2, c, base;
-  int32_t pad[7];
+  int32_t pad[5];
 };
 static_assert(sizeof(SplitJob) == 128, "copied as 32 words per tile");
 
@@ -229,6 +230,8 @@ cudaError_t split_configure();
 // rows (sample-major bits) of every job (at most 65535) from its planes; max_units: the most class
 // words x four 32-SNP columns of a job
 cudaError_t launch_split_rows(const SplitJob* jobs, int n_jobs, int64_t max_units, cudaStream_t stream);
+// packed pair margins of every job; max_tri: the most pairs of a job
+cudaError_t launch_split_pairs(const SplitJob* jobs, int n_jobs, int64_t max_tri, cudaStream_t stream);
 // sample lists and group ends of records [0, n); then their compacted planes (at most max_quads
 // quads and max_cols 32-SNP columns each)
 cudaError_t launch_split_prepare(const SplitJob* jobs, SplitRec* recs, int n, int max_quads, int max_cols,

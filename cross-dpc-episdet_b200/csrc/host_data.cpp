@@ -50,24 +50,24 @@ void build_k2_lut(int64_t n_max, float* lut) { build_k2_lut_range(0, n_max + 1, 
 //   -ln(1 - t1 d)/2  >=  -|t1 d|/2  >=  -K/N - N d^2 t1^2 / (16 K)
 // takes up K/N, so that per cell   ln(P)/2 - (c2 + t1^2 / (16 K)) D^2 / (P - t2 |D|)   remains; log2
 // P is taken from P's FP32 bits (linear between powers of two, never above).  Summed over the 27
-// cells this bounds the K2 score from below, for any p: kp/128 next to the share of controls, which
-// makes 128 D an integer.  base = the terms that are the same for every triplet, less a margin for
+// cells this bounds the K2 score from below, for any p: kp/64 next to the share of controls, which
+// makes 64 D an integer.  base = the terms that are the same for every triplet, less a margin for
 // rounding: of the reference's FP32 table and sums (about 5 ulp of ln n!, 0.1 for the table below
 // 748) and of the FP32 evaluation of the bound.
 ScreenConsts screen_constants(int64_t n0, int64_t n1) {
   const double n = (double)(n0 + n1), kK = 0.22;
-  const int kp = (int)std::min(127.0, std::max(1.0, std::floor(128.0 * ((double)n0 + 13.5) / (n + 27.0) + 0.5)));
-  const double p = kp / 128.0, q = 1.0 - p;
+  const int kp = (int)std::min(63.0, std::max(1.0, std::floor(64.0 * ((double)n0 + 13.5) / (n + 27.0) + 0.5)));
+  const double p = kp / 64.0, q = 1.0 - p;
   const double c2 = 1.0 / (2.0 * p * q);
   const double up = (1.0 + c2 * q * q / std::log(p)) / q;    // 1 - up d meets c2 d^2 / KL at d = q
   const double down = (1.0 + c2 * p * p / std::log(q)) / p;  // 1 - down |d| at d = -p
   const double t1 = (up - down) / 2.0, t2 = (up + down) / 2.0;
   ScreenConsts s{};
-  s.coef = (uint32_t)(uint8_t)(128 - kp) | ((uint32_t)(uint8_t)(-kp) << 8);
-  s.bias = 64 - kp;
-  s.theta1 = (float)(t1 / 128.0);
-  s.theta2 = (float)(t2 * 1.000001 / 128.0);
-  s.c = (float)((c2 + t1 * t1 / (16.0 * kK)) * 1.000001 / (128.0 * 128.0));
+  s.coef = (uint32_t)(uint8_t)(64 - kp) | ((uint32_t)(uint8_t)(-kp) << 8);
+  s.bias = 32 - kp;
+  s.theta1 = (float)(t1 / 64.0);
+  s.theta2 = (float)(t2 * 1.000001 / 64.0);
+  s.c = (float)((c2 + t1 * t1 / (16.0 * kK)) * 1.000001 / (64.0 * 64.0));
   const double margin = 0.3 + 1e-6 * std::lgamma(n + 2.0);
   s.base = (float)(-((double)n0 + 13.5) * std::log(p) - ((double)n1 + 13.5) * std::log(q) -
                    13.5 * std::log(2.0 * 3.14159265358979323846) - margin);

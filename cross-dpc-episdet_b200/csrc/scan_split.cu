@@ -23,21 +23,23 @@
 // Warp roles of a CTA (512 threads), concurrent from tile to tile:
 //   warps 0-5   produce: expand the compacted bit planes into the operand ring (warps 0-3 the 64
 //               SNPs k of this CTA, 4-5 its 28 SNPs j), 256 samples per stage, 4 stages
-//   warp 6      issues the products (even CTA)
+//   warp 6      fences the stored stages and issues the products (even CTA)
 //   warp 7      schedules: takes tiles from the queue, publishes descriptor, record and job
 //   warps 8-15  score: copy a tile's four accumulators out of tensor memory into a 16-bit staging
 //               buffer (class 0 in the low, class 1 in the high half of a word), which frees them
 //               for the next tile, then complete, screen and select while that tile counts
 // Classes of at most 65535 samples (the 16-bit halves).
 //
-// What bounds it: the issue slots of the scoring warps (about 320 instructions per 32 triplets)
-// and, from about 8192 samples on, the round trip of a ring stage (stores, arrival in the even CTA,
-// products, commit).  Cost of the parts of that round trip, which set the roles and hand-offs above
+// What bounds it: the scoring warps (about 350 instructions per 32 triplets) up to about 8192
+// samples; from there on also the round trip of a ring stage (stores, fence and arrival in the even
+// CTA, products, commit).  Cost of the parts of that round trip, which set the roles and hand-offs
 // (clocks, measured alone): a commit of four products 560; an arrival in the other CTA 133, and
 // 447 with a cluster-scope release; issuing four products and their commit 330 from a converged
-// warp, 610 from a lane-0 branch.
-// Measured against k_scan_tc on CTA pairs (kernel time of a whole search): 1024 x 8192 14.1 -> 5.1
-// ms, 3072 x 4096 265 -> 102 ms, 2048 x 8192 103 -> 34.5 ms, an eighth of 4096 x 16384 144 -> 45 ms.
+// warp, 610 from a lane-0 branch.  An eighth of 4096 x 16384 took 45.3 ms with the words of the next
+// four stages in registers and each producing warp fencing its stores (the fence waits for loads in
+// flight), 42.5 with the fence in the issuing warp, 38.8 with cp.async.
+// Measured against k_scan_tc on CTA pairs (kernel time of a whole search): 1024 x 8192 14.1 -> 4.6
+// ms, 3072 x 4096 265 -> 91 ms, 2048 x 8192 103 -> 31.2 ms, an eighth of 4096 x 16384 144 -> 38.8 ms.
 //
 // Every mbarrier wait is bounded; on expiry the kernel sets an error word and ends.
 #include <cfloat>
@@ -88,6 +90,18 @@ __global__ void __launch_bounds__(256) k_split_rows(const SplitJob* __restrict__
   uint4* dst = reinterpret_cast<uint4*>(rows + (32 * w + lane) * (int64_t)mwp + q);
   dst[0] = make_uint4(v[0].x, v[0].y, v[1].x, v[1].y);
   dst[1] = make_uint4(v[2].x, v[2].y, v[3].x, v[3].y);
+}
+
+// Pair margins packed: class 0 in the low, class 1 in the high half of each count (16 bytes per
+// pair instead of 32: one load and no packing per triplet, half the traffic).  Bound by memory.
+__global__ void __launch_bounds__(256) k_split_pairs(const SplitJob* __restrict__ jobs) {
+  const SplitJob& J = jobs[blockIdx.y];
+  const uint4* __restrict__ src = J.pairs;
+  uint4* __restrict__ dst = J.pairs16;
+  for (int64_t x = (int64_t)blockIdx.x * 256 + threadIdx.x; x < J.tri; x += (int64_t)gridDim.x * 256) {
+    const uint4 a = __ldg(src + x), b = __ldg(src + J.tri + x);
+    dst[x] = make_uint4(a.x | (b.x << 16), a.y | (b.y << 16), a.z | (b.z << 16), a.w | (b.w << 16));
+  }
 }
 
 // Sample lists of one record per block: the row numbers of each group's samples, -1 up to the
@@ -258,6 +272,7 @@ constexpr int kSPairJ = 28;          // SNPs j scored by a pair (x 32 SNPs k)
 constexpr int kSFirstScore = kSProd + 2;
 constexpr int kSThreads = 32 * (kSFirstScore + kSScore);
 constexpr int kSStages = 4;
+constexpr int kSRaw = 2;             // raw slots of a producing warp
 constexpr int kSRowBytes = 128;      // 8 words of 32 samples, E2M1
 constexpr uint32_t kSSbo = 8 * kSRowBytes;
 constexpr int kSHalfJ = kSplitJ / 2; // SNPs j expanded by each CTA
@@ -267,9 +282,10 @@ constexpr int kSStagingOff = kSStages * kSStageBytes;  // E[c][j][k]: uint4 word
 constexpr int kSStagingBytes = 2 * kSplitJ * 64 * 16;
 // Per pair of scoring warps: the margins of its SNPs j.
 constexpr int kSPairOff = kSStagingOff + kSStagingBytes;
-constexpr int kMargWords = 28;       // per g_j: forms of (A, g_j), (B, g_j), g_j, 2 unused; offset of row j of the pair table
+constexpr int kMargWords = 20;       // forms of (A, g_j), (B, g_j) for each g_j, then of each g_j; offset of row j of the pair table
 constexpr int kSPairBytes = kSPairJ * kMargWords * 4;
-constexpr int kSSlotOff = kSPairOff + kSPairs * kSPairBytes;
+constexpr int kSRawOff = kSPairOff + kSPairs * kSPairBytes;  // raw words: per producing warp kSRaw slots of 1 KiB
+constexpr int kSSlotOff = kSRawOff + kSProd * kSRaw * 1024;
 constexpr int kSSlotBytes = 64 + 128 + 16;        // record, job, descriptor
 constexpr int kSBarOff = kSSlotOff + kSplitSlots * kSSlotBytes;
 constexpr int kSSmemBytes = kSBarOff + 256;
@@ -297,9 +313,10 @@ __device__ __forceinline__ void split_mma(uint32_t d_tmem, uint64_t a, uint64_t 
           d_tmem),
       "l"(a), "l"(b), "r"(kSIdesc), "r"(accumulate), "r"(sfa), "r"(sfb));
 }
-// Arrival on a barrier of the other CTA.  The stores it announces are to this CTA's own shared
-// memory and for its own tensor core (fence.proxy.async before), so no cluster-scope release: that
-// one waits for earlier accesses of the thread and costs several hundred clocks per stage.
+// Arrival on a barrier of the other CTA.  What it announces are stores to this CTA's own shared
+// memory for its own tensor core (fence.proxy.async before) or completed reads of its own tensor
+// memory, so no cluster-scope release: that one waits for earlier accesses of the thread and costs
+// several hundred clocks.
 __device__ __forceinline__ void bar_arrive_remote(uint32_t cluster_addr) {
   asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
 }
@@ -313,8 +330,16 @@ __device__ __forceinline__ void split_commit(uint32_t bar) {
       : "memory");
 }
 
-__device__ __forceinline__ void tmem_ld2(uint32_t addr, uint32_t (&r)[2]) {
-  asm volatile("tcgen05.ld.sync.aligned.32x32b.x2.b32 {%0, %1}, [%2];" : "=r"(r[0]), "=r"(r[1]) : "r"(addr));
+__device__ __forceinline__ void tmem_ld4(uint32_t addr, uint32_t (&r)[4]) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0, %1, %2, %3}, [%4];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+               : "r"(addr));
+}
+
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int kPending>
+__device__ __forceinline__ void cp_async_wait() {
+  asm volatile("cp.async.wait_group %0;" ::"n"(kPending) : "memory");
 }
 
 // 128 sample bits of one SNP and genotype -> four K groups of 32 E2M1 elements.  Group q holds bit q
@@ -350,25 +375,30 @@ __device__ __forceinline__ int dot2(uint32_t w, uint32_t coef, int c) {
   return r;
 }
 
-// The two linear forms of a cell (a controls, b cases) that the screening bound needs, as integers:
-// n = N = a + b + 1 and d = 128 D = 128 (a + 1/2) - kp N.  A margin over x cells holds the sums of
-// its cells' forms, so that cells complete by subtraction.
+// The two linear forms of a cell (a controls, b cases) that the screening bound needs, as the bits of
+// FP32 numbers: n = 2^23 + N with N = a + b + 1, and d = 1.5 * 2^23 + 64 D with 64 D = 64 (a + 1/2) -
+// kp N.  The integers 64 D stay below 2^22 for 16-bit counts, so adding and subtracting the bits adds
+// and subtracts the numbers, and one FP32 subtraction converts (an integer conversion takes twice
+// the pipe time).  A margin over x cells holds the sums of its cells' bits modulo 2^32, so that cells
+// complete by integer subtraction.
+constexpr uint32_t kBitsN = 0x4B000000u, kBitsD = 0x4B400000u;
 struct Form {
-  int n, d;
+  uint32_t n, d;
 };
 __device__ __forceinline__ Form operator-(Form x, Form y) { return Form{x.n - y.n, x.d - y.d}; }
 struct FormOf {  // counts (class 0 low half, class 1 high half) of a sum over `cells` cells -> forms
-  uint32_t coef;   // bytes (128 - kp, -kp)
-  int bias;        // 64 - kp
+  uint32_t coef;   // bytes (64 - kp, -kp)
+  int bias;        // 32 - kp
   __device__ __forceinline__ Form operator()(uint32_t w, int cells) const {
-    return Form{dot2(w, 0x0101u, cells), dot2(w, coef, bias * cells)};
+    return Form{(uint32_t)dot2(w, 0x0101u, (int)((kBitsN + 1u) * (uint32_t)cells)),
+                (uint32_t)dot2(w, coef, (int)((kBitsD + (uint32_t)bias) * (uint32_t)cells))};
   }
 };
 
-// Lower bound of K2 (screen_constants in host_data.cpp), cell by cell: per cell two conversions,
-// one reciprocal, four FP32 operations and half an integer addition.
+// Lower bound of K2 (screen_constants in host_data.cpp), cell by cell: per cell one reciprocal, six
+// FP32 operations and half an integer addition.
 struct Screen {
-  float theta1, theta2;  // of 128 D
+  float theta1, theta2;  // of 64 D
   float acc;
   uint32_t bits;         // sum of the cells' log2 (N - theta1 D), from below, in units of 2^-23
   template <int kN>
@@ -376,8 +406,8 @@ struct Screen {
     float D[kN], P[kN], r[kN];
 #pragma unroll
     for (int x = 0; x < kN; x++) {
-      D[x] = (float)f[x].d;
-      P[x] = fmaf(D[x], -theta1, (float)f[x].n);
+      D[x] = __uint_as_float(f[x].d) - 12582912.0f;
+      P[x] = fmaf(D[x], -theta1, __uint_as_float(f[x].n) - 8388608.0f);
     }
 #pragma unroll
     for (int x = 0; x < kN; x++) r[x] = rcp_approx(fmaf(fabsf(D[x]), -theta2, P[x]));
@@ -431,11 +461,10 @@ __device__ __forceinline__ void dropped_cells(uint4 jk, uint32_t nj0, uint32_t n
   t[8] = m22 - a[8] - b[8];
 }
 
-// Counts (g_i = g, g_x = 0 and 1) from a pair's counts and the singles of x.
-__device__ __forceinline__ void by_genotype(uint4 c0, uint4 c1, uint32_t n0, uint32_t n1, int g, uint32_t& x0, uint32_t& x1) {
-  const uint32_t a0 = c0.x | (c1.x << 16), a1 = c0.y | (c1.y << 16), b0 = c0.z | (c1.z << 16), b1 = c0.w | (c1.w << 16);
-  x0 = g == 0 ? a0 : g == 1 ? b0 : n0 - a0 - b0;
-  x1 = g == 0 ? a1 : g == 1 ? b1 : n1 - a1 - b1;
+// Counts (g_i = g, g_x = 0 and 1) from the packed counts c of the pair (i, x) and the singles of x.
+__device__ __forceinline__ void by_genotype(uint4 c, uint32_t n0, uint32_t n1, int g, uint32_t& x0, uint32_t& x1) {
+  x0 = g == 0 ? c.x : g == 1 ? c.z : n0 - c.x - c.z;
+  x1 = g == 0 ? c.y : g == 1 ? c.w : n1 - c.y - c.w;
 }
 
 // K2 of triplet (i, j, k) in the reference's arithmetic and order from its eight staged words per
@@ -457,18 +486,14 @@ __device__ __noinline__ float exact_score(uint4 e0, uint4 e1, const SplitJob* J,
   single(k, nk[0], nk[1]);
   ni[2] = all - ni[0] - ni[1];
   nj[2] = all - nj[0] - nj[1];
-  const uint4* pij = J->pairs + tri_offset(m_pad, i, j);
-  const uint4* pik = J->pairs + tri_offset(m_pad, i, k);
-  const uint4* pjk = J->pairs + tri_offset(m_pad, j, k);
-  const uint4 ij0 = __ldg(pij), ij1 = __ldg(pij + J->tri), ik0 = __ldg(pik), ik1 = __ldg(pik + J->tri);
-  const uint4 jk0 = __ldg(pjk), jk1 = __ldg(pjk + J->tri);
-  const uint4 jk = make_uint4(jk0.x | (jk1.x << 16), jk0.y | (jk1.y << 16), jk0.z | (jk1.z << 16), jk0.w | (jk1.w << 16));
+  const uint4 ij = __ldg(J->pairs16 + tri_offset(m_pad, i, j)), ik = __ldg(J->pairs16 + tri_offset(m_pad, i, k));
+  const uint4 jk = __ldg(J->pairs16 + tri_offset(m_pad, j, k));
   uint32_t t[3][9], x0, x1, y0, y1;
-  by_genotype(ij0, ij1, nj[0], nj[1], gA, x0, x1);
-  by_genotype(ik0, ik1, nk[0], nk[1], gA, y0, y1);
+  by_genotype(ij, nj[0], nj[1], gA, x0, x1);
+  by_genotype(ik, nk[0], nk[1], gA, y0, y1);
   counted_cells(e0.x, e1.x, e0.y, e1.y, x0, x1, (gA == 0 ? ni[0] : ni[1]) - x0 - x1, y0, y1, t[0]);
-  by_genotype(ij0, ij1, nj[0], nj[1], gB, x0, x1);
-  by_genotype(ik0, ik1, nk[0], nk[1], gB, y0, y1);
+  by_genotype(ij, nj[0], nj[1], gB, x0, x1);
+  by_genotype(ik, nk[0], nk[1], gB, y0, y1);
   counted_cells(e0.z, e1.z, e0.w, e1.w, x0, x1, (gB == 1 ? ni[1] : ni[2]) - x0 - x1, y0, y1, t[1]);
   dropped_cells(jk, nj[0], nj[1], nj[2], nk[0], nk[1], t[0], t[1], t[2]);
   const float* __restrict__ lut = J->lut;
@@ -509,11 +534,11 @@ __global__ void __launch_bounds__(kSThreads, 1) k_scan_split(const SplitParams p
 
   if (tid == 0) {
     for (int s = 0; s < kSStages; s++) {
-      bar_init(bar(kCFull + s), 2 * kSProd);  // both CTAs' producing warps arrive in the even one
+      bar_init(bar(kCFull + s), kSProd + (even ? 1 : 0));  // + the odd CTA's issuing warp
       bar_init(bar(kCEmpty + s), 1);
     }
     bar_init(bar(kCAcc), 1);
-    bar_init(bar(kCDrained), kSScore + (even ? 1 : 0));
+    bar_init(bar(kCDrained), 2 * kSScore);  // both CTAs' scoring warps arrive in the even one
     for (int s = 0; s < kSplitSlots; s++) {
       bar_init(bar(kCHand + s), 1);
       bar_init(bar(kCDesc + s), 1);
@@ -550,16 +575,19 @@ __global__ void __launch_bounds__(kSThreads, 1) k_scan_split(const SplitParams p
   if (warp < kSProd) {
     // ================= producing warps =================
     // A: rows 64c + kk of this CTA's 64 SNPs k; B: rows 28b + jj of its 28 SNPs j.  A warp takes
-    // one quad (4 words) of a stage for 32 SNPs: 32 bytes loaded, 8 x 16 bytes stored per lane.
+    // one quad (4 words) of a stage for 32 SNPs: 32 bytes loaded, 8 x 16 bytes stored per lane.  The
+    // words come by cp.async through the lane's own two raw slots, a stage ahead; the proxy fence
+    // that the stores need is left to the issuing warp, since a fence here would wait for them.
     const bool isA = warp < 4;
     const int sub = isA ? warp >> 1 : warp - 4;
     const int x = isA ? 32 * (warp & 1) + lane : lane;           // row of genotype 0
     const int row1 = x + (isA ? 64 : kSHalfJ);                   // row of genotype 1
-    const bool mine = isA || lane < kSHalfJ;
+    const bool on = isA || lane < kSHalfJ;
+    const uint32_t raw0 = sbase + kSRawOff + (uint32_t)(warp * kSRaw * 1024 + 16 * lane);
     const uint32_t off_base = (isA ? 0u : (uint32_t)kSStageA) + 512u * (uint32_t)sub;
     const uint32_t off0 = off_base + (uint32_t)(x >> 3) * kSSbo + (uint32_t)(x & 7) * 16;
     const uint32_t off1 = off_base + (uint32_t)(row1 >> 3) * kSSbo + (uint32_t)(row1 & 7) * 16;
-    uint32_t g = 0;
+    uint32_t slot = 0, phase = 1;  // of the ring; the first round finds every slot empty
     for (uint32_t t = 0;; t++) {
       const bool got = bar_wait(bar(kCDesc + (int)(t % kSplitSlots)), (t / kSplitSlots) & 1u, wl);
       if (__any_sync(kFull, !got)) {
@@ -573,59 +601,48 @@ __global__ void __launch_bounds__(kSThreads, 1) k_scan_split(const SplitParams p
       const int j0 = R->i + 1 + kSplitJ * (int)(((uint64_t)desc >> 24) & 0x3FFFF);
       const int k0 = j0 + 1 + kSplitK * (int)(((uint64_t)desc >> 42) & 0xFFFF);
       const int snp = (isA ? k0 + 64 * (int)crank : j0 + kSHalfJ * (int)crank) + x - 32 * R->qlo;
-      const bool on = mine && snp < mlen;
-      const uint4* src = p.cp + R->cp_off + 2 * ((int64_t)sub * mlen + (on ? snp : 0));
+      // (words past a row's end belong to no SNP that is scored; the buffer has room behind its last row)
+      const uint4* next = p.cp + R->cp_off + 2 * ((int64_t)snp + (int64_t)sub * mlen);
       const int64_t step = 4 * (int64_t)mlen;
-      // loads run four stages ahead of their use
-      uint4 va[4], vb[4];
-      auto load = [&](int st, uint4& a, uint4& b) {
-        if (on && 2 * st + sub < nq) {
-          const uint4* s = src + st * step;
-          a = __ldg(s);
-          b = __ldg(s + 1);
+      const int mine = (nq - sub + 1) / 2;  // stages with a quad for this warp
+      auto load = [&](int st) {  // this lane's words of stage st into the raw slot of the stage
+        if (st < mine) {
+          const uint32_t to = raw0 + 1024u * (uint32_t)(st & 1);
+          cp_async16(to, next);
+          cp_async16(to + 512u, next + 1);
+          next += step;
         }
+        cp_async_commit();
       };
-#pragma unroll
-      for (int u = 0; u < 4; u++) {
-        va[u] = vb[u] = make_uint4(0, 0, 0, 0);
-        load(u, va[u], vb[u]);
-      }
+      load(0);
       bool bad = false;
-      for (int st0 = 0; st0 < nst && !bad; st0 += 4) {
-#pragma unroll
-        for (int u = 0; u < 4; u++) {
-          const int st = st0 + u;
-          if (st < nst && !bad) {
-            const uint32_t gg = g + (uint32_t)st;
-            const int s = (int)(gg % kSStages);
-            const uint32_t use = gg / kSStages;
-            bad = __any_sync(kFull, use > 0 && !bar_wait(bar(kCEmpty + s), (use & 1u) ^ 1u, wl));
-            if (!bad) {
-              if (on && 2 * st + sub < nq) {
-                const uint32_t at = sbase + (uint32_t)(s * kSStageBytes);
-                store_quad(at + off0, va[u]);
-                store_quad(at + off1, vb[u]);
-              }
-              load(st + 4, va[u], vb[u]);
-              fence_proxy_async();
-              __syncwarp();
-              if (lane == 0) {
-                if (even) bar_arrive(bar(kCFull + s));
-                else bar_arrive_remote(map_cta(bar(kCFull + s), 0));
-              }
-            }
-          }
+      for (int st = 0; st < nst; st++) {
+        load(st + 1);
+        cp_async_wait<1>();
+        const uint32_t from = raw0 + 1024u * (uint32_t)(st & 1);
+        const uint4 va = lds128(from), vb = lds128(from + 512u);
+        if (!bad) bad = !bar_wait(bar(kCEmpty) + 8u * slot, phase, wl);
+        if (on && st < mine) {
+          const uint32_t at = sbase + slot * (uint32_t)kSStageBytes;
+          store_quad(at + off0, va);
+          store_quad(at + off1, vb);
         }
+        __syncwarp();
+        if (lane == 0) bar_arrive(bar(kCFull) + 8u * slot);
+        slot = slot + 1 == kSStages ? 0 : slot + 1;
+        phase ^= slot == 0;
       }
-      if (bad) {
+      if (__any_sync(kFull, bad)) {
         *abort_flag = 1;
         break;
       }
-      g += (uint32_t)nst;
     }
   } else if (warp == kSProd) {
-    // ================= issuing warp (of the even CTA; the odd one passes its "drained" on) ======
-    uint32_t g = 0;
+    // ================= issuing warp =================
+    // Fences the stored stages for the async proxy; the odd CTA's then tells the even one's, which
+    // issues the products.  Everything it needs per stage stays in uniform registers: slot and phase
+    // of the ring, and the accumulator column and rest of the current sample group.
+    uint32_t slot = 0, phase = 0;
     for (uint32_t t = 0;; t++) {
       bool bad = !bar_wait(bar(kCDesc + (int)(t % kSplitSlots)), (t / kSplitSlots) & 1u, wl);
       if (__any_sync(kFull, bad)) {
@@ -635,45 +652,54 @@ __global__ void __launch_bounds__(kSThreads, 1) k_scan_split(const SplitParams p
       if (__shfl_sync(kFull, *slot_desc(t), 0) < 0) break;
       const SplitRec* R = slot_rec(t);
       const int e0 = __shfl_sync(kFull, R->qend[0], 0), e1 = __shfl_sync(kFull, R->qend[1], 0);
-      const int e2 = __shfl_sync(kFull, R->qend[2], 0), nq = __shfl_sync(kFull, R->qend[3], 0), nst = (nq + 1) / 2;
-      if (t > 0) {  // the previous tile's accumulators have been copied out
-        if (even) {
-          bad = !bar_wait(bar(kCDrained), (t - 1) & 1u, wl);
-        } else {
-          bad = !bar_wait(bar(kCDrained), (t - 1) & 1u, wl);
-          if (!bad && lane == 0) bar_arrive_cluster(map_cta(bar(kCDrained), 0));
+      const int e2 = __shfl_sync(kFull, R->qend[2], 0), nq = __shfl_sync(kFull, R->qend[3], 0);
+      if (!even) {
+        for (int q = 0; q < nq && !bad; q += 2) {
+          bad = __any_sync(kFull, !bar_wait(bar(kCFull) + 8u * slot, phase, wl));
+          fence_proxy_async();
+          if (lane == 0) bar_arrive_remote(map_cta(bar(kCFull) + 8u * slot, 0));
+          slot = slot + 1 == kSStages ? 0 : slot + 1;
+          phase ^= slot == 0;
         }
+        if (bad) {
+          *abort_flag = 1;
+          break;
+        }
+        continue;
       }
-      bad = __any_sync(kFull, bad);
-      if (!even && !bad) continue;  // the odd CTA's operands go to the same products
-      for (int st = 0; st < nst && !bad; st++) {
-        const uint32_t gg = g + (uint32_t)st;
-        const int s = (int)(gg % kSStages);
-        const uint32_t use = gg / kSStages;
-        bad = __any_sync(kFull, !bar_wait(bar(kCFull + s), use & 1u, wl));
+      // the previous tile's accumulators have been copied out of both CTAs
+      if (t > 0) bad = __any_sync(kFull, !bar_wait(bar(kCDrained), (t - 1) & 1u, wl));
+      uint32_t d = tmem, acc = 0;
+      int end = e0;  // of the current group
+      for (int q = 0; q < nq && !bad; q += 2) {
+        bad = __any_sync(kFull, !bar_wait(bar(kCFull) + 8u * slot, phase, wl));
         if (bad) break;
+        fence_proxy_async();
         tc_fence_after();
-        const uint32_t sA = sbase + (uint32_t)(s * kSStageBytes), sB = sA + kSStageA;
-        const uint64_t da = smem_desc(sA, kSSbo), db = smem_desc(sB, kSSbo);
+        const uint32_t sA = sbase + slot * (uint32_t)kSStageBytes;
+        const uint64_t da = smem_desc(sA, kSSbo), db = smem_desc(sA + kSStageA, kSSbo);
 #pragma unroll
         for (int h = 0; h < 2; h++) {
-          const int q = 2 * st + h;
-          if (q < nq) {
-            const int grp = (q >= e0) + (q >= e1) + (q >= e2);
-            const bool first = q == 0 || q == e0 || q == e1 || q == e2;
-            const uint32_t d = tmem + 112u * (uint32_t)grp;
-            split_mma(d, da + 32u * h, db + 32u * h, first ? 0u : 1u, tmem + kSSfCol, tmem + kSSfCol + 16);
+          if (q + h < nq) {
+            split_mma(d, da + 32u * h, db + 32u * h, acc, tmem + kSSfCol, tmem + kSSfCol + 16);
             split_mma(d, da + 32u * h + 16u, db + 32u * h + 16u, 1u, tmem + kSSfCol + 32, tmem + kSSfCol + 48);
+            acc = 1;
+            if (q + h + 1 == end) {  // every group has a quad, so the ends are distinct
+              end = end == e0 ? e1 : (end == e1 ? e2 : nq);
+              d += 112u;
+              acc = 0;
+            }
           }
         }
-        split_commit(bar(kCEmpty + s));
-        if (st == nst - 1) split_commit(bar(kCAcc));
+        split_commit(bar(kCEmpty) + 8u * slot);
+        slot = slot + 1 == kSStages ? 0 : slot + 1;
+        phase ^= slot == 0;
       }
       if (bad) {
         *abort_flag = 1;
         break;
       }
-      g += (uint32_t)nst;
+      split_commit(bar(kCAcc));
     }
   } else if (warp == kSProd + 1) {
     // ================= scheduling warp =================
@@ -769,7 +795,7 @@ __global__ void __launch_bounds__(kSThreads, 1) k_scan_split(const SplitParams p
       int i = 0, m = 0, jp = 0, kb = 0;  // first SNP, SNPs; first SNP j and k of the pair
       // margins of this thread's SNP k and, in the pair's first threads, of a SNP j: in flight while the
       // tile's products complete and its accumulators are copied
-      uint4 ik0, ik1, ij0, ij1;
+      uint4 ik, ij;
       uint2 sk0, sk1, sj0, sj1, si0, si1;
       if (ok && desc >= 0) {
         i = R->i;
@@ -778,15 +804,13 @@ __global__ void __launch_bounds__(kSThreads, 1) k_scan_split(const SplitParams p
         kb = jp + 1 + kSplitK * (int)(((uint64_t)desc >> 42) & 0xFFFF) + 64 * (int)crank + 32 * kh;
         jp += pj;
         const int64_t m_pad = J->m_pad;
-        const uint4* pi = J->pairs + tri_offset(m_pad, i, i + 1) - (i + 1);  // + x: pair (i, x)
+        const uint4* pi = J->pairs16 + tri_offset(m_pad, i, i + 1) - (i + 1);  // + x: pair (i, x)
         const uint2* si = reinterpret_cast<const uint2*>(J->singles);
         const int xk = min(kb + lane, m - 1), xj = min(jp + (pt < nj ? pt : 0), m - 1);  // both > i
-        ik0 = __ldg(pi + xk);
-        ik1 = __ldg(pi + J->tri + xk);
+        ik = __ldg(pi + xk);
         sk0 = __ldg(si + xk);
         sk1 = __ldg(si + m_pad + xk);
-        ij0 = __ldg(pi + xj);
-        ij1 = __ldg(pi + J->tri + xj);
+        ij = __ldg(pi + xj);
         sj0 = __ldg(si + xj);
         sj1 = __ldg(si + m_pad + xj);
         si0 = __ldg(si + i);
@@ -815,17 +839,17 @@ __global__ void __launch_bounds__(kSThreads, 1) k_scan_split(const SplitParams p
         const uint32_t ta = tmem + ((uint32_t)(32 * quarter) << 16);
         const uint32_t dst = Ek + (uint32_t)(c * kSplitJ * 64 * 16);
 #pragma unroll 1
-        for (int jj = 0; jj < nj; jj += 2) {
+        for (int jj = 0; jj < nj; jj += 4) {
           const uint32_t tc = ta + (uint32_t)(pj + jj + (pj + jj >= kSHalfJ ? kSHalfJ : 0));  // SNP j of half h: 28h further
-          uint32_t v[4][2][2];
+          uint32_t v[4][2][4];
 #pragma unroll
           for (int g = 0; g < 4; g++)
 #pragma unroll
-            for (int b = 0; b < 2; b++) tmem_ld2(tc + (uint32_t)(112 * g + kSHalfJ * b), v[g][b]);
+            for (int b = 0; b < 2; b++) tmem_ld4(tc + (uint32_t)(112 * g + kSHalfJ * b), v[g][b]);
           tmem_wait_ld();
           const float magic = 8388608.0f;
 #pragma unroll
-          for (int q = 0; q < 2; q++) {
+          for (int q = 0; q < 4; q++) {
             uint32_t w[4];
 #pragma unroll
             for (int ub = 0; ub < 4; ub++) {
@@ -839,7 +863,10 @@ __global__ void __launch_bounds__(kSThreads, 1) k_scan_split(const SplitParams p
       }
       tc_fence_before();
       __syncwarp();
-      if (lane == 0) bar_arrive(bar(kCDrained));
+      if (lane == 0) {
+        if (even) bar_arrive(bar(kCDrained));
+        else bar_arrive_remote(map_cta(bar(kCDrained), 0));
+      }
       // margins as forms: per j into shared memory, per k (this thread's) in registers
       const uint32_t ntot = (uint32_t)J->n0 | ((uint32_t)J->n1 << 16);
       const FormOf form{J->coef, J->bias};
@@ -849,29 +876,29 @@ __global__ void __launch_bounds__(kSThreads, 1) k_scan_split(const SplitParams p
         const uint32_t n0 = sj0.x | (sj1.x << 16), n1 = sj0.y | (sj1.y << 16);
         uint32_t wA[3], wB[3];
         const uint32_t wj[3] = {n0, n1, ntot - n0 - n1};
-        by_genotype(ij0, ij1, n0, n1, gA, wA[0], wA[1]);
-        by_genotype(ij0, ij1, n0, n1, gB, wB[0], wB[1]);
+        by_genotype(ij, n0, n1, gA, wA[0], wA[1]);
+        by_genotype(ij, n0, n1, gB, wB[0], wB[1]);
         wA[2] = nA - wA[0] - wA[1];
         wB[2] = nB - wB[0] - wB[1];
         int* o = marg + kMargWords * pt;
 #pragma unroll
         for (int b = 0; b < 3; b++) {
           const Form x = form(wA[b], 3), y = form(wB[b], 3), z = form(wj[b], 9);
-          *reinterpret_cast<int4*>(o + 8 * b) = make_int4(x.n, x.d, y.n, y.d);
-          *reinterpret_cast<int2*>(o + 8 * b + 4) = make_int2(z.n, z.d);
+          *reinterpret_cast<uint4*>(o + 4 * b) = make_uint4(x.n, x.d, y.n, y.d);
+          *reinterpret_cast<uint2*>(o + 12 + 2 * b) = make_uint2(z.n, z.d);
         }
         const int64_t j = min(jp + pt, m - 1);
         const int64_t jo = j * (J->m_pad - 1) - (j * (j - 1)) / 2 - j - 1;
-        *reinterpret_cast<int2*>(o + 24) = make_int2((int)(uint32_t)jo, (int)(uint32_t)((uint64_t)jo >> 32));
+        *reinterpret_cast<int2*>(o + 18) = make_int2((int)(uint32_t)jo, (int)(uint32_t)((uint64_t)jo >> 32));
       }
       Form kA0, kA1, kB0, kB1, nk0, nk1;
       {
         const uint32_t n0 = sk0.x | (sk1.x << 16), n1 = sk0.y | (sk1.y << 16);
         uint32_t x0, x1;
-        by_genotype(ik0, ik1, n0, n1, gA, x0, x1);
+        by_genotype(ik, n0, n1, gA, x0, x1);
         kA0 = form(x0, 3);
         kA1 = form(x1, 3);
-        by_genotype(ik0, ik1, n0, n1, gB, x0, x1);
+        by_genotype(ik, n0, n1, gB, x0, x1);
         kB0 = form(x0, 3);
         kB1 = form(x1, 3);
         nk0 = form(n0, 9);
@@ -880,23 +907,20 @@ __global__ void __launch_bounds__(kSThreads, 1) k_scan_split(const SplitParams p
       pair_sync(pbar);  // staging rows and margins are in place
       // complete, screen, select: lane = k, this warp's j = c, c + 2, ...
       const int k = kb + lane;
-      const uint4* pairs = J->pairs + k;
-      const int64_t tri = J->tri;
-      auto load_jk = [&](int jj, uint4& a, uint4& b) {
-        a = b = make_uint4(0, 0, 0, 0);
+      const uint4* pairs = J->pairs16 + k;
+      auto load_jk = [&](int jj, uint4& a) {
+        a = make_uint4(0, 0, 0, 0);
         if (jj < nj && jp + jj < m && k < m && k > jp + jj) {
-          const uint2 o = *reinterpret_cast<const uint2*>(marg + kMargWords * jj + 24);
-          const uint4* q = pairs + (int64_t)(((uint64_t)o.y << 32) | o.x);
-          a = __ldg(q);
-          b = __ldg(q + tri);
+          const uint2 o = *reinterpret_cast<const uint2*>(marg + kMargWords * jj + 18);
+          a = __ldg(pairs + (int64_t)(((uint64_t)o.y << 32) | o.x));
         }
       };
       Screen scr;
       scr.theta1 = J->theta1;
       scr.theta2 = J->theta2;
       const float coef = J->c, base = J->base;
-      uint4 jk0, jk1;
-      load_jk(c, jk0, jk1);
+      uint4 jk;
+      load_jk(c, jk);
       if (kb < m) {
 #pragma unroll 1
         for (int jj = c; jj < nj; jj += 2) {
@@ -907,15 +931,14 @@ __global__ void __launch_bounds__(kSThreads, 1) k_scan_split(const SplitParams p
           const uint4 e1 = lds128(Ek + (uint32_t)((kSplitJ + jj) * 64 * 16));
           bool want = valid;
           if (kDump) {
-            load_jk(jj + 2, jk0, jk1);
+            load_jk(jj + 2, jk);
           } else {
-            const uint32_t w00 = prmt(jk0.x, jk1.x, 0x5410u), w01 = prmt(jk0.y, jk1.y, 0x5410u);
-            const uint32_t w10 = prmt(jk0.z, jk1.z, 0x5410u), w11 = prmt(jk0.w, jk1.w, 0x5410u);
-            load_jk(jj + 2, jk0, jk1);
-            const int4* mj = reinterpret_cast<const int4*>(marg + kMargWords * jj);
+            const Form q00 = form(jk.x, 3), q01 = form(jk.y, 3), q10 = form(jk.z, 3), q11 = form(jk.w, 3);
+            load_jk(jj + 2, jk);
+            const uint4* mj = reinterpret_cast<const uint4*>(marg + kMargWords * jj);
             auto margins = [&](int b, Form& ijA, Form& ijB, Form& nj_b) {
-              const int4 x = mj[2 * b];
-              const int2 y = *reinterpret_cast<const int2*>(mj + 2 * b + 1);
+              const uint4 x = mj[b];
+              const uint2 y = *(reinterpret_cast<const uint2*>(mj + 3) + b);
               ijA = Form{x.x, x.y};
               ijB = Form{x.z, x.w};
               nj_b = Form{y.x, y.y};
@@ -923,7 +946,6 @@ __global__ void __launch_bounds__(kSThreads, 1) k_scan_split(const SplitParams p
             scr.acc = 0.0f;
             scr.bits = 0u;
             Form ijA, ijB, nj_b, r0[9], r1[9], r2[9];
-            const Form q00 = form(w00, 3), q01 = form(w01, 3), q10 = form(w10, 3), q11 = form(w11, 3);
             margins(0, ijA, ijB, nj_b);
             r0[0] = form(e0.x, 1);
             r0[1] = form(e1.x, 1);
@@ -1044,6 +1066,13 @@ cudaError_t split_configure() {
 cudaError_t launch_split_rows(const SplitJob* jobs, int n_jobs, int64_t max_units, cudaStream_t stream) {
   if (n_jobs <= 0 || max_units <= 0) return cudaSuccess;
   k_split_rows<<<dim3((unsigned)((max_units + 7) / 8), (unsigned)n_jobs), 256, 0, stream>>>(jobs);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_split_pairs(const SplitJob* jobs, int n_jobs, int64_t max_tri, cudaStream_t stream) {
+  if (n_jobs <= 0 || max_tri <= 0) return cudaSuccess;
+  const int64_t blocks = (max_tri + 255) / 256;
+  k_split_pairs<<<dim3((unsigned)(blocks < 4096 ? blocks : 4096), (unsigned)n_jobs), 256, 0, stream>>>(jobs);
   return cudaGetLastError();
 }
 
