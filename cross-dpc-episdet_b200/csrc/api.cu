@@ -849,17 +849,19 @@ int run_split(epik2_ctx* ctx, const std::vector<DevDataset*>& ds, int64_t ib, in
       recs.push_back(r);
     }
   }
-  // device: [jobs][recs][runs][jobs of the rescore] uploaded, then [cursors, counters of every chunk][thresholds][results]
+  // uploaded: [jobs][recs][runs][jobs of the rescore][cursor, tickets of every chunk][thresholds]
+  // [error word]; read back: [error word][results][rescored]
   const size_t o_recs = align_up(sizeof(SplitJob) * jobs.size(), 256);
   const size_t o_runs = o_recs + align_up(sizeof(SplitRec) * std::max<size_t>(recs.size(), 1), 256);
   const size_t o_tc = o_runs + align_up(sizeof(SplitRun) * std::max<size_t>(runs.size(), 1), 256);
-  const size_t up_bytes = o_tc + (resc_out ? align_up(sizeof(TcJob) * jobs.size(), 256) : 0);
-  const size_t o_cur = up_bytes, cur_bytes = align_up(8 * std::max<size_t>(chunks.size(), 1) + 4, 256);
-  const size_t o_thr = o_cur + cur_bytes, thr_bytes = align_up(4 * jobs.size(), 256);
-  const size_t o_res = o_thr + thr_bytes, best_bytes = align_up(sizeof(BestSlot) * jobs.size(), 256);
-  const size_t res_bytes = best_bytes + (resc_out ? align_up(sizeof(Rescored) * jobs.size(), 256) : 0);
+  const size_t o_cur = o_tc + (resc_out ? align_up(sizeof(TcJob) * jobs.size(), 256) : 0);
+  const size_t o_thr = o_cur + align_up(8 * std::max<size_t>(chunks.size(), 1), 256);
+  const size_t o_err = o_thr + align_up(4 * jobs.size(), 256);
+  const size_t up_bytes = o_err + 256;  // the error word and, behind it, the results
+  const size_t o_res = o_err + 16, o_resc = align_up(o_res + sizeof(BestSlot) * jobs.size(), 16);
+  const size_t end = align_up(o_resc + (resc_out ? sizeof(Rescored) * jobs.size() : 0) + 256, 256);
   auto reserve = [&]() {
-    cudaError_t e = ctx->sp_small.need(o_res + res_bytes);
+    cudaError_t e = ctx->sp_small.need(end);
     if (e == cudaSuccess) e = ctx->sp_slots.need(sizeof(BestSlot) * (size_t)n_jobs * per_job);
     if (e == cudaSuccess) e = ctx->sp_rows.need(std::max<size_t>(rows_bytes, 256));
     if (e == cudaSuccess) e = ctx->sp_lists.need(std::max<size_t>(lists_max, 256));
@@ -879,7 +881,7 @@ int run_split(epik2_ctx* ctx, const std::vector<DevDataset*>& ds, int64_t ib, in
     return kSplitNoRoom;
   }
   CK(ctx, e, "search workspace");
-  const size_t h_need = up_bytes + res_bytes + 256;
+  const size_t h_need = end;
   if (h_need > ctx->h_small_cap) {
     cudaFreeHost(ctx->h_small);
     ctx->h_small = nullptr;
@@ -906,33 +908,28 @@ int run_split(epik2_ctx* ctx, const std::vector<DevDataset*>& ds, int64_t ib, in
   const SplitJob* d_jobs = reinterpret_cast<const SplitJob*>(dev);
   SplitRec* d_recs = reinterpret_cast<SplitRec*>(dev + o_recs);
   const SplitRun* d_runs = reinterpret_cast<const SplitRun*>(dev + o_runs);
-  unsigned* d_cur = reinterpret_cast<unsigned*>(dev + o_cur);  // per chunk: tile count, tickets; then the error word
-  int* d_err = reinterpret_cast<int*>(d_cur + 2 * chunks.size());
+  memset(ctx->h_small + o_cur, 0, o_thr - o_cur);
+  for (size_t b = 0; b < jobs.size(); b++) reinterpret_cast<float*>(ctx->h_small + o_thr)[b] = 3.0e38f;
+  memset(ctx->h_small + o_err, 0, 16);
+  unsigned* d_cur = reinterpret_cast<unsigned*>(dev + o_cur);  // per chunk: tile count, tickets
+  int* d_err = reinterpret_cast<int*>(dev + o_err);
   unsigned* d_thr = reinterpret_cast<unsigned*>(dev + o_thr);
   BestSlot* d_res = reinterpret_cast<BestSlot*>(dev + o_res);
   BestSlot* d_slots = static_cast<BestSlot*>(ctx->sp_slots.p);
   CK(ctx, cudaEventRecord(ctx->ev_start, ctx->stream), "event");
   CK(ctx, cudaMemcpyAsync(dev, ctx->h_small, up_bytes, cudaMemcpyHostToDevice, ctx->stream), "upload search tables");
   ctx->stats.h2d_bytes += up_bytes;
-  CK(ctx, cudaMemsetAsync(d_cur, 0, cur_bytes, ctx->stream), "reset counters");
-  CK(ctx, cudaMemsetAsync(d_thr, 0x7F, thr_bytes, ctx->stream), "reset thresholds");  // 3.4e38 as FP32
-  CK(ctx, launch_fill_slots(d_slots, (int64_t)n_jobs * per_job, ctx->stream), "reset slots");
-  ctx->stats.kernel_launches += 4;
-  if (top_k > 1) {
-    CK(ctx, launch_fill_slots(ctx->d_cand, (int64_t)grid * split_score_warps() * 32, ctx->stream), "reset candidates");
-    ctx->stats.kernel_launches += 1;
-  }
-  CK(ctx, launch_split_rows(d_jobs, n_jobs, rows_units, ctx->stream), "sample rows");
-  CK(ctx, launch_split_pairs(d_jobs, n_jobs, max_tri, ctx->stream), "packed margins");
+  CK(ctx, launch_split_setup(d_jobs, n_jobs, rows_units, max_tri, d_slots, per_job, ctx->d_cand,
+                             top_k > 1 ? grid * split_score_warps() * 32 : 0, ctx->stream),
+     "search setup");
+  ctx->stats.kernel_launches += 1;
   for (size_t x = 0; x < chunks.size(); x++) {
     const Chunk& c = chunks[x];
     CK(ctx, launch_split_prepare(d_jobs, d_recs + c.rec0, c.n_recs, c.max_quads, c.max_cols,
                                  static_cast<int32_t*>(ctx->sp_lists.p), static_cast<uint4*>(ctx->sp_cp.p),
-                                 ctx->stream),
-       "split planes");
-    CK(ctx, launch_split_tiles(d_jobs, d_recs + c.rec0, d_runs + c.run0, c.n_runs, c.max_blocks,
-                               static_cast<uint64_t*>(ctx->sp_tiles.p), d_cur + 2 * x, ctx->stream),
-       "tile queue");
+                                 d_runs + c.run0, c.n_runs, c.max_blocks, static_cast<uint64_t*>(ctx->sp_tiles.p),
+                                 d_cur + 2 * x, ctx->stream),
+       "split planes and tile queue");
     SplitParams p{};
     p.jobs = d_jobs;
     p.recs = d_recs + c.rec0;
@@ -949,23 +946,20 @@ int run_split(epik2_ctx* ctx, const std::vector<DevDataset*>& ds, int64_t ib, in
     p.err = d_err;
     p.wait_limit = ctx->wait_limit;
     CK(ctx, launch_scan_split(p, grid, dump_tables != nullptr, ctx->stream), "split search kernel");
-    ctx->stats.kernel_launches += 4;
+    ctx->stats.kernel_launches += 3;
   }
   CK(ctx, launch_reduce_jobs(d_slots, n_jobs, per_job, d_res, ctx->stream), "reduce kernel");
   CK(ctx, cudaEventRecord(ctx->ev_stop, ctx->stream), "event");
-  Rescored* d_resc = reinterpret_cast<Rescored*>(reinterpret_cast<char*>(d_res) + best_bytes);
   if (resc_out) {
-    CK(ctx, launch_rescore_jobs(reinterpret_cast<const TcJob*>(dev + o_tc), d_res, n_jobs, d_resc, ctx->stream),
+    CK(ctx, launch_rescore_jobs(reinterpret_cast<const TcJob*>(dev + o_tc), d_res, n_jobs,
+                                reinterpret_cast<Rescored*>(dev + o_resc), ctx->stream),
        "rescore kernel");
     ctx->stats.kernel_launches += 1;
   }
-  BestSlot* h_res = reinterpret_cast<BestSlot*>(ctx->h_small + up_bytes);
-  int* h_err = reinterpret_cast<int*>(ctx->h_small + up_bytes + res_bytes);
-  CK(ctx, cudaMemcpyAsync(h_res, d_res, resc_out ? res_bytes : sizeof(BestSlot) * (size_t)n_jobs,
-                          cudaMemcpyDeviceToHost, ctx->stream),
-     "read results");
-  CK(ctx, cudaMemcpyAsync(h_err, d_err, 4, cudaMemcpyDeviceToHost, ctx->stream), "read error word");
-  ctx->stats.d2h_bytes += sizeof(BestSlot) * (size_t)n_jobs + 4;
+  const size_t back = (resc_out ? o_resc + sizeof(Rescored) * jobs.size() : o_res + sizeof(BestSlot) * jobs.size()) - o_err;
+  CK(ctx, cudaMemcpyAsync(ctx->h_small + o_err, dev + o_err, back, cudaMemcpyDeviceToHost, ctx->stream), "read results");
+  ctx->stats.d2h_bytes += back;
+  const int* h_err = reinterpret_cast<const int*>(ctx->h_small + o_err);
   const cudaError_t done = cudaStreamSynchronize(ctx->stream);
   for (GrowBuf* b : {&ctx->sp_rows, &ctx->sp_lists, &ctx->sp_tiles})
     if (b->cap > kSplitKeepBytes) b->drop();
@@ -975,8 +969,8 @@ int run_split(epik2_ctx* ctx, const std::vector<DevDataset*>& ds, int64_t ib, in
   CK(ctx, cudaEventElapsedTime(&kms, ctx->ev_start, ctx->ev_stop), "event time");
   ctx->stats.last_scan_kernel_ms = kms;
   ctx->stats.last_scan_triplets = trip;
-  memcpy(best_out, h_res, sizeof(BestSlot) * (size_t)n_jobs);
-  if (resc_out) memcpy(resc_out, reinterpret_cast<char*>(h_res) + best_bytes, sizeof(Rescored) * (size_t)n_jobs);
+  memcpy(best_out, ctx->h_small + o_res, sizeof(BestSlot) * (size_t)n_jobs);
+  if (resc_out) memcpy(resc_out, ctx->h_small + o_resc, sizeof(Rescored) * (size_t)n_jobs);
   return EPIK2_OK;
 }
 

@@ -227,18 +227,17 @@ cudaError_t launch_pairs_tc(const TcParams& p, int blocks, cudaStream_t stream);
 cudaError_t launch_scan_reps(const TcParams& p, int blocks, cudaStream_t stream);
 int split_score_warps();  // scoring warps per CTA of the split search
 cudaError_t split_configure();
-// rows (sample-major bits) of every job (at most 65535) from its planes; max_units: the most class
-// words x four 32-SNP columns of a job
-cudaError_t launch_split_rows(const SplitJob* jobs, int n_jobs, int64_t max_units, cudaStream_t stream);
-// packed pair margins of every job; max_tri: the most pairs of a job
-cudaError_t launch_split_pairs(const SplitJob* jobs, int n_jobs, int64_t max_tri, cudaStream_t stream);
-// sample lists and group ends of records [0, n); then their compacted planes (at most max_quads
-// quads and max_cols 32-SNP columns each)
+// rows (sample-major bits) and packed pair margins of every job (at most 65535), its per_job slots
+// emptied, n_cand candidates emptied; max_units: the most class words x four 32-SNP columns of a job,
+// max_tri: the most pairs
+cudaError_t launch_split_setup(const SplitJob* jobs, int n_jobs, int64_t max_units, int64_t max_tri, BestSlot* slots,
+                               int per_job, BestSlot* cand, int n_cand, cudaStream_t stream);
+// sample lists and group ends of records [0, n) and the tile queue of their runs (at most max_blocks
+// j blocks each; *cursor, zeroed by the caller, receives the tile count); then the records' compacted
+// planes (at most max_quads quads and max_cols 32-SNP columns each)
 cudaError_t launch_split_prepare(const SplitJob* jobs, SplitRec* recs, int n, int max_quads, int max_cols,
-                                 int32_t* lists, uint4* cp, cudaStream_t stream);
-// tile queue of a run list; *cursor (zeroed by the caller) receives the tile count
-cudaError_t launch_split_tiles(const SplitJob* jobs, const SplitRec* recs, const SplitRun* runs, int n_runs,
-                               int max_blocks, uint64_t* tiles, unsigned* cursor, cudaStream_t stream);
+                                 int32_t* lists, uint4* cp, const SplitRun* runs, int n_runs, int max_blocks,
+                                 uint64_t* tiles, unsigned* cursor, cudaStream_t stream);
 cudaError_t launch_scan_split(const SplitParams& p, int blocks, bool dump, cudaStream_t stream);
 cudaError_t launch_scan_int(const ScanParams& p, int blocks, bool dump, cudaStream_t stream);
 cudaError_t launch_reduce_best(const BestSlot* slots, int n, BestSlot* out, cudaStream_t stream);

@@ -63,62 +63,118 @@ __device__ __forceinline__ uint32_t transpose32(uint32_t x, int lane) {
   return x;
 }
 
-// rows[32w + b][q] from planes[w][32q ..] of job blockIdx.y: one warp per class word and four
-// 32-SNP columns.
-__global__ void __launch_bounds__(256) k_split_rows(const SplitJob* __restrict__ jobs) {
+// What a search needs once, for job blockIdx.y, by ranges of blockIdx.x:
+// [0, row_blocks): rows[32w + b][q] from planes[w][32q ..], one warp per class word and four 32-SNP
+// columns;
+// [row_blocks, row_blocks + pair_blocks): the pair margins packed, class 0 in the low, class 1 in the
+// high half of each count (16 bytes per pair instead of 32: one load and no packing per triplet, half
+// the traffic; bound by memory);
+// the last block: the job's slots (and, by job 0, the candidate lists) emptied.
+__global__ void __launch_bounds__(256) k_split_setup(const SplitJob* __restrict__ jobs, int row_blocks, int pair_blocks,
+                                                     BestSlot* __restrict__ slots, int per_job,
+                                                     BestSlot* __restrict__ cand, int n_cand) {
   const SplitJob& J = jobs[blockIdx.y];
-  const uint2* __restrict__ planes = J.planes;
-  uint2* __restrict__ rows = J.rows;
-  const int64_t m_pad = J.m_pad, words = (int64_t)J.w0 + J.w1;
-  const int lane = threadIdx.x & 31, mwp = J.mwp;
-  const int nq = mwp / 4;
-  const int64_t unit = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5);
-  const int64_t w = unit / nq;
-  const int q = 4 * (int)(unit - w * nq);
-  if (w >= words) return;
-  uint2 v[4];
+  const int lane = threadIdx.x & 31;
+  if ((int)blockIdx.x < row_blocks) {
+    const int64_t m_pad = J.m_pad, words = (int64_t)J.w0 + J.w1;
+    const int mwp = J.mwp, nq = mwp / 4;
+    const int64_t unit = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5);
+    const int64_t w = unit / nq;
+    const int q = 4 * (int)(unit - w * nq);
+    if (w >= words) return;
+    uint2 v[4];
 #pragma unroll
-  for (int t = 0; t < 4; t++) {
-    const int64_t snp = 32 * (int64_t)(q + t) + lane;
-    v[t] = snp < m_pad ? __ldg(planes + w * m_pad + snp) : make_uint2(0, 0);
-  }
+    for (int t = 0; t < 4; t++) {
+      const int64_t snp = 32 * (int64_t)(q + t) + lane;
+      v[t] = snp < m_pad ? __ldg(J.planes + w * m_pad + snp) : make_uint2(0, 0);
+    }
 #pragma unroll
-  for (int t = 0; t < 4; t++) {
-    v[t].x = transpose32(v[t].x, lane);
-    v[t].y = transpose32(v[t].y, lane);
+    for (int t = 0; t < 4; t++) {
+      v[t].x = transpose32(v[t].x, lane);
+      v[t].y = transpose32(v[t].y, lane);
+    }
+    uint4* dst = reinterpret_cast<uint4*>(J.rows + (32 * w + lane) * (int64_t)mwp + q);
+    dst[0] = make_uint4(v[0].x, v[0].y, v[1].x, v[1].y);
+    dst[1] = make_uint4(v[2].x, v[2].y, v[3].x, v[3].y);
+  } else if ((int)blockIdx.x < row_blocks + pair_blocks) {
+    const uint4* __restrict__ src = J.pairs;
+    uint4* __restrict__ dst = J.pairs16;
+    for (int64_t x = (int64_t)((int)blockIdx.x - row_blocks) * 256 + threadIdx.x; x < J.tri; x += (int64_t)pair_blocks * 256) {
+      const uint4 a = __ldg(src + x), b = __ldg(src + J.tri + x);
+      dst[x] = make_uint4(a.x | (b.x << 16), a.y | (b.y << 16), a.z | (b.z << 16), a.w | (b.w << 16));
+    }
+  } else {
+    BestSlot empty{};
+    empty.score = FLT_MAX;
+    empty.key = ~0ull;
+    for (int x = threadIdx.x; x < per_job; x += 256) slots[(int64_t)blockIdx.y * per_job + x] = empty;
+    if (blockIdx.y == 0)
+      for (int x = threadIdx.x; x < n_cand; x += 256) cand[x] = empty;
   }
-  uint4* dst = reinterpret_cast<uint4*>(rows + (32 * w + lane) * (int64_t)mwp + q);
-  dst[0] = make_uint4(v[0].x, v[0].y, v[1].x, v[1].y);
-  dst[1] = make_uint4(v[2].x, v[2].y, v[3].x, v[3].y);
 }
 
-// Pair margins packed: class 0 in the low, class 1 in the high half of each count (16 bytes per
-// pair instead of 32: one load and no packing per triplet, half the traffic).  Bound by memory.
-__global__ void __launch_bounds__(256) k_split_pairs(const SplitJob* __restrict__ jobs) {
-  const SplitJob& J = jobs[blockIdx.y];
-  const uint4* __restrict__ src = J.pairs;
-  uint4* __restrict__ dst = J.pairs16;
-  for (int64_t x = (int64_t)blockIdx.x * 256 + threadIdx.x; x < J.tri; x += (int64_t)gridDim.x * 256) {
-    const uint4 a = __ldg(src + x), b = __ldg(src + J.tri + x);
-    dst[x] = make_uint4(a.x | (b.x << 16), a.y | (b.y << 16), a.z | (b.z << 16), a.w | (b.w << 16));
-  }
-}
-
-// Sample lists of one record per block: the row numbers of each group's samples, -1 up to the
-// end of its last quad.
+// First of a search's chunk: blocks [0, 2n) make the sample lists of record b / 2, class b % 2; the
+// others the tile queue (split_tiles).
+//
+// Lists: the row numbers of each group's samples, -1 up to the end of its last quad.
+//
+// Tile queue: one block per run of records and j block u; the run's tiles of that j block follow one
+// another record by record, so the CTAs working at the same time share the (j, k) margins through L2.
+// The blocks take their place in the queue from the cursor (any order is correct).
 constexpr int kListThreads = 256;
-__global__ void __launch_bounds__(kListThreads) k_split_lists(const SplitJob* __restrict__ jobs, SplitRec* __restrict__ recs,
-                                                              int32_t* __restrict__ lists) {
+
+__device__ void split_tiles(const SplitJob* __restrict__ jobs, const SplitRec* __restrict__ recs, const SplitRun run,
+                            int u, uint64_t* __restrict__ tiles, unsigned* __restrict__ cursor) {
+  __shared__ unsigned s_warp[kListThreads / 32], s_base;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int m = jobs[recs[run.rec0].job].m, i0 = recs[run.rec0].i;  // the run's records are i0, i0 + 1, ...
+  auto count = [&](int i) { return (unsigned)tiles_of_pair_block((int64_t)i + 1 + kSplitJ * u, m, kSplitK); };
+  if (count(i0) == 0) return;  // the run's smallest i has the most tiles
+  for (int r0 = 0; r0 < run.n; r0 += kListThreads) {
+    const int r = r0 + tid;
+    const unsigned n = r < run.n ? count(i0 + r) : 0u;
+    unsigned x = n;  // inclusive sum over the block
+#pragma unroll
+    for (int off = 1; off < 32; off <<= 1) {
+      const unsigned y = __shfl_up_sync(kFull, x, off);
+      if (lane >= off) x += y;
+    }
+    if (lane == 31) s_warp[warp] = x;
+    __syncthreads();
+    unsigned before = 0, total = 0;
+#pragma unroll
+    for (int w = 0; w < kListThreads / 32; w++) {
+      if (w < warp) before += s_warp[w];
+      total += s_warp[w];
+    }
+    if (tid == 0) s_base = atomicAdd(cursor, total);
+    __syncthreads();
+    const unsigned at = s_base + before + x - n;
+    for (unsigned t = 0; t < n; t++) tiles[at + t] = pack_split_tile((uint32_t)(run.rec0 + r), (uint32_t)u, t);
+    __syncthreads();
+  }
+}
+
+__global__ void __launch_bounds__(kListThreads)
+    k_split_lists(const SplitJob* __restrict__ jobs, SplitRec* __restrict__ recs, int n_recs, int32_t* __restrict__ lists,
+                  const SplitRun* __restrict__ runs, int max_blocks, uint64_t* __restrict__ tiles,
+                  unsigned* __restrict__ cursor) {
   __shared__ uint2 s_sum[kListThreads / 32];
-  SplitRec& rec = recs[blockIdx.x];
+  if (blockIdx.x >= 2u * (unsigned)n_recs) {
+    const int b = (int)(blockIdx.x - 2u * (unsigned)n_recs);
+    split_tiles(jobs, recs, runs[b / max_blocks], b % max_blocks, tiles, cursor);
+    return;
+  }
+  SplitRec& rec = recs[blockIdx.x >> 1];
+  const int c = (int)(blockIdx.x & 1u);
   const SplitJob& J = jobs[rec.job];
   const int i = rec.i, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   int n[2][3];
 #pragma unroll
-  for (int c = 0; c < 2; c++) {
-    n[c][0] = (int)J.singles[((int64_t)c * J.m_pad + i) * 2];
-    n[c][1] = (int)J.singles[((int64_t)c * J.m_pad + i) * 2 + 1];
-    n[c][2] = (c ? J.n1 : J.n0) - n[c][0] - n[c][1];
+  for (int x = 0; x < 2; x++) {
+    n[x][0] = (int)J.singles[((int64_t)x * J.m_pad + i) * 2];
+    n[x][1] = (int)J.singles[((int64_t)x * J.m_pad + i) * 2 + 1];
+    n[x][2] = (x ? J.n1 : J.n0) - n[x][0] - n[x][1];
   }
   const int t0 = n[0][0] + n[1][0], t1 = n[0][1] + n[1][1], t2 = n[0][2] + n[1][2];
   const int gC = (t0 >= t1 && t0 >= t2) ? 0 : (t1 >= t2 ? 1 : 2);
@@ -126,69 +182,71 @@ __global__ void __launch_bounds__(kListThreads) k_split_lists(const SplitJob* __
   int qend[4], q = 0;
 #pragma unroll
   for (int g = 0; g < 4; g++) {
-    const int cnt = n[g >> 1][(g & 1) ? gB : gA];
+    const int* nc = n[g >> 1];
+    const int want = (g & 1) ? gB : gA;
+    const int cnt = want == 0 ? nc[0] : want == 1 ? nc[1] : nc[2];
     q += cnt > 0 ? (cnt + 127) / 128 : 1;
     qend[g] = q;
   }
-  if (tid < 4) rec.qend[tid] = qend[tid];
-  if (tid == 4) rec.genos = gA | (gB << 2) | (gC << 4);
-  int32_t* list = lists + rec.list_off;
-#pragma unroll 1
-  for (int c = 0; c < 2; c++) {
-    const int words = c ? J.w1 : J.w0, wb = c ? J.w0 : 0, ncls = c ? J.n1 : J.n0;
-    int posA = 128 * (c ? qend[1] : 0), posB = 128 * (c ? qend[2] : qend[0]);
-    for (int base = 0; base < words; base += kListThreads) {
-      const int w = base + tid;
-      uint32_t ma = 0, mb = 0;
-      if (w < words) {
-        const uint2 v = __ldg(J.planes + (int64_t)(wb + w) * J.m_pad + i);
-        const int left = ncls - 32 * w;
-        const uint32_t valid = left >= 32 ? kFull : ((1u << left) - 1u);
-        const uint32_t m2 = ~(v.x | v.y) & valid;
-        ma = gA == 0 ? v.x : v.y;
-        mb = gB == 1 ? v.y : m2;
-      }
-      const int ca = __popc(ma), cb = __popc(mb);
-      int xa = ca, xb = cb;  // inclusive sums over the block
+  if (c == 0 && tid == 0) {
 #pragma unroll
-      for (int off = 1; off < 32; off <<= 1) {
-        const int ya = __shfl_up_sync(kFull, xa, off), yb = __shfl_up_sync(kFull, xb, off);
-        if (lane >= off) {
-          xa += ya;
-          xb += yb;
-        }
-      }
-      if (lane == 31) s_sum[warp] = make_uint2((uint32_t)xa, (uint32_t)xb);
-      __syncthreads();
-      int ba = 0, bb = 0, ta = 0, tb = 0;
-#pragma unroll
-      for (int x = 0; x < kListThreads / 32; x++) {
-        const uint2 v = s_sum[x];
-        if (x < warp) {
-          ba += (int)v.x;
-          bb += (int)v.y;
-        }
-        ta += (int)v.x;
-        tb += (int)v.y;
-      }
-      int pa = posA + ba + xa - ca, pb = posB + bb + xb - cb;
-      const int row = 32 * (wb + w);
-      while (ma) {
-        list[pa++] = row + __ffs(ma) - 1;
-        ma &= ma - 1;
-      }
-      while (mb) {
-        list[pb++] = row + __ffs(mb) - 1;
-        mb &= mb - 1;
-      }
-      posA += ta;
-      posB += tb;
-      __syncthreads();
-    }
-    const int endA = 128 * (c ? qend[2] : qend[0]), endB = 128 * (c ? qend[3] : qend[1]);
-    for (int x = posA + tid; x < endA; x += kListThreads) list[x] = -1;
-    for (int x = posB + tid; x < endB; x += kListThreads) list[x] = -1;
+    for (int g = 0; g < 4; g++) rec.qend[g] = qend[g];
+    rec.genos = gA | (gB << 2) | (gC << 4);
   }
+  int32_t* list = lists + rec.list_off;
+  const int words = c ? J.w1 : J.w0, wb = c ? J.w0 : 0, ncls = c ? J.n1 : J.n0;
+  int posA = 128 * (c ? qend[1] : 0), posB = 128 * (c ? qend[2] : qend[0]);
+  for (int base = 0; base < words; base += kListThreads) {
+    const int w = base + tid;
+    uint32_t ma = 0, mb = 0;
+    if (w < words) {
+      const uint2 v = __ldg(J.planes + (int64_t)(wb + w) * J.m_pad + i);
+      const int left = ncls - 32 * w;
+      const uint32_t valid = left >= 32 ? kFull : ((1u << left) - 1u);
+      const uint32_t m2 = ~(v.x | v.y) & valid;
+      ma = gA == 0 ? v.x : v.y;
+      mb = gB == 1 ? v.y : m2;
+    }
+    const int ca = __popc(ma), cb = __popc(mb);
+    int xa = ca, xb = cb;  // inclusive sums over the block
+#pragma unroll
+    for (int off = 1; off < 32; off <<= 1) {
+      const int ya = __shfl_up_sync(kFull, xa, off), yb = __shfl_up_sync(kFull, xb, off);
+      if (lane >= off) {
+        xa += ya;
+        xb += yb;
+      }
+    }
+    if (lane == 31) s_sum[warp] = make_uint2((uint32_t)xa, (uint32_t)xb);
+    __syncthreads();
+    int ba = 0, bb = 0, ta = 0, tb = 0;
+#pragma unroll
+    for (int x = 0; x < kListThreads / 32; x++) {
+      const uint2 v = s_sum[x];
+      if (x < warp) {
+        ba += (int)v.x;
+        bb += (int)v.y;
+      }
+      ta += (int)v.x;
+      tb += (int)v.y;
+    }
+    int pa = posA + ba + xa - ca, pb = posB + bb + xb - cb;
+    const int row = 32 * (wb + w);
+    while (ma) {
+      list[pa++] = row + __ffs(ma) - 1;
+      ma &= ma - 1;
+    }
+    while (mb) {
+      list[pb++] = row + __ffs(mb) - 1;
+      mb &= mb - 1;
+    }
+    posA += ta;
+    posB += tb;
+    __syncthreads();
+  }
+  const int endA = 128 * (c ? qend[2] : qend[0]), endB = 128 * (c ? qend[3] : qend[1]);
+  for (int x = posA + tid; x < endA; x += kListThreads) list[x] = -1;
+  for (int x = posB + tid; x < endB; x += kListThreads) list[x] = -1;
 }
 
 // Compacted planes: one warp per record, quad and four 32-SNP columns.  Lane l gathers the row
@@ -229,37 +287,6 @@ __global__ void __launch_bounds__(256) k_split_planes(const SplitJob* __restrict
     }
     dst[64 * t] = make_uint4(x[t][0], x[t][1], x[t][2], x[t][3]);
     dst[64 * t + 1] = make_uint4(y[t][0], y[t][1], y[t][2], y[t][3]);
-  }
-}
-
-// Tile queue: one block per run of records and j block u; the run's tiles of that j block follow
-// one another record by record, so the CTAs working at the same time share the (j, k) margins
-// through L2.  The blocks take their place in the queue from the cursor (any order is correct).
-__global__ void __launch_bounds__(128) k_split_tiles(const SplitJob* __restrict__ jobs, const SplitRec* __restrict__ recs,
-                                                     const SplitRun* __restrict__ runs, uint64_t* __restrict__ tiles,
-                                                     unsigned* __restrict__ cursor) {
-  __shared__ unsigned s_base;
-  const SplitRun run = runs[blockIdx.y];
-  const int u = blockIdx.x;
-  const int m = jobs[recs[run.rec0].job].m;
-  auto count = [&](int i) { return (int)tiles_of_pair_block((int64_t)i + 1 + kSplitJ * u, m, kSplitK); };
-  if (count(recs[run.rec0].i) == 0) return;  // the run's smallest i has the most tiles
-  unsigned total = 0;
-  for (int r = threadIdx.x; r < run.n; r += blockDim.x) total += (unsigned)count(recs[run.rec0 + r].i);
-  // block sum through a shared accumulator (few records per run)
-  __shared__ unsigned s_total;
-  if (threadIdx.x == 0) s_total = 0;
-  __syncthreads();
-  if (total) atomicAdd(&s_total, total);
-  __syncthreads();
-  if (threadIdx.x == 0) s_base = atomicAdd(cursor, s_total);
-  __syncthreads();
-  unsigned at = s_base;
-  for (int r = 0; r < run.n; r++) {
-    const int n = count(recs[run.rec0 + r].i);
-    for (int t = threadIdx.x; t < n; t += blockDim.x)
-      tiles[at + t] = pack_split_tile((uint32_t)(run.rec0 + r), (uint32_t)u, (uint32_t)t);
-    at += (unsigned)n;
   }
 }
 
@@ -1011,10 +1038,10 @@ __global__ void __launch_bounds__(kSThreads, 1) k_scan_split(const SplitParams p
             reach = __float_as_uint(__shfl_sync(kFull, list_s, 31));
           }
           reach = __reduce_min_sync(kFull, reach);
-          if (reach < thr) {
-            if (lane == 0) thr = min(reach, atomicMin(p.thr + cur_job, reach));
-            thr = __shfl_sync(kFull, thr, 0);
-          }
+          // also without an improvement the lowest score known by now is read back: early in a search
+          // the warps learn from one another within a tile
+          if (lane == 0) thr = min(reach, atomicMin(p.thr + cur_job, reach));
+          thr = __shfl_sync(kFull, thr, 0);
         }
       }
       __syncwarp();
@@ -1063,23 +1090,22 @@ cudaError_t split_configure() {
   return e;
 }
 
-cudaError_t launch_split_rows(const SplitJob* jobs, int n_jobs, int64_t max_units, cudaStream_t stream) {
-  if (n_jobs <= 0 || max_units <= 0) return cudaSuccess;
-  k_split_rows<<<dim3((unsigned)((max_units + 7) / 8), (unsigned)n_jobs), 256, 0, stream>>>(jobs);
-  return cudaGetLastError();
-}
-
-cudaError_t launch_split_pairs(const SplitJob* jobs, int n_jobs, int64_t max_tri, cudaStream_t stream) {
-  if (n_jobs <= 0 || max_tri <= 0) return cudaSuccess;
-  const int64_t blocks = (max_tri + 255) / 256;
-  k_split_pairs<<<dim3((unsigned)(blocks < 4096 ? blocks : 4096), (unsigned)n_jobs), 256, 0, stream>>>(jobs);
+cudaError_t launch_split_setup(const SplitJob* jobs, int n_jobs, int64_t max_units, int64_t max_tri, BestSlot* slots,
+                               int per_job, BestSlot* cand, int n_cand, cudaStream_t stream) {
+  if (n_jobs <= 0) return cudaSuccess;
+  const int row_blocks = (int)((max_units + 7) / 8);
+  const int pair_blocks = (int)(max_tri / 256 < 4095 ? max_tri / 256 + 1 : 4096);
+  k_split_setup<<<dim3((unsigned)(row_blocks + pair_blocks + 1), (unsigned)n_jobs), 256, 0, stream>>>(
+      jobs, row_blocks, pair_blocks, slots, per_job, cand, n_cand);
   return cudaGetLastError();
 }
 
 cudaError_t launch_split_prepare(const SplitJob* jobs, SplitRec* recs, int n, int max_quads, int max_cols,
-                                 int32_t* lists, uint4* cp, cudaStream_t stream) {
+                                 int32_t* lists, uint4* cp, const SplitRun* runs, int n_runs, int max_blocks,
+                                 uint64_t* tiles, unsigned* cursor, cudaStream_t stream) {
   if (n <= 0) return cudaSuccess;
-  k_split_lists<<<(unsigned)n, kListThreads, 0, stream>>>(jobs, recs, lists);
+  const int64_t blocks = 2 * (int64_t)n + (int64_t)n_runs * max_blocks;
+  k_split_lists<<<(unsigned)blocks, kListThreads, 0, stream>>>(jobs, recs, n, lists, runs, max_blocks, tiles, cursor);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return e;
   const int64_t units = (int64_t)max_quads * ((max_cols + 3) / 4);
@@ -1087,18 +1113,6 @@ cudaError_t launch_split_prepare(const SplitJob* jobs, SplitRec* recs, int n, in
     const int c = n - at < 65535 ? n - at : 65535;
     k_split_planes<<<dim3((unsigned)((units + 7) / 8), (unsigned)c), 256, 0, stream>>>(jobs, recs + at, lists, cp);
     e = cudaGetLastError();
-    if (e != cudaSuccess) return e;
-  }
-  return cudaSuccess;
-}
-
-cudaError_t launch_split_tiles(const SplitJob* jobs, const SplitRec* recs, const SplitRun* runs, int n_runs,
-                               int max_blocks, uint64_t* tiles, unsigned* cursor, cudaStream_t stream) {
-  if (n_runs <= 0 || max_blocks <= 0) return cudaSuccess;
-  for (int at = 0; at < n_runs; at += 65535) {
-    const int c = n_runs - at < 65535 ? n_runs - at : 65535;
-    k_split_tiles<<<dim3((unsigned)max_blocks, (unsigned)c), 128, 0, stream>>>(jobs, recs, runs + at, tiles, cursor);
-    const cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
   }
   return cudaSuccess;
