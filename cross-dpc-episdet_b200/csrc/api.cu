@@ -802,7 +802,7 @@ int run_split(epik2_ctx* ctx, const std::vector<DevDataset*>& ds, int64_t ib, in
     J.base = sc.base;
     J.rows = reinterpret_cast<uint2*>(rows_bytes);  // offset, made an address below
     rows_units = std::max(rows_units, (d.w0 + d.w1) * (J.mwp / 4));
-    rows_bytes += align_up((size_t)(32 * (d.w0 + d.w1)) * J.mwp * 8, 256);
+    rows_bytes += align_up((size_t)(32 * (d.w0 + d.w1) + 1) * J.mwp * 8, 256);
     J.pairs16 = reinterpret_cast<uint4*>(rows_bytes);
     rows_bytes += align_up((size_t)d.tri * 16, 256);
     max_tri = std::max(max_tri, d.tri);

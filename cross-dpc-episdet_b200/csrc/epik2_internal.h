@@ -159,7 +159,7 @@ struct ScreenConsts {
 // One dataset of a split search.
 struct SplitJob {
   const uint2* planes;
-  uint2* rows;             // [32*(w0+w1)][mwp] {g0, g1} bits of 32 SNPs per entry, class-sorted samples
+  uint2* rows;             // [32*(w0+w1) + 1][mwp] {g0, g1} bits of 32 SNPs per entry, class-sorted samples
   const uint32_t* singles;
   const uint4* pairs;
   uint4* pairs16;          // `pairs` with both classes' counts in one word

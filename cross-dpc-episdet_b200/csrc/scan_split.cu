@@ -69,7 +69,8 @@ __device__ __forceinline__ uint32_t transpose32(uint32_t x, int lane) {
 // [row_blocks, row_blocks + pair_blocks): the pair margins packed, class 0 in the low, class 1 in the
 // high half of each count (16 bytes per pair instead of 32: one load and no packing per triplet, half
 // the traffic; bound by memory);
-// the last block: the job's slots (and, by job 0, the candidate lists) emptied.
+// the last block: the row of no genotypes behind the others; the job's slots (and, by job 0, the
+// candidate lists) emptied.
 __global__ void __launch_bounds__(256) k_split_setup(const SplitJob* __restrict__ jobs, int row_blocks, int pair_blocks,
                                                      BestSlot* __restrict__ slots, int per_job,
                                                      BestSlot* __restrict__ cand, int n_cand) {
@@ -104,6 +105,7 @@ __global__ void __launch_bounds__(256) k_split_setup(const SplitJob* __restrict_
       dst[x] = make_uint4(a.x | (b.x << 16), a.y | (b.y << 16), a.z | (b.z << 16), a.w | (b.w << 16));
     }
   } else {
+    for (int x = threadIdx.x; x < J.mwp; x += 256) J.rows[32 * ((int64_t)J.w0 + J.w1) * J.mwp + x] = make_uint2(0, 0);
     BestSlot empty{};
     empty.score = FLT_MAX;
     empty.key = ~0ull;
@@ -116,7 +118,7 @@ __global__ void __launch_bounds__(256) k_split_setup(const SplitJob* __restrict_
 // First of a search's chunk: blocks [0, 2n) make the sample lists of record b / 2, class b % 2; the
 // others the tile queue (split_tiles).
 //
-// Lists: the row numbers of each group's samples, -1 up to the end of its last quad.
+// Lists: the row numbers of each group's samples, up to the end of its last quad the empty row's.
 //
 // Tile queue: one block per run of records and j block u; the run's tiles of that j block follow one
 // another record by record, so the CTAs working at the same time share the (j, k) margins through L2.
@@ -245,48 +247,90 @@ __global__ void __launch_bounds__(kListThreads)
     __syncthreads();
   }
   const int endA = 128 * (c ? qend[2] : qend[0]), endB = 128 * (c ? qend[3] : qend[1]);
-  for (int x = posA + tid; x < endA; x += kListThreads) list[x] = -1;
-  for (int x = posB + tid; x < endB; x += kListThreads) list[x] = -1;
+  const int empty = 32 * (J.w0 + J.w1);
+  for (int x = posA + tid; x < endA; x += kListThreads) list[x] = empty;
+  for (int x = posB + tid; x < endB; x += kListThreads) list[x] = empty;
 }
 
-// Compacted planes: one warp per record, quad and four 32-SNP columns.  Lane l gathers the row
-// pieces (32 bytes) of four samples, the warp transposes them and lane l writes the 32 bytes of
-// SNP 32q + l: its four words of g0, then of g1.  Bound by the transposes (shuffles).
-__global__ void __launch_bounds__(256) k_split_planes(const SplitJob* __restrict__ jobs, const SplitRec* __restrict__ recs,
-                                                      const int32_t* __restrict__ lists, uint4* __restrict__ cp) {
-  const SplitRec& rec = recs[blockIdx.y];
-  const int lane = threadIdx.x & 31;
-  const int ncol = rec.mlen / 128;
-  const int unit = blockIdx.x * 8 + (threadIdx.x >> 5);
-  const int quad = unit / ncol, col = unit - quad * ncol;
-  if (quad >= rec.qend[3]) return;
-  const SplitJob& J = jobs[rec.job];
-  const int q = rec.qlo + 4 * col;
-  uint32_t x[4][4], y[4][4];  // [column][word]
-  int s[4];
+// 32 x 32 bit transpose inside a thread: word s, bit b -> word b, bit s (16 exchanges per step: two
+// byte permutes each for the steps of 16 and 8 bits, four shifts and selects for the others).
+__device__ __forceinline__ void transpose_words(uint32_t (&a)[32]) {
 #pragma unroll
-  for (int w = 0; w < 4; w++) s[w] = __ldg(lists + rec.list_off + 128 * quad + 32 * w + lane);
-#pragma unroll
-  for (int w = 0; w < 4; w++) {
-    uint4 a = make_uint4(0, 0, 0, 0), b = a;
-    if (s[w] >= 0) {
-      const uint4* src = reinterpret_cast<const uint4*>(J.rows + (int64_t)s[w] * J.mwp + q);
-      a = __ldg(src);
-      b = __ldg(src + 1);
-    }
-    x[0][w] = a.x; y[0][w] = a.y; x[1][w] = a.z; y[1][w] = a.w;
-    x[2][w] = b.x; y[2][w] = b.y; x[3][w] = b.z; y[3][w] = b.w;
+  for (int k = 0; k < 16; k++) {
+    const uint32_t x = a[k], y = a[k + 16];
+    a[k] = prmt(x, y, 0x5410u);
+    a[k + 16] = prmt(x, y, 0x7632u);
   }
-  uint4* dst = cp + rec.cp_off + 2 * ((int64_t)quad * rec.mlen + 128 * col + lane);
 #pragma unroll
-  for (int t = 0; t < 4; t++) {
-#pragma unroll
-    for (int w = 0; w < 4; w++) {
-      x[t][w] = transpose32(x[t][w], lane);
-      y[t][w] = transpose32(y[t][w], lane);
+  for (int k = 0; k < 32; k++)
+    if (!(k & 8)) {
+      const uint32_t x = a[k], y = a[k + 8];
+      a[k] = prmt(x, y, 0x6240u);
+      a[k + 8] = prmt(x, y, 0x7351u);
     }
-    dst[64 * t] = make_uint4(x[t][0], x[t][1], x[t][2], x[t][3]);
-    dst[64 * t + 1] = make_uint4(y[t][0], y[t][1], y[t][2], y[t][3]);
+#pragma unroll
+  for (int j = 4; j > 0; j >>= 1) {
+    const uint32_t m = j == 4 ? 0x0F0F0F0Fu : j == 2 ? 0x33333333u : 0x55555555u;
+#pragma unroll
+    for (int k = 0; k < 32; k++)
+      if (!(k & j)) {
+        const uint32_t x = a[k], y = a[k + j];
+        a[k] = (x & m) | ((y << j) & ~m);
+        a[k + j] = ((x >> j) & m) | (y & ~m);
+      }
+  }
+}
+
+// Compacted planes: per record and quad of 128 samples, the four words of g0 and of g1 of every SNP
+// (32 bytes, so that a warp of the search reads 1 KiB).  A block of four warps takes 32 pieces of 32
+// SNPs each (a piece: one quad and one 32-SNP column; as many quads as columns are short of 32);
+// warp w makes word w: each lane reads the row words of its column for the 32 samples (coalesced
+// across the lanes) and transposes them in its registers.  The words meet in shared memory, [plane,
+// w][bit][piece] with rows of 33, and leave as whole SNPs.  Bound by the transposes (integer pipe):
+// 1024 x 8192 with uniform genotypes takes 267 us per search, 450 with transposes by shuffles across
+// the lanes.
+constexpr int kPlaneThreads = 128;
+__global__ void __launch_bounds__(kPlaneThreads) k_split_planes(const SplitJob* __restrict__ jobs, const SplitRec* __restrict__ recs,
+                                                                const int32_t* __restrict__ lists, uint4* __restrict__ cp) {
+  __shared__ uint32_t s_word[8 * 32 * 33];
+  const SplitRec& rec = recs[blockIdx.y];
+  const int mlen = rec.mlen, ncol = mlen / 32, nq = rec.qend[3];
+  const int span = ncol > 16 ? 32 : ncol > 8 ? 16 : ncol > 4 ? 8 : 4;  // columns of a block
+  const int sets = 32 / span, cblocks = (ncol + span - 1) / span;      // quads of a block; blocks across
+  const int quad0 = (int)(blockIdx.x / (unsigned)cblocks) * sets, col0 = (int)(blockIdx.x % (unsigned)cblocks) * span;
+  if (quad0 >= nq) return;
+  const SplitJob& J = jobs[rec.job];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  {
+    const int quad = quad0 + lane / span, col = col0 + lane % span;
+    const bool on = quad < nq && col < ncol;
+    const int4* list = reinterpret_cast<const int4*>(lists + rec.list_off + 128 * (on ? quad : quad0) + 32 * w);
+    const uint2* rows = J.rows + rec.qlo + (on ? col : col0);
+    const int mwp = J.mwp;
+    uint32_t x[32], y[32];
+#pragma unroll
+    for (int t = 0; t < 8; t++) {
+      const int4 s = __ldg(list + t);
+      const uint2 r0 = __ldg(rows + (int64_t)s.x * mwp), r1 = __ldg(rows + (int64_t)s.y * mwp);
+      const uint2 r2 = __ldg(rows + (int64_t)s.z * mwp), r3 = __ldg(rows + (int64_t)s.w * mwp);
+      x[4 * t] = r0.x; x[4 * t + 1] = r1.x; x[4 * t + 2] = r2.x; x[4 * t + 3] = r3.x;
+      y[4 * t] = r0.y; y[4 * t + 1] = r1.y; y[4 * t + 2] = r2.y; y[4 * t + 3] = r3.y;
+    }
+    transpose_words(x);
+#pragma unroll
+    for (int b = 0; b < 32; b++) s_word[(w * 32 + b) * 33 + lane] = x[b];
+    transpose_words(y);
+#pragma unroll
+    for (int b = 0; b < 32; b++) s_word[((4 + w) * 32 + b) * 33 + lane] = y[b];
+  }
+  __syncthreads();
+  for (int piece = w; piece < 32; piece += kPlaneThreads / 32) {  // lane = SNP of the piece's column
+    const int quad = quad0 + piece / span, col = col0 + piece % span;
+    if (quad >= nq || col >= ncol) continue;
+    const uint32_t* p = s_word + lane * 33 + piece;
+    uint4* dst = cp + rec.cp_off + 2 * ((int64_t)quad * mlen + 32 * col + lane);
+    dst[0] = make_uint4(p[0], p[32 * 33], p[2 * 32 * 33], p[3 * 32 * 33]);
+    dst[1] = make_uint4(p[4 * 32 * 33], p[5 * 32 * 33], p[6 * 32 * 33], p[7 * 32 * 33]);
   }
 }
 
@@ -1108,10 +1152,12 @@ cudaError_t launch_split_prepare(const SplitJob* jobs, SplitRec* recs, int n, in
   k_split_lists<<<(unsigned)blocks, kListThreads, 0, stream>>>(jobs, recs, n, lists, runs, max_blocks, tiles, cursor);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return e;
-  const int64_t units = (int64_t)max_quads * ((max_cols + 3) / 4);
+  // blocks of a record: at most those of max_cols columns (fewer columns take more quads per block)
+  const int span = max_cols > 16 ? 32 : max_cols > 8 ? 16 : max_cols > 4 ? 8 : 4;
+  const int64_t units = (int64_t)((max_quads + 32 / span - 1) / (32 / span)) * ((max_cols + span - 1) / span);
   for (int at = 0; at < n; at += 65535) {
     const int c = n - at < 65535 ? n - at : 65535;
-    k_split_planes<<<dim3((unsigned)((units + 7) / 8), (unsigned)c), 256, 0, stream>>>(jobs, recs + at, lists, cp);
+    k_split_planes<<<dim3((unsigned)units, (unsigned)c), kPlaneThreads, 0, stream>>>(jobs, recs + at, lists, cp);
     e = cudaGetLastError();
     if (e != cudaSuccess) return e;
   }
