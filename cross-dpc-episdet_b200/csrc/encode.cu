@@ -41,37 +41,48 @@ __global__ void k_encode(const uint8_t* __restrict__ geno, const int32_t* __rest
 }
 
 // The same encoding, 16 SNPs per thread, for matrices whose rows are whole 16-byte pieces
-// (n_snps a multiple of 16): one 128-bit load per sample gives the thread all 16 genotypes,
-// so a warp reads 512 consecutive bytes of a sample row per load.  Per 32-bit piece,
-// __vcmpeq4 marks the bytes equal to 0 and to 1; bit b of a plane word is sample b of the
-// class word, as in k_encode.  Groups past n_snps (up to m_pad) write zero planes.
-__global__ void k_encode16(const uint8_t* __restrict__ geno, const int32_t* __restrict__ perm,
+// (n_snps a multiple of 16): one 128-bit load per sample gives the thread all 16 genotypes.  Threads
+// are numbered over (class word, group of 16 SNPs), groups fastest, so a warp reads up to 512
+// consecutive bytes of a sample row per load and narrow matrices fill their warps too.  Eight samples
+// are in flight at a time (100000 x 256 takes 26 us, 61 with one after the other).  Per
+// 32-bit piece, __vcmpeq4 marks the bytes equal to 0 and to 1; bit b of a plane word is sample b of
+// the class word, as in k_encode.  Groups past n_snps (up to m_pad) write zero planes.
+__global__ void __launch_bounds__(128) k_encode16(const uint8_t* __restrict__ geno, const int32_t* __restrict__ perm,
                            uint2* __restrict__ planes, int64_t n_snps, int64_t m_pad, int64_t w0, int64_t w1,
                            int64_t n0, int64_t n1) {
-  const int64_t m0 = 16 * ((int64_t)blockIdx.x * blockDim.x + threadIdx.x);
-  if (m0 >= m_pad) return;
-  const int64_t wt = w0 + w1;
-  for (int64_t w = blockIdx.y; w < wt; w += gridDim.y) {
+  const int64_t groups = m_pad / 16, units = groups * (w0 + w1);
+  for (int64_t unit = (int64_t)blockIdx.x * 128 + threadIdx.x; unit < units; unit += (int64_t)gridDim.x * 128) {
+    const int64_t w = unit / groups, m0 = 16 * (unit - w * groups);
     const bool cases = w >= w0;
     const int64_t base = 32 * (cases ? w - w0 : w);
     const int64_t n_class = cases ? n1 : n0;
-    const int32_t* pc = perm + (cases ? n0 : 0);
+    const int32_t* pc = perm + (cases ? n0 : 0) + base;
+    const int lim = (int)(n_class - base < 32 ? n_class - base : 32);
     uint32_t g0[16], g1[16];
 #pragma unroll
     for (int q = 0; q < 16; q++) g0[q] = g1[q] = 0;
     if (m0 < n_snps) {
-      const int64_t lim = n_class - base < 32 ? n_class - base : 32;
-      for (int64_t b = 0; b < lim; b++) {
-        const int64_t s = pc[base + b];
-        const uint4 v = __ldg(reinterpret_cast<const uint4*>(geno + s * n_snps + m0));
-        const uint32_t x[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll 1
+      for (int b0 = 0; b0 < 32; b0 += 8) {
+        if (b0 >= lim) break;
+        int64_t s[8];
+        uint4 v[8];
 #pragma unroll
-        for (int h = 0; h < 4; h++) {
-          const uint32_t z = __vcmpeq4(x[h], 0u), o = __vcmpeq4(x[h], 0x01010101u);
+        for (int b = 0; b < 8; b++) s[b] = __ldg(pc + (b0 + b < lim ? b0 + b : b0));
 #pragma unroll
-          for (int t = 0; t < 4; t++) {
-            g0[4 * h + t] |= ((z >> (8 * t)) & 1u) << b;
-            g1[4 * h + t] |= ((o >> (8 * t)) & 1u) << b;
+        for (int b = 0; b < 8; b++) v[b] = __ldg(reinterpret_cast<const uint4*>(geno + s[b] * n_snps + m0));
+#pragma unroll
+        for (int b = 0; b < 8; b++) {
+          const uint32_t keep = b0 + b < lim ? 0xFFFFFFFFu : 0u;
+          const uint32_t x[4] = {v[b].x, v[b].y, v[b].z, v[b].w};
+#pragma unroll
+          for (int h = 0; h < 4; h++) {
+            const uint32_t z = __vcmpeq4(x[h], 0u) & keep, o = __vcmpeq4(x[h], 0x01010101u) & keep;
+#pragma unroll
+            for (int t = 0; t < 4; t++) {
+              g0[4 * h + t] |= ((z >> (8 * t)) & 1u) << (b0 + b);
+              g1[4 * h + t] |= ((o >> (8 * t)) & 1u) << (b0 + b);
+            }
           }
         }
       }
@@ -82,26 +93,33 @@ __global__ void k_encode16(const uint8_t* __restrict__ geno, const int32_t* __re
   }
 }
 
-// singles[c][m][g] = popcount over class c's words of plane g of SNP m.
-__global__ void k_singles(const uint2* __restrict__ planes, uint32_t* __restrict__ singles, int64_t m_pad, int64_t w0,
-                          int64_t w1) {
-  const int64_t m = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (m >= m_pad) return;
-  uint32_t c0g0 = 0, c0g1 = 0, c1g0 = 0, c1g1 = 0;
-  for (int64_t w = 0; w < w0; w++) {
-    const uint2 v = planes[w * m_pad + m];
-    c0g0 += __popc(v.x);
-    c0g1 += __popc(v.y);
+// singles[c][m][g] = popcount over class c's words of plane g of SNP m.  A block counts 32 SNPs
+// (lanes, 256-byte rows) of one class, its 32 warps every 32nd word each: with one thread per SNP
+// and class pair 100000 samples x 256 SNPs took 527 us, a chain of loads.
+__global__ void __launch_bounds__(1024) k_singles(const uint2* __restrict__ planes, uint32_t* __restrict__ singles,
+                                                  int64_t m_pad, int64_t w0, int64_t w1) {
+  __shared__ uint2 s_cnt[32][32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, c = (int)blockIdx.y;
+  const int64_t m = 32 * (int64_t)blockIdx.x + lane;  // m_pad is a multiple of 32
+  const int64_t we = c ? w0 + w1 : w0;
+  uint32_t g0 = 0, g1 = 0;
+#pragma unroll 4
+  for (int64_t w = (c ? w0 : 0) + warp; w < we; w += 32) {
+    const uint2 v = __ldg(planes + w * m_pad + m);
+    g0 += __popc(v.x);
+    g1 += __popc(v.y);
   }
-  for (int64_t w = w0; w < w0 + w1; w++) {
-    const uint2 v = planes[w * m_pad + m];
-    c1g0 += __popc(v.x);
-    c1g1 += __popc(v.y);
+  s_cnt[warp][lane] = make_uint2(g0, g1);
+  __syncthreads();
+  if (warp == 0) {
+    uint2 t = make_uint2(0, 0);
+#pragma unroll
+    for (int x = 0; x < 32; x++) {
+      t.x += s_cnt[x][lane].x;
+      t.y += s_cnt[x][lane].y;
+    }
+    reinterpret_cast<uint2*>(singles)[c * m_pad + m] = t;
   }
-  singles[(0 * m_pad + m) * 2 + 0] = c0g0;
-  singles[(0 * m_pad + m) * 2 + 1] = c0g1;
-  singles[(1 * m_pad + m) * 2 + 0] = c1g0;
-  singles[(1 * m_pad + m) * 2 + 1] = c1g1;
 }
 
 // pairs[c][tri(x,y)] = (n(0,0), n(0,1), n(1,0), n(1,1)) of SNPs x < y in class c.
@@ -132,11 +150,12 @@ __global__ void k_pairs(const uint2* __restrict__ planes, uint4* __restrict__ pa
 cudaError_t launch_encode(const DevDataset& d, cudaStream_t stream) {
   const int64_t wt = d.w0 + d.w1;
   if (wt == 0 || d.m_pad == 0) return cudaSuccess;
-  const bool vec = d.n_snps % 16 == 0 && ((uintptr_t)d.geno % 16) == 0 && ((uintptr_t)d.planes % 16) == 0;
+  // 16 SNPs per thread from 16384 threads on, where both take about 18 us (8192 x 1024); below that
+  // there are too few threads to hide the loads (2048 x 128: 18 us against 8).
+  const bool vec = d.m_pad / 16 * wt >= 16384 && d.n_snps % 16 == 0 && ((uintptr_t)d.geno % 16) == 0 && ((uintptr_t)d.planes % 16) == 0;
   if (vec) {  // 16 SNPs per thread
-    const int64_t groups = d.m_pad / 16;
-    dim3 grid((unsigned)((groups + 127) / 128), (unsigned)(wt < 65535 ? wt : 65535));
-    k_encode16<<<grid, 128, 0, stream>>>(d.geno, d.perm, d.planes, d.n_snps, d.m_pad, d.w0, d.w1, d.n_controls,
+    const int64_t blocks = (d.m_pad / 16 * wt + 127) / 128;
+    k_encode16<<<(unsigned)(blocks < (1 << 20) ? blocks : (1 << 20)), 128, 0, stream>>>(d.geno, d.perm, d.planes, d.n_snps, d.m_pad, d.w0, d.w1, d.n_controls,
                                          d.n_cases);
   } else {
     dim3 grid((unsigned)((d.m_pad + 255) / 256), (unsigned)(wt < 65535 ? wt : 65535));
@@ -148,7 +167,7 @@ cudaError_t launch_encode(const DevDataset& d, cudaStream_t stream) {
 
 cudaError_t launch_counts(const DevDataset& d, cudaStream_t stream, bool pairs) {
   if (d.m_pad == 0) return cudaSuccess;
-  k_singles<<<(unsigned)((d.m_pad + 255) / 256), 256, 0, stream>>>(d.planes, d.singles, d.m_pad, d.w0, d.w1);
+  k_singles<<<dim3((unsigned)(d.m_pad / 32), 2), 1024, 0, stream>>>(d.planes, d.singles, d.m_pad, d.w0, d.w1);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return e;
   if (d.m_pad < 2 || !pairs) return cudaSuccess;
