@@ -94,7 +94,7 @@ struct epik2_ctx {
   int64_t rep_cap = 0, rep_slot_cap = 0;
   // split search workspace (kept while it is at most kSplitKeepBytes; given back when another
   // allocation needs the room and with the context)
-  GrowBuf sp_rows, sp_lists, sp_cp, sp_tiles, sp_small, sp_slots;
+  GrowBuf sp_rows, sp_lists, sp_cp, sp_tiles, sp_small, sp_slots, sp_cand;
   unsigned char* h_small = nullptr;  // pinned image of the uploaded part of sp_small, and results
   size_t h_small_cap = 0;
 };
@@ -167,11 +167,11 @@ void drop_spare(epik2_ctx* ctx) {
 
 size_t split_bytes(const epik2_ctx* ctx) {
   return ctx->sp_rows.cap + ctx->sp_lists.cap + ctx->sp_cp.cap + ctx->sp_tiles.cap + ctx->sp_small.cap +
-         ctx->sp_slots.cap;
+         ctx->sp_slots.cap + ctx->sp_cand.cap;
 }
 
 void drop_split(epik2_ctx* ctx) {
-  for (GrowBuf* b : {&ctx->sp_rows, &ctx->sp_lists, &ctx->sp_cp, &ctx->sp_tiles, &ctx->sp_small, &ctx->sp_slots})
+  for (GrowBuf* b : {&ctx->sp_rows, &ctx->sp_lists, &ctx->sp_cp, &ctx->sp_tiles, &ctx->sp_small, &ctx->sp_slots, &ctx->sp_cand})
     b->drop();
 }
 
@@ -308,7 +308,8 @@ int ensure_pgoff(epik2_ctx* ctx, int64_t n) {
   return EPIK2_OK;
 }
 
-int collect_topk(epik2_ctx* ctx, DevDataset& d, const epik2_opts* opts, int top_k, int n_warps);
+int collect_topk(epik2_ctx* ctx, DevDataset& d, const epik2_opts* opts, int top_k, const BestSlot* d_cand,
+                 int64_t n_cand);
 int run_scan_tc(epik2_ctx* ctx, DevDataset& d, int64_t ib, int64_t ie, int top_k, uint32_t* dump_tables,
                 float* dump_scores, BestSlot* best_out, const epik2_opts* opts, int kw, bool fp4, bool pair,
                 bool overlap);
@@ -395,7 +396,8 @@ int run_scan(epik2_ctx* ctx, DevDataset& d, const epik2_opts* opts, uint32_t* du
 constexpr int kSplitNoRoom = 1;  // run_split: the workspace does not fit (the caller takes the other kernels)
 bool split_fits(const DevDataset& d);
 int run_split(epik2_ctx* ctx, const std::vector<DevDataset*>& ds, int64_t ib, int64_t ie, int top_k,
-              uint32_t* dump_tables, float* dump_scores, BestSlot* best_out, Rescored* resc_out = nullptr);
+              uint32_t* dump_tables, float* dump_scores, BestSlot* best_out, Rescored* resc_out = nullptr,
+              int* n_cand_out = nullptr);
 
 // Pair groups of first index i: j0 = i+1, i+5, ... while j0 <= m-2.
 int64_t groups_of(int64_t m, int64_t i) { return (i <= m - 3) ? (m - 2 - i + kPairsPerWarp) / kPairsPerWarp : 0; }
@@ -430,11 +432,12 @@ int run_scan(epik2_ctx* ctx, DevDataset& d, const epik2_opts* opts, uint32_t* du
   // Nothing pinned beyond the format: the genotype-split kernel wherever its 16-bit cells hold
   // (it is the fastest at every shape measured); the other kernels for larger classes.
   if ((engine == 0 || engine == 3) && kw == 0 && pt == 0 && ov == 0 && split_fits(d)) {
-    const int r = run_split(ctx, {&d}, ib, ie, top_k, dump_tables, dump_scores, best_out);
+    int n_cand = 0;
+    const int r = run_split(ctx, {&d}, ib, ie, top_k, dump_tables, dump_scores, best_out, nullptr, &n_cand);
     if (r != kSplitNoRoom) {
       if (r) return r;
       ctx->stats.last_scan_words = d.w0 + d.w1;
-      return collect_topk(ctx, d, opts, top_k, tc_pair_blocks(ctx->tc_blocks) * split_score_warps());
+      return collect_topk(ctx, d, opts, top_k, static_cast<const BestSlot*>(ctx->sp_cand.p), n_cand);
     }
   }
   if (engine == 0 || ((engine == 2 || engine == 3) && kw == 0)) {
@@ -510,14 +513,15 @@ int run_scan(epik2_ctx* ctx, DevDataset& d, const epik2_opts* opts, uint32_t* du
   ctx->stats.last_scan_triplets = trip;
   ctx->stats.last_scan_words = d.w0 + d.w1;
   *best_out = *ctx->h_best;
-  return collect_topk(ctx, d, opts, top_k, n_warps);
+  return collect_topk(ctx, d, opts, top_k, ctx->d_cand, (int64_t)n_warps * 32);
 }
 
-int collect_topk(epik2_ctx* ctx, DevDataset& d, const epik2_opts* opts, int top_k, int n_warps) {
+int collect_topk(epik2_ctx* ctx, DevDataset& d, const epik2_opts* opts, int top_k, const BestSlot* d_cand,
+                 int64_t n_cand) {
   const bool rescore = opts && opts->rescore_fp64;
   if (top_k > 1 && rescore) {
-    const int64_t nc = (int64_t)n_warps * 32;
-    CK(ctx, launch_rescore(d, ctx->d_cand, nc, ctx->d_resc, ctx->stream), "rescore kernel");
+    const int64_t nc = n_cand;
+    CK(ctx, launch_rescore(d, d_cand, nc, ctx->d_resc, ctx->stream), "rescore kernel");
     ctx->stats.kernel_launches += 1;
     std::vector<Rescored> res((size_t)nc);
     CK(ctx, cudaMemcpyAsync(res.data(), ctx->d_resc, res.size() * sizeof(Rescored), cudaMemcpyDeviceToHost,
@@ -540,8 +544,8 @@ int collect_topk(epik2_ctx* ctx, DevDataset& d, const epik2_opts* opts, int top_
       ctx->last_topk.push_back(e);
     }
   } else if (top_k > 1) {
-    std::vector<BestSlot> cand((size_t)n_warps * 32);
-    CK(ctx, cudaMemcpyAsync(cand.data(), ctx->d_cand, cand.size() * sizeof(BestSlot), cudaMemcpyDeviceToHost,
+    std::vector<BestSlot> cand((size_t)n_cand);
+    CK(ctx, cudaMemcpyAsync(cand.data(), d_cand, cand.size() * sizeof(BestSlot), cudaMemcpyDeviceToHost,
                             ctx->stream),
        "read candidates");
     CK(ctx, cudaStreamSynchronize(ctx->stream), "read candidates");
@@ -732,7 +736,7 @@ int run_scan_tc(epik2_ctx* ctx, DevDataset& d, int64_t ib, int64_t ie, int top_k
   ctx->stats.last_scan_triplets = trip;
   ctx->stats.last_scan_words = d.w0 + d.w1;
   *best_out = *ctx->h_best;
-  return collect_topk(ctx, d, opts, top_k, n_warps);
+  return collect_topk(ctx, d, opts, top_k, ctx->d_cand, (int64_t)n_warps * 32);
 }
 
 // Triplets with first index in [0, ie).
@@ -757,12 +761,13 @@ constexpr size_t kSplitKeepBytes = (size_t)1 << 30;
 constexpr size_t kSplitRunBytes = (size_t)40 << 20;
 
 // Best triplet of each dataset over first indices [ib, ie) (clipped to the dataset); resc_out (may
-// be null): their FP64 rescores.  top_k > 1 (one dataset): candidates in ctx->d_cand,
-// split_score_warps() lists per CTA.
+// be null): their FP64 rescores.  top_k > 1 (one dataset): *n_cand_out candidates in ctx->sp_cand,
+// all that can be among the 32 best.
 int run_split(epik2_ctx* ctx, const std::vector<DevDataset*>& ds, int64_t ib, int64_t ie, int top_k,
-              uint32_t* dump_tables, float* dump_scores, BestSlot* best_out, Rescored* resc_out) {
+              uint32_t* dump_tables, float* dump_scores, BestSlot* best_out, Rescored* resc_out, int* n_cand_out) {
   const int n_jobs = (int)ds.size();
   const int grid = tc_pair_blocks(ctx->tc_blocks), per_job = grid * split_score_warps();
+  const int n_cand = top_k > 1 ? per_job * 32 : 0;
   struct Chunk {
     int rec0, n_recs, run0, n_runs, max_quads, max_cols, max_blocks;
   };
@@ -773,6 +778,7 @@ int run_split(epik2_ctx* ctx, const std::vector<DevDataset*>& ds, int64_t ib, in
   size_t rows_bytes = 0, cp_max = 0, lists_max = 0, tiles_max = 0;
   size_t cp = 0, lists = 0, tiles = 0;  // of the current chunk: bytes, bytes, descriptors
   int64_t trip = 0, rows_units = 0, max_tri = 0;
+  float margin = 0.0f;
   // datasets with the most samples first: their tiles last longest, the short ones fill the end
   std::vector<int> order((size_t)n_jobs);
   for (int b = 0; b < n_jobs; b++) order[(size_t)b] = b;
@@ -799,7 +805,9 @@ int run_split(epik2_ctx* ctx, const std::vector<DevDataset*>& ds, int64_t ib, in
     J.theta1 = sc.theta1;
     J.theta2 = sc.theta2;
     J.c = sc.c;
-    J.base = sc.base;
+    // top-k: also what FP64 may rank among the best must be scored (twice the rounding margin)
+    J.base = top_k > 1 ? sc.base - sc.margin : sc.base;
+    margin = sc.margin;
     J.rows = reinterpret_cast<uint2*>(rows_bytes);  // offset, made an address below
     rows_units = std::max(rows_units, (d.w0 + d.w1) * (J.mwp / 4));
     rows_bytes += align_up((size_t)(32 * (d.w0 + d.w1) + 1) * J.mwp * 8, 256);
@@ -863,6 +871,7 @@ int run_split(epik2_ctx* ctx, const std::vector<DevDataset*>& ds, int64_t ib, in
   auto reserve = [&]() {
     cudaError_t e = ctx->sp_small.need(end);
     if (e == cudaSuccess) e = ctx->sp_slots.need(sizeof(BestSlot) * (size_t)n_jobs * per_job);
+    if (e == cudaSuccess && top_k > 1) e = ctx->sp_cand.need(sizeof(BestSlot) * (size_t)n_cand);
     if (e == cudaSuccess) e = ctx->sp_rows.need(std::max<size_t>(rows_bytes, 256));
     if (e == cudaSuccess) e = ctx->sp_lists.need(std::max<size_t>(lists_max, 256));
     if (e == cudaSuccess) e = ctx->sp_cp.need(cp_max + 8192);  // tiles past the last SNP read up to 128 columns on
@@ -919,8 +928,8 @@ int run_split(epik2_ctx* ctx, const std::vector<DevDataset*>& ds, int64_t ib, in
   CK(ctx, cudaEventRecord(ctx->ev_start, ctx->stream), "event");
   CK(ctx, cudaMemcpyAsync(dev, ctx->h_small, up_bytes, cudaMemcpyHostToDevice, ctx->stream), "upload search tables");
   ctx->stats.h2d_bytes += up_bytes;
-  CK(ctx, launch_split_setup(d_jobs, n_jobs, rows_units, max_tri, d_slots, per_job, ctx->d_cand,
-                             top_k > 1 ? grid * split_score_warps() * 32 : 0, ctx->stream),
+  CK(ctx, launch_split_setup(d_jobs, n_jobs, rows_units, max_tri, d_slots, per_job, ctx->d_cand, n_cand,
+                             ctx->stream),
      "search setup");
   ctx->stats.kernel_launches += 1;
   for (size_t x = 0; x < chunks.size(); x++) {
@@ -950,6 +959,12 @@ int run_split(epik2_ctx* ctx, const std::vector<DevDataset*>& ds, int64_t ib, in
   }
   CK(ctx, launch_reduce_jobs(d_slots, n_jobs, per_job, d_res, ctx->stream), "reduce kernel");
   CK(ctx, cudaEventRecord(ctx->ev_stop, ctx->stream), "event");
+  if (top_k > 1) {  // the candidates' number goes behind the error word
+    CK(ctx, launch_split_collect(ctx->d_cand, n_cand, d_thr, margin, static_cast<BestSlot*>(ctx->sp_cand.p),
+                                 reinterpret_cast<unsigned*>(dev + o_err) + 1, ctx->stream),
+       "collect candidates");
+    ctx->stats.kernel_launches += 1;
+  }
   if (resc_out) {
     CK(ctx, launch_rescore_jobs(reinterpret_cast<const TcJob*>(dev + o_tc), d_res, n_jobs,
                                 reinterpret_cast<Rescored*>(dev + o_resc), ctx->stream),
@@ -969,6 +984,7 @@ int run_split(epik2_ctx* ctx, const std::vector<DevDataset*>& ds, int64_t ib, in
   CK(ctx, cudaEventElapsedTime(&kms, ctx->ev_start, ctx->ev_stop), "event time");
   ctx->stats.last_scan_kernel_ms = kms;
   ctx->stats.last_scan_triplets = trip;
+  if (n_cand_out) *n_cand_out = h_err[1];
   memcpy(best_out, ctx->h_small + o_res, sizeof(BestSlot) * (size_t)n_jobs);
   if (resc_out) memcpy(resc_out, ctx->h_small + o_resc, sizeof(Rescored) * (size_t)n_jobs);
   return EPIK2_OK;

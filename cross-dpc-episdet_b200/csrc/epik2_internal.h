@@ -155,6 +155,7 @@ struct ScreenConsts {
   float theta1, theta2;    // of 64 D
   float c;                 // of (64 D)^2 / den
   float base;
+  float margin;            // for rounding, taken off in base
 };
 // One dataset of a split search.
 struct SplitJob {
@@ -238,6 +239,9 @@ cudaError_t launch_split_setup(const SplitJob* jobs, int n_jobs, int64_t max_uni
 cudaError_t launch_split_prepare(const SplitJob* jobs, SplitRec* recs, int n, int max_quads, int max_cols,
                                  int32_t* lists, uint4* cp, const SplitRun* runs, int n_runs, int max_blocks,
                                  uint64_t* tiles, unsigned* cursor, cudaStream_t stream);
+// candidates within margin of *thr into out, their number added to *count
+cudaError_t launch_split_collect(const BestSlot* cand, int n, const unsigned* thr, float margin, BestSlot* out,
+                                 unsigned* count, cudaStream_t stream);
 cudaError_t launch_scan_split(const SplitParams& p, int blocks, bool dump, cudaStream_t stream);
 cudaError_t launch_scan_int(const ScanParams& p, int blocks, bool dump, cudaStream_t stream);
 cudaError_t launch_reduce_best(const BestSlot* slots, int n, BestSlot* out, cudaStream_t stream);

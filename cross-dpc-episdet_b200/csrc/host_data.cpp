@@ -69,6 +69,7 @@ ScreenConsts screen_constants(int64_t n0, int64_t n1) {
   s.theta2 = (float)(t2 * 1.000001 / 64.0);
   s.c = (float)((c2 + t1 * t1 / (16.0 * kK)) * 1.000001 / (64.0 * 64.0));
   const double margin = 0.3 + 1e-6 * std::lgamma(n + 2.0);
+  s.margin = (float)margin;
   s.base = (float)(-((double)n0 + 13.5) * std::log(p) - ((double)n1 + 13.5) * std::log(q) -
                    13.5 * std::log(2.0 * 3.14159265358979323846) - margin);
   return s;

@@ -1041,9 +1041,7 @@ __global__ void __launch_bounds__(kSThreads, 1) k_scan_split(const SplitParams p
             // sum of logs: bits - 27 * 127 * 2^23 (modulo 2^32) in units of 2^-23 / log2 e * 2
             const float lg = __uint2float_rn(scr.bits - 27u * 0x3F800000u);
             const float low = fmaf(4.1315582e-8f, lg, -coef * scr.acc);
-            float reach = __uint_as_float(thr);
-            if (kTopK) reach = fminf(reach, __shfl_sync(kFull, list_s, 31));
-            want = valid && !(low >= reach - base);  // not a number: take the exact path
+            want = valid && !(low >= __uint_as_float(thr) - base);  // not a number: take the exact path
           }
           if (!__any_sync(kFull, want)) continue;
           float sc = FLT_MAX;
@@ -1132,6 +1130,23 @@ cudaError_t split_configure() {
   if (e == cudaSuccess) e = split_set_smem<false, true>();
   if (e == cudaSuccess) configured = true;
   return e;
+}
+
+// Candidates that can be among the best 32 in double precision: those within `margin` (twice the
+// most that FP32 and FP64 scores differ by) of the score that 32 candidates of one warp reach.
+__global__ void __launch_bounds__(256) k_split_collect(const BestSlot* __restrict__ cand, int n,
+                                                       const unsigned* __restrict__ thr, float margin,
+                                                       BestSlot* __restrict__ out, unsigned* __restrict__ count) {
+  const int x = (int)(blockIdx.x * 256 + threadIdx.x);
+  if (x >= n) return;
+  const BestSlot c = cand[x];
+  if (c.key != ~0ull && c.score <= __uint_as_float(*thr) + margin) out[atomicAdd(count, 1u)] = c;
+}
+
+cudaError_t launch_split_collect(const BestSlot* cand, int n, const unsigned* thr, float margin, BestSlot* out,
+                                 unsigned* count, cudaStream_t stream) {
+  k_split_collect<<<(unsigned)((n + 255) / 256), 256, 0, stream>>>(cand, n, thr, margin, out, count);
+  return cudaGetLastError();
 }
 
 cudaError_t launch_split_setup(const SplitJob* jobs, int n_jobs, int64_t max_units, int64_t max_tri, BestSlot* slots,
