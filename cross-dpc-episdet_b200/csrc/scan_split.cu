@@ -339,6 +339,7 @@ __global__ void __launch_bounds__(kPlaneThreads) k_split_planes(const SplitJob* 
 constexpr int kSProd = 6;            // producing warps
 constexpr int kSScore = 8;           // scoring warps (the last ones): four pairs of warps
 constexpr int kSPairs = kSScore / 2;
+constexpr int kSPairJ = 28;          // SNPs j scored by a pair (x 32 SNPs k)
 constexpr int kSFirstScore = kSProd + 2;
 constexpr int kSThreads = 32 * (kSFirstScore + kSScore);
 constexpr int kSStages = 4;
@@ -350,18 +351,17 @@ constexpr int kSStageA = 128 * kSRowBytes;
 constexpr int kSStageBytes = (128 + 2 * kSHalfJ) * kSRowBytes;
 constexpr int kSStagingOff = kSStages * kSStageBytes;  // E[c][j][k]: uint4 words (u, b) = (A,0) (A,1) (B,0) (B,1)
 constexpr int kSStagingBytes = 2 * kSplitJ * 64 * 16;
-// Margins of the tile's SNPs j, per half of the SNPs k (a pair of scoring warps writes and reads its
-// own rows).
+// Per pair of scoring warps: the margins of its SNPs j.
 constexpr int kSPairOff = kSStagingOff + kSStagingBytes;
 constexpr int kMargWords = 20;       // forms of (A, g_j), (B, g_j) for each g_j, then of each g_j; offset of row j of the pair table
-constexpr int kSMargBytes = 2 * kSplitJ * kMargWords * 4;
-constexpr int kSRawOff = kSPairOff + kSMargBytes;  // raw words: per producing warp kSRaw slots of 1 KiB
+constexpr int kSPairBytes = kSPairJ * kMargWords * 4;
+constexpr int kSRawOff = kSPairOff + kSPairs * kSPairBytes;  // raw words: per producing warp kSRaw slots of 1 KiB
 constexpr int kSSlotOff = kSRawOff + kSProd * kSRaw * 1024;
 constexpr int kSSlotBytes = 64 + 128 + 16;        // record, job, descriptor
 constexpr int kSBarOff = kSSlotOff + kSplitSlots * kSSlotBytes;
 constexpr int kSSmemBytes = kSBarOff + 256;
 static_assert(kSSmemBytes <= 232448 - 1024, "shared memory of one CTA");
-static_assert(kMargWords % 4 == 0 && kSStagingOff % 128 == 0, "alignment");
+static_assert(kSPairBytes % 16 == 0 && kSStagingOff % 128 == 0, "alignment");
 
 constexpr int kCFull = 0, kCEmpty = 4, kCAcc = 8, kCDrained = 9, kCHand = 10, kCDesc = 13, kCRel = 16, kCFinal = 19;
 // Accumulators of group g: columns [112g, 112g + 112).  Scale factors (UE8M0, per row and K group):
@@ -825,8 +825,8 @@ __global__ void __launch_bounds__(kSThreads, 1) k_scan_split(const SplitParams p
     const int pt = 32 * c + lane;  // thread of the pair
     const int pair = kh + 2 * part, pbar = 1 + pair;
     const int pj = 28 * part, nj = 28;  // its SNPs j in the tile
-    int* const marg = reinterpret_cast<int*>(smem + kSPairOff) + (kSplitJ * kh + pj) * kMargWords;
     volatile int* const fail = &s_fail[pair];
+    int* const marg = reinterpret_cast<int*>(smem + kSPairOff + pair * kSPairBytes);
     float best_s = FLT_MAX, list_s = FLT_MAX;
     unsigned long long best_k = ~0ull, list_k = ~0ull;
     unsigned thr = 0x7F7F7F7Fu, known = thr;  // bits of the score to reach; of the one last read
