@@ -779,6 +779,7 @@ int run_split(epik2_ctx* ctx, const std::vector<DevDataset*>& ds, int64_t ib, in
   size_t cp = 0, lists = 0, tiles = 0;  // of the current chunk: bytes, bytes, descriptors
   int64_t trip = 0, rows_units = 0, max_tri = 0;
   float margin = 0.0f;
+  bool even = true;
   // datasets with the most samples first: their tiles last longest, the short ones fill the end
   std::vector<int> order((size_t)n_jobs);
   for (int b = 0; b < n_jobs; b++) order[(size_t)b] = b;
@@ -808,6 +809,7 @@ int run_split(epik2_ctx* ctx, const std::vector<DevDataset*>& ds, int64_t ib, in
     // top-k: also what FP64 may rank among the best must be scored (twice the rounding margin)
     J.base = top_k > 1 ? sc.base - sc.margin : sc.base;
     margin = sc.margin;
+    even = even && J.theta1 == 0.0f;
     J.rows = reinterpret_cast<uint2*>(rows_bytes);  // offset, made an address below
     rows_units = std::max(rows_units, (d.w0 + d.w1) * (J.mwp / 4));
     rows_bytes += align_up((size_t)(32 * (d.w0 + d.w1) + 1) * J.mwp * 8, 256);
@@ -954,7 +956,7 @@ int run_split(epik2_ctx* ctx, const std::vector<DevDataset*>& ds, int64_t ib, in
     p.dump_scores = dump_scores;
     p.err = d_err;
     p.wait_limit = ctx->wait_limit;
-    CK(ctx, launch_scan_split(p, grid, dump_tables != nullptr, ctx->stream), "split search kernel");
+    CK(ctx, launch_scan_split(p, grid, dump_tables != nullptr, even, ctx->stream), "split search kernel");
     ctx->stats.kernel_launches += 3;
   }
   CK(ctx, launch_reduce_jobs(d_slots, n_jobs, per_job, d_res, ctx->stream), "reduce kernel");

@@ -242,7 +242,8 @@ cudaError_t launch_split_prepare(const SplitJob* jobs, SplitRec* recs, int n, in
 // candidates within margin of *thr into out, their number added to *count
 cudaError_t launch_split_collect(const BestSlot* cand, int n, const unsigned* thr, float margin, BestSlot* out,
                                  unsigned* count, cudaStream_t stream);
-cudaError_t launch_scan_split(const SplitParams& p, int blocks, bool dump, cudaStream_t stream);
+// even: every job's theta1 is 0
+cudaError_t launch_scan_split(const SplitParams& p, int blocks, bool dump, bool even, cudaStream_t stream);
 cudaError_t launch_scan_int(const ScanParams& p, int blocks, bool dump, cudaStream_t stream);
 cudaError_t launch_reduce_best(const BestSlot* slots, int n, BestSlot* out, cudaStream_t stream);
 cudaError_t launch_tables(const DevDataset& d, const uint32_t* triplets, int64_t n, uint32_t* out,

@@ -30,7 +30,8 @@
 //               for the next tile, then complete, screen and select while that tile counts
 // Classes of at most 65535 samples (the 16-bit halves).
 //
-// What bounds it: the scoring warps (about 350 instructions per 32 triplets) up to about 8192
+// What bounds it: the scoring warps (about 330 instructions per 32 triplets, 27 more where the classes
+// are not even: screen_constants) up to about 8192
 // samples; from there on also the round trip of a ring stage (stores, fence and arrival in the even
 // CTA, products, commit).  Cost of the parts of that round trip, which set the roles and hand-offs
 // (clocks, measured alone): a commit of four products 560; an arrival in the other CTA 133, and
@@ -467,7 +468,8 @@ struct FormOf {  // counts (class 0 low half, class 1 high half) of a sum over `
 };
 
 // Lower bound of K2 (screen_constants in host_data.cpp), cell by cell: per cell one reciprocal, six
-// FP32 operations and half an integer addition.
+// FP32 operations (five for even classes, where theta1 is 0) and half an integer addition.
+template <bool kEven>
 struct Screen {
   float theta1, theta2;  // of 64 D
   float acc;
@@ -478,7 +480,8 @@ struct Screen {
 #pragma unroll
     for (int x = 0; x < kN; x++) {
       D[x] = __uint_as_float(f[x].d) - 12582912.0f;
-      P[x] = fmaf(D[x], -theta1, __uint_as_float(f[x].n) - 8388608.0f);
+      const float N = __uint_as_float(f[x].n) - 8388608.0f;
+      P[x] = kEven ? N : fmaf(D[x], -theta1, N);
     }
 #pragma unroll
     for (int x = 0; x < kN; x++) r[x] = rcp_approx(fmaf(fabsf(D[x]), -theta2, P[x]));
@@ -586,7 +589,7 @@ __device__ __noinline__ float exact_score(uint4 e0, uint4 e1, const SplitJob* J,
   return fabsf(score);
 }
 
-template <bool kDump, bool kTopK>
+template <bool kDump, bool kTopK, bool kEven>
 __global__ void __launch_bounds__(kSThreads, 1) k_scan_split(const SplitParams p) {
   extern __shared__ __align__(1024) unsigned char smem[];
   __shared__ uint32_t s_tmem;
@@ -959,8 +962,7 @@ __global__ void __launch_bounds__(kSThreads, 1) k_scan_split(const SplitParams p
           *reinterpret_cast<uint2*>(o + 12 + 2 * b) = make_uint2(z.n, z.d);
         }
         const int64_t j = min(jp + pt, m - 1);
-        const int64_t jo = j * (J->m_pad - 1) - (j * (j - 1)) / 2 - j - 1;
-        *reinterpret_cast<int2*>(o + 18) = make_int2((int)(uint32_t)jo, (int)(uint32_t)((uint64_t)jo >> 32));
+        *reinterpret_cast<const uint4**>(o + 18) = J->pairs16 + (j * (J->m_pad - 1) - (j * (j - 1)) / 2 - j - 1);
       }
       Form kA0, kA1, kB0, kB1, nk0, nk1;
       {
@@ -978,19 +980,18 @@ __global__ void __launch_bounds__(kSThreads, 1) k_scan_split(const SplitParams p
       pair_sync(pbar);  // staging rows and margins are in place
       // complete, screen, select: lane = k, this warp's j = c, c + 2, ...
       const int k = kb + lane;
-      const uint4* pairs = J->pairs16 + k;
-      auto load_jk = [&](int jj, uint4& a) {
-        a = make_uint4(0, 0, 0, 0);
-        if (jj < nj && jp + jj < m && k < m && k > jp + jj) {
-          const uint2 o = *reinterpret_cast<const uint2*>(marg + kMargWords * jj + 18);
-          a = __ldg(pairs + (int64_t)(((uint64_t)o.y << 32) | o.x));
-        }
-      };
-      Screen scr;
+      Screen<kEven> scr;
       scr.theta1 = J->theta1;
       scr.theta2 = J->theta2;
-      const float coef = J->c, base = J->base;
+      const float coef = -J->c, base = J->base;
+      float limit = __uint_as_float(thr) - base;
       uint4 jk;
+      // (j, k) margins of the pair's row jj
+      auto load_jk = [&](int jj, uint4& a) {
+        a = make_uint4(0, 0, 0, 0);
+        if (jj < nj && jp + jj < m && k < m && k > jp + jj)
+          a = __ldg(*reinterpret_cast<const uint4* const*>(marg + kMargWords * jj + 18) + k);
+      };
       load_jk(c, jk);
       if (kb < m) {
 #pragma unroll 1
@@ -1040,8 +1041,8 @@ __global__ void __launch_bounds__(kSThreads, 1) k_scan_split(const SplitParams p
             scr.cells(r2);
             // sum of logs: bits - 27 * 127 * 2^23 (modulo 2^32) in units of 2^-23 / log2 e * 2
             const float lg = __uint2float_rn(scr.bits - 27u * 0x3F800000u);
-            const float low = fmaf(4.1315582e-8f, lg, -coef * scr.acc);
-            want = valid && !(low >= __uint_as_float(thr) - base);  // not a number: take the exact path
+            const float low = fmaf(4.1315582e-8f, lg, coef * scr.acc);
+            want = valid && !(low >= limit);  // not a number: take the exact path
           }
           if (!__any_sync(kFull, want)) continue;
           float sc = FLT_MAX;
@@ -1084,6 +1085,7 @@ __global__ void __launch_bounds__(kSThreads, 1) k_scan_split(const SplitParams p
           // the warps learn from one another within a tile
           if (lane == 0) thr = min(reach, atomicMin(p.thr + cur_job, reach));
           thr = __shfl_sync(kFull, thr, 0);
+          limit = __uint_as_float(thr) - base;
         }
       }
       __syncwarp();
@@ -1117,17 +1119,19 @@ __global__ void __launch_bounds__(kSThreads, 1) k_scan_split(const SplitParams p
 
 int split_score_warps() { return kSScore; }
 
-template <bool kD, bool kT>
+template <bool kD, bool kT, bool kE>
 static cudaError_t split_set_smem() {
-  return cudaFuncSetAttribute(k_scan_split<kD, kT>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSSmemBytes);
+  return cudaFuncSetAttribute(k_scan_split<kD, kT, kE>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSSmemBytes);
 }
 
 cudaError_t split_configure() {
   static bool configured = false;
   if (configured) return cudaSuccess;
-  cudaError_t e = split_set_smem<false, false>();
-  if (e == cudaSuccess) e = split_set_smem<true, false>();
-  if (e == cudaSuccess) e = split_set_smem<false, true>();
+  cudaError_t e = split_set_smem<false, false, false>();
+  if (e == cudaSuccess) e = split_set_smem<false, false, true>();
+  if (e == cudaSuccess) e = split_set_smem<true, false, false>();
+  if (e == cudaSuccess) e = split_set_smem<false, true, false>();
+  if (e == cudaSuccess) e = split_set_smem<false, true, true>();
   if (e == cudaSuccess) configured = true;
   return e;
 }
@@ -1179,7 +1183,7 @@ cudaError_t launch_split_prepare(const SplitJob* jobs, SplitRec* recs, int n, in
   return cudaSuccess;
 }
 
-template <bool kD, bool kT>
+template <bool kD, bool kT, bool kE>
 static cudaError_t launch_split(const SplitParams& p, int blocks, cudaStream_t stream) {
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3((unsigned)blocks);
@@ -1193,15 +1197,20 @@ static cudaError_t launch_split(const SplitParams& p, int blocks, cudaStream_t s
   attr[0].val.clusterDim.z = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, k_scan_split<kD, kT>, p);
+  return cudaLaunchKernelEx(&cfg, k_scan_split<kD, kT, kE>, p);
 }
 
-cudaError_t launch_scan_split(const SplitParams& p, int blocks, bool dump, cudaStream_t stream) {
+cudaError_t launch_scan_split(const SplitParams& p, int blocks, bool dump, bool even, cudaStream_t stream) {
   const cudaError_t ce = split_configure();
   if (ce != cudaSuccess) return ce;
-  const cudaError_t e = dump ? launch_split<true, false>(p, blocks & ~1, stream)
-                        : p.top_k > 1 ? launch_split<false, true>(p, blocks & ~1, stream)
-                                      : launch_split<false, false>(p, blocks & ~1, stream);
+  const int grid = blocks & ~1;
+  cudaError_t e;
+  if (dump)
+    e = launch_split<true, false, false>(p, grid, stream);
+  else if (p.top_k > 1)
+    e = even ? launch_split<false, true, true>(p, grid, stream) : launch_split<false, true, false>(p, grid, stream);
+  else
+    e = even ? launch_split<false, false, true>(p, grid, stream) : launch_split<false, false, false>(p, grid, stream);
   return e != cudaSuccess ? e : cudaGetLastError();
 }
 

@@ -76,6 +76,44 @@ def test_class_splits(auto, cases):
     _check(auto, g, p)
 
 
+def _even(S, cases):
+    """The class split whose screening bound has p = 1/2."""
+    return 1.115 * S * abs((S - cases + 13.5) / (S + 27.0) - 0.5) ** 3 <= 1.0
+
+
+@pytest.mark.parametrize("S", [150, 1000, 9000])
+@pytest.mark.parametrize("top_k", [1, 32])
+def test_even_and_uneven_classes(auto, S, top_k):
+    """The last even split and the first uneven one on either side, and an even and an uneven dataset in
+    one batch: triplets and scores as the oracle's (exact, the scores are FP32 sums in its order)."""
+    rng = np.random.default_rng(S)
+    g = _genotypes(rng, S, 40, (0.5, 0.35, 0.15))
+    few = next(c for c in range(S) if _even(S, c))
+    many = next(c for c in range(S, 0, -1) if _even(S, c))
+    splits = [few, few - 1, many, many + 1]
+    dids = []
+    try:
+        for cases in splits:
+            p = np.zeros(S, np.uint8)
+            p[rng.permutation(S)[:cases]] = 1
+            r = O.scan(g, p, with_tables=True)
+            did = auto.load(g, p)
+            dids.append((did, r))
+            if top_k == 1:
+                b = auto.scan(did)
+                assert b.ijk == r["ijk"] and f32_bits(b.score) == f32_bits(r["score"])
+            else:
+                best = np.sort(r["scores"].astype(np.float64))[:top_k]
+                got = [x.score for x in auto.scan_topk(did, top_k)]
+                assert np.array_equal(np.sort(np.float32(got)), best.astype(np.float32))
+        if top_k == 1:
+            for (_, r), b in zip(dids, auto.scan_batch([d for d, _ in dids])):
+                assert b.ijk == r["ijk"] and f32_bits(b.score) == f32_bits(r["score"])
+    finally:
+        for did, _ in dids:
+            auto.unload(did)
+
+
 def test_rare_alleles_and_strong_effects(auto):
     """Scores far from the bulk, sparse tables: where the screening bound is loosest."""
     rng = np.random.default_rng(17)
