@@ -343,9 +343,9 @@ constexpr int kSPairs = kSScore / 2;
 constexpr int kSPairJ = 28;          // SNPs j scored by a pair (x 32 SNPs k)
 constexpr int kSFirstScore = kSProd + 2;
 constexpr int kSThreads = 32 * (kSFirstScore + kSScore);
-constexpr int kSStages = 4;
+constexpr int kSStages = 8;
 constexpr int kSRaw = 2;             // raw slots of a producing warp
-constexpr int kSRowBytes = 128;      // 8 words of 32 samples, E2M1
+constexpr int kSRowBytes = 64;       // a quad: 4 words of 32 samples, E2M1
 constexpr uint32_t kSSbo = 8 * kSRowBytes;
 constexpr int kSHalfJ = kSplitJ / 2; // SNPs j expanded by each CTA
 constexpr int kSStageA = 128 * kSRowBytes;
@@ -364,7 +364,7 @@ constexpr int kSSmemBytes = kSBarOff + 256;
 static_assert(kSSmemBytes <= 232448 - 1024, "shared memory of one CTA");
 static_assert(kSPairBytes % 16 == 0 && kSStagingOff % 128 == 0, "alignment");
 
-constexpr int kCFull = 0, kCEmpty = 4, kCAcc = 8, kCDrained = 9, kCHand = 10, kCDesc = 13, kCRel = 16, kCFinal = 19;
+constexpr int kCFull = 0, kCEmpty = 8, kCAcc = 16, kCDrained = 17, kCHand = 18, kCDesc = 21, kCRel = 24, kCFinal = 27;
 // Accumulators of group g: columns [112g, 112g + 112).  Scale factors (UE8M0, per row and K group):
 // columns [448, 480) for the first two K groups of a quad (2 and 1), [480, 512) for the others (1/2).
 constexpr uint32_t kSSfCol = 448;
@@ -424,6 +424,18 @@ __device__ __forceinline__ void store_quad(uint32_t at, uint4 w) {
   sts128(at + 256, make_uint4(w.x & 0x44444444u, w.y & 0x44444444u, w.z & 0x44444444u, w.w & 0x44444444u));
   sts128(at + 384, make_uint4((w.x >> 1) & 0x44444444u, (w.y >> 1) & 0x44444444u, (w.z >> 1) & 0x44444444u,
                               (w.w >> 1) & 0x44444444u));
+}
+
+__device__ __forceinline__ bool bar_test(uint32_t bar, uint32_t parity) {  // without waiting
+  uint32_t ok;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}\n"
+      : "=r"(ok)
+      : "r"(bar), "r"(parity)
+      : "memory");
+  return ok != 0;
 }
 
 __device__ __forceinline__ uint4 lds128(uint32_t saddr) {
@@ -608,7 +620,7 @@ __global__ void __launch_bounds__(kSThreads, 1) k_scan_split(const SplitParams p
 
   if (tid == 0) {
     for (int s = 0; s < kSStages; s++) {
-      bar_init(bar(kCFull + s), kSProd + (even ? 1 : 0));  // + the odd CTA's issuing warp
+      bar_init(bar(kCFull + s), kSProd / 2 + (even ? 1 : 0));  // + the odd CTA's issuing warp
       bar_init(bar(kCEmpty + s), 1);
     }
     bar_init(bar(kCAcc), 1);
@@ -658,10 +670,11 @@ __global__ void __launch_bounds__(kSThreads, 1) k_scan_split(const SplitParams p
     const int row1 = x + (isA ? 64 : kSHalfJ);                   // row of genotype 1
     const bool on = isA || lane < kSHalfJ;
     const uint32_t raw0 = sbase + kSRawOff + (uint32_t)(warp * kSRaw * 1024 + 16 * lane);
-    const uint32_t off_base = (isA ? 0u : (uint32_t)kSStageA) + 512u * (uint32_t)sub;
+    const uint32_t off_base = isA ? 0u : (uint32_t)kSStageA;
     const uint32_t off0 = off_base + (uint32_t)(x >> 3) * kSSbo + (uint32_t)(x & 7) * 16;
     const uint32_t off1 = off_base + (uint32_t)(row1 >> 3) * kSSbo + (uint32_t)(row1 & 7) * 16;
-    uint32_t slot = 0, phase = 1;  // of the ring; the first round finds every slot empty
+    const uint32_t zero = (uint32_t)(wl >> 63);  // 0, unknown to the compiler
+    uint32_t stage = 0;  // of the ring, counted over all tiles
     for (uint32_t t = 0;; t++) {
       const bool got = bar_wait(bar(kCDesc + (int)(t % kSplitSlots)), (t / kSplitSlots) & 1u, wl);
       if (__any_sync(kFull, !got)) {
@@ -671,41 +684,44 @@ __global__ void __launch_bounds__(kSThreads, 1) k_scan_split(const SplitParams p
       const long long desc = *slot_desc(t);
       if (desc < 0) break;
       const SplitRec* R = slot_rec(t);
-      const int nq = R->qend[3], nst = (nq + 1) / 2, mlen = R->mlen;
+      const int nq = R->qend[3], mlen = R->mlen, first = (int)((stage + (uint32_t)sub) & 1u);
       const int j0 = R->i + 1 + kSplitJ * (int)(((uint64_t)desc >> 24) & 0x3FFFF);
       const int k0 = j0 + 1 + kSplitK * (int)(((uint64_t)desc >> 42) & 0xFFFF);
       const int snp = (isA ? k0 + 64 * (int)crank : j0 + kSHalfJ * (int)crank) + x - 32 * R->qlo;
       // (words past a row's end belong to no SNP that is scored; the buffer has room behind its last row)
-      const uint4* next = p.cp + R->cp_off + 2 * ((int64_t)snp + (int64_t)sub * mlen);
+      const uint4* next = p.cp + R->cp_off + 2 * ((int64_t)snp + (int64_t)first * mlen);
       const int64_t step = 4 * (int64_t)mlen;
-      const int mine = (nq - sub + 1) / 2;  // stages with a quad for this warp
-      auto load = [&](int st) {  // this lane's words of stage st into the raw slot of the stage
+      const int mine = (nq - first + 1) / 2;  // quads of this warp
+      auto load = [&](int st, uint32_t after) {  // this lane's words of the warp's quad st into its raw slot
         if (st < mine) {
-          const uint32_t to = raw0 + 1024u * (uint32_t)(st & 1);
+          const uint32_t to = raw0 + 1024u * (uint32_t)(st & 1) + after;
           cp_async16(to, next);
           cp_async16(to + 512u, next + 1);
           next += step;
         }
         cp_async_commit();
       };
-      load(0);
+      load(0, 0);
+      load(1, 0);
       bool bad = false;
-      for (int st = 0; st < nst; st++) {
-        load(st + 1);
+      for (int st = 0; st < mine; st++) {
         cp_async_wait<1>();
         const uint32_t from = raw0 + 1024u * (uint32_t)(st & 1);
         const uint4 va = lds128(from), vb = lds128(from + 512u);
-        if (!bad) bad = !bar_wait(bar(kCEmpty) + 8u * slot, phase, wl);
-        if (on && st < mine) {
+        const uint32_t g = stage + (uint32_t)(first + 2 * st), slot = g % kSStages;
+        const uint32_t phase = (g / kSStages & 1u) ^ 1u;  // the first round finds every slot empty
+        const bool empty = bar_test(bar(kCEmpty) + 8u * slot, phase);
+        load(st + 2, (va.w | vb.w) & zero);  // into the slot just read: not issued before the words are here
+        if (!bad && !empty) bad = !bar_wait(bar(kCEmpty) + 8u * slot, phase, wl);
+        if (on) {
           const uint32_t at = sbase + slot * (uint32_t)kSStageBytes;
           store_quad(at + off0, va);
           store_quad(at + off1, vb);
         }
         __syncwarp();
         if (lane == 0) bar_arrive(bar(kCFull) + 8u * slot);
-        slot = slot + 1 == kSStages ? 0 : slot + 1;
-        phase ^= slot == 0;
       }
+      stage += (uint32_t)nq;
       if (__any_sync(kFull, bad)) {
         *abort_flag = 1;
         break;
@@ -717,6 +733,7 @@ __global__ void __launch_bounds__(kSThreads, 1) k_scan_split(const SplitParams p
     // issues the products.  Everything it needs per stage stays in uniform registers: slot and phase
     // of the ring, and the accumulator column and rest of the current sample group.
     uint32_t slot = 0, phase = 0;
+    bool ready = false;  // stage `slot` was found full already
     for (uint32_t t = 0;; t++) {
       bool bad = !bar_wait(bar(kCDesc + (int)(t % kSplitSlots)), (t / kSplitSlots) & 1u, wl);
       if (__any_sync(kFull, bad)) {
@@ -728,12 +745,13 @@ __global__ void __launch_bounds__(kSThreads, 1) k_scan_split(const SplitParams p
       const int e0 = __shfl_sync(kFull, R->qend[0], 0), e1 = __shfl_sync(kFull, R->qend[1], 0);
       const int e2 = __shfl_sync(kFull, R->qend[2], 0), nq = __shfl_sync(kFull, R->qend[3], 0);
       if (!even) {
-        for (int q = 0; q < nq && !bad; q += 2) {
-          bad = __any_sync(kFull, !bar_wait(bar(kCFull) + 8u * slot, phase, wl));
+        for (int q = 0; q < nq && !bad; q++) {
+          if (!ready) bad = __any_sync(kFull, !bar_wait(bar(kCFull) + 8u * slot, phase, wl));
           fence_proxy_async();
           if (lane == 0) bar_arrive_remote(map_cta(bar(kCFull) + 8u * slot, 0));
           slot = slot + 1 == kSStages ? 0 : slot + 1;
           phase ^= slot == 0;
+          ready = __all_sync(kFull, bar_test(bar(kCFull) + 8u * slot, phase));
         }
         if (bad) {
           *abort_flag = 1;
@@ -745,29 +763,27 @@ __global__ void __launch_bounds__(kSThreads, 1) k_scan_split(const SplitParams p
       if (t > 0) bad = __any_sync(kFull, !bar_wait(bar(kCDrained), (t - 1) & 1u, wl));
       uint32_t d = tmem, acc = 0;
       int end = e0;  // of the current group
-      for (int q = 0; q < nq && !bad; q += 2) {
-        bad = __any_sync(kFull, !bar_wait(bar(kCFull) + 8u * slot, phase, wl));
+      for (int q = 0; q < nq && !bad; q++) {
+        if (!ready) bad = __any_sync(kFull, !bar_wait(bar(kCFull) + 8u * slot, phase, wl));
         if (bad) break;
         fence_proxy_async();
         tc_fence_after();
+        const uint32_t slot1 = slot + 1 == kSStages ? 0 : slot + 1, phase1 = phase ^ (slot1 == 0);
+        const bool next = bar_test(bar(kCFull) + 8u * slot1, phase1);  // its latency passes during the issue
         const uint32_t sA = sbase + slot * (uint32_t)kSStageBytes;
         const uint64_t da = smem_desc(sA, kSSbo), db = smem_desc(sA + kSStageA, kSSbo);
-#pragma unroll
-        for (int h = 0; h < 2; h++) {
-          if (q + h < nq) {
-            split_mma(d, da + 32u * h, db + 32u * h, acc, tmem + kSSfCol, tmem + kSSfCol + 16);
-            split_mma(d, da + 32u * h + 16u, db + 32u * h + 16u, 1u, tmem + kSSfCol + 32, tmem + kSSfCol + 48);
-            acc = 1;
-            if (q + h + 1 == end) {  // every group has a quad, so the ends are distinct
-              end = end == e0 ? e1 : (end == e1 ? e2 : nq);
-              d += 112u;
-              acc = 0;
-            }
-          }
+        split_mma(d, da, db, acc, tmem + kSSfCol, tmem + kSSfCol + 16);
+        split_mma(d, da + 16u, db + 16u, 1u, tmem + kSSfCol + 32, tmem + kSSfCol + 48);
+        acc = 1;
+        if (q + 1 == end) {  // every group has a quad, so the ends are distinct
+          end = end == e0 ? e1 : (end == e1 ? e2 : nq);
+          d += 112u;
+          acc = 0;
         }
         split_commit(bar(kCEmpty) + 8u * slot);
-        slot = slot + 1 == kSStages ? 0 : slot + 1;
-        phase ^= slot == 0;
+        ready = __all_sync(kFull, next);
+        slot = slot1;
+        phase = phase1;
       }
       if (bad) {
         *abort_flag = 1;
