@@ -354,7 +354,7 @@ constexpr int kSStagingOff = kSStages * kSStageBytes;  // E[c][j][k]: uint4 word
 constexpr int kSStagingBytes = 2 * kSplitJ * 64 * 16;
 // Per pair of scoring warps: the margins of its SNPs j.
 constexpr int kSPairOff = kSStagingOff + kSStagingBytes;
-constexpr int kMargWords = 20;       // forms of (A, g_j), (B, g_j) for each g_j, then of each g_j; offset of row j of the pair table
+constexpr int kMargWords = 20;       // forms of (A, g_j), (B, g_j) for each g_j, then of each (C, g_j); row j of the pair table
 constexpr int kSPairBytes = kSPairJ * kMargWords * 4;
 constexpr int kSRawOff = kSPairOff + kSPairs * kSPairBytes;  // raw words: per producing warp kSRaw slots of 1 KiB
 constexpr int kSSlotOff = kSRawOff + kSProd * kSRaw * 1024;
@@ -505,15 +505,12 @@ struct Screen {
   }
 };
 
-// The nine cells of one genotype of j from those with g_k = 0 and 1 of the two counted genotypes of
-// i (f[0], f[1]: A; f[3], f[4]: B) and the margins: (A, j), (B, j), j, and (j, k) with g_k = 0 and 1.
-// f[6 ..]: C.
-__device__ __forceinline__ void row_forms(Form ijA, Form ijB, Form nj, Form jk0, Form jk1, Form (&f)[9]) {
+// The other cells of one genotype of j, from those with g_k = 0 and 1 (f[0], f[1]: A; f[3], f[4]: B;
+// f[6], f[7]: C) and the margins (A, j), (B, j), (C, j): one subtraction of three terms per form.
+__device__ __forceinline__ void row_forms(Form ijA, Form ijB, Form ijC, Form (&f)[9]) {
   f[2] = ijA - f[0] - f[1];
   f[5] = ijB - f[3] - f[4];
-  f[6] = jk0 - f[0] - f[3];
-  f[7] = jk1 - f[1] - f[4];
-  f[8] = nj - jk0 - jk1 - f[2] - f[5];
+  f[8] = ijC - f[6] - f[7];
 }
 
 // Cells of one counted genotype of i from its four counts: t[3b + c].
@@ -973,29 +970,31 @@ __global__ void __launch_bounds__(kSThreads, 1) k_scan_split(const SplitParams p
         int* o = marg + kMargWords * pt;
 #pragma unroll
         for (int b = 0; b < 3; b++) {
-          const Form x = form(wA[b], 3), y = form(wB[b], 3), z = form(wj[b], 9);
+          const Form x = form(wA[b], 3), y = form(wB[b], 3), z = form(wj[b] - wA[b] - wB[b], 3);
           *reinterpret_cast<uint4*>(o + 4 * b) = make_uint4(x.n, x.d, y.n, y.d);
           *reinterpret_cast<uint2*>(o + 12 + 2 * b) = make_uint2(z.n, z.d);
         }
         const int64_t j = min(jp + pt, m - 1);
         *reinterpret_cast<const uint4**>(o + 18) = J->pairs16 + (j * (J->m_pad - 1) - (j * (j - 1)) / 2 - j - 1);
       }
-      Form kA0, kA1, kB0, kB1, nk0, nk1;
+      Form kA0, kA1, kB0, kB1, kC0, kC1;
       {
         const uint32_t n0 = sk0.x | (sk1.x << 16), n1 = sk0.y | (sk1.y << 16);
-        uint32_t x0, x1;
-        by_genotype(ik, n0, n1, gA, x0, x1);
-        kA0 = form(x0, 3);
-        kA1 = form(x1, 3);
-        by_genotype(ik, n0, n1, gB, x0, x1);
-        kB0 = form(x0, 3);
-        kB1 = form(x1, 3);
-        nk0 = form(n0, 9);
-        nk1 = form(n1, 9);
+        uint32_t a0, a1, b0, b1;
+        by_genotype(ik, n0, n1, gA, a0, a1);
+        by_genotype(ik, n0, n1, gB, b0, b1);
+        kA0 = form(a0, 3);
+        kA1 = form(a1, 3);
+        kB0 = form(b0, 3);
+        kB1 = form(b1, 3);
+        kC0 = form(n0 - a0 - b0, 3);
+        kC1 = form(n1 - a1 - b1, 3);
       }
       pair_sync(pbar);  // staging rows and margins are in place
       // complete, screen, select: lane = k, this warp's j = c, c + 2, ...
+      // SNP jj of the pair makes a triplet with this lane's k if jj < lane_end (j < k < m)
       const int k = kb + lane;
+      const int lane_end = k < m ? min(nj, k - jp) : 0, warp_end = min(nj, min(m - 1, kb + 31) - jp);
       Screen<kEven> scr;
       scr.theta1 = J->theta1;
       scr.theta2 = J->theta2;
@@ -1005,16 +1004,15 @@ __global__ void __launch_bounds__(kSThreads, 1) k_scan_split(const SplitParams p
       // (j, k) margins of the pair's row jj
       auto load_jk = [&](int jj, uint4& a) {
         a = make_uint4(0, 0, 0, 0);
-        if (jj < nj && jp + jj < m && k < m && k > jp + jj)
+        if (jj < lane_end)
           a = __ldg(*reinterpret_cast<const uint4* const*>(marg + kMargWords * jj + 18) + k);
       };
       load_jk(c, jk);
       if (kb < m) {
 #pragma unroll 1
-        for (int jj = c; jj < nj; jj += 2) {
+        for (int jj = c; jj < warp_end; jj += 2) {
           const int j = jp + jj;
-          if (j >= m || kb + 31 <= j) break;  // no valid lane from here on
-          const bool valid = k < m && k > j;
+          const bool valid = jj < lane_end;
           const uint4 e0 = lds128(Ek + (uint32_t)(jj * 64 * 16));
           const uint4 e1 = lds128(Ek + (uint32_t)((kSplitJ + jj) * 64 * 16));
           bool want = valid;
@@ -1024,36 +1022,42 @@ __global__ void __launch_bounds__(kSThreads, 1) k_scan_split(const SplitParams p
             const Form q00 = form(jk.x, 3), q01 = form(jk.y, 3), q10 = form(jk.z, 3), q11 = form(jk.w, 3);
             load_jk(jj + 2, jk);
             const uint4* mj = reinterpret_cast<const uint4*>(marg + kMargWords * jj);
-            auto margins = [&](int b, Form& ijA, Form& ijB, Form& nj_b) {
+            auto margins = [&](int b, Form& ijA, Form& ijB, Form& ijC) {
               const uint4 x = mj[b];
               const uint2 y = *(reinterpret_cast<const uint2*>(mj + 3) + b);
               ijA = Form{x.x, x.y};
               ijB = Form{x.z, x.w};
-              nj_b = Form{y.x, y.y};
+              ijC = Form{y.x, y.y};
             };
             scr.acc = 0.0f;
             scr.bits = 0u;
-            Form ijA, ijB, nj_b, r0[9], r1[9], r2[9];
-            margins(0, ijA, ijB, nj_b);
+            Form ijA, ijB, ijC, r0[9], r1[9], r2[9];
+            margins(0, ijA, ijB, ijC);
             r0[0] = form(e0.x, 1);
             r0[1] = form(e1.x, 1);
             r0[3] = form(e0.z, 1);
             r0[4] = form(e1.z, 1);
-            row_forms(ijA, ijB, nj_b, q00, q01, r0);
+            r0[6] = q00 - r0[0] - r0[3];
+            r0[7] = q01 - r0[1] - r0[4];
+            row_forms(ijA, ijB, ijC, r0);
             scr.cells(r0);
-            margins(1, ijA, ijB, nj_b);
+            margins(1, ijA, ijB, ijC);
             r1[0] = form(e0.y, 1);
             r1[1] = form(e1.y, 1);
             r1[3] = form(e0.w, 1);
             r1[4] = form(e1.w, 1);
-            row_forms(ijA, ijB, nj_b, q10, q11, r1);
+            r1[6] = q10 - r1[0] - r1[3];
+            r1[7] = q11 - r1[1] - r1[4];
+            row_forms(ijA, ijB, ijC, r1);
             scr.cells(r1);
-            margins(2, ijA, ijB, nj_b);
+            margins(2, ijA, ijB, ijC);
             r2[0] = kA0 - r0[0] - r1[0];
             r2[1] = kA1 - r0[1] - r1[1];
             r2[3] = kB0 - r0[3] - r1[3];
             r2[4] = kB1 - r0[4] - r1[4];
-            row_forms(ijA, ijB, nj_b, nk0 - q00 - q10, nk1 - q01 - q11, r2);
+            r2[6] = kC0 - r0[6] - r1[6];
+            r2[7] = kC1 - r0[7] - r1[7];
+            row_forms(ijA, ijB, ijC, r2);
             scr.cells(r2);
             // sum of logs: bits - 27 * 127 * 2^23 (modulo 2^32) in units of 2^-23 / log2 e * 2
             const float lg = __uint2float_rn(scr.bits - 27u * 0x3F800000u);
