@@ -571,33 +571,18 @@ int collect_topk(epik2_ctx* ctx, DevDataset& d, const epik2_opts* opts, int top_
 // on; every (j, k), j < k < m_pad, is written once.  Waits for the result (stream sync).
 int run_pairs_tc(epik2_ctx* ctx, DevDataset& d) {
   const int64_t m_pad = d.m_pad, kk = tc_k_per_tile(true);
-  std::vector<uint32_t> ij;
-  std::vector<int64_t> off(1, 0);
-  for (int64_t j0 = 0; j0 <= m_pad - 2; j0 += 64) {
-    ij.push_back(0);
-    ij.push_back((uint32_t)j0);
-    off.push_back(off.back() + tiles_of_pair_block(j0, m_pad, kk));
-  }
-  const int64_t n_pb = (int64_t)off.size() - 1;
-  int r = ensure_pb(ctx, std::max<int64_t>(n_pb, 1));
+  int64_t n_tiles = 0;
+  for (int64_t j0 = 0; j0 <= m_pad - 2; j0 += 64) n_tiles += tiles_of_pair_block(j0, m_pad, kk);
+  int r = ensure_tiles(ctx, std::max<int64_t>(n_tiles, 1));
   if (r) return r;
-  r = ensure_tiles(ctx, std::max<int64_t>(off.back(), 1));
-  if (r) return r;
-  CK(ctx, cudaMemcpyAsync(ctx->d_pb_off, off.data(), off.size() * 8, cudaMemcpyHostToDevice, ctx->stream),
-     "upload pair-margin tiles");
-  CK(ctx, cudaMemcpyAsync(ctx->d_pb_ij, ij.data(), ij.size() * 4, cudaMemcpyHostToDevice, ctx->stream),
-     "upload pair-margin tiles");
-  CK(ctx, launch_expand_tiles(ctx->d_pb_off, ctx->d_pb_ij, n_pb, true, 0, ctx->d_tiles, ctx->stream),
-     "expand pair-margin tiles");
-  CK(ctx, cudaMemsetAsync(ctx->d_counter, 0, 8, ctx->stream), "reset counter");
-  CK(ctx, cudaMemsetAsync(ctx->d_err, 0, 4, ctx->stream), "reset error word");
+  CK(ctx, launch_pair_tiles(m_pad, ctx->d_tiles, ctx->d_counter, ctx->d_err, ctx->stream), "pair-margin tiles");
   TcParams p{};
   p.planes = d.planes;
   p.singles = d.singles;
   p.pairs = d.pairs;
   p.lut = d.lut;
   p.tiles = ctx->d_tiles;
-  p.n_tiles = off.back();
+  p.n_tiles = n_tiles;
   p.tri = d.tri;
   p.m = (int32_t)d.n_snps;
   p.m_pad = (int32_t)d.m_pad;

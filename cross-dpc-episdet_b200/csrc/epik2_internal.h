@@ -224,6 +224,8 @@ cudaError_t launch_encode(const DevDataset& d, cudaStream_t stream);
 cudaError_t launch_counts(const DevDataset& d, cudaStream_t stream, bool pairs = true);
 // pair margins on tensor cores (the CTA-pair FP4 kernel; exact for classes below 2^24)
 cudaError_t launch_pairs_tc(const TcParams& p, int blocks, cudaStream_t stream);
+// tiles of launch_pairs_tc for m_pad >= 2 SNPs into out; *counter and *err set to 0
+cudaError_t launch_pair_tiles(int64_t m_pad, uint64_t* out, unsigned long long* counter, int* err, cudaStream_t stream);
 // replicate form of the CTA-pair FP4 search (16 words per stage): see TcParams::n_reps
 cudaError_t launch_scan_reps(const TcParams& p, int blocks, cudaStream_t stream);
 int split_score_warps();  // scoring warps per CTA of the split search

@@ -687,6 +687,34 @@ cudaError_t launch_expand_tiles(const int64_t* pb_off, const uint32_t* pb_ij, in
   return cudaGetLastError();
 }
 
+// Tiles of the pair margins (i = 0; block u: the SNPs j from 64u); the tile counter and the error word
+// are reset with them.  Bound by the launch: one call where there were two copies of a list made on the
+// host, two memsets and its expansion (a new phenotype for 128 x 2048: 68 -> 59 us,
+// a one-call search of it 202 -> 195).  A block adds up
+// the tiles of those before it.
+__global__ void __launch_bounds__(256) k_pair_tiles(int64_t m_pad, int64_t kK, uint64_t* __restrict__ out,
+                                                    unsigned long long* __restrict__ counter, int* __restrict__ err) {
+  __shared__ unsigned long long s_before;
+  const int u = blockIdx.x, tid = threadIdx.x;
+  if (tid == 0) s_before = 0;
+  if (u == 0 && tid == 0) {
+    *counter = 0;
+    *err = 0;
+  }
+  __syncthreads();
+  unsigned long long before = 0;
+  for (int v = tid; v < u; v += 256) before += (unsigned long long)tiles_of_pair_block(64 * (int64_t)v, m_pad, kK);
+  if (before) atomicAdd(&s_before, before);
+  __syncthreads();
+  const int64_t n = tiles_of_pair_block(64 * (int64_t)u, m_pad, kK);
+  for (int64_t t = tid; t < n; t += 256) out[s_before + t] = pack_tile(0, (uint32_t)(64 * u), (uint32_t)t, 0);
+}
+
+cudaError_t launch_pair_tiles(int64_t m_pad, uint64_t* out, unsigned long long* counter, int* err, cudaStream_t stream) {
+  k_pair_tiles<<<(unsigned)((m_pad - 2) / 64 + 1), 256, 0, stream>>>(m_pad, tc_k_per_tile(true), out, counter, err);
+  return cudaGetLastError();
+}
+
 // Per-dataset reduction of the batched search's per-CTA slots: block b reduces dataset b.
 __global__ void k_reduce_jobs(const BestSlot* __restrict__ slots, int per_job, BestSlot* __restrict__ out) {
   __shared__ float ss[32];

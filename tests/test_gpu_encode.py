@@ -6,6 +6,8 @@ import numpy as np
 import pytest
 
 import epik2
+import oracle as O
+from conftest import f32_bits
 
 pytestmark = pytest.mark.gpu
 
@@ -31,3 +33,26 @@ def test_tables_from_planes(S, M, cases):
     for t, tab in zip(trip, got):
         assert np.array_equal(tab, _table(g, p, t)), t
     assert best.ijk == one.ijk and best.score == one.score
+
+
+@pytest.mark.parametrize("M", [3, 32, 33, 64, 65, 66, 97, 176, 177, 178, 16500])
+def test_pair_margin_tiles(M):
+    """The tile list of the pair margins (64 SNPs j x 112 SNPs k; from 16385 SNPs more blocks than a
+    block of its kernel has threads): the last 24 SNPs' tables, which complete from their margins, and
+    for a small dataset all of them.  Counts, so exact."""
+    rng = np.random.default_rng(M)
+    S = 70
+    g = rng.integers(0, 3, (S, M)).astype(np.uint8)
+    p = (rng.random(S) < 0.5).astype(np.uint8)
+    b = max(0, M - 24)
+    want = O.scan(np.ascontiguousarray(g[:, b:]), p)
+    with epik2.Context(0) as c:
+        did = c.load(g, p)
+        got = c.scan(did, snp_begin=b, snp_end=M)
+        assert tuple(x - b for x in got.ijk) == tuple(want["ijk"]) and f32_bits(got.score) == f32_bits(want["score"])
+        if M < 1000:
+            assert c.scan(did).score == np.float32(O.scan(g, p)["score"])
+        c.set_pheno(did, 1 - p)
+        want = O.scan(np.ascontiguousarray(g[:, b:]), 1 - p)
+        got = c.scan(did, snp_begin=b, snp_end=M)
+        assert f32_bits(got.score) == f32_bits(want["score"])
