@@ -736,9 +736,10 @@ int64_t triplets_before(int64_t m, int64_t ie) {
 // Its cells are 16-bit halves of a word: classes of at most 65535 samples.
 bool split_fits(const DevDataset& d) { return d.n_snps >= 3 && d.n_controls <= 65535 && d.n_cases <= 65535; }
 
-// Compacted planes of the first SNPs searched per launch: launches of the large workload then
-// last 6 ms or more, and their ends (one tile, about 10 us) stay below 0.3 %.
-constexpr size_t kSplitChunkBytes = (size_t)768 << 20;
+// Compacted planes of the first SNPs searched per launch: launches of the large workload then last 8
+// ms or more, and their ends (one tile, about 10 us) stay below 0.3 %.  Most searches take one launch:
+// with 768 MiB 256 x 100000 took a second one for its last 7 first SNPs (1.07 ms instead of 0.99).
+constexpr size_t kSplitChunkBytes = (size_t)1 << 30;
 // A larger workspace of a part is released after the search that needed it.
 constexpr size_t kSplitKeepBytes = (size_t)1 << 30;
 // Planes of the first SNPs whose tiles are interleaved in the queue: what may stay in L2 (126 MB)
