@@ -770,80 +770,105 @@ int run_split(epik2_ctx* ctx, const std::vector<DevDataset*>& ds, int64_t ib, in
   std::vector<int> order((size_t)n_jobs);
   for (int b = 0; b < n_jobs; b++) order[(size_t)b] = b;
   std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return ds[(size_t)a]->n_samples > ds[(size_t)b]->n_samples; });
-  for (int b : order) {
-    const DevDataset& d = *ds[(size_t)b];
-    SplitJob& J = jobs[(size_t)b];
-    J = SplitJob{};
-    J.planes = d.planes;
-    J.singles = d.singles;
-    J.pairs = d.pairs;
-    J.lut = d.lut;
-    J.tri = d.tri;
-    J.m = (int32_t)d.n_snps;
-    J.m_pad = (int32_t)d.m_pad;
-    J.mwp = (int32_t)((d.m_pad / 32 + 3) / 4 * 4);
-    J.w0 = (int32_t)d.w0;
-    J.w1 = (int32_t)d.w1;
-    J.n0 = (int32_t)d.n_controls;
-    J.n1 = (int32_t)d.n_cases;
-    const ScreenConsts sc = screen_constants(d.n_controls, d.n_cases);
-    J.coef = sc.coef;
-    J.bias = sc.bias;
-    J.theta1 = sc.theta1;
-    J.theta2 = sc.theta2;
-    J.c = sc.c;
-    // top-k: also what FP64 may rank among the best must be scored (twice the rounding margin)
-    J.base = top_k > 1 ? sc.base - sc.margin : sc.base;
-    margin = sc.margin;
-    even = even && J.theta1 == 0.0f;
-    J.rows = reinterpret_cast<uint2*>(rows_bytes);  // offset, made an address below
-    rows_units = std::max(rows_units, (d.w0 + d.w1) * (J.mwp / 4));
-    rows_bytes += align_up((size_t)(32 * (d.w0 + d.w1) + 1) * J.mwp * 8, 256);
-    J.pairs16 = reinterpret_cast<uint4*>(rows_bytes);
-    rows_bytes += align_up((size_t)d.tri * 16, 256);
-    max_tri = std::max(max_tri, d.tri);
-    const int64_t m = d.n_snps;
-    const int max_quads = (int)(2 * d.n_samples / 3 / 128) + 5;  // the dropped genotype is the most frequent
-    const int64_t i0 = std::max<int64_t>(ib, 0), i1 = std::min<int64_t>(ie, m - 2);
-    size_t run_bytes = 0;
-    for (int64_t i = i0; i < i1; i++) {
-      SplitRec r{};
-      r.job = b;
-      r.i = (int32_t)i;
-      r.qlo = (int32_t)((i + 1) / 32 / 4 * 4);
-      r.mlen = 32 * (J.mwp - r.qlo);
-      const size_t rec_cp = (size_t)max_quads * r.mlen * 32, rec_list = (size_t)max_quads * 128 * 4;
-      const bool new_chunk = chunks.empty() || cp + rec_cp > kSplitChunkBytes || recs.size() - chunks.back().rec0 >= (1u << 23);
-      if (new_chunk) {
-        chunks.push_back(Chunk{(int)recs.size(), 0, (int)runs.size(), 0, 0, 0, 0});
-        cp = lists = tiles = 0;
+  auto lay_out = [&](int64_t ib, int64_t ie) {  // the jobs, records, runs and chunks of first indices [ib, ie)
+    recs.clear();
+    runs.clear();
+    chunks.clear();
+    rows_bytes = cp_max = lists_max = tiles_max = 0;
+    trip = rows_units = max_tri = 0;
+    even = true;
+    for (int b : order) {
+      const DevDataset& d = *ds[(size_t)b];
+      SplitJob& J = jobs[(size_t)b];
+      J = SplitJob{};
+      J.planes = d.planes;
+      J.singles = d.singles;
+      J.pairs = d.pairs;
+      J.lut = d.lut;
+      J.tri = d.tri;
+      J.m = (int32_t)d.n_snps;
+      J.m_pad = (int32_t)d.m_pad;
+      J.mwp = (int32_t)((d.m_pad / 32 + 3) / 4 * 4);
+      J.w0 = (int32_t)d.w0;
+      J.w1 = (int32_t)d.w1;
+      J.n0 = (int32_t)d.n_controls;
+      J.n1 = (int32_t)d.n_cases;
+      const ScreenConsts sc = screen_constants(d.n_controls, d.n_cases);
+      J.coef = sc.coef;
+      J.bias = sc.bias;
+      J.theta1 = sc.theta1;
+      J.theta2 = sc.theta2;
+      J.c = sc.c;
+      // top-k: also what FP64 may rank among the best must be scored (twice the rounding margin)
+      J.base = top_k > 1 ? sc.base - sc.margin : sc.base;
+      margin = sc.margin;
+      even = even && J.theta1 == 0.0f;
+      J.rows = reinterpret_cast<uint2*>(rows_bytes);  // offset, made an address below
+      rows_units = std::max(rows_units, (d.w0 + d.w1) * (J.mwp / 4));
+      rows_bytes += align_up((size_t)(32 * (d.w0 + d.w1) + 1) * J.mwp * 8, 256);
+      J.pairs16 = reinterpret_cast<uint4*>(rows_bytes);
+      rows_bytes += align_up((size_t)d.tri * 16, 256);
+      max_tri = std::max(max_tri, d.tri);
+      const int64_t m = d.n_snps;
+      const int max_quads = (int)(2 * d.n_samples / 3 / 128) + 5;  // the dropped genotype is the most frequent
+      const int64_t i0 = std::max<int64_t>(ib, 0), i1 = std::min<int64_t>(ie, m - 2);
+      size_t run_bytes = 0;
+      for (int64_t i = i0; i < i1; i++) {
+        SplitRec r{};
+        r.job = b;
+        r.i = (int32_t)i;
+        r.qlo = (int32_t)((i + 1) / 32 / 4 * 4);
+        r.mlen = 32 * (J.mwp - r.qlo);
+        const size_t rec_cp = (size_t)max_quads * r.mlen * 32, rec_list = (size_t)max_quads * 128 * 4;
+        const bool new_chunk = chunks.empty() || cp + rec_cp > kSplitChunkBytes || recs.size() - chunks.back().rec0 >= (1u << 23);
+        if (new_chunk) {
+          chunks.push_back(Chunk{(int)recs.size(), 0, (int)runs.size(), 0, 0, 0, 0});
+          cp = lists = tiles = 0;
+        }
+        Chunk& c = chunks.back();
+        const size_t est = (size_t)((max_quads * 5 + 7) / 8) * r.mlen * 32;  // usual size: 0.41 of the samples
+        if (new_chunk || runs.empty() || recs[(size_t)runs.back().rec0 + c.rec0].job != b || run_bytes + est > kSplitRunBytes) {
+          runs.push_back(SplitRun{(int32_t)recs.size() - c.rec0, 0});
+          c.n_runs++;
+          run_bytes = 0;
+        }
+        run_bytes += est;
+        runs.back().n++;
+        r.cp_off = (int64_t)(cp / 16);
+        r.list_off = (int64_t)(lists / 4);
+        cp += rec_cp;
+        lists += rec_list;
+        const int64_t left = m - 2 - i;  // SNPs j from i + 1 to m - 2
+        const int64_t blocks = (left + kSplitJ - 1) / kSplitJ;
+        tiles += (size_t)(blocks + (blocks * left - kSplitJ * blocks * (blocks - 1) / 2) / kSplitK + 1);
+        trip += (m - 1 - i) * (m - 2 - i) / 2;
+        c.n_recs++;
+        c.max_quads = std::max(c.max_quads, max_quads);
+        c.max_cols = std::max(c.max_cols, r.mlen / 32);
+        c.max_blocks = std::max(c.max_blocks, (int)blocks);
+        cp_max = std::max(cp_max, cp);
+        lists_max = std::max(lists_max, lists);
+        tiles_max = std::max(tiles_max, tiles);
+        recs.push_back(r);
       }
-      Chunk& c = chunks.back();
-      const size_t est = (size_t)((max_quads * 5 + 7) / 8) * r.mlen * 32;  // usual size: 0.41 of the samples
-      if (new_chunk || runs.empty() || recs[(size_t)runs.back().rec0 + c.rec0].job != b || run_bytes + est > kSplitRunBytes) {
-        runs.push_back(SplitRun{(int32_t)recs.size() - c.rec0, 0});
-        c.n_runs++;
-        run_bytes = 0;
-      }
-      run_bytes += est;
-      runs.back().n++;
-      r.cp_off = (int64_t)(cp / 16);
-      r.list_off = (int64_t)(lists / 4);
-      cp += rec_cp;
-      lists += rec_list;
-      const int64_t left = m - 2 - i;  // SNPs j from i + 1 to m - 2
-      const int64_t blocks = (left + kSplitJ - 1) / kSplitJ;
-      tiles += (size_t)(blocks + (blocks * left - kSplitJ * blocks * (blocks - 1) / 2) / kSplitK + 1);
-      trip += (m - 1 - i) * (m - 2 - i) / 2;
-      c.n_recs++;
-      c.max_quads = std::max(c.max_quads, max_quads);
-      c.max_cols = std::max(c.max_cols, r.mlen / 32);
-      c.max_blocks = std::max(c.max_blocks, (int)blocks);
-      cp_max = std::max(cp_max, cp);
-      lists_max = std::max(lists_max, lists);
-      tiles_max = std::max(tiles_max, tiles);
-      recs.push_back(r);
     }
+  };
+  lay_out(ib, ie);
+  // What is too small for a shard grows at once to what the whole search needs, if there is room: a
+  // search's shards then reallocate once (which synchronises the device; eight shards of 4096 x 16384
+  // after five of them: 1.8 ms a shard).
+  int64_t all = 0;
+  for (const DevDataset* d : ds) all = std::max(all, d->n_snps - 2);
+  if ((ib > 0 || ie < all) &&
+      (cp_max + 8192 > ctx->sp_cp.cap || lists_max > ctx->sp_lists.cap || 8 * tiles_max > ctx->sp_tiles.cap)) {
+    lay_out(0, all);
+    cudaError_t e = ctx->sp_cp.need(cp_max + 8192);
+    if (e == cudaSuccess) e = ctx->sp_lists.need(lists_max);
+    if (e == cudaSuccess) e = ctx->sp_tiles.need(8 * tiles_max);
+    const size_t tables = sizeof(SplitRec) * recs.size() + sizeof(SplitRun) * runs.size() + 8 * chunks.size();
+    if (e == cudaSuccess) e = ctx->sp_small.need(tables + (sizeof(SplitJob) + sizeof(TcJob) + 256) * jobs.size() + 4096);
+    if (e != cudaSuccess) cudaGetLastError();
+    lay_out(ib, ie);
   }
   // uploaded: [jobs][recs][runs][jobs of the rescore][cursor, tickets of every chunk][thresholds]
   // [error word]; read back: [error word][results][rescored]
@@ -883,8 +908,9 @@ int run_split(epik2_ctx* ctx, const std::vector<DevDataset*>& ds, int64_t ib, in
     cudaFreeHost(ctx->h_small);
     ctx->h_small = nullptr;
     ctx->h_small_cap = 0;
-    CK(ctx, cudaMallocHost(&ctx->h_small, 2 * h_need), "pinned search tables");
-    ctx->h_small_cap = 2 * h_need;
+    const size_t h_new = std::max(2 * h_need, ctx->sp_small.cap);
+    CK(ctx, cudaMallocHost(&ctx->h_small, h_new), "pinned search tables");
+    ctx->h_small_cap = h_new;
   }
   unsigned char* const dev = static_cast<unsigned char*>(ctx->sp_small.p);
   for (SplitJob& J : jobs) {
