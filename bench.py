@@ -255,8 +255,11 @@ def run_ours(args, rank, world, local_rank):
     if args.overlap:
         ctx.set_overlap(args.overlap)
         tune = dict(tune, overlap=1 if args.overlap == 2 else 0)
-    engine_tc = tune["engine"] in (epik2.ENGINE_TC, epik2.ENGINE_TC_FP4)
-    engine_fp4 = tune["engine"] == epik2.ENGINE_TC_FP4
+    # the library's own choice: the genotype-split search, unless an option pins another kernel
+    split = (args.engine in ("auto", "fp4") and not (args.stage_words or args.pair_tile or args.overlap)
+             and max(info["n_cases"], info["n_samples"] - info["n_cases"]) <= 65535)
+    engine_tc = split or tune["engine"] in (epik2.ENGINE_TC, epik2.ENGINE_TC_FP4)
+    engine_fp4 = split or tune["engine"] == epik2.ENGINE_TC_FP4
     flush = torch.empty(args.flush_mb << 20, dtype=torch.uint8, device=f"cuda:{local_rank}")
 
     def shard_of(t):
@@ -318,13 +321,13 @@ def run_ours(args, rank, world, local_rank):
     value = ts_total / (elapsed_max / 1e3)
 
     # roofline of the search kernel over its own event-timed duration.  Tensor-core engine:
-    # algorithmic int8 ops = 2 x 8 multiply-accumulates (the 8 counted cells) per triplet
+    # algorithmic ops = 2 x 8 multiply-accumulates (the 8 counted cells) per triplet
     # per sample, against the measured dense int8 tcgen05 rate.  Integer engine: 8 POPC per
     # triplet per 32-sample class word, against the measured POPC rate.
     kernel_s = sum(kernel_ms) / 1e3
     achieved_popc = popc_local / kernel_s
     ref_form_popc = sum(step_trip) * words * 27 / kernel_s
-    kernel_name = ("k_scan_pipe" if tune.get("overlap") else "k_scan_tc") if engine_tc else "k_scan_int"
+    kernel_name = ("k_scan_split" if split else "k_scan_pipe" if tune.get("overlap") else "k_scan_tc") if engine_tc else "k_scan_int"
     traffic = None
     try:
         tr = json.load(open(os.path.join(ROOT, "profiles", "traffic.json")))[kernel_name]
@@ -334,14 +337,24 @@ def run_ours(args, rank, world, local_rank):
         pass
     peak_key = "tc_fp4_mac_per_s" if engine_fp4 else "tc_i8_mac_per_s"
     if engine_tc and peak_key in peaks:
-        # 8 counted cells per triplet and sample = 8 multiply-accumulates = 16 operations
-        ops = 16.0 * ts_local / kernel_s
+        # 8 counted cells per triplet and sample = 8 multiply-accumulates = 16 operations; the split
+        # search: 4 multiply-accumulates per triplet and sample whose genotype of the first SNP is
+        # not that SNP's most frequent one
+        per_ts = 16.0
+        if split:
+            rest = S - np.max([np.count_nonzero(g == v, axis=0) for v in range(3)], axis=0)
+            after = M - 1 - np.arange(M, dtype=np.float64)
+            per_i = after * (after - 1) / 2
+            done = [shard_of(t) for t in range(args.warmup, args.warmup + args.steps)]
+            per_ts = 8.0 * sum(float((per_i * rest)[a:b].sum()) for a, b in done) / (
+                S * sum(float(per_i[a:b].sum()) for a, b in done))
+        ops = per_ts * ts_local / kernel_s
         roof = {"bound": "tensor", "achieved": ops / 1e12, "peak": 2 * peaks[peak_key] / 1e12,
                 "unit": "TOPS (fp4)" if engine_fp4 else "TOPS (int8)", "frac": ops / (2 * peaks[peak_key]),
                 "peak_source": ("measured live by epik2_probe_tc_fp4 on this GPU (dense tcgen05 kind::mxf4, "
                                 "M128 N224 K64)" if engine_fp4 else
                                 "measured live by epik2_probe_tc_i8 on this GPU (dense tcgen05 kind::i8)"),
-                "algorithmic_ops_per_triplet_sample": 16}
+                "algorithmic_ops_per_triplet_sample": per_ts}
     else:
         roof = {"bound": "popc", "achieved": achieved_popc / 1e9, "peak": peaks["popc_per_s"] / 1e9,
                 "unit": "Gpopc/s", "frac": achieved_popc / peaks["popc_per_s"],
@@ -446,7 +459,8 @@ def run_ours(args, rank, world, local_rank):
                        "n_cases": info["n_cases"], "step": f"1/{parts} of the triplet space (first-index shard)",
                        "l2": f"flushed before every step ({args.flush_mb} MiB write)",
                        "parallelism": f"{world} GPU(s), shard-parallel",
-                       "engine": ("tensor cores (tcgen05 %s), %d words per stage, %d SNPs j per tile%s"
+                       "engine": "tensor cores (tcgen05 block-scaled FP4), genotype-split search" if split else
+                       ("tensor cores (tcgen05 %s), %d words per stage, %d SNPs j per tile%s"
                                   % ("block-scaled FP4" if engine_fp4 else "int8", tune["stage_words"],
                                      tune["pair_tile"], ", overlapped scoring" if tune.get("overlap") else ""))
                        if engine_tc else "integer (LOP3+POPC)",
