@@ -13,7 +13,7 @@
 //    uniform in [0.05, 0.5]); the cells of the most frequent genotype follow from the (j, k)
 //    margins by inclusion-exclusion, as the cells with genotype 2 of j or k do.  No operand holds
 //    a product of two SNPs any more: both are plain indicator rows.  The sorting itself is one
-//    pass of bit transposes per i (k_split_lists, k_split_planes), 3-5 % of a search.
+//    pass of bit transposes per i (k_split_lists, k_split_planes), 1-7 % of a search.
 // 2. A triplet's 27 cells are first put through a lower bound of K2 (screen_constants in
 //    host_data.cpp: one reciprocal per cell and a few FP32 operations, no table).  Only where the
 //    bound does not exceed the best score found so far (of the whole launch) is the score computed
@@ -22,7 +22,8 @@
 //
 // Warp roles of a CTA (512 threads), concurrent from tile to tile:
 //   warps 0-5   produce: expand the compacted bit planes into the operand ring (warps 0-3 the 64
-//               SNPs k of this CTA, 4-5 its 28 SNPs j), 256 samples per stage, 4 stages
+//               SNPs k of this CTA, 4-5 its 28 SNPs j), a quad of 128 samples per stage, 8 stages; half of
+//               them take the even, half the odd stages
 //   warp 6      fences the stored stages and issues the products (even CTA)
 //   warp 7      schedules: takes tiles from the queue, publishes descriptor, record and job
 //   warps 8-15  score: copy a tile's four accumulators out of tensor memory into a 16-bit staging
@@ -31,18 +32,22 @@
 // Classes of at most 65535 samples (the 16-bit halves).
 //
 // What bounds it: the scoring warps (about 330 instructions per 32 triplets, 27 more where the classes
-// are not even: screen_constants) up to about 8192
-// samples; from there on also the round trip of a ring stage (stores, fence and arrival in the even
-// CTA, products, commit).  Cost of the parts of that round trip, which set the roles and hand-offs
-// (clocks, measured alone): a commit of four products 560; an arrival in the other CTA 133, and
-// 447 with a cluster-scope release; issuing four products and their commit 330 from a converged
-// warp, 610 from a lane-0 branch.  An eighth of 4096 x 16384 took 45.3 ms with the words of the next
-// four stages in registers and each producing warp fencing its stores (the fence waits for loads in
-// flight), 42.5 with the fence in the issuing warp, 38.8 with cp.async.
-// Measured against k_scan_tc on CTA pairs (kernel time of a whole search): 1024 x 8192 14.1 -> 4.6
-// ms, 3072 x 4096 265 -> 91 ms, 2048 x 8192 103 -> 31.2 ms, an eighth of 4096 x 16384 144 -> 38.8 ms.
+// are not even: screen_constants) up to about 8192 samples: the loop alone takes 340 clocks per
+// scheduler and 32 triplets, in the kernel 430 to 530, for the producing warps issue beside it.  From
+// there on also the round trip of a ring stage (stores, fence and arrival in the even CTA, products,
+// commit).  Cost of the parts of that round trip, which set the roles and hand-offs (clocks, measured
+// alone): a commit of four products 560; an arrival in the other CTA 133, and 447 with a cluster-scope
+// release; issuing four products and their commit 330 from a converged warp, 610 from a lane-0 branch;
+// a wait on a barrier that is complete 111, which passes during the issue of the stage before.
+// An eighth of 4096 x 16384 took 45.3 ms with the words of the next four stages in registers and each
+// producing warp fencing its stores (the fence waits for loads in flight), 42.5 with the fence in the
+// issuing warp, 38.8 with cp.async, 36.0 with stages of two quads whose words were loaded a stage ahead,
+// 33.2 so.  (One commit per two quads: +1.3 ms; seven stages and three raw slots: +2.8 ms.)
+// Measured against k_scan_tc on CTA pairs (kernel time of a whole search): 1024 x 8192 14.1 -> 4.07
+// ms, 3072 x 4096 265 -> 82.9 ms, 2048 x 8192 103 -> 27.9 ms, an eighth of 4096 x 16384 144 -> 33.2 ms.
 //
 // Every mbarrier wait is bounded; on expiry the kernel sets an error word and ends.
+#include <atomic>
 #include <cfloat>
 
 #include "epik2_internal.h"
@@ -838,7 +843,7 @@ __global__ void __launch_bounds__(kSThreads, 1) k_scan_split(const SplitParams p
     }
   } else if (warp >= kSFirstScore) {
     // ================= scoring warps =================
-    // Warp (c, kh, part): drains rows c of the SNPs k 32kh.. and columns of a third of the SNPs
+    // Warp (c, kh, part): drains rows c of the SNPs k 32kh.. and columns of half of the SNPs
     // j; the pair of warps with the same (kh, part) shares its part of the staging buffer and its margins
     // and nothing else, so the pairs go from tile to tile by themselves (less than a tile apart).
     const int sw = warp - kSFirstScore;
@@ -1150,14 +1155,18 @@ static cudaError_t split_set_smem() {
 }
 
 cudaError_t split_configure() {
-  static bool configured = false;
-  if (configured) return cudaSuccess;
-  cudaError_t e = split_set_smem<false, false, false>();
+  static std::atomic<uint64_t> configured{0};  // bit per device: the attribute belongs to one
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  const uint64_t bit = dev < 64 ? 1ull << dev : 0;
+  if (configured.load() & bit) return cudaSuccess;
+  e = split_set_smem<false, false, false>();
   if (e == cudaSuccess) e = split_set_smem<false, false, true>();
   if (e == cudaSuccess) e = split_set_smem<true, false, false>();
   if (e == cudaSuccess) e = split_set_smem<false, true, false>();
   if (e == cudaSuccess) e = split_set_smem<false, true, true>();
-  if (e == cudaSuccess) configured = true;
+  if (e == cudaSuccess) configured |= bit;
   return e;
 }
 

@@ -7,8 +7,7 @@
 // behind a large one); create each admitted scan's dataset (a replicate sharing a
 // resident genotype matrix, or a freshly uploaded matrix); run one batched launch over
 // all of them (epik2_scan_batch) -- except that three or more replicates of one resident matrix
-// admitted together run in the replicate form (epik2_scan_replicates: each tile's all-sample
-// counts shared by them); release the datasets; and complete the requests whose scans are
+// admitted together run in the replicate form (epik2_scan_replicates); release the datasets; and complete the requests whose scans are
 // all done.  Requests that arrive during a launch join the next admission
 // round.  Submitting never waits for the device: it copies the request and queues it.
 #include <algorithm>
@@ -169,9 +168,9 @@ struct epik2_server {
         std::this_thread::sleep_for(std::chrono::microseconds(100));
       {
         std::lock_guard<std::mutex> g(ctx_mu);
-        // replicate scans of one resident matrix run in the replicate form (each tile's
-        // all-sample counts shared by the replicates) when this launch holds three or more of
-        // them: below that the all-sample pass costs about what it saves
+        // replicate scans of one resident matrix run in the replicate form when this launch holds
+        // three or more of them: where that form shares the all-sample counts (classes of more than
+        // 65535 samples) fewer replicates cost about what it saves
         std::map<int32_t, std::vector<size_t>> by_matrix;
         for (size_t b = 0; b < batch.size(); b++)
           if (batch[b].req->dataset >= 0) by_matrix[batch[b].req->dataset].push_back(b);

@@ -98,7 +98,10 @@ int epik2_device_name(const epik2_ctx *ctx, char *buf, size_t len);
 int epik2_mem_info(const epik2_ctx *ctx, size_t *free_bytes, size_t *total_bytes);
 
 /* Default search engine of the context (EPIK2_ENGINE_*).  All engines give identical
- * tables, scores and triplets; AUTO takes the autotuner's choice for the dataset's shape. */
+ * tables, scores and triplets.  AUTO, and FP4 with no tuning option given, take the genotype-split
+ * FP4 search where both classes have at most 65535 samples (for each first SNP only the samples of its
+ * two rarer genotypes are counted); beyond, AUTO takes the autotuner's choice for the dataset's
+ * shape. */
 #define EPIK2_ENGINE_AUTO 0
 #define EPIK2_ENGINE_INT 1 /* integer pipe: 8 LOP3+POPC per triplet and 32-sample word */
 #define EPIK2_ENGINE_TC 2  /* tcgen05 int8 matrix products on 0/1 operands, int32 accumulators */
@@ -222,7 +225,8 @@ int epik2_scan_u8(epik2_ctx *ctx, const uint8_t *geno, const uint8_t *pheno, int
                   int64_t n_snps, const epik2_opts *opts, epik2_best *out);
 
 /* --------------------------------------------------------------------------------
- * Batched form (no reference counterpart).  One persistent tensor-core launch over many
+ * Batched form (no reference counterpart).  With no tuning option given and every class of at most
+ * 65535 samples: one genotype-split search over all the datasets.  Otherwise one persistent tensor-core launch over many
  * resident datasets: the triplet tiles of all of them go on one shared queue (datasets with
  * the most samples first), each CTA folds its candidates into per-dataset slots, and a
  * per-dataset reduction writes out[0..n).  The launch sequence is captured once per set of
@@ -240,7 +244,9 @@ int epik2_scan_batch(epik2_ctx *ctx, const int32_t *dataset_ids, int32_t n, cons
  * tensor cores): the best triplet of each of n_reps phenotype-permutation replicates of a
  * resident dataset (phenos: n_reps x n_samples bytes, 1 = case).  Each tile of the search
  * counts the all-sample contingency cells of the base matrix once, then for every replicate
- * only its cases; its controls are the totals minus its cases.  Runs the FP4 CTA-pair kernel
+ * only its cases; its controls are the totals minus its cases (where every class has at most 65535
+ * samples, the replicates are instead the datasets of one genotype-split search, which counts less
+ * still).  Runs the FP4 CTA-pair kernel
  * (EPIK2_E_TOO_LARGE for classes of 2^24 samples or more), as many replicates per launch as
  * free device memory allows (at most 256).  out[r] equals epik2_scan of the dataset with
  * phenotype r; with opts->rescore_fp64, out[r].score_fp64 is its best triplet rescored in FP64
@@ -255,7 +261,8 @@ int epik2_scan_replicates(epik2_ctx *ctx, int32_t dataset_id, const uint8_t *phe
  * stage, each with a pair tile of 32 SNPs j (one CTA) and of 64 (a cluster of two CTAs), and
  * the overlapped FP4 CTA-pair kernel at 4 and 8 words per stage (classes <= 65535 samples).
  * Caches the fastest per shape bucket (log2 of samples and SNPs); EPIK2_ENGINE_AUTO scans and
- * the batched form use the cached rates.  Reports the choice and the measured rates
+ * the batched form use the cached rates where the genotype-split search, which is not among them, does
+ * not apply.  Reports the choice and the measured rates
  * (triplet*samples/s; 0 = not a candidate).  The k-strip (SNPs k per tile: 128 int8, 112
  * FP4) is fixed by the tensor-memory budget: both classes' accumulators and the scale
  * factors fill 480 of the 512 columns. */
