@@ -42,9 +42,9 @@
 // An eighth of 4096 x 16384 took 45.3 ms with the words of the next four stages in registers and each
 // producing warp fencing its stores (the fence waits for loads in flight), 42.5 with the fence in the
 // issuing warp, 38.8 with cp.async, 36.0 with stages of two quads whose words were loaded a stage ahead,
-// 33.2 so.  (One commit per two quads: +1.3 ms; seven stages and three raw slots: +2.8 ms.)
-// Measured against k_scan_tc on CTA pairs (kernel time of a whole search): 1024 x 8192 14.1 -> 4.07
-// ms, 3072 x 4096 265 -> 82.9 ms, 2048 x 8192 103 -> 27.9 ms, an eighth of 4096 x 16384 144 -> 33.2 ms.
+// 33.2 with stages of one quad, 32.1 with the accumulators copied eight SNPs j per wait.  (One commit per two quads: +1.3 ms; seven stages and three raw slots: +2.8 ms.)
+// Measured against k_scan_tc on CTA pairs (kernel time of a whole search): 1024 x 8192 14.1 -> 3.90
+// ms, 3072 x 4096 265 -> 79.1 ms, 2048 x 8192 103 -> 26.9 ms, an eighth of 4096 x 16384 144 -> 32.1 ms.
 //
 // Every mbarrier wait is bounded; on expiry the kernel sets an error word and ends.
 #include <atomic>

@@ -226,8 +226,8 @@ int epik2_scan_u8(epik2_ctx *ctx, const uint8_t *geno, const uint8_t *pheno, int
 
 /* --------------------------------------------------------------------------------
  * Batched form (no reference counterpart).  With no tuning option given and every class of at most
- * 65535 samples: one genotype-split search over all the datasets.  Otherwise one persistent tensor-core launch over many
- * resident datasets: the triplet tiles of all of them go on one shared queue (datasets with
+ * 65535 samples: one genotype-split search over all the datasets.  Otherwise one persistent
+ * tensor-core launch over many resident datasets: the triplet tiles of all of them go on one shared queue (datasets with
  * the most samples first), each CTA folds its candidates into per-dataset slots, and a
  * per-dataset reduction writes out[0..n).  The launch sequence is captured once per set of
  * dataset shapes into a CUDA graph and replayed (phenotype re-encodings via epik2_set_pheno
