@@ -1783,7 +1783,7 @@ int epik2_scan_batch(epik2_ctx* ctx, const int32_t* dataset_ids, int32_t n, cons
   if (ov_req == 2 && !all_overlap)
     return fail(ctx, EPIK2_E_TOO_LARGE, "overlapped kernel: classes of at most 65535 samples");
   // Nothing pinned beyond the format and every class within the split search's cells: one split
-  // search over all the datasets (16 datasets of 128-1536 SNPs: 32.9 against 84.5 ms).
+  // search over all the datasets (16 datasets of 128-1536 SNPs: 32.4 against 84.6 ms).
   bool all_split = true;
   for (DevDataset* d : ds) all_split = all_split && split_fits(*d);
   if (engine_req != EPIK2_ENGINE_TC && kw_req == 0 && pt_req == 0 && ov_req == 0 && all_split) {
@@ -1973,7 +1973,7 @@ int epik2_scan_replicates(epik2_ctx* ctx, int32_t dataset_id, const uint8_t* phe
     encode_ms += std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t_enc).count();
     // Each replicate as a dataset of one split search, wherever their classes fit its cells: counting
     // only the rarer genotypes of i saves more than sharing the all-sample counts (8 replicates of
-    // 1024 x 8192: 33.5 against 100.4 ms), which remains the form for larger classes.
+    // 1024 x 8192: 32.4 against 100.7 ms), which remains the form for larger classes.
     bool all_split = true;
     for (int32_t t = 0; t < g; t++) all_split = all_split && split_fits(reps[(size_t)t]);
     if (all_split) {
