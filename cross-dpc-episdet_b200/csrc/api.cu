@@ -1439,6 +1439,14 @@ int epik2_test_withhold_arrival(epik2_ctx* ctx) {
   return EPIK2_OK;
 }
 
+int epik2_test_screen_bound(int64_t n_controls, int64_t n_cases, const uint32_t* tables, int64_t n, float* bounds) {
+  if (n_controls < 0 || n_cases < 0 || n_controls > 65535 || n_cases > 65535 || n_controls + n_cases < 1 || n < 0 ||
+      (n > 0 && (!tables || !bounds)))
+    return EPIK2_E_INVALID;
+  for (int64_t t = 0; t < n; t++) bounds[t] = screen_bound(n_controls, n_cases, tables + 54 * t);
+  return EPIK2_OK;
+}
+
 int epik2_set_overlap(epik2_ctx* ctx, int overlap) {
   if (!ctx) return EPIK2_E_INVALID;
   if (overlap < 0 || overlap > 2) return fail(ctx, EPIK2_E_INVALID, "overlap must be 0, 1 or 2");

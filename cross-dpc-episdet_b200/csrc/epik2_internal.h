@@ -148,6 +148,12 @@ constexpr int kSplitK = 128;   // SNPs k per tile (64 per CTA of the pair)
 constexpr int kSplitJ = 56;    // SNPs j per tile
 constexpr int kSplitSlots = 3; // tiles in flight per CTA pair: scored, in tensor memory, produced
 
+// The screening bound (screen_constants): the logarithm of a cell is taken at N + kScreenShift;
+// kScreenLog is half of ln 2 in units of 2^-23, not above it.
+constexpr float kScreenShift = 7.0f / 16.0f;
+constexpr float kScreenLog = 0x1.62e42ep-25f;
+static_assert((double)kScreenLog * 8388608.0 <= 0.34657359027997264 && (double)kScreenLog * 8388608.0 > 0.3465735,
+              "half of ln 2, rounded down");
 // Constants of the screening bound for a class split (screen_constants).
 struct ScreenConsts {
   uint32_t coef;           // bytes (64 - kp, -kp): 64 D = (64 - kp) a - kp b + bias
@@ -275,6 +281,7 @@ int tc_warps_per_block();
 
 // Host helpers (host_data.cpp).
 ScreenConsts screen_constants(int64_t n0, int64_t n1);
+float screen_bound(int64_t n0, int64_t n1, const uint32_t* table);  // of a 54-count table, as k_scan_split takes it
 void build_k2_lut(int64_t n_max, float* lut);
 void build_k2_lut_range(int64_t n_begin, int64_t n_end, float* out);  // out[n - n_begin], n in [begin, end)
 void build_k2_lut64(int64_t n_max, double* lut);

@@ -6,6 +6,7 @@
 #include <cmath>
 #include <cstdint>
 #include <cstdlib>
+#include <cstring>
 #include <random>
 #include <vector>
 
@@ -41,21 +42,27 @@ void build_k2_lut(int64_t n_max, float* lut) { build_k2_lut_range(0, n_max + 1, 
 
 // Screening bound of the split search.  With A = a + 1/2, N = a + b + 1 for a cell of a controls
 // and b cases, p in (0, 1), q = 1 - p, D = A - p N and d = D / N:
-//   ln (a+b+1)! - ln a! - ln b!  >=  -A ln p - (N - A) ln q + ln(N)/2 - ln(2 pi)/2 + K/N - N KL(p + d || p)
-// with K = 0.22 (Stirling at half-integers; the smallest slack times N over all a, b is 0.2258, at
+//   ln (a+b+1)! - ln a! - ln b!  =  -A ln p - (N - A) ln q + ln(N)/2 - ln(2 pi)/2 - N KL(p + d || p) + S
+// with S about 1/(12 N) + 1/(24 A) + 1/(24 (N - A)) (Stirling at half-integers; S N is least, 0.2258, at
 // a = b = 0).  KL / d^2 is c2 = 1 / (2 p q) at d = 0 and known at both ends, d = q and d = -p; its
 // inverse is concave on either side, so it lies above the chords:
-//   KL(p + d || p)  <=  c2 d^2 / (1 - t1 d - t2 |d|).
-// And with P = N - t1 D:  ln(N)/2 = ln(P)/2 - ln(1 - t1 d)/2, where
-//   -ln(1 - t1 d)/2  >=  -|t1 d|/2  >=  -K/N - N d^2 t1^2 / (16 K)
-// takes up K/N, so that per cell   ln(P)/2 - (c2 + t1^2 / (16 K)) D^2 / (P - t2 |D|)   remains; log2
-// P is taken from P's FP32 bits (linear between powers of two, never above).  Summed over the 27
+//   N KL(p + d || p)  <=  c2 D^2 / (N - t1 D - t2 |D|).
+// The cell's bound takes both at M = N + 7/16 instead of N, which costs nothing:
+//   -A ln p - (N - A) ln q + ln(M)/2 - ln(2 pi)/2 - c2 D^2 / (M - t1 D - t2 |D|),
+// log2 M from M's FP32 bits (linear between powers of two, never above).  What M adds, at most 7/(32 N)
+// to the logarithm and a share 7/(16 M) of the quotient, is less than S, what the chord leaves and what
+// the linear logarithm leaves together: the least slack, times N, is 0.019 over every p = kp/64 with all
+// a, b < 5000, and positive on grids, edges, the ridge a = p N and around powers of two up to 65535 (M = N
+// + 1/2 fails at (0, 1) for p near 1/4).  A table of rare alleles is mostly empty cells, each of which
+// loses S = 0.2258 at M = N: 1000 samples, minor-allele frequencies 0.001 to 0.005: 1.5 below the score
+// instead of 5.6 (512 SNPs x 2000 samples, 5 % cases, frequencies 0.005 to 0.02: 1.97 -> 0.60 ms with
+// it and without a term t1^2 / 3.5 beside c2 that the logarithm of N - t1 D costs).  Summed over the 27
 // cells this bounds the K2 score from below, for any p: kp/64 next to the share of controls, which
 // makes 64 D an integer.  base = the terms that are the same for every triplet, less a margin for
-// rounding: of the reference's FP32 table and sums (about 5 ulp of ln n!, 0.1 for the table below
-// 748) and of the FP32 evaluation of the bound.
+// rounding: of the reference's FP32 table and sums (about 5 ulp of ln n!, 0.1 for the table below 748)
+// and of the FP32 evaluation of the bound.
 ScreenConsts screen_constants(int64_t n0, int64_t n1) {
-  const double n = (double)(n0 + n1), kK = 0.22;
+  const double n = (double)(n0 + n1);
   int kp = (int)std::min(63.0, std::max(1.0, std::floor(64.0 * ((double)n0 + 13.5) / (n + 27.0) + 0.5)));
   // Nearly even classes take p = 1/2, where t1 = 0 and a cell costs an operation less (3072 x 4096: 84.9
   // ms, with the operation 91.0, before the loop's later changes).  At a distance x of the controls' share from 1/2 the bound loses about
@@ -72,12 +79,29 @@ ScreenConsts screen_constants(int64_t n0, int64_t n1) {
   s.bias = 32 - kp;
   s.theta1 = (float)(t1 / 64.0);
   s.theta2 = (float)(t2 * 1.000001 / 64.0);
-  s.c = (float)((c2 + t1 * t1 / (16.0 * kK)) * 1.000001 / (64.0 * 64.0));
+  s.c = (float)(c2 * 1.000001 / (64.0 * 64.0));
   const double margin = 0.3 + 1e-6 * std::lgamma(n + 2.0);
   s.margin = (float)margin;
   s.base = (float)(-((double)n0 + 13.5) * std::log(p) - ((double)n1 + 13.5) * std::log(q) -
                    13.5 * std::log(2.0 * 3.14159265358979323846) - margin);
   return s;
+}
+
+float screen_bound(int64_t n0, int64_t n1, const uint32_t* table) {
+  const ScreenConsts s = screen_constants(n0, n1);
+  const int ka = (int8_t)(s.coef & 0xFF), kb = (int8_t)(s.coef >> 8);
+  float acc = 0.0f;
+  uint32_t bits = 0;
+  for (int x = 0; x < 27; x++) {
+    const int a = (int)table[x], b = (int)table[27 + x];
+    const float D = (float)(ka * a + kb * b + s.bias), M = (float)(a + b + 1) + kScreenShift;
+    uint32_t m;
+    std::memcpy(&m, &M, 4);
+    bits += m;
+    const float P = s.theta1 == 0.0f ? M : std::fma(D, -s.theta1, M);
+    acc = std::fma(D * (1.0f / std::fma(std::fabs(D), -s.theta2, P)), D, acc);
+  }
+  return std::fma(kScreenLog, (float)(bits - 27u * 0x3F800000u), -s.c * acc) + s.base;
 }
 
 // The same ln n! evaluated entirely in double (precision form's FP64 rescore): the table

@@ -17,8 +17,8 @@
 // 2. A triplet's 27 cells are first put through a lower bound of K2 (screen_constants in
 //    host_data.cpp: one reciprocal per cell and a few FP32 operations, no table).  Only where the
 //    bound does not exceed the best score found so far (of the whole launch) is the score computed
-//    in the reference's arithmetic.  The bound is below the score by 2 to 4 on average; 0.002 % to
-//    0.04 % of the warps' steps go on to the score.
+//    in the reference's arithmetic.  The bound is below the score by 1 to 2 on average for common
+//    alleles and classes of at least a twentieth of the samples, by 5 to 6 for alleles of 0.5 to 5 %.
 //
 // Warp roles of a CTA (512 threads), concurrent from tile to tile:
 //   warps 0-5   produce: expand the compacted bit planes into the operand ring (warps 0-3 the 64
@@ -471,12 +471,14 @@ __device__ __forceinline__ int dot2(uint32_t w, uint32_t coef, int c) {
 }
 
 // The two linear forms of a cell (a controls, b cases) that the screening bound needs, as the bits of
-// FP32 numbers: n = 2^23 + N with N = a + b + 1, and d = 1.5 * 2^23 + 64 D with 64 D = 64 (a + 1/2) -
-// kp N.  The integers 64 D stay below 2^22 for 16-bit counts, so adding and subtracting the bits adds
-// and subtracts the numbers, and one FP32 subtraction converts (an integer conversion takes twice
-// the pipe time).  A margin over x cells holds the sums of its cells' bits modulo 2^32, so that cells
-// complete by integer subtraction.
-constexpr uint32_t kBitsN = 0x4B000000u, kBitsD = 0x4B400000u;
+// FP32 numbers: n = 2^20 + N with N = a + b + 1 (a step of the bits is 1/8), and d = 1.5 * 2^23 + 64 D
+// with 64 D = 64 (a + 1/2) - kp N.  N stays below 2^18 and 64 D below 2^22 for 16-bit counts, so adding
+// and subtracting the bits adds and subtracts the numbers, and one FP32 subtraction converts (an integer
+// conversion takes twice the pipe time); that of n leaves N + 7/16, the number the bound wants, whose
+// sixteenths 2^20 - 7/16 can hold.  A margin over x cells holds the sums of its cells' bits modulo 2^32,
+// so that cells complete by integer subtraction.
+constexpr uint32_t kBitsN = 0x49800000u, kBitsD = 0x4B400000u;
+constexpr float kLessN = 1048576.0f - kScreenShift;
 struct Form {
   uint32_t n, d;
 };
@@ -485,7 +487,7 @@ struct FormOf {  // counts (class 0 low half, class 1 high half) of a sum over `
   uint32_t coef;   // bytes (64 - kp, -kp)
   int bias;        // 32 - kp
   __device__ __forceinline__ Form operator()(uint32_t w, int cells) const {
-    return Form{(uint32_t)dot2(w, 0x0101u, (int)((kBitsN + 1u) * (uint32_t)cells)),
+    return Form{(uint32_t)dot2(w, 0x0808u, (int)((kBitsN + 8u) * (uint32_t)cells)),
                 (uint32_t)dot2(w, coef, (int)((kBitsD + (uint32_t)bias) * (uint32_t)cells))};
   }
 };
@@ -496,21 +498,21 @@ template <bool kEven>
 struct Screen {
   float theta1, theta2;  // of 64 D
   float acc;
-  uint32_t bits;         // sum of the cells' log2 (N - theta1 D), from below, in units of 2^-23
+  uint32_t bits;         // sum of the cells' log2 (N + 7/16), from below, in units of 2^-23
   template <int kN>
   __device__ __forceinline__ void cells(const Form (&f)[kN]) {
-    float D[kN], P[kN], r[kN];
+    float D[kN], M[kN], P[kN], r[kN];
 #pragma unroll
     for (int x = 0; x < kN; x++) {
       D[x] = __uint_as_float(f[x].d) - 12582912.0f;
-      const float N = __uint_as_float(f[x].n) - 8388608.0f;
-      P[x] = kEven ? N : fmaf(D[x], -theta1, N);
+      M[x] = __uint_as_float(f[x].n) - kLessN;
+      P[x] = kEven ? M[x] : fmaf(D[x], -theta1, M[x]);
     }
 #pragma unroll
     for (int x = 0; x < kN; x++) r[x] = rcp_approx(fmaf(fabsf(D[x]), -theta2, P[x]));
 #pragma unroll
-    for (int x = 0; x + 1 < kN; x += 2) bits += __float_as_uint(P[x]) + __float_as_uint(P[x + 1]);
-    if (kN & 1) bits += __float_as_uint(P[kN - 1]);
+    for (int x = 0; x + 1 < kN; x += 2) bits += __float_as_uint(M[x]) + __float_as_uint(M[x + 1]);
+    if (kN & 1) bits += __float_as_uint(M[kN - 1]);
 #pragma unroll
     for (int x = 0; x < kN; x++) acc = fmaf(D[x] * r[x], D[x], acc);
   }
@@ -1079,9 +1081,9 @@ __global__ void __launch_bounds__(kSThreads, 1) k_scan_split(const SplitParams p
             r2[7] = kC1 - r0[7] - r1[7];
             row_forms(ijA, ijB, ijC, r2);
             scr.cells(r2);
-            // sum of logs: bits - 27 * 127 * 2^23 (modulo 2^32) in units of 2^-23 / log2 e * 2
+            // sum of logs: bits - 27 * 127 * 2^23 (modulo 2^32) in units of 2^-23 log2, half of it in ln
             const float lg = __uint2float_rn(scr.bits - 27u * 0x3F800000u);
-            const float low = fmaf(4.1315582e-8f, lg, coef * scr.acc);
+            const float low = fmaf(kScreenLog, lg, coef * scr.acc);
             want = valid && !(low >= limit);  // not a number: take the exact path
           }
           if (!__any_sync(kFull, want)) continue;

@@ -154,6 +154,7 @@ def library():
         "epik2_set_pair_tile": ([p, ctypes.c_int], ctypes.c_int),
         "epik2_set_overlap": ([p, ctypes.c_int], ctypes.c_int),
         "epik2_test_withhold_arrival": ([p], ctypes.c_int),
+        "epik2_test_screen_bound": ([i64, i64, p, i64, p], ctypes.c_int),
         "epik2_plink_dims": ([ctypes.c_char_p, ctypes.POINTER(ctypes.c_int64), ctypes.POINTER(ctypes.c_int64)],
                              ctypes.c_int),
         "epik2_read_plink": ([ctypes.c_char_p, ctypes.c_uint8, p, p], ctypes.c_int),

@@ -136,6 +136,10 @@ int epik2_set_wait_limit(epik2_ctx *ctx, int64_t sm_clocks);
  * before any matrix product is issued and the search returns EPIK2_E_TIMEOUT.  One-shot:
  * the search after it runs normally. */
 int epik2_test_withhold_arrival(epik2_ctx *ctx);
+/* Test hook (host only): the lower bound of K2 by which the genotype-split search leaves out
+ * triplets, for n tables of 54 counts (27 of controls, 27 of cases) of a dataset with n_controls
+ * and n_cases samples (at most 65535 each), in the FP32 arithmetic of the search. */
+int epik2_test_screen_bound(int64_t n_controls, int64_t n_cases, const uint32_t *tables, int64_t n, float *bounds);
 
 /* Counters kept by the context (no reference counterpart: the reference's only
  * instrument is a TSC timer around its launch loop, GPU/v4.cpp:282, 609). */
