@@ -62,7 +62,8 @@ struct epik2_ctx {
   int scan_blocks = 0;          // integer engine grid
   int tc_blocks = 0;            // tensor-core engine grid (one CTA per SM)
   int n_slots = 0;              // per-warp slots, enough for either grid
-  int* d_err = nullptr;
+  int* d_err = nullptr;         // error word; sum of the flat SNPs of every dataset encoded
+  int flat_seen = 0;            // that sum as last read
   int64_t wait_limit = 0;       // SM clocks of a bounded device-side wait (0 = kernel default)
   int test_withhold = 0;        // one-shot test hook of the bounded-wait error path
   int64_t* d_pb_off = nullptr;
@@ -395,6 +396,7 @@ int run_scan(epik2_ctx* ctx, DevDataset& d, const epik2_opts* opts, uint32_t* du
              BestSlot* best_out);
 constexpr int kSplitNoRoom = 1;  // run_split: the workspace does not fit (the caller takes the other kernels)
 bool split_fits(const DevDataset& d);
+bool split_screens(const std::vector<DevDataset*>& ds, int top_k = 0);
 int run_split(epik2_ctx* ctx, const std::vector<DevDataset*>& ds, int64_t ib, int64_t ie, int top_k,
               uint32_t* dump_tables, float* dump_scores, BestSlot* best_out, Rescored* resc_out = nullptr,
               int* n_cand_out = nullptr);
@@ -429,9 +431,10 @@ int run_scan(epik2_ctx* ctx, DevDataset& d, const epik2_opts* opts, uint32_t* du
   const bool can_overlap = fp4_exact(d) && pipe_fits(d.n_controls, d.n_cases);
   if (ov == 2 && !can_overlap)
     return fail(ctx, EPIK2_E_TOO_LARGE, "overlapped kernel: classes of at most 65535 samples");
-  // Nothing pinned beyond the format: the genotype-split kernel wherever its 16-bit cells hold
-  // (it is the fastest at every shape measured); the other kernels for larger classes.
-  if ((engine == 0 || engine == 3) && kw == 0 && pt == 0 && ov == 0 && split_fits(d)) {
+  // Nothing pinned beyond the format: the genotype-split kernel wherever its 16-bit cells hold and its
+  // screen keeps something back (a dump scores every triplet anyway); else the other kernels.
+  if ((engine == 0 || engine == 3) && kw == 0 && pt == 0 && ov == 0 && split_fits(d) &&
+      (dump_tables || split_screens({&d}, top_k))) {
     int n_cand = 0;
     const int r = run_split(ctx, {&d}, ib, ie, top_k, dump_tables, dump_scores, best_out, nullptr, &n_cand);
     if (r != kSplitNoRoom) {
@@ -575,7 +578,7 @@ int run_pairs_tc(epik2_ctx* ctx, DevDataset& d) {
   for (int64_t j0 = 0; j0 <= m_pad - 2; j0 += 64) n_tiles += tiles_of_pair_block(j0, m_pad, kk);
   int r = ensure_tiles(ctx, std::max<int64_t>(n_tiles, 1));
   if (r) return r;
-  CK(ctx, launch_pair_tiles(m_pad, ctx->d_tiles, ctx->d_counter, ctx->d_err, ctx->stream), "pair-margin tiles");
+  CK(ctx, launch_pair_tiles(d, ctx->d_tiles, ctx->d_counter, ctx->d_err, ctx->stream), "pair-margin tiles");
   TcParams p{};
   p.planes = d.planes;
   p.singles = d.singles;
@@ -597,10 +600,12 @@ int run_pairs_tc(epik2_ctx* ctx, DevDataset& d) {
   p.pairs_out = d.pairs;
   CK(ctx, launch_pairs_tc(p, tc_pair_blocks(ctx->tc_blocks), ctx->stream), "pair-margin kernel");
   ctx->stats.kernel_launches += 2;
-  int err_word = 0;
-  CK(ctx, cudaMemcpyAsync(&err_word, ctx->d_err, 4, cudaMemcpyDeviceToHost, ctx->stream), "read error word");
+  int back[2] = {0, 0};
+  CK(ctx, cudaMemcpyAsync(back, ctx->d_err, 8, cudaMemcpyDeviceToHost, ctx->stream), "read error word");
   CK(ctx, cudaStreamSynchronize(ctx->stream), "encode");
-  if (err_word) return fail(ctx, EPIK2_E_TIMEOUT, "pair margins: a bounded wait expired");
+  d.flat = std::min<int64_t>((unsigned)back[1] - (unsigned)ctx->flat_seen, d.n_snps);
+  ctx->flat_seen = back[1];
+  if (back[0]) return fail(ctx, EPIK2_E_TIMEOUT, "pair margins: a bounded wait expired");
   return EPIK2_OK;
 }
 
@@ -735,6 +740,28 @@ int64_t triplets_before(int64_t m, int64_t ie) {
 
 // Its cells are 16-bit halves of a word: classes of at most 65535 samples.
 bool split_fits(const DevDataset& d) { return d.n_snps >= 3 && d.n_controls <= 65535 && d.n_cases <= 65535; }
+
+// Whether the screen keeps most triplets from being scored.  No bound can between equal scores, and a scored
+// step costs four times a screened one, twice a step of the other kernels at 1000 samples.  Equal scores
+// come with SNPs that are constant or nearly so (at most kFlatRest samples off the most frequent
+// genotype): the split search can be slower where more than about half of the SNPs are such (1024 SNPs x
+// 1000 samples all constant: 11.2 against 6.1 ms, half of them 3.2 against 6.5; 512 x 500 at frequencies of
+// 0.0005 to 0.001, 96 % flat, 1.03 against 0.84, at 0.001 to 0.005, 46 % flat, 0.55), and less often the
+// longer the counting of all samples takes the other kernels: never from 8000 samples on (512 x
+// 8192 all constant: 1.73 against 1.89 ms).  Of several datasets those decide that hold most triplets.  The
+// 32 best of up to 6e7 triplets are found sooner by it all the same, since the other kernels' lists of
+// every warp take the host 2 to 4 ms (512 SNPs x 500 samples all constant: 3.1 against 3.4 ms, 1024
+// x 1000 13.1 against 9.2).
+bool split_screens(const std::vector<DevDataset*>& ds, int top_k) {
+  double flat = 0.0, all = 0.0;
+  for (const DevDataset* d : ds) {
+    const double m = (double)d->n_snps, s = (double)d->n_samples;
+    all += m * m * m;
+    if (top_k > 1 && m * m * m < 3.6e8) continue;
+    if (s < 8000.0 && (double)d->flat > (0.5 + 0.04e-3 * s) * m) flat += m * m * m;
+  }
+  return 2.0 * flat <= all;
+}
 
 // Compacted planes of the first SNPs searched per launch: launches of the large workload then last 8
 // ms or more, and their ends (one tile, about 10 us) stay below 0.3 %.  Most searches take one launch:
@@ -1344,7 +1371,7 @@ int epik2_create(epik2_ctx** out, int device) {
   ctx->tc_blocks = ctx->prop.multiProcessorCount;
   const int n_warps = std::max(ctx->scan_blocks * (kScanThreads / 32), ctx->tc_blocks * tc_warps_per_block());
   ctx->n_slots = n_warps;
-  if (cudaMalloc(&ctx->d_counter, 64) != cudaSuccess || cudaMalloc(&ctx->d_err, 64) != cudaSuccess || cudaMalloc(&ctx->d_slots, sizeof(BestSlot) * n_warps) ||
+  if (cudaMalloc(&ctx->d_counter, 64) != cudaSuccess || cudaMalloc(&ctx->d_err, 64) != cudaSuccess || cudaMemset(ctx->d_err, 0, 64) != cudaSuccess || cudaMalloc(&ctx->d_slots, sizeof(BestSlot) * n_warps) ||
       cudaMalloc(&ctx->d_best, sizeof(BestSlot)) || cudaMalloc(&ctx->d_cand, sizeof(BestSlot) * n_warps * 32) ||
       cudaMalloc(&ctx->d_resc, sizeof(Rescored) * n_warps * 32) ||
       cudaMallocHost(&ctx->h_best, sizeof(BestSlot))) {
@@ -1794,6 +1821,7 @@ int epik2_scan_batch(epik2_ctx* ctx, const int32_t* dataset_ids, int32_t n, cons
   // search over all the datasets (16 datasets of 128-1536 SNPs: 32.4 against 84.6 ms).
   bool all_split = true;
   for (DevDataset* d : ds) all_split = all_split && split_fits(*d);
+  all_split = all_split && split_screens(ds);
   if (engine_req != EPIK2_ENGINE_TC && kw_req == 0 && pt_req == 0 && ov_req == 0 && all_split) {
     const bool rescore = opts && opts->rescore_fp64;
     std::vector<BestSlot> best((size_t)n);
@@ -1983,10 +2011,12 @@ int epik2_scan_replicates(epik2_ctx* ctx, int32_t dataset_id, const uint8_t* phe
     // only the rarer genotypes of i saves more than sharing the all-sample counts (8 replicates of
     // 1024 x 8192: 32.4 against 100.7 ms), which remains the form for larger classes.
     bool all_split = true;
-    for (int32_t t = 0; t < g; t++) all_split = all_split && split_fits(reps[(size_t)t]);
-    if (all_split) {
-      std::vector<DevDataset*> ds;
-      for (int32_t t = 0; t < g; t++) ds.push_back(&reps[(size_t)t]);
+    std::vector<DevDataset*> ds;
+    for (int32_t t = 0; t < g; t++) {
+      all_split = all_split && split_fits(reps[(size_t)t]);
+      ds.push_back(&reps[(size_t)t]);
+    }
+    if (all_split && split_screens(ds)) {
       r = run_split(ctx, ds, 0, INT64_MAX, 0, nullptr, nullptr, res.data(), rescore ? resc.data() : nullptr);
       if (r < 0) {
         release();

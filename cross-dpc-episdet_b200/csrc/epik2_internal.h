@@ -14,6 +14,7 @@ constexpr int kTableMaxSize = 748;    // reference TABLE_MAX_SIZE (GPU/v4.cpp:15
 // (controls' words first, then cases'), one uint2 {g0 bits, g1 bits} per SNP, rows of
 // m_pad SNPs.  Bit b of class word w is the sample of rank 32*w' + b in its class
 // (w' = word index inside the class); padding bits and padding SNPs are zero.
+constexpr int64_t kFlatRest = 2;
 struct DevDataset {
   int64_t n_samples = 0, n_snps = 0, n_cases = 0, n_controls = 0;
   int64_t m_pad = 0;      // n_snps rounded up to 32
@@ -26,6 +27,7 @@ struct DevDataset {
   float* lut = nullptr;         // ln n! in the reference CPU arithmetic, [0, n_samples+1]
   double* lut64 = nullptr;      // ln n! in double (precision form), [0, n_samples+1]
   int64_t tri = 0;              // entries per class in `pairs`
+  int64_t flat = 0;             // SNPs with at most kFlatRest samples off their most frequent genotype
   void* block = nullptr;        // single allocation holding all of the above
   size_t bytes = 0;             // bytes the layout needs
   size_t block_bytes = 0;       // size of `block` (at least `bytes`)
@@ -230,8 +232,9 @@ cudaError_t launch_encode(const DevDataset& d, cudaStream_t stream);
 cudaError_t launch_counts(const DevDataset& d, cudaStream_t stream, bool pairs = true);
 // pair margins on tensor cores (the CTA-pair FP4 kernel; exact for classes below 2^24)
 cudaError_t launch_pairs_tc(const TcParams& p, int blocks, cudaStream_t stream);
-// tiles of launch_pairs_tc for m_pad >= 2 SNPs into out; *counter and *err set to 0
-cudaError_t launch_pair_tiles(int64_t m_pad, uint64_t* out, unsigned long long* counter, int* err, cudaStream_t stream);
+// tiles of launch_pairs_tc for d (m_pad >= 2) into out; *counter and err[0] set to 0, d's flat SNPs
+// (DevDataset::flat) added to err[1]
+cudaError_t launch_pair_tiles(const DevDataset& d, uint64_t* out, unsigned long long* counter, int* err, cudaStream_t stream);
 // replicate form of the CTA-pair FP4 search (16 words per stage): see TcParams::n_reps
 cudaError_t launch_scan_reps(const TcParams& p, int blocks, cudaStream_t stream);
 int split_score_warps();  // scoring warps per CTA of the split search

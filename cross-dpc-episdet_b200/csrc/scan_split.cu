@@ -1123,10 +1123,12 @@ __global__ void __launch_bounds__(kSThreads, 1) k_scan_split(const SplitParams p
             reach = __float_as_uint(__shfl_sync(kFull, list_s, 31));
           }
           reach = __reduce_min_sync(kFull, reach);
-          // also without an improvement the lowest score known by now is read back: early in a search
-          // the warps learn from one another within a tile
-          if (lane == 0) thr = min(reach, atomicMin(p.thr + cur_job, reach));
-          thr = __shfl_sync(kFull, thr, 0);
+          // Also without an improvement the lowest score known by now is read: early in a search the warps
+          // learn from one another within a tile.  Only a lower one is written: an atomic at every such
+          // step took 1.97 ms instead of 1.73 for 512 x 8192 constant SNPs, which are all scored.
+          const unsigned now = *reinterpret_cast<volatile unsigned*>(p.thr + cur_job);
+          if (lane == 0 && reach < now) atomicMin(p.thr + cur_job, reach);
+          thr = min(reach, now);
           limit = __uint_as_float(thr) - base;
         }
       }

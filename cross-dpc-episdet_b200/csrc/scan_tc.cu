@@ -691,8 +691,9 @@ cudaError_t launch_expand_tiles(const int64_t* pb_off, const uint32_t* pb_ij, in
 // are reset with them.  Bound by the launch: one call where there were two copies of a list made on the
 // host, two memsets and its expansion (a new phenotype for 128 x 2048: 68 -> 59 us,
 // a one-call search of it 202 -> 195).  A block adds up
-// the tiles of those before it.
-__global__ void __launch_bounds__(256) k_pair_tiles(int64_t m_pad, int64_t kK, uint64_t* __restrict__ out,
+// the tiles of those before it, and counts the flat ones among its SNPs (DevDataset::flat).
+__global__ void __launch_bounds__(256) k_pair_tiles(const uint2* __restrict__ singles, int m, int n_samples, int64_t m_pad,
+                                                    int64_t kK, uint64_t* __restrict__ out,
                                                     unsigned long long* __restrict__ counter, int* __restrict__ err) {
   __shared__ unsigned long long s_before;
   const int u = blockIdx.x, tid = threadIdx.x;
@@ -701,7 +702,15 @@ __global__ void __launch_bounds__(256) k_pair_tiles(int64_t m_pad, int64_t kK, u
     *counter = 0;
     *err = 0;
   }
-  __syncthreads();
+  bool flat = false;
+  const int snp = 64 * u + tid;
+  if (tid < 64 && snp < m) {
+    const uint2 a = __ldg(singles + snp), b = __ldg(singles + m_pad + snp);
+    const int n0 = (int)(a.x + b.x), n1 = (int)(a.y + b.y);
+    flat = n_samples - max(max(n0, n1), n_samples - n0 - n1) <= kFlatRest;
+  }
+  const int n_flat = __syncthreads_count(flat);  // (also: s_before is 0)
+  if (tid == 0 && n_flat) atomicAdd(err + 1, n_flat);
   unsigned long long before = 0;
   for (int v = tid; v < u; v += 256) before += (unsigned long long)tiles_of_pair_block(64 * (int64_t)v, m_pad, kK);
   if (before) atomicAdd(&s_before, before);
@@ -710,8 +719,9 @@ __global__ void __launch_bounds__(256) k_pair_tiles(int64_t m_pad, int64_t kK, u
   for (int64_t t = tid; t < n; t += 256) out[s_before + t] = pack_tile(0, (uint32_t)(64 * u), (uint32_t)t, 0);
 }
 
-cudaError_t launch_pair_tiles(int64_t m_pad, uint64_t* out, unsigned long long* counter, int* err, cudaStream_t stream) {
-  k_pair_tiles<<<(unsigned)((m_pad - 2) / 64 + 1), 256, 0, stream>>>(m_pad, tc_k_per_tile(true), out, counter, err);
+cudaError_t launch_pair_tiles(const DevDataset& d, uint64_t* out, unsigned long long* counter, int* err, cudaStream_t stream) {
+  k_pair_tiles<<<(unsigned)((d.m_pad - 2) / 64 + 1), 256, 0, stream>>>(
+      reinterpret_cast<const uint2*>(d.singles), (int)d.n_snps, (int)d.n_samples, d.m_pad, tc_k_per_tile(true), out, counter, err);
   return cudaGetLastError();
 }
 
