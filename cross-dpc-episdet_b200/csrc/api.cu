@@ -401,6 +401,28 @@ int run_split(epik2_ctx* ctx, const std::vector<DevDataset*>& ds, int64_t ib, in
               uint32_t* dump_tables, float* dump_scores, BestSlot* best_out, Rescored* resc_out = nullptr,
               int* n_cand_out = nullptr);
 
+// Triplets with first index in [ib, ie) of m SNPs.
+double triplets_in(int64_t m, int64_t ib, int64_t ie) {
+  auto c3 = [](double n) { return n > 2 ? n * (n - 1) * (n - 2) / 6 : 0.0; };
+  return c3((double)(m - ib)) - c3((double)(m - std::max(ib, ie)));
+}
+
+// The smallest searches last as long as their launches: the split search's five against two to four of
+// the other kernels.  Without asking the tuner (it times 18 searches): the integer engine, which needs
+// no tile list either, or single FP4 CTAs; engine is set to the one to take.  Measured, us a call (split,
+// integer, FP4): 8 SNPs x 100 samples 62, 41, 56; 100 x 50 95, 62, 75; 64 x 500 80, 62, 58; 100 x 500 81, 97,
+// 75; 160 x 500 98, 111, 104; 64 x 2048 73, 117, 71; 128 x 2048 93, 196, 99; 16 x 8192 68, 134, 83.
+// A part of a search (whole = false) takes the integer engine or none, since the tile list of
+// the other kernels grows to that of all parts at once.
+bool small_search(double triplets, int64_t samples, bool whole, int& engine) {
+  const double ts = triplets * (double)samples;
+  if (samples > 4096 || ts >= 2.5e8) return false;
+  if (engine == EPIK2_ENGINE_AUTO && (samples <= 64 || ts < (whole || samples > 1000 ? 3e6 : 4e7))) engine = EPIK2_ENGINE_INT;
+  else if (whole) engine = EPIK2_ENGINE_TC_FP4;
+  else return false;
+  return true;
+}
+
 // Pair groups of first index i: j0 = i+1, i+5, ... while j0 <= m-2.
 int64_t groups_of(int64_t m, int64_t i) { return (i <= m - 3) ? (m - 2 - i + kPairsPerWarp) / kPairsPerWarp : 0; }
 
@@ -433,8 +455,15 @@ int run_scan(epik2_ctx* ctx, DevDataset& d, const epik2_opts* opts, uint32_t* du
     return fail(ctx, EPIK2_E_TOO_LARGE, "overlapped kernel: classes of at most 65535 samples");
   // Nothing pinned beyond the format: the genotype-split kernel wherever its 16-bit cells hold and its
   // screen keeps something back (a dump scores every triplet anyway); else the other kernels.
-  if ((engine == 0 || engine == 3) && kw == 0 && pt == 0 && ov == 0 && split_fits(d) &&
-      (dump_tables || split_screens({&d}, top_k))) {
+  const bool free_choice = (engine == 0 || engine == 3) && kw == 0 && pt == 0 && ov == 0 && split_fits(d);
+  // (of the 32 best it is always the faster one: the other kernels' lists of every warp go through the host)
+  if (free_choice && top_k < 2 && small_search(triplets_in(m, ib, ie), d.n_samples, ib == 0 && ie >= m - 2, engine)) {
+    if (engine == EPIK2_ENGINE_TC_FP4) {
+      kw = 8;
+      pt = 32;
+      ov = 1;
+    }
+  } else if (free_choice && (dump_tables || split_screens({&d}, top_k))) {
     int n_cand = 0;
     const int r = run_split(ctx, {&d}, ib, ie, top_k, dump_tables, dump_scores, best_out, nullptr, &n_cand);
     if (r != kSplitNoRoom) {
@@ -1822,7 +1851,19 @@ int epik2_scan_batch(epik2_ctx* ctx, const int32_t* dataset_ids, int32_t n, cons
   bool all_split = true;
   for (DevDataset* d : ds) all_split = all_split && split_fits(*d);
   all_split = all_split && split_screens(ds);
-  if (engine_req != EPIK2_ENGINE_TC && kw_req == 0 && pt_req == 0 && ov_req == 0 && all_split) {
+  const bool free_choice = engine_req != EPIK2_ENGINE_TC && kw_req == 0 && pt_req == 0 && ov_req == 0 && all_split;
+  // Many tiny datasets, or little in all: the persistent launch below on single CTAs, whose tiles are
+  // cheaper when nearly empty (us a call, split and FP4: 512 datasets of 32 SNPs x 500 samples 2179 and 1180,
+  // of 64 x 500 4581 and 3672, of 64 x 2000 4800 and 5164, of 128 x 500 12062 and 14240; one of 128 x 2000
+  // 97 and 92, 16 of 64 x 2000 212 and 209); int8 for the fewest samples (512 of 64 x 500 3433).
+  double ts = 0.0;
+  int64_t most_samples = 0;
+  for (DevDataset* d : ds) {
+    ts += triplets_in(d->n_snps, 0, d->n_snps) * (double)d->n_samples;
+    most_samples = std::max(most_samples, d->n_samples);
+  }
+  const bool tiny = free_choice && most_samples <= 4096 && (ts < 8e8 || ts < 6e7 * (double)n);
+  if (free_choice && !tiny) {
     const bool rescore = opts && opts->rescore_fp64;
     std::vector<BestSlot> best((size_t)n);
     std::vector<Rescored> resc(rescore ? (size_t)n : 0);
@@ -1840,7 +1881,11 @@ int epik2_scan_batch(epik2_ctx* ctx, const int32_t* dataset_ids, int32_t n, cons
   }
   TcConfig pick{0, 0, false, false};
   bool have = false;
-  if (engine_req != 0 && kw_req != 0 && (pt_req != 0 || engine_req == EPIK2_ENGINE_TC) && ov_req != 0) {
+  if (tiny) {
+    const bool int8 = most_samples <= 1000 && engine_req == EPIK2_ENGINE_AUTO;
+    pick = int8 ? TcConfig{EPIK2_ENGINE_TC, 4, false, false} : TcConfig{EPIK2_ENGINE_TC_FP4, 8, false, false};
+    have = true;
+  } else if (engine_req != 0 && kw_req != 0 && (pt_req != 0 || engine_req == EPIK2_ENGINE_TC) && ov_req != 0) {
     pick = TcConfig{engine_req, kw_req, pt_req == 64, ov_req == 2};
     have = true;
   } else if (engine_req == EPIK2_ENGINE_TC && kw_req != 0) {

@@ -70,6 +70,21 @@ def test_rare_alleles_and_uneven_classes(auto, S, M, maf, cases):
     _with(auto, *_hwe(S, M, maf, cases))
 
 
+@pytest.mark.parametrize("S,M", [(50, 4), (100, 8), (50, 100), (50, 200), (500, 32), (500, 64), (1000, 64), (2048, 40)])
+def test_small_searches(auto, S, M):
+    _with(auto, *_hwe(S, M, (0.05, 0.5), S // 2))
+
+
+@pytest.mark.parametrize("n,S,M", [(3, 100, 8), (512, 100, 8), (256, 500, 32), (200, 500, 64)])
+def test_batches_of_small_datasets(auto, n, S, M):
+    ids = [auto.load(*_hwe(S, M, (0.05, 0.5), S // 2, seed=t)) for t in range(n)]
+    try:
+        _compare(lambda **kw: auto.scan_batch(ids, **kw), PINNED[1:])
+    finally:
+        for d in ids:
+            auto.unload(d)
+
+
 @pytest.mark.parametrize("S,M,constant", [(200, 700, 1.0), (1000, 1024, 1.0), (2000, 1024, 1.0), (4000, 1024, 0.95),
                                           (8192, 512, 1.0), (9500, 512, 1.0), (1000, 1024, 0.4)])
 def test_constant_snps(auto, S, M, constant):
