@@ -20,9 +20,19 @@ using namespace epik2;
 struct GrowBuf {
   void* p = nullptr;
   size_t cap = 0;
-  cudaError_t need(size_t bytes) {
+  // at least bytes; a buffer that was too small grows to twice its size at once, but not beyond most
+  cudaError_t need(size_t bytes, size_t most = 0) {
     if (bytes <= cap) return cudaSuccess;
+    const size_t more = std::min(2 * cap, most);
     drop();
+    if (more > bytes) {
+      if (cudaMalloc(&p, more) == cudaSuccess) {
+        cap = more;
+        return cudaSuccess;
+      }
+      cudaGetLastError();
+      p = nullptr;
+    }
     const cudaError_t e = cudaMalloc(&p, bytes);
     if (e == cudaSuccess) cap = bytes;
     else p = nullptr;
@@ -93,8 +103,9 @@ struct epik2_ctx {
   BestSlot* d_rep_res = nullptr;
   Rescored* d_rep_resc = nullptr;
   int64_t rep_cap = 0, rep_slot_cap = 0;
-  // split search workspace (kept while it is at most kSplitKeepBytes; given back when another
-  // allocation needs the room and with the context)
+  size_t lent_bytes = 0;  // allocation of the replicates being searched
+  // split search workspace (trim_split: what is kept; given back when another allocation needs the
+  // room and with the context)
   GrowBuf sp_rows, sp_lists, sp_cp, sp_tiles, sp_small, sp_slots, sp_cand;
   unsigned char* h_small = nullptr;  // pinned image of the uploaded part of sp_small, and results
   size_t h_small_cap = 0;
@@ -174,6 +185,20 @@ size_t split_bytes(const epik2_ctx* ctx) {
 void drop_split(epik2_ctx* ctx) {
   for (GrowBuf* b : {&ctx->sp_rows, &ctx->sp_lists, &ctx->sp_cp, &ctx->sp_tiles, &ctx->sp_small, &ctx->sp_slots, &ctx->sp_cand})
     b->drop();
+}
+
+// The search workspace that a context keeps: up to as much as its datasets hold, at least 4 GiB (256
+// replicates of 1024 x 8192 need 3.9).  What goes beyond is released after the search that needed it, the
+// largest parts first; allocating and releasing it for every part of a search of 24000 x 300 took 5 ms
+// of a call's 8.
+constexpr size_t kSplitKeepBytes = (size_t)4 << 30;
+
+void trim_split(epik2_ctx* ctx) {  // no search is running
+  size_t held = ctx->spare_bytes + ctx->lent_bytes;
+  for (const auto& kv : ctx->datasets) held += kv.second->block_bytes;
+  const size_t keep = std::max(kSplitKeepBytes, held);
+  for (GrowBuf* b : {&ctx->sp_rows, &ctx->sp_cp, &ctx->sp_tiles, &ctx->sp_lists})
+    if (split_bytes(ctx) > keep) b->drop();
 }
 
 // A dataset allocation of at least `bytes`: the context's spare block when it fits without
@@ -796,8 +821,6 @@ bool split_screens(const std::vector<DevDataset*>& ds, int top_k) {
 // ms or more, and their ends (one tile, about 10 us) stay below 0.3 %.  Most searches take one launch:
 // with 768 MiB 256 x 100000 took a second one for its last 7 first SNPs (1.07 ms instead of 0.99).
 constexpr size_t kSplitChunkBytes = (size_t)1 << 30;
-// A larger workspace of a part is released after the search that needed it.
-constexpr size_t kSplitKeepBytes = (size_t)1 << 30;
 // Planes of the first SNPs whose tiles are interleaved in the queue: what may stay in L2 (126 MB)
 // beside the margins.
 constexpr size_t kSplitRunBytes = (size_t)40 << 20;
@@ -817,7 +840,7 @@ int run_split(epik2_ctx* ctx, const std::vector<DevDataset*>& ds, int64_t ib, in
   std::vector<SplitRec> recs;
   std::vector<SplitRun> runs;
   std::vector<Chunk> chunks;
-  size_t rows_bytes = 0, cp_max = 0, lists_max = 0, tiles_max = 0;
+  size_t rows_bytes = 0, rows_all = 0, cp_max = 0, lists_max = 0, tiles_max = 0;
   size_t cp = 0, lists = 0, tiles = 0;  // of the current chunk: bytes, bytes, descriptors
   int64_t trip = 0, rows_units = 0, max_tri = 0;
   float margin = 0.0f;
@@ -830,7 +853,7 @@ int run_split(epik2_ctx* ctx, const std::vector<DevDataset*>& ds, int64_t ib, in
     recs.clear();
     runs.clear();
     chunks.clear();
-    rows_bytes = cp_max = lists_max = tiles_max = 0;
+    rows_bytes = rows_all = cp_max = lists_max = tiles_max = 0;
     trip = rows_units = max_tri = 0;
     even = true;
     for (int b : order) {
@@ -844,7 +867,14 @@ int run_split(epik2_ctx* ctx, const std::vector<DevDataset*>& ds, int64_t ib, in
       J.tri = d.tri;
       J.m = (int32_t)d.n_snps;
       J.m_pad = (int32_t)d.m_pad;
-      J.mwp = (int32_t)((d.m_pad / 32 + 3) / 4 * 4);
+      // rows and packed margins from the first searched SNP on: for the last 100 first SNPs of 16384
+      // those of the whole matrix took 1 ms to make and 2 to 4 ms to allocate
+      const int64_t m = d.n_snps, i0 = std::max<int64_t>(ib, 0), i1 = std::min<int64_t>(ie, m - 2);
+      const int64_t from = std::min(i0, m - 3);
+      const int32_t cols = (int32_t)((d.m_pad / 32 + 3) / 4 * 4);
+      J.q0 = (int32_t)((from + 1) / 32 / 4 * 4);
+      J.mwp = cols - J.q0;
+      J.pair0 = tri_offset(d.m_pad, from, from + 1);
       J.w0 = (int32_t)d.w0;
       J.w1 = (int32_t)d.w1;
       J.n0 = (int32_t)d.n_controls;
@@ -863,18 +893,17 @@ int run_split(epik2_ctx* ctx, const std::vector<DevDataset*>& ds, int64_t ib, in
       rows_units = std::max(rows_units, (d.w0 + d.w1) * (J.mwp / 4));
       rows_bytes += align_up((size_t)(32 * (d.w0 + d.w1) + 1) * J.mwp * 8, 256);
       J.pairs16 = reinterpret_cast<uint4*>(rows_bytes);
-      rows_bytes += align_up((size_t)d.tri * 16, 256);
-      max_tri = std::max(max_tri, d.tri);
-      const int64_t m = d.n_snps;
+      rows_bytes += align_up((size_t)(d.tri - J.pair0) * 16, 256);
+      rows_all += align_up((size_t)(32 * (d.w0 + d.w1) + 1) * cols * 8, 256) + align_up((size_t)d.tri * 16, 256);
+      max_tri = std::max(max_tri, d.tri - J.pair0);
       const int max_quads = (int)(2 * d.n_samples / 3 / 128) + 5;  // the dropped genotype is the most frequent
-      const int64_t i0 = std::max<int64_t>(ib, 0), i1 = std::min<int64_t>(ie, m - 2);
       size_t run_bytes = 0;
       for (int64_t i = i0; i < i1; i++) {
         SplitRec r{};
         r.job = b;
         r.i = (int32_t)i;
         r.qlo = (int32_t)((i + 1) / 32 / 4 * 4);
-        r.mlen = 32 * (J.mwp - r.qlo);
+        r.mlen = 32 * (cols - r.qlo);
         const size_t rec_cp = (size_t)max_quads * r.mlen * 32, rec_list = (size_t)max_quads * 128 * 4;
         const bool new_chunk = chunks.empty() || cp + rec_cp > kSplitChunkBytes || recs.size() - chunks.back().rec0 >= (1u << 23);
         if (new_chunk) {
@@ -941,7 +970,7 @@ int run_split(epik2_ctx* ctx, const std::vector<DevDataset*>& ds, int64_t ib, in
     cudaError_t e = ctx->sp_small.need(end);
     if (e == cudaSuccess) e = ctx->sp_slots.need(sizeof(BestSlot) * (size_t)n_jobs * per_job);
     if (e == cudaSuccess && top_k > 1) e = ctx->sp_cand.need(sizeof(BestSlot) * (size_t)n_cand);
-    if (e == cudaSuccess) e = ctx->sp_rows.need(std::max<size_t>(rows_bytes, 256));
+    if (e == cudaSuccess) e = ctx->sp_rows.need(std::max<size_t>(rows_bytes, 256), rows_all);
     if (e == cudaSuccess) e = ctx->sp_lists.need(std::max<size_t>(lists_max, 256));
     if (e == cudaSuccess) e = ctx->sp_cp.need(cp_max + 8192);  // tiles past the last SNP read up to 128 columns on
     if (e == cudaSuccess) e = ctx->sp_tiles.need(8 * std::max<size_t>(tiles_max, 32));
@@ -971,7 +1000,7 @@ int run_split(epik2_ctx* ctx, const std::vector<DevDataset*>& ds, int64_t ib, in
   unsigned char* const dev = static_cast<unsigned char*>(ctx->sp_small.p);
   for (SplitJob& J : jobs) {
     J.rows = reinterpret_cast<uint2*>(static_cast<char*>(ctx->sp_rows.p) + reinterpret_cast<size_t>(J.rows));
-    J.pairs16 = reinterpret_cast<uint4*>(static_cast<char*>(ctx->sp_rows.p) + reinterpret_cast<size_t>(J.pairs16));
+    J.pairs16 = reinterpret_cast<uint4*>(static_cast<char*>(ctx->sp_rows.p) + reinterpret_cast<size_t>(J.pairs16)) - J.pair0;
   }
   memcpy(ctx->h_small, jobs.data(), sizeof(SplitJob) * jobs.size());
   if (!recs.empty()) memcpy(ctx->h_small + o_recs, recs.data(), sizeof(SplitRec) * recs.size());
@@ -1046,8 +1075,7 @@ int run_split(epik2_ctx* ctx, const std::vector<DevDataset*>& ds, int64_t ib, in
   ctx->stats.d2h_bytes += back;
   const int* h_err = reinterpret_cast<const int*>(ctx->h_small + o_err);
   const cudaError_t done = cudaStreamSynchronize(ctx->stream);
-  for (GrowBuf* b : {&ctx->sp_rows, &ctx->sp_lists, &ctx->sp_tiles})
-    if (b->cap > kSplitKeepBytes) b->drop();
+  trim_split(ctx);
   CK(ctx, done, "search");
   if (*h_err) return fail(ctx, EPIK2_E_TIMEOUT, "tensor-core scan: a bounded wait expired");
   float kms = 0.0f;
@@ -1725,6 +1753,7 @@ int unload_dataset(epik2_ctx* ctx, int32_t dataset_id, bool keep) {
     cudaFree(it->second->block);
   }
   ctx->datasets.erase(it);
+  trim_split(ctx);
   return EPIK2_OK;
 }
 }  // namespace
@@ -2002,8 +2031,10 @@ int epik2_scan_replicates(epik2_ctx* ctx, int32_t dataset_id, const uint8_t* phe
   Rescored* d_resc = ctx->d_rep_resc;
   const double alloc_ms = std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t_call).count();
   double encode_ms = 0.0;
+  ctx->lent_bytes = arena ? arena_bytes : 0;
   auto release = [&]() {
     cudaStreamSynchronize(ctx->stream);
+    ctx->lent_bytes = 0;
     if (arena) {  // becomes the context's spare allocation
       drop_spare(ctx);
       ctx->spare_block = arena;

@@ -168,17 +168,19 @@ struct ScreenConsts {
 // One dataset of a split search.
 struct SplitJob {
   const uint2* planes;
-  uint2* rows;             // [32*(w0+w1) + 1][mwp] {g0, g1} bits of 32 SNPs per entry, class-sorted samples
+  uint2* rows;             // [32*(w0+w1) + 1][mwp] {g0, g1} bits of 32 SNPs per entry from column q0 on, class-sorted samples
   const uint32_t* singles;
   const uint4* pairs;
-  uint4* pairs16;          // `pairs` with both classes' counts in one word
+  uint4* pairs16;          // `pairs` with both classes' counts in one word, entries [pair0, tri) only
   const float* lut;
   int64_t tri;
   int32_t m, m_pad, mwp, w0, w1, n0, n1;
   uint32_t coef;           // ScreenConsts
   int32_t bias;
   float theta1, theta2, c, base;
-  int32_t pad[5];
+  int32_t q0;
+  int64_t pair0;
+  int32_t pad[2];
 };
 static_assert(sizeof(SplitJob) == 128, "copied as 32 words per tile");
 
@@ -239,9 +241,9 @@ cudaError_t launch_pair_tiles(const DevDataset& d, uint64_t* out, unsigned long 
 cudaError_t launch_scan_reps(const TcParams& p, int blocks, cudaStream_t stream);
 int split_score_warps();  // scoring warps per CTA of the split search
 cudaError_t split_configure();
-// rows (sample-major bits) and packed pair margins of every job (at most 65535), its per_job slots
-// emptied, n_cand candidates emptied; max_units: the most class words x four 32-SNP columns of a job,
-// max_tri: the most pairs
+// rows (sample-major bits) and packed pair margins of every job (at most 65535) from its first searched
+// SNP on, its per_job slots emptied, n_cand candidates emptied; max_units: the most class words x four
+// 32-SNP columns of a job, max_tri: the most pairs
 cudaError_t launch_split_setup(const SplitJob* jobs, int n_jobs, int64_t max_units, int64_t max_tri, BestSlot* slots,
                                int per_job, BestSlot* cand, int n_cand, cudaStream_t stream);
 // sample lists and group ends of records [0, n) and the tile queue of their runs (at most max_blocks

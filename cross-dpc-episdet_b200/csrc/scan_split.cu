@@ -70,7 +70,8 @@ __device__ __forceinline__ uint32_t transpose32(uint32_t x, int lane) {
   return x;
 }
 
-// What a search needs once, for job blockIdx.y, by ranges of blockIdx.x:
+// What a search needs once, for job blockIdx.y, by ranges of blockIdx.x (a part of a search: from its
+// first SNP on):
 // [0, row_blocks): rows[32w + b][q] from planes[w][32q ..], one warp per class word and four 32-SNP
 // columns;
 // [row_blocks, row_blocks + pair_blocks): the pair margins packed, class 0 in the low, class 1 in the
@@ -93,7 +94,7 @@ __global__ void __launch_bounds__(256) k_split_setup(const SplitJob* __restrict_
     uint2 v[4];
 #pragma unroll
     for (int t = 0; t < 4; t++) {
-      const int64_t snp = 32 * (int64_t)(q + t) + lane;
+      const int64_t snp = 32 * (int64_t)(J.q0 + q + t) + lane;
       v[t] = snp < m_pad ? __ldg(J.planes + w * m_pad + snp) : make_uint2(0, 0);
     }
 #pragma unroll
@@ -107,7 +108,7 @@ __global__ void __launch_bounds__(256) k_split_setup(const SplitJob* __restrict_
   } else if ((int)blockIdx.x < row_blocks + pair_blocks) {
     const uint4* __restrict__ src = J.pairs;
     uint4* __restrict__ dst = J.pairs16;
-    for (int64_t x = (int64_t)((int)blockIdx.x - row_blocks) * 256 + threadIdx.x; x < J.tri; x += (int64_t)pair_blocks * 256) {
+    for (int64_t x = J.pair0 + (int64_t)((int)blockIdx.x - row_blocks) * 256 + threadIdx.x; x < J.tri; x += (int64_t)pair_blocks * 256) {
       const uint4 a = __ldg(src + x), b = __ldg(src + J.tri + x);
       dst[x] = make_uint4(a.x | (b.x << 16), a.y | (b.y << 16), a.z | (b.z << 16), a.w | (b.w << 16));
     }
@@ -317,7 +318,7 @@ __global__ void __launch_bounds__(kPlaneThreads) k_split_planes(const SplitJob* 
     const int quad = quad0 + lane / span, col = col0 + lane % span;
     const bool on = quad < nq && col < ncol;
     const int4* list = reinterpret_cast<const int4*>(lists + rec.list_off + 128 * (on ? quad : quad0) + 32 * w);
-    const uint2* rows = J.rows + rec.qlo + (on ? col : col0);
+    const uint2* rows = J.rows + (rec.qlo - J.q0) + (on ? col : col0);
     const int mwp = J.mwp;
     uint32_t x[32], y[32];
 #pragma unroll

@@ -85,6 +85,19 @@ def test_batches_of_small_datasets(auto, n, S, M):
             auto.unload(d)
 
 
+@pytest.mark.parametrize("S,M", [(2000, 4096), (500, 12000)])
+def test_parts_of_a_large_search(auto, S, M):
+    """Also the last first SNPs, whose triplets are few beside the matrix."""
+    rng = np.random.default_rng(M)
+    g = rng.integers(0, 3, (S, M), dtype=np.uint8)
+    did = auto.load(g, (rng.random(S) < 0.5).astype(np.uint8))
+    try:
+        for a, e in ((M - 10, M), (M - 100, M), (M // 2, M // 2 + 1), (M // 2, M // 2 + 8), (0, 1)):
+            _compare(lambda **kw: auto.scan(did, snp_begin=a, snp_end=e, **kw), PINNED[1:] if e < M else PINNED, slack=1.6)
+    finally:
+        auto.unload(did)
+
+
 @pytest.mark.parametrize("S,M,constant", [(200, 700, 1.0), (1000, 1024, 1.0), (2000, 1024, 1.0), (4000, 1024, 0.95),
                                           (8192, 512, 1.0), (9500, 512, 1.0), (1000, 1024, 0.4)])
 def test_constant_snps(auto, S, M, constant):
