@@ -16,28 +16,10 @@
 
 using namespace epik2;
 
-// A device buffer that only grows.
+// A device buffer that only grows (grow).
 struct GrowBuf {
   void* p = nullptr;
   size_t cap = 0;
-  // at least bytes; a buffer that was too small grows to twice its size at once, but not beyond most
-  cudaError_t need(size_t bytes, size_t most = 0) {
-    if (bytes <= cap) return cudaSuccess;
-    const size_t more = std::min(2 * cap, most);
-    drop();
-    if (more > bytes) {
-      if (cudaMalloc(&p, more) == cudaSuccess) {
-        cap = more;
-        return cudaSuccess;
-      }
-      cudaGetLastError();
-      p = nullptr;
-    }
-    const cudaError_t e = cudaMalloc(&p, bytes);
-    if (e == cudaSuccess) cap = bytes;
-    else p = nullptr;
-    return e;
-  }
   void drop() {
     if (p) cudaFree(p);
     p = nullptr;
@@ -76,6 +58,7 @@ struct epik2_ctx {
   int flat_seen = 0;            // that sum as last read
   int64_t wait_limit = 0;       // SM clocks of a bounded device-side wait (0 = kernel default)
   int test_withhold = 0;        // one-shot test hook of the bounded-wait error path
+  int64_t test_limit = 0;       // test hook: device memory the context may hold (0 = what there is)
   int64_t* d_pb_off = nullptr;
   uint32_t* d_pb_ij = nullptr;
   int64_t pb_cap = 0;
@@ -182,6 +165,48 @@ size_t split_bytes(const epik2_ctx* ctx) {
          ctx->sp_slots.cap + ctx->sp_cand.cap;
 }
 
+// Device memory of the context's datasets (with the spare allocation) and of all its large buffers.
+size_t dataset_bytes(const epik2_ctx* ctx) {
+  size_t held = ctx->spare_bytes + ctx->lent_bytes;
+  for (const auto& kv : ctx->datasets) held += kv.second->block_bytes;
+  return held;
+}
+
+size_t held_bytes(const epik2_ctx* ctx) {
+  return dataset_bytes(ctx) + split_bytes(ctx) + 8 * (size_t)ctx->tiles_cap + 16 * (size_t)ctx->pb_cap;
+}
+
+cudaError_t raw_malloc(epik2_ctx* ctx, void** p, size_t bytes) {
+  *p = nullptr;
+  if (ctx->test_limit && held_bytes(ctx) + bytes > (size_t)ctx->test_limit) return cudaErrorMemoryAllocation;
+  const cudaError_t e = cudaMalloc(p, bytes);
+  if (e == cudaErrorMemoryAllocation) cudaGetLastError();
+  return e;
+}
+
+cudaError_t free_memory(const epik2_ctx* ctx, size_t* free_bytes, size_t* total_bytes) {
+  const cudaError_t e = cudaMemGetInfo(free_bytes, total_bytes);
+  if (e == cudaSuccess && ctx->test_limit) {
+    const size_t held = held_bytes(ctx), limit = (size_t)ctx->test_limit;
+    *free_bytes = std::min(*free_bytes, limit > held ? limit - held : 0);
+  }
+  return e;
+}
+
+// At least bytes; a buffer that was too small grows to twice its size at once, but not beyond most.
+cudaError_t grow(epik2_ctx* ctx, GrowBuf& b, size_t bytes, size_t most = 0) {
+  if (bytes <= b.cap) return cudaSuccess;
+  const size_t more = std::min(2 * b.cap, most);
+  b.drop();
+  if (more > bytes && raw_malloc(ctx, &b.p, more) == cudaSuccess) {
+    b.cap = more;
+    return cudaSuccess;
+  }
+  const cudaError_t e = raw_malloc(ctx, &b.p, bytes);
+  if (e == cudaSuccess) b.cap = bytes;
+  return e;
+}
+
 void drop_split(epik2_ctx* ctx) {
   for (GrowBuf* b : {&ctx->sp_rows, &ctx->sp_lists, &ctx->sp_cp, &ctx->sp_tiles, &ctx->sp_small, &ctx->sp_slots, &ctx->sp_cand})
     b->drop();
@@ -194,11 +219,23 @@ void drop_split(epik2_ctx* ctx) {
 constexpr size_t kSplitKeepBytes = (size_t)4 << 30;
 
 void trim_split(epik2_ctx* ctx) {  // no search is running
-  size_t held = ctx->spare_bytes + ctx->lent_bytes;
-  for (const auto& kv : ctx->datasets) held += kv.second->block_bytes;
-  const size_t keep = std::max(kSplitKeepBytes, held);
+  const size_t keep = std::max(kSplitKeepBytes, dataset_bytes(ctx));
   for (GrowBuf* b : {&ctx->sp_rows, &ctx->sp_cp, &ctx->sp_tiles, &ctx->sp_lists})
     if (split_bytes(ctx) > keep) b->drop();
+}
+
+// Device memory for anything but the search workspace, which gives way to it.
+template <typename T>
+cudaError_t dev_malloc(epik2_ctx* ctx, T** out, size_t bytes) {
+  void* p = nullptr;
+  cudaError_t e = raw_malloc(ctx, &p, bytes);
+  if (e == cudaErrorMemoryAllocation && split_bytes(ctx) > 0) {
+    cudaStreamSynchronize(ctx->stream);
+    drop_split(ctx);
+    e = raw_malloc(ctx, &p, bytes);
+  }
+  *out = static_cast<T*>(p);
+  return e;
 }
 
 // A dataset allocation of at least `bytes`: the context's spare block when it fits without
@@ -213,14 +250,7 @@ cudaError_t take_block(epik2_ctx* ctx, size_t bytes, void** out, size_t* got) {
   }
   drop_spare(ctx);
   *got = bytes;
-  cudaError_t e = cudaMalloc(out, bytes);
-  if (e == cudaErrorMemoryAllocation && split_bytes(ctx) > 0) {  // the search workspace gives way
-    cudaGetLastError();
-    cudaStreamSynchronize(ctx->stream);
-    drop_split(ctx);
-    e = cudaMalloc(out, bytes);
-  }
-  return e;
+  return dev_malloc(ctx, out, bytes);
 }
 
 struct Layout {
@@ -306,8 +336,8 @@ int ensure_pb(epik2_ctx* ctx, int64_t n) {
   ctx->d_pb_off = nullptr;
   ctx->d_pb_ij = nullptr;
   ctx->pb_cap = 0;
-  CK(ctx, cudaMalloc(&ctx->d_pb_off, (size_t)(n + 1) * 8), "alloc tile list");
-  CK(ctx, cudaMalloc(&ctx->d_pb_ij, (size_t)n * 8), "alloc tile list");
+  CK(ctx, dev_malloc(ctx, &ctx->d_pb_off, (size_t)(n + 1) * 8), "alloc tile list");
+  CK(ctx, dev_malloc(ctx, &ctx->d_pb_ij, (size_t)n * 8), "alloc tile list");
   ctx->pb_cap = n;
   return EPIK2_OK;
 }
@@ -318,7 +348,7 @@ int ensure_tiles(epik2_ctx* ctx, int64_t n) {
   cudaFree(ctx->d_tiles);
   ctx->d_tiles = nullptr;
   ctx->tiles_cap = 0;
-  CK(ctx, cudaMalloc(&ctx->d_tiles, (size_t)n * 8), "alloc tile descriptors");
+  CK(ctx, dev_malloc(ctx, &ctx->d_tiles, (size_t)n * 8), "alloc tile descriptors");
   ctx->tiles_cap = n;
   return EPIK2_OK;
 }
@@ -329,7 +359,7 @@ int ensure_pgoff(epik2_ctx* ctx, int64_t n) {
   if (ctx->d_pgoff) cudaFree(ctx->d_pgoff);
   ctx->d_pgoff = nullptr;
   ctx->pgoff_cap = 0;
-  CK(ctx, cudaMalloc(&ctx->d_pgoff, (size_t)n * 8), "alloc pair-group offsets");
+  CK(ctx, dev_malloc(ctx, &ctx->d_pgoff, (size_t)n * 8), "alloc pair-group offsets");
   ctx->pgoff_cap = n;
   return EPIK2_OK;
 }
@@ -947,11 +977,11 @@ int run_split(epik2_ctx* ctx, const std::vector<DevDataset*>& ds, int64_t ib, in
   if ((ib > 0 || ie < all) &&
       (cp_max + 8192 > ctx->sp_cp.cap || lists_max > ctx->sp_lists.cap || 8 * tiles_max > ctx->sp_tiles.cap)) {
     lay_out(0, all);
-    cudaError_t e = ctx->sp_cp.need(cp_max + 8192);
-    if (e == cudaSuccess) e = ctx->sp_lists.need(lists_max);
-    if (e == cudaSuccess) e = ctx->sp_tiles.need(8 * tiles_max);
+    cudaError_t e = grow(ctx, ctx->sp_cp, cp_max + 8192);
+    if (e == cudaSuccess) e = grow(ctx, ctx->sp_lists, lists_max);
+    if (e == cudaSuccess) e = grow(ctx, ctx->sp_tiles, 8 * tiles_max);
     const size_t tables = sizeof(SplitRec) * recs.size() + sizeof(SplitRun) * runs.size() + 8 * chunks.size();
-    if (e == cudaSuccess) e = ctx->sp_small.need(tables + (sizeof(SplitJob) + sizeof(TcJob) + 256) * jobs.size() + 4096);
+    if (e == cudaSuccess) e = grow(ctx, ctx->sp_small, tables + (sizeof(SplitJob) + sizeof(TcJob) + 256) * jobs.size() + 4096);
     if (e != cudaSuccess) cudaGetLastError();
     lay_out(ib, ie);
   }
@@ -967,13 +997,13 @@ int run_split(epik2_ctx* ctx, const std::vector<DevDataset*>& ds, int64_t ib, in
   const size_t o_res = o_err + 16, o_resc = align_up(o_res + sizeof(BestSlot) * jobs.size(), 16);
   const size_t end = align_up(o_resc + (resc_out ? sizeof(Rescored) * jobs.size() : 0) + 256, 256);
   auto reserve = [&]() {
-    cudaError_t e = ctx->sp_small.need(end);
-    if (e == cudaSuccess) e = ctx->sp_slots.need(sizeof(BestSlot) * (size_t)n_jobs * per_job);
-    if (e == cudaSuccess && top_k > 1) e = ctx->sp_cand.need(sizeof(BestSlot) * (size_t)n_cand);
-    if (e == cudaSuccess) e = ctx->sp_rows.need(std::max<size_t>(rows_bytes, 256), rows_all);
-    if (e == cudaSuccess) e = ctx->sp_lists.need(std::max<size_t>(lists_max, 256));
-    if (e == cudaSuccess) e = ctx->sp_cp.need(cp_max + 8192);  // tiles past the last SNP read up to 128 columns on
-    if (e == cudaSuccess) e = ctx->sp_tiles.need(8 * std::max<size_t>(tiles_max, 32));
+    cudaError_t e = grow(ctx, ctx->sp_small, end);
+    if (e == cudaSuccess) e = grow(ctx, ctx->sp_slots, sizeof(BestSlot) * (size_t)n_jobs * per_job);
+    if (e == cudaSuccess && top_k > 1) e = grow(ctx, ctx->sp_cand, sizeof(BestSlot) * (size_t)n_cand);
+    if (e == cudaSuccess) e = grow(ctx, ctx->sp_rows, std::max<size_t>(rows_bytes, 256), rows_all);
+    if (e == cudaSuccess) e = grow(ctx, ctx->sp_lists, std::max<size_t>(lists_max, 256));
+    if (e == cudaSuccess) e = grow(ctx, ctx->sp_cp, cp_max + 8192);  // tiles past the last SNP read up to 128 columns on
+    if (e == cudaSuccess) e = grow(ctx, ctx->sp_tiles, 8 * std::max<size_t>(tiles_max, 32));
     return e;
   };
   cudaError_t e = reserve();
@@ -1271,13 +1301,13 @@ int run_batch(epik2_ctx* ctx, const std::vector<DevDataset*>& ds, const std::vec
     for (int g = 1; g <= n_groups; g++) pl->group_off[g] = std::max(pl->group_off[g], pl->group_off[g - 1]);
     pl->group_code = group_code;
     const size_t pb_ij_bytes = std::max<size_t>(pb_ij_all.size(), 2) * 4;
-    if (cudaMalloc(&pl->d_jobs, sizeof(TcJob) * n) ||
-        cudaMalloc(&pl->d_tiles, 8 * (size_t)std::max<int64_t>(pl->n_tiles, 1)) ||
-        cudaMalloc(&pl->d_counters, 8 * (size_t)n_groups) ||
-        cudaMalloc(&pl->d_pb_off, 8 * pb_off_all.size()) || cudaMalloc(&pl->d_pb_ij, pb_ij_bytes) ||
-        cudaMalloc(&pl->d_job_slots, sizeof(BestSlot) * (size_t)n * grid) ||
-        cudaMalloc(&pl->d_results, sizeof(BestSlot) * n) || cudaMallocHost(&pl->h_results, sizeof(BestSlot) * n) ||
-        cudaMallocHost(&pl->h_err, sizeof(int)) || cudaMalloc(&pl->d_resc, sizeof(Rescored) * n) ||
+    if (dev_malloc(ctx, &pl->d_jobs, sizeof(TcJob) * n) ||
+        dev_malloc(ctx, &pl->d_tiles, 8 * (size_t)std::max<int64_t>(pl->n_tiles, 1)) ||
+        dev_malloc(ctx, &pl->d_counters, 8 * (size_t)n_groups) ||
+        dev_malloc(ctx, &pl->d_pb_off, 8 * pb_off_all.size()) || dev_malloc(ctx, &pl->d_pb_ij, pb_ij_bytes) ||
+        dev_malloc(ctx, &pl->d_job_slots, sizeof(BestSlot) * (size_t)n * grid) ||
+        dev_malloc(ctx, &pl->d_results, sizeof(BestSlot) * n) || cudaMallocHost(&pl->h_results, sizeof(BestSlot) * n) ||
+        cudaMallocHost(&pl->h_err, sizeof(int)) || dev_malloc(ctx, &pl->d_resc, sizeof(Rescored) * n) ||
         cudaMallocHost(&pl->h_resc, sizeof(Rescored) * n))
       return fail(ctx, EPIK2_E_NOMEM, "batched plan: device memory");
     CK(ctx, cudaMemcpyAsync(pl->d_pb_off, pb_off_all.data(), 8 * pb_off_all.size(), cudaMemcpyHostToDevice,
@@ -1481,7 +1511,7 @@ int epik2_device_name(const epik2_ctx* ctx, char* buf, size_t len) {
 int epik2_mem_info(const epik2_ctx* ctx, size_t* free_bytes, size_t* total_bytes) {
   if (!ctx || !free_bytes || !total_bytes) return EPIK2_E_INVALID;
   cudaSetDevice(ctx->device);
-  if (cudaMemGetInfo(free_bytes, total_bytes) != cudaSuccess) return EPIK2_E_CUDA;
+  if (free_memory(ctx, free_bytes, total_bytes) != cudaSuccess) return EPIK2_E_CUDA;
   // the context's spare allocation and search workspace are reused or released on demand
   *free_bytes += ctx->spare_bytes + split_bytes(ctx);
   return EPIK2_OK;
@@ -1520,6 +1550,12 @@ int epik2_set_wait_limit(epik2_ctx* ctx, int64_t sm_clocks) {
 int epik2_test_withhold_arrival(epik2_ctx* ctx) {
   if (!ctx) return EPIK2_E_INVALID;
   ctx->test_withhold = 1;
+  return EPIK2_OK;
+}
+
+int epik2_test_memory_limit(epik2_ctx* ctx, int64_t bytes) {
+  if (!ctx || bytes < 0) return EPIK2_E_INVALID;
+  ctx->test_limit = bytes;
   return EPIK2_OK;
 }
 
@@ -1603,7 +1639,7 @@ int epik2_load_u8(epik2_ctx* ctx, const uint8_t* geno, const uint8_t* pheno, int
   const bool reuse = ctx->spare_block && ctx->spare_bytes >= L.total && ctx->spare_bytes <= 2 * L.total;
   if (!reuse) {
     size_t fr = 0, tot = 0;
-    CK(ctx, cudaMemGetInfo(&fr, &tot), "mem info");
+    CK(ctx, free_memory(ctx, &fr, &tot), "mem info");
     if (L.total + (size_t)(256u << 20) > fr + ctx->spare_bytes + split_bytes(ctx))
       return fail(ctx, EPIK2_E_NOMEM, "dataset does not fit in free device memory");
   }
@@ -1691,7 +1727,7 @@ int epik2_load_replicate(epik2_ctx* ctx, int32_t base_dataset_id, const uint8_t*
   const Layout L = dataset_layout(root->n_samples, root->n_snps, false);
   if (!(ctx->spare_block && ctx->spare_bytes >= L.total && ctx->spare_bytes <= 2 * L.total)) {
     size_t fr = 0, tot = 0;  // a new allocation: ask for free memory (about a millisecond)
-    CK(ctx, cudaMemGetInfo(&fr, &tot), "mem info");
+    CK(ctx, free_memory(ctx, &fr, &tot), "mem info");
     if (L.total + (size_t)(256u << 20) > fr + ctx->spare_bytes + split_bytes(ctx))
       return fail(ctx, EPIK2_E_NOMEM, "replicate does not fit in free device memory");
   }
@@ -1987,7 +2023,7 @@ int epik2_scan_replicates(epik2_ctx* ctx, int32_t dataset_id, const uint8_t* phe
   int64_t fit = want;  // a spare allocation that holds them all needs no free-memory query
   if (!(ctx->spare_block && ctx->spare_bytes >= rep_bytes * (size_t)want)) {
     size_t fr = 0, tot = 0;
-    CK(ctx, cudaMemGetInfo(&fr, &tot), "mem info");
+    CK(ctx, free_memory(ctx, &fr, &tot), "mem info");
     fr += ctx->spare_bytes + split_bytes(ctx);
     fit = ((int64_t)fr - ((int64_t)1 << 30)) / (int64_t)rep_bytes;
   }
@@ -2017,10 +2053,10 @@ int epik2_scan_replicates(epik2_ctx* ctx, int32_t dataset_id, const uint8_t* phe
     ctx->d_rep_resc = nullptr;
     ctx->rep_cap = ctx->rep_slot_cap = 0;
     const int64_t cap = std::max<int64_t>(group, 64);
-    e = cudaMalloc(&ctx->d_rep_jobs, sizeof(TcJob) * cap);
-    if (e == cudaSuccess) e = cudaMalloc(&ctx->d_rep_slots, sizeof(BestSlot) * (size_t)cap * grid);
-    if (e == cudaSuccess) e = cudaMalloc(&ctx->d_rep_res, sizeof(BestSlot) * cap);
-    if (e == cudaSuccess) e = cudaMalloc(&ctx->d_rep_resc, sizeof(Rescored) * cap);
+    e = dev_malloc(ctx, &ctx->d_rep_jobs, sizeof(TcJob) * cap);
+    if (e == cudaSuccess) e = dev_malloc(ctx, &ctx->d_rep_slots, sizeof(BestSlot) * (size_t)cap * grid);
+    if (e == cudaSuccess) e = dev_malloc(ctx, &ctx->d_rep_res, sizeof(BestSlot) * cap);
+    if (e == cudaSuccess) e = dev_malloc(ctx, &ctx->d_rep_resc, sizeof(Rescored) * cap);
     if (e == cudaSuccess) {
       ctx->rep_cap = cap;
       ctx->rep_slot_cap = cap * grid;
@@ -2198,8 +2234,8 @@ int epik2_dump_tables(epik2_ctx* ctx, int32_t dataset_id, uint32_t* tables, floa
   const int64_t T = m * (m - 1) * (m - 2) / 6;
   uint32_t* dt = nullptr;
   float* ds = nullptr;
-  CK(ctx, cudaMalloc(&dt, (size_t)T * 54 * 4), "alloc dump");
-  cudaError_t e = cudaMalloc(&ds, (size_t)T * 4);
+  CK(ctx, dev_malloc(ctx, &dt, (size_t)T * 54 * 4), "alloc dump");
+  cudaError_t e = dev_malloc(ctx, &ds, (size_t)T * 4);
   if (e != cudaSuccess) {
     cudaFree(dt);
     return cuda_fail(ctx, e, "alloc dump");
@@ -2230,8 +2266,8 @@ int epik2_tables(epik2_ctx* ctx, int32_t dataset_id, const uint32_t* triplets, i
   }
   CK(ctx, cudaSetDevice(ctx->device), "set device");
   uint32_t *dtrip = nullptr, *dout = nullptr;
-  CK(ctx, cudaMalloc(&dtrip, (size_t)n * 12), "alloc triplets");
-  cudaError_t e = cudaMalloc(&dout, (size_t)n * 54 * 4);
+  CK(ctx, dev_malloc(ctx, &dtrip, (size_t)n * 12), "alloc triplets");
+  cudaError_t e = dev_malloc(ctx, &dout, (size_t)n * 54 * 4);
   if (e == cudaSuccess) e = cudaMemcpy(dtrip, triplets, (size_t)n * 12, cudaMemcpyHostToDevice);
   if (e == cudaSuccess) e = launch_tables(*d, dtrip, n, dout, ctx->stream);
   ctx->stats.kernel_launches += 1;

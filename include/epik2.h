@@ -94,7 +94,11 @@ const char *epik2_strerror(int status);
 const char *epik2_last_error(const epik2_ctx *ctx);
 /* Device name as the reference prints it ("Selected device: ...", GPU/v4.cpp:251). */
 int epik2_device_name(const epik2_ctx *ctx, char *buf, size_t len);
-/* Bytes of device memory currently free / total on the context's device. */
+/* Bytes of device memory currently free / total on the context's device.  A context keeps the
+ * workspace of its last searches (as much as its datasets hold, or 4 GiB if that is more) and one dataset
+ * allocation for its next calls.  Both count as free here, because any allocation of this context
+ * takes them back; other contexts and libraries on the device see that much less.
+ * epik2_destroy releases them. */
 int epik2_mem_info(const epik2_ctx *ctx, size_t *free_bytes, size_t *total_bytes);
 
 /* Default search engine of the context (EPIK2_ENGINE_*).  All engines give identical
@@ -136,6 +140,9 @@ int epik2_set_wait_limit(epik2_ctx *ctx, int64_t sm_clocks);
  * before any matrix product is issued and the search returns EPIK2_E_TIMEOUT.  One-shot:
  * the search after it runs normally. */
 int epik2_test_withhold_arrival(epik2_ctx *ctx);
+/* Test hook (host only, no reference counterpart): the context refuses to hold more than this many
+ * bytes of device memory in datasets and large buffers, as if the device had no more (0 = no limit). */
+int epik2_test_memory_limit(epik2_ctx *ctx, int64_t bytes);
 /* Test hook (host only): the lower bound of K2 by which the genotype-split search leaves out
  * triplets, for n tables of 54 counts (27 of controls, 27 of cases) of a dataset with n_controls
  * and n_cases samples (at most 65535 each), in the FP32 arithmetic of the search. */
