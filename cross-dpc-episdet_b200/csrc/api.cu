@@ -455,6 +455,7 @@ bool split_screens(const std::vector<DevDataset*>& ds, int top_k = 0);
 int run_split(epik2_ctx* ctx, const std::vector<DevDataset*>& ds, int64_t ib, int64_t ie, int top_k,
               uint32_t* dump_tables, float* dump_scores, BestSlot* best_out, Rescored* resc_out = nullptr,
               int* n_cand_out = nullptr);
+int run_split_all(epik2_ctx* ctx, const std::vector<DevDataset*>& ds, BestSlot* best_out, Rescored* resc_out);
 
 // Triplets with first index in [ib, ie) of m SNPs.
 double triplets_in(int64_t m, int64_t ib, int64_t ie) {
@@ -1116,6 +1117,35 @@ int run_split(epik2_ctx* ctx, const std::vector<DevDataset*>& ds, int64_t ib, in
   memcpy(best_out, ctx->h_small + o_res, sizeof(BestSlot) * (size_t)n_jobs);
   if (resc_out) memcpy(resc_out, ctx->h_small + o_resc, sizeof(Rescored) * (size_t)n_jobs);
   return EPIK2_OK;
+}
+
+// Best triplet of each of many datasets; those whose workspaces do not fit together are searched in halves.
+int run_split_all(epik2_ctx* ctx, const std::vector<DevDataset*>& ds, BestSlot* best_out, Rescored* resc_out) {
+  const int r = run_split(ctx, ds, 0, INT64_MAX, 0, nullptr, nullptr, best_out, resc_out);
+  if (r != kSplitNoRoom || ds.size() < 2) return r;
+  double kms = 0.0;
+  int64_t trip = 0;
+  for (size_t a = 0, half = ds.size() / 2; a < ds.size(); a += half, half = ds.size() - a) {
+    const std::vector<DevDataset*> part(ds.begin() + (ptrdiff_t)a, ds.begin() + (ptrdiff_t)(a + half));
+    const int h = run_split_all(ctx, part, best_out + a, resc_out ? resc_out + a : nullptr);
+    if (h) return h;
+    kms += ctx->stats.last_scan_kernel_ms;
+    trip += ctx->stats.last_scan_triplets;
+  }
+  ctx->stats.last_scan_kernel_ms = kms;
+  ctx->stats.last_scan_triplets = trip;
+  return EPIK2_OK;
+}
+
+// Device memory that the split search of n replicates of an S x m matrix needs beside them: rows and
+// packed margins each; planes, lists and tiles of one chunk.
+size_t split_replicate_bytes(int64_t S, int64_t m) {
+  const int64_t m_pad = (m + 31) / 32 * 32, cols = (m_pad / 32 + 3) / 4 * 4;
+  return (size_t)(S + 65) * (size_t)cols * 8 + (size_t)tri_size(m_pad) * 16 + (1 << 16);
+}
+size_t split_chunk_bytes(int64_t S, int64_t m, int64_t n) {
+  const double quads = 2.0 * (double)S / 3.0 / 128.0 + 5.0, all = quads * 32.0 * ((double)m + 128.0) * (double)m * (double)n;
+  return (size_t)(1.25 * std::min((double)kSplitChunkBytes, all)) + ((size_t)64 << 20);
 }
 
 // Autotuner: time each candidate on a slice of the dataset (first indices [0, ie) holding
@@ -1932,7 +1962,7 @@ int epik2_scan_batch(epik2_ctx* ctx, const int32_t* dataset_ids, int32_t n, cons
     const bool rescore = opts && opts->rescore_fp64;
     std::vector<BestSlot> best((size_t)n);
     std::vector<Rescored> resc(rescore ? (size_t)n : 0);
-    const int r = run_split(ctx, ds, 0, INT64_MAX, 0, nullptr, nullptr, best.data(), rescore ? resc.data() : nullptr);
+    const int r = run_split_all(ctx, ds, best.data(), rescore ? resc.data() : nullptr);
     if (r != kSplitNoRoom) {
       if (r) return r;
       ctx->stats.last_scan_words = 0;
@@ -2011,7 +2041,8 @@ int epik2_scan_replicates(epik2_ctx* ctx, int32_t dataset_id, const uint8_t* phe
   CK(ctx, cudaSetDevice(ctx->device), "set device");
   const int64_t S = base->n_samples, m = base->n_snps;
   const int grid = tc_pair_blocks(ctx->tc_blocks);
-  // replicates per launch: as many as fit in free device memory above 1 GiB, at most 256.
+  // replicates per launch: as many as fit in free device memory (above 1 GiB, or with what their split
+  // search needs), at most 256.
   // Their class orders, planes and margins live in one allocation for the whole call, kept
   // afterwards as the context's spare allocation (the next call of the same shape reuses it;
   // any other allocation of the context releases it first); their genotypes and ln n! tables
@@ -2026,6 +2057,13 @@ int epik2_scan_replicates(epik2_ctx* ctx, int32_t dataset_id, const uint8_t* phe
     CK(ctx, free_memory(ctx, &fr, &tot), "mem info");
     fr += ctx->spare_bytes + split_bytes(ctx);
     fit = ((int64_t)fr - ((int64_t)1 << 30)) / (int64_t)rep_bytes;
+    // Room for the split search of them, which is worth more than a larger group: 16 replicates of 2000 x
+    // 1536 with room for 12 of them and 1 GiB take 162 ms in groups, 445 in the form below.
+    if (split_fits(*base) && split_screens({base})) {
+      const int64_t room = (int64_t)fr - (int64_t)split_chunk_bytes(S, m, want);
+      const int64_t split_fit = room / (int64_t)(rep_bytes + split_replicate_bytes(S, m));
+      if (split_fit >= 1) fit = std::min(fit, split_fit);
+    }
   }
   const int32_t group = (int32_t)std::max<int64_t>(1, std::min<int64_t>(fit, want));
   int r = EPIK2_OK;
@@ -2129,7 +2167,7 @@ int epik2_scan_replicates(epik2_ctx* ctx, int32_t dataset_id, const uint8_t* phe
       ds.push_back(&reps[(size_t)t]);
     }
     if (all_split && split_screens(ds)) {
-      r = run_split(ctx, ds, 0, INT64_MAX, 0, nullptr, nullptr, res.data(), rescore ? resc.data() : nullptr);
+      r = run_split_all(ctx, ds, res.data(), rescore ? resc.data() : nullptr);
       if (r < 0) {
         release();
         return r;
