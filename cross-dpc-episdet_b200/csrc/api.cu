@@ -1088,6 +1088,7 @@ int run_split(epik2_ctx* ctx, const std::vector<DevDataset*>& ds, int64_t ib, in
     ctx->stats.kernel_launches += 3;
   }
   CK(ctx, launch_reduce_jobs(d_slots, n_jobs, per_job, d_res, ctx->stream), "reduce kernel");
+  ctx->stats.kernel_launches += 1;
   CK(ctx, cudaEventRecord(ctx->ev_stop, ctx->stream), "event");
   if (top_k > 1) {  // the candidates' number goes behind the error word
     CK(ctx, launch_split_collect(ctx->d_cand, n_cand, d_thr, margin, static_cast<BestSlot*>(ctx->sp_cand.p),
