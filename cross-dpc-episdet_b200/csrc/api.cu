@@ -848,13 +848,18 @@ bool split_screens(const std::vector<DevDataset*>& ds, int top_k) {
   return 2.0 * flat <= all;
 }
 
-// Compacted planes of the first SNPs searched per launch: launches of the large workload then last 8
-// ms or more, and their ends (one tile, about 10 us) stay below 0.3 %.  Most searches take one launch:
-// with 768 MiB 256 x 100000 took a second one for its last 7 first SNPs (1.07 ms instead of 0.99).
+// Most compacted planes of the first SNPs searched per launch, a bound on memory: launches then last
+// 1 ms or more, and their ends (one tile, about 10 us) cost less than 1 %.  A search that needs more
+// takes launches of about equal planes, so that none holds a handful of first SNPs.
 constexpr size_t kSplitChunkBytes = (size_t)1 << 30;
 // Planes of the first SNPs whose tiles are interleaved in the queue: what may stay in L2 (126 MB)
 // beside the margins.
 constexpr size_t kSplitRunBytes = (size_t)40 << 20;
+
+// Quads of samples of a first SNP at most (the dropped genotype is the most frequent one); SNPs that its
+// planes hold.
+int split_quads(const DevDataset& d) { return (int)(2 * d.n_samples / 3 / 128) + 5; }
+int64_t split_row(const DevDataset& d, int64_t i) { return 32 * ((d.m_pad / 32 + 3) / 4 * 4 - (i + 1) / 32 / 4 * 4); }
 
 // Best triplet of each dataset over first indices [ib, ie) (clipped to the dataset); resc_out (may
 // be null): their FP64 rescores.  top_k > 1 (one dataset): *n_cand_out candidates in ctx->sp_cand,
@@ -887,6 +892,19 @@ int run_split(epik2_ctx* ctx, const std::vector<DevDataset*>& ds, int64_t ib, in
     rows_bytes = rows_all = cp_max = lists_max = tiles_max = 0;
     trip = rows_units = max_tri = 0;
     even = true;
+    // planes of all launches and of the largest record, then of one launch: a launch ends where the sum
+    // of the planes passes a multiple of that
+    size_t planes = 0, planes_rec = 0, done = 0;
+    for (const DevDataset* d : ds) {
+      const size_t quads = (size_t)split_quads(*d) * 32;
+      for (int64_t i = std::max<int64_t>(ib, 0); i < std::min<int64_t>(ie, d->n_snps - 2); i++) {
+        const size_t bytes = quads * (size_t)split_row(*d, i);
+        planes += bytes;
+        planes_rec = std::max(planes_rec, bytes);
+      }
+    }
+    const size_t most = std::max(kSplitChunkBytes - std::min(planes_rec, kSplitChunkBytes / 2), kSplitChunkBytes / 2);
+    const size_t launches = std::max<size_t>((planes + most - 1) / most, 1), share = (planes + launches - 1) / launches;
     for (int b : order) {
       const DevDataset& d = *ds[(size_t)b];
       SplitJob& J = jobs[(size_t)b];
@@ -927,16 +945,17 @@ int run_split(epik2_ctx* ctx, const std::vector<DevDataset*>& ds, int64_t ib, in
       rows_bytes += align_up((size_t)(d.tri - J.pair0) * 16, 256);
       rows_all += align_up((size_t)(32 * (d.w0 + d.w1) + 1) * cols * 8, 256) + align_up((size_t)d.tri * 16, 256);
       max_tri = std::max(max_tri, d.tri - J.pair0);
-      const int max_quads = (int)(2 * d.n_samples / 3 / 128) + 5;  // the dropped genotype is the most frequent
+      const int max_quads = split_quads(d);
       size_t run_bytes = 0;
       for (int64_t i = i0; i < i1; i++) {
         SplitRec r{};
         r.job = b;
         r.i = (int32_t)i;
         r.qlo = (int32_t)((i + 1) / 32 / 4 * 4);
-        r.mlen = 32 * (cols - r.qlo);
+        r.mlen = (int32_t)split_row(d, i);
         const size_t rec_cp = (size_t)max_quads * r.mlen * 32, rec_list = (size_t)max_quads * 128 * 4;
-        const bool new_chunk = chunks.empty() || cp + rec_cp > kSplitChunkBytes || recs.size() - chunks.back().rec0 >= (1u << 23);
+        const bool new_chunk = chunks.empty() || done >= share * chunks.size() || cp + rec_cp > kSplitChunkBytes ||
+                               recs.size() - chunks.back().rec0 >= (1u << 23);
         if (new_chunk) {
           chunks.push_back(Chunk{(int)recs.size(), 0, (int)runs.size(), 0, 0, 0, 0});
           cp = lists = tiles = 0;
@@ -953,6 +972,7 @@ int run_split(epik2_ctx* ctx, const std::vector<DevDataset*>& ds, int64_t ib, in
         r.cp_off = (int64_t)(cp / 16);
         r.list_off = (int64_t)(lists / 4);
         cp += rec_cp;
+        done += rec_cp;
         lists += rec_list;
         const int64_t left = m - 2 - i;  // SNPs j from i + 1 to m - 2
         const int64_t blocks = (left + kSplitJ - 1) / kSplitJ;
