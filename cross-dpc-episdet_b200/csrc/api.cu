@@ -257,13 +257,19 @@ struct Layout {
   size_t geno, perm, planes, singles, pairs, lut, lut64, total;
 };
 
-Layout dataset_layout(int64_t s, int64_t m, bool with_geno = true) {
+// At least kLutRead bytes can be read from the ln n! table on: the split search looks up
+// a + b + 1 of two 16-bit counts, which may be any after a bounded wait has expired.
+constexpr size_t kLutRead = 4 * (2 * 65535 + 2);
+
+Layout dataset_layout(int64_t s, int64_t m, bool with_geno = true, bool own_lut = true) {
   const int64_t m_pad = (m + 31) / 32 * 32;
   const int64_t words = (s + 31) / 32 + 1;  // enough for any class split
   Layout L{};
   size_t off = 0;
   L.geno = off;
   off = align_up(off + (with_geno ? (size_t)(s * m) : 0), 256);
+  L.lut = off;
+  off = align_up(off + (size_t)(s + 2) * 4, 256);
   L.perm = off;
   off = align_up(off + (size_t)s * 4, 256);
   L.planes = off;
@@ -272,11 +278,9 @@ Layout dataset_layout(int64_t s, int64_t m, bool with_geno = true) {
   off = align_up(off + (size_t)m_pad * 16, 256);
   L.pairs = off;
   off = align_up(off + (size_t)(2 * tri_size(m_pad)) * 16, 256);
-  L.lut = off;
-  off = align_up(off + (size_t)(s + 2) * 4, 256);
   L.lut64 = off;
   off = align_up(off + (size_t)(s + 2) * 8, 256);
-  L.total = off;
+  L.total = own_lut ? std::max(off, L.lut + kLutRead) : off;
   return L;
 }
 
@@ -2069,7 +2073,7 @@ int epik2_scan_replicates(epik2_ctx* ctx, int32_t dataset_id, const uint8_t* phe
   // any other allocation of the context releases it first); their genotypes and ln n! tables
   // are the base dataset's.
   const auto t_call = std::chrono::steady_clock::now();
-  const Layout L = dataset_layout(S, m, false);
+  const Layout L = dataset_layout(S, m, false, false);  // the ln n! tables are the base dataset's
   const size_t rep_bytes = align_up(L.total, 256);
   const int64_t want = std::min<int64_t>(n_reps, 256);
   int64_t fit = want;  // a spare allocation that holds them all needs no free-memory query

@@ -46,7 +46,9 @@
 // Measured against k_scan_tc on CTA pairs (kernel time of a whole search): 1024 x 8192 14.1 -> 3.90
 // ms, 3072 x 4096 265 -> 79.1 ms, 2048 x 8192 103 -> 26.9 ms, an eighth of 4096 x 16384 144 -> 32.1 ms.
 //
-// Every mbarrier wait is bounded; on expiry the kernel sets an error word and ends.
+// Every mbarrier wait is bounded; on expiry the kernel sets an error word and ends.  A producing warp then
+// goes on to the end of its tile and may overwrite a stage that is still to be multiplied: counts that come
+// of it are wrong, but 16 bits wide, and the ln n! table can be read for any such (dataset_layout).
 #include <atomic>
 #include <cfloat>
 #include <type_traits>
