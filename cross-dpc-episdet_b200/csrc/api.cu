@@ -786,7 +786,7 @@ int run_scan_tc(epik2_ctx* ctx, DevDataset& d, int64_t ib, int64_t ie, int top_k
   p.dump_scores = dump_scores;
   p.err = ctx->d_err;
   p.wait_limit = ctx->wait_limit;
-  p.test_withhold = pair ? 0 : ctx->test_withhold;
+  p.test_withhold = pair ? 0 : ctx->test_withhold == 1;
   if (!pair) ctx->test_withhold = 0;
   CK(ctx, cudaEventRecord(ctx->ev_start, ctx->stream), "event");
   if (overlap)
@@ -1108,6 +1108,8 @@ int run_split(epik2_ctx* ctx, const std::vector<DevDataset*>& ds, int64_t ib, in
     p.dump_scores = dump_scores;
     p.err = d_err;
     p.wait_limit = ctx->wait_limit;
+    p.test_withhold = ctx->test_withhold;
+    ctx->test_withhold = 0;
     CK(ctx, launch_scan_split(p, grid, dump_tables != nullptr, even, ctx->stream), "split search kernel");
     ctx->stats.kernel_launches += 3;
   }
@@ -1605,6 +1607,12 @@ int epik2_set_wait_limit(epik2_ctx* ctx, int64_t sm_clocks) {
 int epik2_test_withhold_arrival(epik2_ctx* ctx) {
   if (!ctx) return EPIK2_E_INVALID;
   ctx->test_withhold = 1;
+  return EPIK2_OK;
+}
+
+int epik2_test_withhold_odd_arrival(epik2_ctx* ctx) {
+  if (!ctx) return EPIK2_E_INVALID;
+  ctx->test_withhold = 2;
   return EPIK2_OK;
 }
 

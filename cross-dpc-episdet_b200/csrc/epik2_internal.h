@@ -227,6 +227,7 @@ struct SplitParams {
   float* dump_scores;
   int* err;
   long long wait_limit;
+  int32_t test_withhold;         // test hook: CTA (from 1) whose first stage waits for one arrival too many
 };
 
 // Kernel launchers (scan_int.cu / scan_tc.cu / encode.cu); all asynchronous on `stream`.

@@ -633,7 +633,8 @@ __global__ void __launch_bounds__(kSThreads, 1) k_scan_split(const SplitParams p
 
   if (tid == 0) {
     for (int s = 0; s < kSStages; s++) {
-      bar_init(bar(kCFull + s), kSProd / 2 + (even ? 1 : 0));  // + the odd CTA's issuing warp
+      // + the odd CTA's issuing warp, + some that never come (test hook)
+      bar_init(bar(kCFull + s), kSProd / 2 + (even ? 1 : 0) + (s == 0 && p.test_withhold == (int)blockIdx.x + 1 ? 1000 : 0));
       bar_init(bar(kCEmpty + s), 1);
     }
     bar_init(bar(kCAcc), 1);

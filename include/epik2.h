@@ -134,12 +134,15 @@ int epik2_get_stream(const epik2_ctx *ctx, void **cuda_stream);
  * memory and ends; the call returns EPIK2_E_TIMEOUT and the context stays usable (the
  * reference has no device-side wait to bound).  0 = the default, about 2 s. */
 int epik2_set_wait_limit(epik2_ctx *ctx, int64_t sm_clocks);
-/* Test hook of that error path (no reference counterpart): in the next tensor-core search
- * that runs on single CTAs (int8, or FP4 at 8 words per stage), one producing warp of the
- * first CTA leaves out its first "stage stored" arrival, so the issuing warp's wait expires
+/* Test hook of that error path (no reference counterpart): in the next genotype-split search, or
+ * tensor-core search that runs on single CTAs (int8, or FP4 at 8 words per stage), the first
+ * stage of the first CTA misses a "stage stored" arrival, so the issuing warp's wait expires
  * before any matrix product is issued and the search returns EPIK2_E_TIMEOUT.  One-shot:
- * the search after it runs normally. */
+ * the search after it runs normally.  The other kernels (integer, FP4 on CTA pairs) neither heed
+ * nor clear it. */
 int epik2_test_withhold_arrival(epik2_ctx *ctx);
+/* The same for the second CTA of the first pair (genotype-split search only). */
+int epik2_test_withhold_odd_arrival(epik2_ctx *ctx);
 /* Test hook (host only, no reference counterpart): the context refuses to hold more than this many
  * bytes of device memory in datasets and large buffers, as if the device had no more (0 = no limit). */
 int epik2_test_memory_limit(epik2_ctx *ctx, int64_t bytes);
