@@ -98,8 +98,8 @@ float screen_bound(int64_t n0, int64_t n1, const uint32_t* table) {
     uint32_t m;
     std::memcpy(&m, &M, 4);
     bits += m;
-    const float P = s.theta1 == 0.0f ? M : std::fma(D, -s.theta1, M);
-    acc = std::fma(D * (1.0f / std::fma(std::fabs(D), -s.theta2, P)), D, acc);
+    const float P = std::fma(std::fabs(D), -s.theta2, M);
+    acc = std::fma(D * (1.0f / (s.theta1 == 0.0f ? P : std::fma(D, -s.theta1, P))), D, acc);
   }
   return std::fma(kScreenLog, (float)(bits - 27u * 0x3F800000u), -s.c * acc) + s.base;
 }

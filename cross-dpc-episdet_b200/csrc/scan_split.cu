@@ -504,20 +504,32 @@ struct Screen {
   uint32_t bits;         // sum of the cells' log2 (N + 7/16), from below, in units of 2^-23
   template <int kN>
   __device__ __forceinline__ void cells(const Form (&f)[kN]) {
-    float D[kN], M[kN], P[kN], r[kN];
+    float D[kN], M[kN], r[kN];
 #pragma unroll
     for (int x = 0; x < kN; x++) {
       D[x] = __uint_as_float(f[x].d) - 12582912.0f;
       M[x] = __uint_as_float(f[x].n) - kLessN;
-      P[x] = kEven ? M[x] : fmaf(D[x], -theta1, M[x]);
     }
 #pragma unroll
-    for (int x = 0; x < kN; x++) r[x] = rcp_approx(fmaf(fabsf(D[x]), -theta2, P[x]));
+    for (int x = 0; x < kN; x++) {
+      const float P = fmaf(fabsf(D[x]), -theta2, M[x]);
+      r[x] = rcp_approx(kEven ? P : fmaf(D[x], -theta1, P));
+    }
+    // (the order of the sums is the faster one of either form: 4096 x 16384 with the other one 2 % slower,
+    // 1136 x 18638 with a third of cases 1.5 %)
+    if (kEven) {
 #pragma unroll
-    for (int x = 0; x + 1 < kN; x += 2) bits += __float_as_uint(M[x]) + __float_as_uint(M[x + 1]);
-    if (kN & 1) bits += __float_as_uint(M[kN - 1]);
+      for (int x = 0; x + 1 < kN; x += 2) bits += __float_as_uint(M[x]) + __float_as_uint(M[x + 1]);
+      if (kN & 1) bits += __float_as_uint(M[kN - 1]);
 #pragma unroll
-    for (int x = 0; x < kN; x++) acc = fmaf(D[x] * r[x], D[x], acc);
+      for (int x = 0; x < kN; x++) acc = fmaf(D[x] * r[x], D[x], acc);
+    } else {
+#pragma unroll
+      for (int x = 0; x < kN; x++) {
+        acc = fmaf(D[x] * r[x], D[x], acc);
+        bits += __float_as_uint(M[x]);
+      }
+    }
   }
 };
 
