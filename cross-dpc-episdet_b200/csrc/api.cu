@@ -58,6 +58,7 @@ struct epik2_ctx {
   int flat_seen = 0;            // that sum as last read
   int64_t wait_limit = 0;       // SM clocks of a bounded device-side wait (0 = kernel default)
   int test_withhold = 0;        // one-shot test hook of the bounded-wait error path
+  bool test_split = false;      // test hook: the split search wherever it fits
   int64_t test_limit = 0;       // test hook: device memory the context may hold (0 = what there is)
   int64_t* d_pb_off = nullptr;
   uint32_t* d_pb_ij = nullptr;
@@ -517,13 +518,13 @@ int run_scan(epik2_ctx* ctx, DevDataset& d, const epik2_opts* opts, uint32_t* du
   // screen keeps something back (a dump scores every triplet anyway); else the other kernels.
   const bool free_choice = (engine == 0 || engine == 3) && kw == 0 && pt == 0 && ov == 0 && split_fits(d);
   // (of the 32 best it is always the faster one: the other kernels' lists of every warp go through the host)
-  if (free_choice && top_k < 2 && small_search(triplets_in(m, ib, ie), d.n_samples, ib == 0 && ie >= m - 2, engine)) {
+  if (free_choice && top_k < 2 && !ctx->test_split && small_search(triplets_in(m, ib, ie), d.n_samples, ib == 0 && ie >= m - 2, engine)) {
     if (engine == EPIK2_ENGINE_TC_FP4) {
       kw = 8;
       pt = 32;
       ov = 1;
     }
-  } else if (free_choice && (dump_tables || split_screens({&d}, top_k))) {
+  } else if (free_choice && (dump_tables || ctx->test_split || split_screens({&d}, top_k))) {
     int n_cand = 0;
     const int r = run_split(ctx, {&d}, ib, ie, top_k, dump_tables, dump_scores, best_out, nullptr, &n_cand);
     if (r != kSplitNoRoom) {
@@ -1616,6 +1617,12 @@ int epik2_test_withhold_odd_arrival(epik2_ctx* ctx) {
   return EPIK2_OK;
 }
 
+int epik2_test_always_split(epik2_ctx* ctx, int on) {
+  if (!ctx) return EPIK2_E_INVALID;
+  ctx->test_split = on != 0;
+  return EPIK2_OK;
+}
+
 int epik2_test_memory_limit(epik2_ctx* ctx, int64_t bytes) {
   if (!ctx || bytes < 0) return EPIK2_E_INVALID;
   ctx->test_limit = bytes;
@@ -1978,7 +1985,7 @@ int epik2_scan_batch(epik2_ctx* ctx, const int32_t* dataset_ids, int32_t n, cons
   // search over all the datasets (16 datasets of 128-1536 SNPs: 32.4 against 84.6 ms).
   bool all_split = true;
   for (DevDataset* d : ds) all_split = all_split && split_fits(*d);
-  all_split = all_split && split_screens(ds);
+  all_split = all_split && (ctx->test_split || split_screens(ds));
   const bool free_choice = engine_req != EPIK2_ENGINE_TC && kw_req == 0 && pt_req == 0 && ov_req == 0 && all_split;
   // Many tiny datasets, or little in all: the persistent launch below on single CTAs, whose tiles are
   // cheaper when nearly empty (us a call, split and FP4: 512 datasets of 32 SNPs x 500 samples 2179 and 1180,
@@ -1990,7 +1997,7 @@ int epik2_scan_batch(epik2_ctx* ctx, const int32_t* dataset_ids, int32_t n, cons
     ts += triplets_in(d->n_snps, 0, d->n_snps) * (double)d->n_samples;
     most_samples = std::max(most_samples, d->n_samples);
   }
-  const bool tiny = free_choice && most_samples <= 4096 && (ts < 8e8 || ts < 6e7 * (double)n);
+  const bool tiny = free_choice && !ctx->test_split && most_samples <= 4096 && (ts < 8e8 || ts < 6e7 * (double)n);
   if (free_choice && !tiny) {
     const bool rescore = opts && opts->rescore_fp64;
     std::vector<BestSlot> best((size_t)n);
@@ -2199,7 +2206,7 @@ int epik2_scan_replicates(epik2_ctx* ctx, int32_t dataset_id, const uint8_t* phe
       all_split = all_split && split_fits(reps[(size_t)t]);
       ds.push_back(&reps[(size_t)t]);
     }
-    if (all_split && split_screens(ds)) {
+    if (all_split && (ctx->test_split || split_screens(ds))) {
       r = run_split_all(ctx, ds, res.data(), rescore ? resc.data() : nullptr);
       if (r < 0) {
         release();

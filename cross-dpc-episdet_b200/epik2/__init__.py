@@ -155,6 +155,7 @@ def library():
         "epik2_set_overlap": ([p, ctypes.c_int], ctypes.c_int),
         "epik2_test_withhold_arrival": ([p], ctypes.c_int),
         "epik2_test_withhold_odd_arrival": ([p], ctypes.c_int),
+        "epik2_test_always_split": ([p, ctypes.c_int], ctypes.c_int),
         "epik2_test_memory_limit": ([p, i64], ctypes.c_int),
         "epik2_test_screen_bound": ([i64, i64, p, i64, p], ctypes.c_int),
         "epik2_plink_dims": ([ctypes.c_char_p, ctypes.POINTER(ctypes.c_int64), ctypes.POINTER(ctypes.c_int64)],
@@ -344,6 +345,10 @@ class Context:
     def test_withhold_odd_arrival(self):
         """Test hook: the next genotype-split search times out in the second CTA of a pair."""
         self._check(self._lib.epik2_test_withhold_odd_arrival(self._h))
+
+    def test_always_split(self, on=True):
+        """Test hook: the genotype-split search wherever its counts fit."""
+        self._check(self._lib.epik2_test_always_split(self._h, int(on)))
 
     def test_memory_limit(self, n_bytes):
         """Test hook: device memory the context may hold (0 = what there is)."""

@@ -143,6 +143,10 @@ int epik2_set_wait_limit(epik2_ctx *ctx, int64_t sm_clocks);
 int epik2_test_withhold_arrival(epik2_ctx *ctx);
 /* The same for the second CTA of the first pair (genotype-split search only). */
 int epik2_test_withhold_odd_arrival(epik2_ctx *ctx);
+/* Test hook (host only, no reference counterpart): with nothing pinned the context takes the
+ * genotype-split search wherever its counts fit, also where other kernels are faster (the smallest
+ * searches, matrices of nearly constant SNPs). */
+int epik2_test_always_split(epik2_ctx *ctx, int on);
 /* Test hook (host only, no reference counterpart): the context refuses to hold more than this many
  * bytes of device memory in datasets and large buffers, as if the device had no more (0 = no limit). */
 int epik2_test_memory_limit(epik2_ctx *ctx, int64_t bytes);
