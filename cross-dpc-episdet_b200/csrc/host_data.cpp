@@ -64,9 +64,9 @@ void build_k2_lut(int64_t n_max, float* lut) { build_k2_lut_range(0, n_max + 1, 
 ScreenConsts screen_constants(int64_t n0, int64_t n1) {
   const double n = (double)(n0 + n1);
   int kp = (int)std::min(63.0, std::max(1.0, std::floor(64.0 * ((double)n0 + 13.5) / (n + 27.0) + 0.5)));
-  // Nearly even classes take p = 1/2, where t1 = 0 and a cell costs an operation less (3072 x 4096: 84.9
-  // ms, with the operation 91.0, before the loop's later changes).  At a distance x of the controls' share from 1/2 the bound loses about
-  // 2 n t2 x^3, which at most 1 keeps small beside the 2 to 4 it is below the score anyway.
+  // Nearly even classes take p = 1/2, where t1 = 0 and a cell costs an operation less (1024 x 8192: 3.94
+  // ms, with the operation 4.21).  At a distance x of the controls' share from 1/2 the bound loses about
+  // 2 n t2 x^3, which at most 1 keeps no larger than the 1 to 2 it is below the score anyway.
   const double x = ((double)n0 + 13.5) / (n + 27.0) - 0.5;
   if (1.115 * n * std::fabs(x * x * x) <= 1.0) kp = 32;
   const double p = kp / 64.0, q = 1.0 - p;

@@ -17,8 +17,8 @@
 // 2. A triplet's 27 cells are first put through a lower bound of K2 (screen_constants in
 //    host_data.cpp: one reciprocal per cell and a few FP32 operations, no table).  Only where the
 //    bound does not exceed the best score found so far (of the whole launch) is the score computed
-//    in the reference's arithmetic.  The bound is below the score by 1 to 2 on average for common
-//    alleles and classes of at least a twentieth of the samples, by 5 to 6 for alleles of 0.5 to 5 %.
+//    in the reference's arithmetic.  The bound is below the score by 1 to 2 on average, by 3 to 6
+//    where cases are 5 % or fewer.
 //
 // Warp roles of a CTA (512 threads), concurrent from tile to tile:
 //   warps 0-5   produce: expand the compacted bit planes into the operand ring (warps 0-3 the 64
@@ -35,16 +35,16 @@
 // are not even: screen_constants) up to about 8192 samples: the loop alone takes 340 clocks per
 // scheduler and 32 triplets, in the kernel 430 to 530, for the producing warps issue beside it.  From
 // there on also the round trip of a ring stage (stores, fence and arrival in the even CTA, products,
-// commit).  Cost of the parts of that round trip, which set the roles and hand-offs (clocks, measured
+// commit).  What the parts of that round trip cost sets the roles and hand-offs (clocks, measured
 // alone): a commit of four products 560; an arrival in the other CTA 133, and 447 with a cluster-scope
 // release; issuing four products and their commit 330 from a converged warp, 610 from a lane-0 branch;
 // a wait on a barrier that is complete 111, which passes during the issue of the stage before.
-// An eighth of 4096 x 16384 took 45.3 ms with the words of the next four stages in registers and each
-// producing warp fencing its stores (the fence waits for loads in flight), 42.5 with the fence in the
-// issuing warp, 38.8 with cp.async, 36.0 with stages of two quads whose words were loaded a stage ahead,
-// 33.2 with stages of one quad, 32.1 with the accumulators copied eight SNPs j per wait.  (One commit per two quads: +1.3 ms; seven stages and three raw slots: +2.8 ms.)
-// Measured against k_scan_tc on CTA pairs (kernel time of a whole search): 1024 x 8192 14.1 -> 3.90
-// ms, 3072 x 4096 265 -> 79.1 ms, 2048 x 8192 103 -> 26.9 ms, an eighth of 4096 x 16384 144 -> 32.1 ms.
+// Whole calls against what the other kernels take in their fastest configuration: 1024 x 8192 12.9 -> 3.94
+// ms, 3072 x 4096 224 -> 79.2, 2048 x 8192 97 -> 26.9, an eighth of 4096 x 16384 141 -> 32.5.
+//
+// A step that is scored (exact_score) costs four times a screened one.  Usual data score 1e-5 to 2e-3
+// of the steps, the more the fewer triplets there are to learn the threshold from; data whose scores
+// are equal (constant or equal SNPs) all of them: split_screens in api.cu keeps most of those away.
 //
 // Every mbarrier wait is bounded; on expiry the kernel sets an error word and ends.  A producing warp then
 // goes on to the end of its tile and may overwrite a stage that is still to be multiplied: counts that come
@@ -580,7 +580,7 @@ __device__ __forceinline__ void by_genotype(uint4 c, uint32_t n0, uint32_t n1, i
 
 // K2 of triplet (i, j, k) in the reference's arithmetic and order from its eight staged words per
 // class (e0: g_k = 0, e1: g_k = 1) and the margins in device memory; its table where one is
-// wanted.  Not inlined: the search takes it for a few triplets in a million.
+// wanted.  Not inlined: the search takes it for one triplet in a thousand or fewer.
 __device__ __noinline__ float exact_score(uint4 e0, uint4 e1, const SplitJob* J, int i, int j, int k, int genos,
                                           uint32_t* table) {
   const int gA = genos & 3, gB = (genos >> 2) & 3, gC = genos >> 4;
@@ -955,8 +955,7 @@ __global__ void __launch_bounds__(kSThreads, 1) k_scan_split(const SplitParams p
         const uint32_t ta = tmem + ((uint32_t)(32 * quarter) << 16);
         const uint32_t dst = Ek + (uint32_t)(c * kSplitJ * 64 * 16);
         // Eight SNPs j per wait, then four: the loads' latency is paid four times instead of seven
-        // (3072 x 4096 82.9 -> 79.1 ms).  Twelve per wait 81.3, one load of eight columns instead of two
-        // of four 80.9, the loop unrolled 83.2 (the kernel's code then passes the instruction caches).
+        // (3072 x 4096 82.9 -> 79.1 ms).
         auto drain = [&](int jj, auto quads) {
           constexpr int kQ = decltype(quads)::value;
           const uint32_t tc = ta + (uint32_t)(2 * kSHalfJ * part + jj);  // SNP j of half h: 28h further
