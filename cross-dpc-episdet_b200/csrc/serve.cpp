@@ -7,8 +7,8 @@
 // behind a large one); create each admitted scan's dataset (a replicate sharing a
 // resident genotype matrix, or a freshly uploaded matrix); run one batched launch over
 // all of them (epik2_scan_batch) -- except that three or more replicates of one resident matrix
-// admitted together run in the replicate form (epik2_scan_replicates); release the datasets; and complete the requests whose scans are
-// all done.  Requests that arrive during a launch join the next admission
+// admitted together run in the replicate form (epik2_scan_replicates); release the datasets; and
+// complete the requests whose scans are all done.  Requests that arrive during a launch join the next admission
 // round.  Submitting never waits for the device: it copies the request and queues it.
 #include <algorithm>
 #include <atomic>

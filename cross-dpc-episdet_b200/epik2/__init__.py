@@ -434,7 +434,7 @@ class Context:
         return b
 
     def scan_batch(self, datasets, **opts):
-        """Best triplet of each dataset from one batched, graph-captured launch."""
+        """Best triplet of each dataset from one call (epik2_scan_batch)."""
         ids = np.ascontiguousarray(np.asarray(datasets, dtype=np.int32))
         o = self._opts(**opts)
         arr = (Best * len(ids))()
@@ -443,7 +443,7 @@ class Context:
 
     def scan_replicates(self, dataset, phenos, **opts):
         """Best triplet of each phenotype-permutation replicate (rows of phenos) of a resident
-        dataset, the all-sample counts shared across replicates (epik2_scan_replicates)."""
+        dataset from one call (epik2_scan_replicates)."""
         phenos = np.ascontiguousarray(np.atleast_2d(phenos), dtype=np.uint8)
         arr = (Best * len(phenos))()
         o = self._opts(**opts)

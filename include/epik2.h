@@ -104,8 +104,9 @@ int epik2_mem_info(const epik2_ctx *ctx, size_t *free_bytes, size_t *total_bytes
 /* Default search engine of the context (EPIK2_ENGINE_*).  All engines give identical
  * tables, scores and triplets.  AUTO, and FP4 with no tuning option given, take the genotype-split
  * FP4 search where both classes have at most 65535 samples (for each first SNP only the samples of its
- * two rarer genotypes are counted); beyond, AUTO takes the autotuner's choice for the dataset's
- * shape. */
+ * two rarer genotypes are counted); beyond, below 8000 samples where most SNPs are nearly constant, and
+ * where the workspace does not fit, AUTO takes the autotuner's choice for the dataset's shape.  The
+ * smallest searches (triplets x samples below 2.5e8) take the integer engine or single FP4 CTAs. */
 #define EPIK2_ENGINE_AUTO 0
 #define EPIK2_ENGINE_INT 1 /* integer pipe: 8 LOP3+POPC per triplet and 32-sample word */
 #define EPIK2_ENGINE_TC 2  /* tcgen05 int8 matrix products on 0/1 operands, int32 accumulators */
@@ -260,13 +261,12 @@ int epik2_scan_batch(epik2_ctx *ctx, const int32_t *dataset_ids, int32_t n, cons
 
 /* Replicate form (no reference counterpart; the phenotype-mask idea of GPU/v1.cpp:264-289 on
  * tensor cores): the best triplet of each of n_reps phenotype-permutation replicates of a
- * resident dataset (phenos: n_reps x n_samples bytes, 1 = case).  Each tile of the search
- * counts the all-sample contingency cells of the base matrix once, then for every replicate
- * only its cases; its controls are the totals minus its cases (where every class has at most 65535
- * samples, the replicates are instead the datasets of one genotype-split search, which counts less
- * still).  Runs the FP4 CTA-pair kernel
- * (EPIK2_E_TOO_LARGE for classes of 2^24 samples or more), as many replicates per launch as
- * free device memory allows (at most 256).  out[r] equals epik2_scan of the dataset with
+ * resident dataset (phenos: n_reps x n_samples bytes, 1 = case).  The replicates are the datasets of
+ * one genotype-split search; where that does not apply (classes of more than 65535 samples, mostly
+ * nearly constant SNPs, no room) each tile counts the all-sample contingency cells of the base
+ * matrix once, then for every replicate only its cases, its controls being the totals minus its
+ * cases (FP4 CTA pairs).  EPIK2_E_TOO_LARGE for classes of 2^24 samples or more; as many replicates
+ * per launch as free device memory allows (at most 256).  out[r] equals epik2_scan of the dataset with
  * phenotype r; with opts->rescore_fp64, out[r].score_fp64 is its best triplet rescored in FP64
  * on the GPU (other options are ignored). */
 int epik2_scan_replicates(epik2_ctx *ctx, int32_t dataset_id, const uint8_t *phenos, int32_t n_reps,
