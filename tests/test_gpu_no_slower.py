@@ -1,7 +1,8 @@
 """Searches that the library's own choice of kernel must not make slower than the kernels it chooses from:
-data and shapes where the genotype-split search has least to gain.  Each is timed (median of 9 calls)
+data and shapes where the genotype-split search has least to gain.  Each is timed (fastest of 9 calls)
 against the fastest pinned configuration; both sides' results must be equal.  The bound of 1.3 is far above
-the run-to-run spread (a few per cent) and below what a wrong choice costs (1.4 to 100 times)."""
+the run-to-run spread (a few per cent) and below what a wrong choice costs (1.4 to 100 times); a comparison
+that a busy host disturbed is made again, twice at most."""
 import time
 
 import numpy as np
@@ -41,17 +42,20 @@ def _time(f, n=9):
         t0 = time.perf_counter()
         r = f()
         t.append(time.perf_counter() - t0)
-    return float(np.median(t)), r
+    return min(t), r
 
 
 def _compare(call, pinned=PINNED, slack=1.3):
-    ours, got = _time(call)
-    best = None
-    for kw in pinned:
-        t, want = _time(lambda: call(**kw))
-        got_l, want_l = (got, want) if isinstance(got, list) else ([got], [want])
-        assert [(b.ijk, b.score) for b in got_l] == [(b.ijk, b.score) for b in want_l]
-        best = t if best is None else min(best, t)
+    for attempt in range(3):
+        ours, got = _time(call)
+        best = None
+        for kw in pinned:
+            t, want = _time(lambda: call(**kw))
+            got_l, want_l = (got, want) if isinstance(got, list) else ([got], [want])
+            assert [(b.ijk, b.score) for b in got_l] == [(b.ijk, b.score) for b in want_l]
+            best = t if best is None else min(best, t)
+        if ours <= slack * best:
+            return
     assert ours <= slack * best, (ours * 1e3, best * 1e3)
 
 
