@@ -98,6 +98,7 @@ __global__ void __launch_bounds__(kPipeThreads, 1) k_scan_pipe(const TcParams p)
   __shared__ long long s_hand[4];           // odd CTA: descriptors handed over by the even CTA
   __shared__ long long s_desc[4];           // this CTA's descriptor of tile t at t % 4
   __shared__ int s_abort, s_pfail, s_sfail;
+  __shared__ int s_read;                    // tiles whose descriptor the scoring warps have read
   __shared__ float s_red_s[8];
   __shared__ unsigned long long s_red_k[8];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -109,6 +110,7 @@ __global__ void __launch_bounds__(kPipeThreads, 1) k_scan_pipe(const TcParams p)
   volatile int* abort_flag = &s_abort;
   volatile int* pfail = &s_pfail;
   volatile int* sfail = &s_sfail;
+  volatile int* tiles_read = &s_read;
 
   if (tid == 0) {
     for (int s = 0; s < kStages; s++) {
@@ -126,6 +128,7 @@ __global__ void __launch_bounds__(kPipeThreads, 1) k_scan_pipe(const TcParams p)
     s_abort = 0;
     s_pfail = 0;
     s_sfail = 0;
+    s_read = 0;
   }
   cluster_sync_all();  // both CTAs' barriers exist before any remote arrival
   if (warp == 0) {
@@ -167,6 +170,14 @@ __global__ void __launch_bounds__(kPipeThreads, 1) k_scan_pipe(const TcParams p)
     for (uint32_t t = 0;; t++) {
       if (tid == 0) {  // tile t's descriptor: fetched by the even CTA, handed to the odd one
         long long d = -1;
+        // Descriptor slot t % 4 is written again only after the scoring warps have read tile t - 4's.  Where a
+        // tile is one stage (a class without samples, few in the other), the ring alone lets the
+        // producing warps run five tiles ahead of them.
+        if (t >= 4) {
+          const long long t0 = clock64();
+          while (*tiles_read < (int)t - 3 && !*abort_flag && !*sfail)
+            if (clock64() - t0 > wl) *abort_flag = 1;
+        }
         if (even) {
           if (t == 0) {
             pf_t = atomicAdd(p.counter, 1ull);
@@ -328,6 +339,7 @@ __global__ void __launch_bounds__(kPipeThreads, 1) k_scan_pipe(const TcParams p)
       if (!ok || *abort_flag) *sfail = 1;  // written only here, before the barrier
       named_sync(1, 256);
       if (desc < 0 || *sfail) break;
+      if (st == 0) *tiles_read = (int)t + 1;  // every scoring thread read it before the barrier
       const int job = kBatched ? tile_job((uint64_t)desc) : 0;
       const JobRef jv = job_of(desc);
       if (kBatched && job != cur_job) {
