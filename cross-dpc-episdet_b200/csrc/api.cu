@@ -81,6 +81,7 @@ struct epik2_ctx {
   // pointer: the job table is rewritten before every replay), least recently used first
   std::map<std::vector<int64_t>, std::unique_ptr<struct BatchPlan>> plans;
   std::vector<std::vector<int64_t>> plan_lru;
+  std::vector<std::vector<int64_t>> tiny_seen;  // shapes of the last batches of tiny datasets, oldest first
   // replicate form scratch: job table, per-CTA slots, results (grown, never shrunk)
   TcJob* d_rep_jobs = nullptr;
   BestSlot* d_rep_slots = nullptr;
@@ -1260,6 +1261,25 @@ int tuned(epik2_ctx* ctx, DevDataset& d, epik2_tune* out) {
   return EPIK2_OK;
 }
 
+// What a batched plan is kept by: the datasets' SNP counts, their configurations' codes, rescore.
+std::vector<int64_t> batch_key(const std::vector<DevDataset*>& ds, const std::vector<int>& codes, bool rescore) {
+  std::vector<int64_t> key;
+  for (const DevDataset* d : ds) key.push_back(d->n_snps);
+  for (int c : codes) key.push_back(c);
+  key.push_back(rescore ? 1 : 0);
+  return key;
+}
+
+// Whether the plan for a batch of tiny datasets is worth having: there is one, or the same shapes came
+// before (of the last kMaxPlans; else they are noted).
+bool tiny_batch_again(epik2_ctx* ctx, const std::vector<int64_t>& key) {
+  if (ctx->plans.count(key) || std::find(ctx->tiny_seen.begin(), ctx->tiny_seen.end(), key) != ctx->tiny_seen.end())
+    return true;
+  if (ctx->tiny_seen.size() >= kMaxPlans) ctx->tiny_seen.erase(ctx->tiny_seen.begin());
+  ctx->tiny_seen.push_back(key);
+  return false;
+}
+
 // Batched form: build (or reuse) the plan for these datasets, refresh the job table from
 // the datasets' current class split, replay the captured launch sequence.  codes[b] =
 // tc_code() of dataset b's configuration; datasets with the same code form a group, one
@@ -1269,10 +1289,7 @@ int tuned(epik2_ctx* ctx, DevDataset& d, epik2_tune* out) {
 int run_batch(epik2_ctx* ctx, const std::vector<DevDataset*>& ds, const std::vector<int32_t>& ids,
               const std::vector<int>& codes, bool rescore, epik2_best* out) {
   (void)ids;
-  std::vector<int64_t> key;
-  for (const DevDataset* d : ds) key.push_back(d->n_snps);
-  for (int c : codes) key.push_back(c);
-  key.push_back(rescore ? 1 : 0);
+  const std::vector<int64_t> key = batch_key(ds, codes, rescore);
   BatchPlan* plan = nullptr;
   auto it = ctx->plans.find(key);
   const int32_t n = (int32_t)ds.size();
@@ -1990,7 +2007,9 @@ int epik2_scan_batch(epik2_ctx* ctx, const int32_t* dataset_ids, int32_t n, cons
   // Many tiny datasets, or little in all: the persistent launch below on single CTAs, whose tiles are
   // cheaper when nearly empty (us a call, split and FP4: 512 datasets of 32 SNPs x 500 samples 2179 and 1180,
   // of 64 x 500 4581 and 3672, of 64 x 2000 4800 and 5164, of 128 x 500 12062 and 14240; one of 128 x 2000
-  // 97 and 92, 16 of 64 x 2000 212 and 209); int8 for the fewest samples (512 of 64 x 500 3433).
+  // 97 and 92, 16 of 64 x 2000 212 and 209); int8 for the fewest samples (512 of 64 x 500 3433).  Its plan takes
+  // 150 to 500 us to make, so shapes that come for the first time are searched by the split search
+  // (16 of 8 to 39 SNPs x 300 samples: 112 us, with a new plan 287, with the plan at hand 86).
   double ts = 0.0;
   int64_t most_samples = 0;
   for (DevDataset* d : ds) {
@@ -1998,8 +2017,11 @@ int epik2_scan_batch(epik2_ctx* ctx, const int32_t* dataset_ids, int32_t n, cons
     most_samples = std::max(most_samples, d->n_samples);
   }
   const bool tiny = free_choice && !ctx->test_split && most_samples <= 4096 && (ts < 8e8 || ts < 6e7 * (double)n);
-  if (free_choice && !tiny) {
-    const bool rescore = opts && opts->rescore_fp64;
+  const bool rescore = opts && opts->rescore_fp64;
+  const bool int8 = most_samples <= 1000 && engine_req == EPIK2_ENGINE_AUTO;
+  const TcConfig tiny_pick = int8 ? TcConfig{EPIK2_ENGINE_TC, 4, false, false} : TcConfig{EPIK2_ENGINE_TC_FP4, 8, false, false};
+  if (free_choice &&
+      !(tiny && tiny_batch_again(ctx, batch_key(ds, std::vector<int>(ds.size(), tc_code(tiny_pick.kw, !int8, false, false)), rescore)))) {
     std::vector<BestSlot> best((size_t)n);
     std::vector<Rescored> resc(rescore ? (size_t)n : 0);
     const int r = run_split_all(ctx, ds, best.data(), rescore ? resc.data() : nullptr);
@@ -2017,8 +2039,7 @@ int epik2_scan_batch(epik2_ctx* ctx, const int32_t* dataset_ids, int32_t n, cons
   TcConfig pick{0, 0, false, false};
   bool have = false;
   if (tiny) {
-    const bool int8 = most_samples <= 1000 && engine_req == EPIK2_ENGINE_AUTO;
-    pick = int8 ? TcConfig{EPIK2_ENGINE_TC, 4, false, false} : TcConfig{EPIK2_ENGINE_TC_FP4, 8, false, false};
+    pick = tiny_pick;
     have = true;
   } else if (engine_req != 0 && kw_req != 0 && (pt_req != 0 || engine_req == EPIK2_ENGINE_TC) && ov_req != 0) {
     pick = TcConfig{engine_req, kw_req, pt_req == 64, ov_req == 2};
@@ -2066,7 +2087,7 @@ int epik2_scan_batch(epik2_ctx* ctx, const int32_t* dataset_ids, int32_t n, cons
                 "tensor-core configuration: int8 takes 4 or 8 words per stage on 32-SNP tiles; FP4 takes 8 or 16 "
                 "(32- or 64-SNP tiles), or 4 or 8 overlapped on 64-SNP tiles");
   const std::vector<int> codes(ds.size(), tc_code(pick.kw, fp4, pick.pair && fp4, pick.overlap));
-  return run_batch(ctx, ds, ids, codes, opts && opts->rescore_fp64, out);
+  return run_batch(ctx, ds, ids, codes, rescore, out);
 }
 
 int epik2_scan_replicates(epik2_ctx* ctx, int32_t dataset_id, const uint8_t* phenos, int32_t n_reps,

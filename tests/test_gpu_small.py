@@ -50,9 +50,11 @@ def test_batches(n, S, M):
             for (g, p), b in zip(data, c.scan_batch(ids, rescore_fp64=rescore)):
                 r = O.scan(g, p)
                 assert b.ijk == r["ijk"] and f32_bits(b.score) == f32_bits(r["score"])
-        # a new phenotype follows into the next call
-        q = rng.permutation(data[0][1])
-        c.set_pheno(ids[0], q)
-        r = O.scan(data[0][0], q)
-        b = c.scan_batch(ids)[0]
-        assert b.ijk == r["ijk"] and f32_bits(b.score) == f32_bits(r["score"])
+        # a new phenotype follows into the next calls (shapes seen once, a new plan, its replay), and
+        # other shapes between them
+        for _ in range(4):
+            q = rng.permutation(data[0][1])
+            c.set_pheno(ids[0], q)
+            r = O.scan(data[0][0], q)
+            for got in (c.scan_batch(ids)[0], c.scan_batch(ids[::-1])[-1], c.scan_batch(ids + ids[:1])[-1]):
+                assert got.ijk == r["ijk"] and f32_bits(got.score) == f32_bits(r["score"])
